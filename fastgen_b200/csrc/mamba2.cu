@@ -84,6 +84,97 @@ conv_silu_kernel(const T* __restrict__ in, long in_stride, TO* __restrict__ out,
   }
 }
 
+// The same for four taps, four channels a thread and CONV_RUN consecutive tokens: where those tokens and the
+// three before them are one sequence's, every input is read once, 8 or 16 bytes at a time, and all reads are
+// in flight together (the kernel above reads every input four times, a channel at a time).  Other runs (a
+// sequence's start, padding) look up each tap's place as above.  The sums are the kernel's above, bit for bit.
+// 2,048 tokens of 6,144 channels, bfloat16 -> float32: 105 -> 23 us (its 75 MB take 11.5).
+constexpr int CONV_RUN = 8;
+
+template <typename T>
+__device__ __forceinline__ float4 conv_load4(const T* p);
+template <>
+__device__ __forceinline__ float4 conv_load4<float>(const float* p) {
+  return *reinterpret_cast<const float4*>(p);
+}
+template <>
+__device__ __forceinline__ float4 conv_load4<__nv_bfloat16>(const __nv_bfloat16* p) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void conv_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void conv_store4(__nv_bfloat16* p, float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  uint2 r;
+  r.x = *reinterpret_cast<const uint32_t*>(&a);
+  r.y = *reinterpret_cast<const uint32_t*>(&b);
+  *reinterpret_cast<uint2*>(p) = r;
+}
+
+template <typename T, typename TO, bool SILU>
+__global__ void __launch_bounds__(CONV_THREADS)
+conv4_silu_kernel(const T* __restrict__ in, long in_stride, TO* __restrict__ out, long out_stride,
+                  const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ state,
+                  long state_stride, long conv_offset, const int* __restrict__ req, int n_tokens, int channels) {
+  constexpr int TAPS = 4, BACK = TAPS - 1;
+  const int c = (blockIdx.y * CONV_THREADS + threadIdx.x) * 4;
+  if (c >= channels) return;
+  const int t0 = blockIdx.x * CONV_RUN;
+  int rq[CONV_RUN + BACK];  // rq[j]: the slot of token t0 - BACK + j
+  bool one = t0 >= BACK && t0 + CONV_RUN <= n_tokens;
+#pragma unroll
+  for (int j = 0; j < CONV_RUN + BACK; ++j) {
+    const int t = t0 - BACK + j;
+    rq[j] = (t >= 0 && t < n_tokens) ? req[t] : -1;
+    one = one && rq[j] == rq[0];
+  }
+  one = one && rq[0] >= 0;
+  float wk[4][TAPS];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    *reinterpret_cast<float4*>(wk[e]) = *reinterpret_cast<const float4*>(w + (size_t)(c + e) * TAPS);
+  const float4 bc = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  auto emit = [&](int t, const float4& v0, const float4& v1, const float4& v2, const float4& v3) {
+    float r[4] = {bc.x, bc.y, bc.z, bc.w};
+    const float x[TAPS][4] = {{v0.x, v0.y, v0.z, v0.w}, {v1.x, v1.y, v1.z, v1.w}, {v2.x, v2.y, v2.z, v2.w}, {v3.x, v3.y, v3.z, v3.w}};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+#pragma unroll
+      for (int k = 0; k < TAPS; ++k) r[e] = fmaf(wk[e][k], x[k][e], r[e]);
+      if (SILU) r[e] = r[e] / (1.f + expf(-r[e]));
+    }
+    conv_store4(out + (size_t)t * out_stride + c, make_float4(r[0], r[1], r[2], r[3]));
+  };
+  if (one) {
+    float4 v[CONV_RUN + BACK];
+#pragma unroll
+    for (int j = 0; j < CONV_RUN + BACK; ++j) v[j] = conv_load4<T>(in + (size_t)(t0 - BACK + j) * in_stride + c);
+#pragma unroll
+    for (int u = 0; u < CONV_RUN; ++u) emit(t0 + u, v[u], v[u + 1], v[u + 2], v[u + 3]);
+    return;
+  }
+#pragma unroll
+  for (int u = 0; u < CONV_RUN; ++u) {
+    const int t = t0 + u, slot = rq[u + BACK];
+    if (slot < 0) continue;
+    int have = 0;  // how many of the three tokens before t the step itself brings
+#pragma unroll
+    for (int b = 1; b <= BACK; ++b)
+      if (have == b - 1 && rq[u + BACK - b] == slot) have = b;
+    float4 v[TAPS];
+#pragma unroll
+    for (int k = 0; k < TAPS; ++k) {
+      const int back = BACK - k;
+      v[k] = back <= have ? conv_load4<T>(in + (size_t)(t - back) * in_stride + c)
+                          : *reinterpret_cast<const float4*>(state + (size_t)slot * state_stride + conv_offset +
+                                                             (size_t)(BACK + have - back) * channels + c);
+    }
+    emit(t, v[0], v[1], v[2], v[3]);
+  }
+}
+
 // The state's convolution inputs after the step: the last taps-1 of (old inputs, new inputs).
 template <typename T>
 __global__ void __launch_bounds__(CONV_THREADS)
@@ -446,6 +537,41 @@ gated_part_norm_warp_kernel(const float* __restrict__ y, long y_stride, const T*
   }
 }
 
+// Parts of 128, 256, 512 or 1,024 columns: the same sums with a compile-time number of columns a lane, so that
+// all of a part's loads are in flight together and nothing is tested (2,048 tokens of 8 parts of 512: 43 -> 19 us;
+// its 67 MB take 10).
+template <typename T, int ITEMS>
+__global__ void __launch_bounds__(GW_WARPS * 32)
+gated_part_norm_whole_kernel(const float* __restrict__ y, long y_stride, const T* __restrict__ z, long z_stride,
+                             const float* __restrict__ w, T* __restrict__ out, long out_stride,
+                             const int* __restrict__ req, int n_tokens, int parts, float eps) {
+  constexpr int PART = ITEMS * 32;
+  const int lane = threadIdx.x & 31;
+  const long item = (long)blockIdx.x * GW_WARPS + (threadIdx.x >> 5);
+  if (item >= (long)n_tokens * parts) return;
+  const int t = item / parts, c0 = (int)(item - (long)t * parts) * PART;
+  if (req[t] < 0) return;
+  const float* yr = y + (size_t)t * y_stride + c0 + lane;
+  const T* zr = z + (size_t)t * z_stride + c0 + lane;
+  float v[ITEMS], zv[ITEMS];
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    v[i] = yr[32 * i];
+    zv[i] = to_f32<T>(zr[32 * i]);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    v[i] *= zv[i] / (1.f + expf(-zv[i]));
+    ss += v[i] * v[i];
+  }
+  ss = warp_sum(ss);
+  const float rstd = 1.f / sqrtf(ss / (float)PART + eps);
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i)
+    out[(size_t)t * out_stride + c0 + lane + 32 * i] = from_f32<T>(v[i] * rstd * w[c0 + lane + 32 * i]);
+}
+
 // ---- C interface -----------------------------------------------------------------------------------
 
 // A causal convolution over time per channel, from and into the state's last inputs, with a choice
@@ -457,7 +583,18 @@ static int launch_time_conv(const T* in, long proj_stride, TO* out, long out_str
                             cudaStream_t stream) {
   const dim3 grid((n_tokens + CONV_TOKENS - 1) / CONV_TOKENS, (channels + CONV_THREADS - 1) / CONV_THREADS);
   const dim3 sgrid(n_seqs, grid.y);
-  if (act)
+  // four taps, and every row of inputs, weights, state and results in whole aligned groups of four channels
+  const bool fours = taps == 4 && channels % 4 == 0 && proj_stride % 4 == 0 && out_stride % 4 == 0 && state_stride % 4 == 0 &&
+                     conv_offset % 4 == 0 && (uintptr_t)in % (4 * sizeof(T)) == 0 && (uintptr_t)out % (4 * sizeof(TO)) == 0 &&
+                     (((uintptr_t)w | (uintptr_t)bias | (uintptr_t)state) & 15) == 0;
+  const dim3 fgrid((n_tokens + CONV_RUN - 1) / CONV_RUN, (channels / 4 + CONV_THREADS - 1) / CONV_THREADS);
+  if (fours && act)
+    conv4_silu_kernel<T, TO, true><<<fgrid, CONV_THREADS, 0, stream>>>(in, proj_stride, out, out_stride, w, bias, state,
+                                                                       state_stride, conv_offset, req, n_tokens, channels);
+  else if (fours)
+    conv4_silu_kernel<T, TO, false><<<fgrid, CONV_THREADS, 0, stream>>>(in, proj_stride, out, out_stride, w, bias, state,
+                                                                        state_stride, conv_offset, req, n_tokens, channels);
+  else if (act)
     conv_silu_kernel<T, TO, true><<<grid, CONV_THREADS, 0, stream>>>(in, proj_stride, out, out_stride, w, bias, state,
                                                                      state_stride, conv_offset, req, n_tokens, channels,
                                                                      taps);
@@ -576,6 +713,25 @@ extern "C" int fg_gated_part_norm(const float* y, long y_stride, const void* z, 
   FG_CHECK_ARG(parts > 0 && width % parts == 0, "fg_gated_part_norm: %d columns in %d parts", width, parts);
   const dim3 grid(n_tokens, parts);
   const int part = width / parts;
+  if ((dtype == FG_F32 || dtype == FG_BF16) && (part == 128 || part == 256 || part == 512 || part == 1024)) {
+    const int blocks = (int)(((long)n_tokens * parts + GW_WARPS - 1) / GW_WARPS);
+#define GATED(T, I)                                                                                                       \
+  gated_part_norm_whole_kernel<T, I><<<blocks, GW_WARPS * 32, 0, stream>>>(y, y_stride, (const T*)z, z_stride, w, (T*)out, \
+                                                                           out_stride, req, n_tokens, parts, eps)
+#define GATED_I(T)                      \
+  do {                                  \
+    if (part == 128) GATED(T, 4);       \
+    else if (part == 256) GATED(T, 8);  \
+    else if (part == 512) GATED(T, 16); \
+    else GATED(T, 32);                  \
+  } while (0)
+    if (dtype == FG_F32) GATED_I(float);
+    else GATED_I(__nv_bfloat16);
+#undef GATED_I
+#undef GATED
+    FG_CHECK_LAUNCH("fg_gated_part_norm");
+    return 0;
+  }
   if (part <= 32 * GW_ITEMS) {
     const long items = (long)n_tokens * parts;
     const int blocks = (int)((items + GW_WARPS - 1) / GW_WARPS);

@@ -53,3 +53,60 @@ def test_float32_product_routes(ops32, m, n, k):
     ref = x.double() @ w.double().T
     bound = k * EPS * (x.double().abs() @ w.double().abs().T)
     assert bool(((got.double() - ref).abs() <= bound + 1e-30).all())
+
+
+# -- convolution, gate and norms -----------------------------------------------------------------------
+
+def _sequences(lengths, pad=0, slots=None):
+    """A step's arrays for sequences of these lengths, ``pad`` tokens of slot -1 behind them."""
+    slots = slots or list(range(len(lengths)))
+    req, start = [], [0]
+    for n, s in zip(lengths, slots):
+        req += [s] * n
+        start.append(start[-1] + n)
+    to = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    return SimpleNamespace(req=to(req + [-1] * pad), seq_slot=to(slots), seq_start=to(start), n_seqs=len(lengths),
+                           n_tokens=len(req) + pad)
+
+
+@pytest.mark.parametrize("act", ["silu", None])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lengths,pad", [([1], 0), ([2, 3, 1, 1], 2), ([40], 0), ([11, 1, 8, 30], 5), ([3, 8, 9, 64], 0)])
+def test_convolution_four_channels_at_a_time(ops32, ops16, dtype, lengths, pad, act):
+    """Aligned channels against the same channels one column further (the kernel of one channel a thread)."""
+    ops = ops32 if dtype == torch.float32 else ops16
+    channels, taps = 136, 4
+    ctx = _sequences(lengths, pad, slots=list(range(1, len(lengths) + 1)))
+    g = torch.Generator().manual_seed(sum(lengths))
+    t = ctx.n_tokens
+    rows = _randn(g, t, channels).to(dtype)
+    w, bias = _randn(g, channels, taps), _randn(g, channels)
+    state = _randn(g, len(lengths) + 2, 8 + (taps - 1) * channels)
+    outs = []
+    for shift in (0, 1):
+        proj = torch.zeros(t, channels + 4, dtype=dtype, device=DEV)
+        proj[:, shift : shift + channels] = rows
+        st = state.clone()
+        out = ops.time_conv(proj, shift, channels, w, bias, st, 8, taps, ctx, act=act, out_dtype=dtype)
+        live = ctx.req >= 0
+        outs.append((out[live], st))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("part,parts", [(128, 3), (256, 1), (512, 8), (1024, 2), (96, 2), (640, 1)])
+def test_gate_and_norm_in_parts(ops32, ops16, dtype, part, parts):
+    ops = ops32 if dtype == torch.float32 else ops16
+    ctx = _sequences([5, 12], 2)
+    t, width = ctx.n_tokens, part * parts
+    g = torch.Generator().manual_seed(part)
+    y, w = _randn(g, t, width), 1 + _randn(g, width, scale=0.1)
+    proj = _randn(g, t, width + 24).to(dtype)
+    z = proj[:, 8 : 8 + width]
+    got = ops.gated_part_norm(y, z, w, parts, 1e-5, ctx)[:17].double()
+    v = (y.double() * torch.nn.functional.silu(z.double())).reshape(t, parts, part)
+    ref = (v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-5)).reshape(t, width) * w.double()
+    ref = ref[:17]
+    # float32: the sum of squares and a handful of operations; bfloat16: one rounding more
+    rel = (part + 16) * EPS + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+    assert bool(((got - ref).abs() <= rel * ref.abs() + 1e-6).all())
