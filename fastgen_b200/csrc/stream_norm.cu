@@ -119,6 +119,94 @@ stream_norm_kernel(float* h, int n_streams, const TD* delta, const float* __rest
   }
 }
 
+// The same for up to four streams and rows that fit a block's registers (up to COLS columns a thread): all
+// streams' loads are in flight at once, and the row waits between the passes of the variance in registers.  The
+// sums are the kernel's above, bit for bit (a thread's columns are the same ones in the same order).
+// 2,048 tokens of two streams of 2,048: 30 -> 21 us (its 84 MB take 13).
+template <typename TD, typename TO, int S, int COLS>
+__global__ void __launch_bounds__(SN_THREADS)
+stream_norm_reg_kernel(float* h, const TD* delta, const float* __restrict__ mix, const float* __restrict__ out_coef,
+                       const float* __restrict__ in_coef, const float* __restrict__ w, const float* __restrict__ b,
+                       TO* __restrict__ out, const int* rows, int dim, float eps, int kind) {
+  __shared__ float scratch[32];
+  pdl_trigger();
+  float mx[S][S], oc[S], ic[S];
+#pragma unroll
+  for (int a = 0; a < S; ++a) {
+    oc[a] = out_coef ? out_coef[a] : 1.f;
+    ic[a] = in_coef ? in_coef[a] : 1.f;
+#pragma unroll
+    for (int c = 0; c < S; ++c) mx[a][c] = mix ? mix[a * S + c] : (a == c ? 1.f : 0.f);
+  }
+  const int tid = threadIdx.x;
+  float w_r[COLS], b_r[COLS];
+#pragma unroll
+  for (int i = 0; i < COLS; ++i) {
+    const int d = tid + SN_THREADS * i;
+    w_r[i] = out != nullptr && d < dim ? w[d] : 0.f;
+    b_r[i] = out != nullptr && b != nullptr && d < dim ? b[d] : 0.f;
+  }
+  pdl_wait();
+  const size_t row = rows ? ld_global_4(rows + blockIdx.x) : blockIdx.x;
+  float* x = h + row * (size_t)S * dim;
+  const TD* dl = delta + row * dim;
+  const bool store = delta != nullptr && rows == nullptr;
+  const bool has_mix = mix != nullptr, has_in = in_coef != nullptr;
+  float xs[COLS][S], y[COLS];
+#pragma unroll
+  for (int i = 0; i < COLS; ++i) {
+    const int d = tid + SN_THREADS * i;
+#pragma unroll
+    for (int s = 0; s < S; ++s) xs[i][s] = d < dim ? x[(size_t)s * dim + d] : 0.f;
+    y[i] = delta != nullptr && d < dim ? to_f32<TD>(dl[d]) : 0.f;
+  }
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < COLS; ++i) {  // (columns beyond dim hold zeros)
+    const int d = tid + SN_THREADS * i;
+    float u = 0.f;
+    float v[S];
+#pragma unroll
+    for (int t = 0; t < S; ++t) {
+      v[t] = xs[i][t];
+      if (delta != nullptr) {
+        if (has_mix) {
+          v[t] = 0.f;
+#pragma unroll
+          for (int s = 0; s < S; ++s) v[t] = fmaf(mx[s][t], xs[i][s], v[t]);
+        }
+        v[t] = fmaf(oc[t], y[i], v[t]);
+        if (store && d < dim) x[(size_t)t * dim + d] = v[t];
+      }
+      u = has_in ? fmaf(ic[t], v[t], u) : u + v[t];
+    }
+    y[i] = u;
+    sum += kind == 0 ? u : u * u;
+  }
+  if (out == nullptr) return;
+  sum = block_sum(sum, scratch);
+  float mean = 0.f, rstd;
+  if (kind == 0) {
+    mean = sum / (float)dim;
+    float sq = 0.f;
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) {
+      const float c = y[i] - mean;
+      if (tid + SN_THREADS * i < dim) sq += c * c;
+    }
+    sq = block_sum(sq, scratch);
+    rstd = 1.f / sqrtf(sq / (float)dim + eps);
+  } else {
+    rstd = 1.f / sqrtf(sum / (float)dim + eps);
+  }
+  TO* o = out + (size_t)blockIdx.x * dim;
+#pragma unroll
+  for (int i = 0; i < COLS; ++i) {
+    const int d = tid + SN_THREADS * i;
+    if (d < dim) o[d] = from_f32<TO>((y[i] - mean) * rstd * w_r[i] + b_r[i]);
+  }
+}
+
 extern "C" int fg_stream_norm(float* h, int n_streams, const void* delta, int delta_dtype, const float* mix,
                               const float* out_coef, const float* in_coef, const float* w, const float* b,
                               void* out, int out_dtype, const int* rows, int n_rows, int dim, float eps, int kind,
@@ -137,9 +225,23 @@ extern "C" int fg_stream_norm(float* h, int n_streams, const void* delta, int de
     fg_launch_pdl(kern, dim3(n_rows), dim3(SN_THREADS), smem, stream, h, n_streams, (const TD*)delta, mix,   \
                   out_coef, in_coef, w, b, (TO*)out, rows, dim, eps, kind);                                  \
   } while (0)
+  // rows that fit the registers: at most 16 columns a thread, streams as the instantiations below have them
+  const int cols = n_streams <= 4 && dim <= 16 * SN_THREADS ? (dim <= 8 * SN_THREADS ? 8 : 16) : 0;
+#define LAUNCH_R(TD, TO, S, COLS)                                                                                       \
+  fg_launch_pdl(stream_norm_reg_kernel<TD, TO, S, COLS>, dim3(n_rows), dim3(SN_THREADS), 0, stream, h, (const TD*)delta, \
+                mix, out_coef, in_coef, w, b, (TO*)out, rows, dim, eps, kind)
+#define LAUNCH_C(TD, TO, S)                 \
+  do {                                      \
+    if (cols == 8) LAUNCH_R(TD, TO, S, 8);  \
+    else LAUNCH_R(TD, TO, S, 16);           \
+  } while (0)
 #define LAUNCH(TD, TO)                          \
   do {                                          \
-    if (n_streams == 1) LAUNCH_S(TD, TO, 1);    \
+    if (cols != 0 && n_streams == 1) LAUNCH_C(TD, TO, 1);      \
+    else if (cols != 0 && n_streams == 2) LAUNCH_C(TD, TO, 2); \
+    else if (cols != 0 && n_streams == 3) LAUNCH_C(TD, TO, 3); \
+    else if (cols != 0) LAUNCH_C(TD, TO, 4);   \
+    else if (n_streams == 1) LAUNCH_S(TD, TO, 1);    \
     else if (n_streams == 2) LAUNCH_S(TD, TO, 2); \
     else if (n_streams == 3) LAUNCH_S(TD, TO, 3); \
     else if (n_streams == 4) LAUNCH_S(TD, TO, 4); \
@@ -152,6 +254,8 @@ extern "C" int fg_stream_norm(float* h, int n_streams, const void* delta, int de
   else LAUNCH(__nv_bfloat16, __nv_bfloat16);
 #undef LAUNCH
 #undef LAUNCH_S
+#undef LAUNCH_C
+#undef LAUNCH_R
   FG_CHECK_LAUNCH("fg_stream_norm");
   return 0;
 }

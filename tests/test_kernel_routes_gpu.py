@@ -110,3 +110,38 @@ def test_gate_and_norm_in_parts(ops32, ops16, dtype, part, parts):
     # float32: the sum of squares and a handful of operations; bfloat16: one rounding more
     rel = (part + 16) * EPS + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
     assert bool(((got - ref).abs() <= rel * ref.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("kind", ["layer", "rms"])
+@pytest.mark.parametrize("streams,dim", [(1, 4), (2, 2047), (2, 2048), (3, 2049), (4, 4096), (2, 4097), (5, 100)])
+def test_stream_norm_rows_in_registers(ops32, streams, dim, kind):
+    g = torch.Generator().manual_seed(dim + streams)
+    t = 5
+    h, delta = _randn(g, t, streams, dim), _randn(g, t, dim).to(torch.bfloat16)
+    mix, oc, ic = torch.rand(streams, streams, generator=g).to(DEV), torch.rand(streams, generator=g).to(DEV), torch.rand(streams, generator=g).to(DEV)
+    w, b = 1 + _randn(g, dim, scale=0.1), _randn(g, dim, scale=0.1)
+    want = torch.einsum("ast,nsd->ntd", mix.double()[None], h.double()) + oc.double()[:, None] * delta.double()[:, None]
+    u = (ic.double()[:, None] * want).sum(1)
+    if kind == "layer":
+        c = u - u.mean(-1, keepdim=True)
+        ref = c / torch.sqrt((c * c).mean(-1, keepdim=True) + 1e-5) * w.double() + b.double()
+    else:
+        ref = u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-5) * w.double()
+    out = torch.empty(t, dim, dtype=torch.float32, device=DEV)
+    rows = torch.tensor([3, 0], dtype=torch.int32, device=DEV)
+    some = torch.empty(2, dim, dtype=torch.float32, device=DEV)
+    args = dict(delta=delta, mix=mix, out_coef=oc, in_coef=ic, bias=b if kind == "layer" else None, eps=1e-5, rms=kind == "rms")
+    _stream_norm(ops32, h, w, some, rows=rows, **args)
+    _stream_norm(ops32, h, w, out, **args)
+    bound = (dim + 32) * EPS
+    assert float((h.double() - want).abs().max()) <= 8 * EPS * float(want.abs().max()) * (streams + 1)
+    assert float((out.double() - ref).abs().max()) <= bound * float(ref.abs().max())
+    assert torch.equal(some, out[rows.long()])
+
+
+def _stream_norm(ops, h, w, out, delta, mix, out_coef, in_coef, bias, eps, rms, rows=None):
+    from fastgen_b200.csrc.ops import _check, _code, _ptr, _stream
+    n = out.shape[0]
+    _check(ops.lib, ops.lib.fg_stream_norm(_ptr(h), h.shape[1], _ptr(delta), _code(delta.dtype), _ptr(mix), _ptr(out_coef),
+                                           _ptr(in_coef), _ptr(w), _ptr(bias), _ptr(out), _code(out.dtype), _ptr(rows), n,
+                                           h.shape[2], eps, int(rms), _stream()))
