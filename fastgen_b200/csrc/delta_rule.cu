@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(DELTA_THREADS)
 delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ rec,
                   const float* __restrict__ vp, float* __restrict__ out, long out_stride, float* __restrict__ state,
                   long state_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_heads,
-                  int n_kv_heads, int d, int dv, int DVP) {
+                  int n_kv_heads, int d, int dv, int DVP, int most) {
   constexpr int DP = LPC * RPL;            // rows, padded
   constexpr int CPW = 32 / LPC;            // columns a warp
   constexpr int COLS = DELTA_WARPS * CPW;  // columns a block
@@ -124,7 +124,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   const int slot = seq_slot[blockIdx.z];
   if (slot < 0) return;
   const int start = seq_start[blockIdx.z], n = seq_start[blockIdx.z + 1] - start;
-  if (n <= 0) return;
+  if (n <= 0 || n > most) return;  // (more than `most`: delta_chunk_kernel's)
   const int h = blockIdx.y, hk = h / (n_heads / n_kv_heads);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane % LPC, cw = warp * CPW + lane / LPC;  // the lane's part of a column; its column in the block
@@ -233,13 +233,295 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   }
 }
 
+// ---- sequences of many tokens with one decay a head: chunks ------------------------------------------
+// The recurrence above is a chain of about 450 cycles a token.  Over a chunk of C = 32 tokens from state S0 it
+// is also, with D[i][j] = g_{j+1} .. g_i (a product, never a quotient) and c_i = g_1 .. g_i,
+//
+//     (I + A) U = beta (V - c K S0),   A[i][j] = beta_i D[i][j] k_i . k_j  (j < i)
+//     O = c Q S0 + (D o Q K^T) U       S <- c_C S0 + (D[C] o K)^T U
+//
+// and all that does not hold S0 is each chunk's own.  delta_wy_kernel forms it for all chunks side by side
+// (a block a (chunk, head); the triangular system by forward substitution, a thread a column):
+//     W = (I + A)^-1 beta c K,  V' = (I + A)^-1 beta V,  c Q,  (D[C] o K)^T,  D o Q K^T
+// and delta_chunk_kernel walks the chunks: U = V' - W S0, then O and the next state, two small products
+// and two barriers for 32 tokens.  1,501 tokens, 16 heads of 64: 347 -> 77 us and 24 of forming the chunks.
+// float32 throughout; the order of the sums is not the token kernel's, so the
+// float32 mode, whose results do not depend on how a prompt is cut, keeps the kernel above.
+constexpr int CHUNK = 32;
+constexpr int CHUNK_THREADS = 128;
+constexpr int CHUNK_COLS = 8;    // columns of the state a block of the walk
+constexpr int CHUNK_STAGES = 3;  // chunks in its ring
+constexpr int CHUNK_MIN = 64;    // fewest tokens of a sequence that takes this way (64 tokens: 15 us above, about 20 here; 128: 30 and 22)
+
+// floats of a (chunk, head): W [32][D], c Q [32][D], (D[C] o K)^T [D][32], D o Q K^T [32][32], V' [32][DVP], c_C
+__host__ __device__ constexpr long chunk_floats(int D, int DVP) { return 96L * D + CHUNK * CHUNK + CHUNK * DVP + 4; }
+
+// Sequence b's tokens take the chunks (else the token kernel).
+__device__ __forceinline__ bool chunked_sequence(const int* seq_slot, const int* seq_start, int b, int& n) {
+  n = seq_start[b + 1] - seq_start[b];
+  return seq_slot[b] >= 0 && n >= CHUNK_MIN;
+}
+
+template <int D>
+__global__ void __launch_bounds__(CHUNK_THREADS)
+delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ rec,
+                const float* __restrict__ vp, float* __restrict__ chunks, const int* __restrict__ seq_slot,
+                const int* __restrict__ seq_start, int n_seqs, int n_heads, int n_kv_heads, int DVP) {
+  constexpr int SK = D + 4, SA = CHUNK + 4;
+  __shared__ __align__(16) float ks[CHUNK][SK];
+  __shared__ __align__(16) float qs[CHUNK][SK];
+  __shared__ __align__(16) float at[CHUNK][SA];  // A transposed: [m][i]
+  __shared__ float dm[CHUNK][CHUNK + 1];         // D[i][j], j <= i
+  __shared__ float gs[CHUNK], betas[CHUNK], cs[CHUNK];
+  const int h = blockIdx.y, hk = h / (n_heads / n_kv_heads), tid = threadIdx.x;
+  int c = blockIdx.x, b = 0, n = 0;
+  for (; b < n_seqs; ++b) {
+    if (!chunked_sequence(seq_slot, seq_start, b, n)) continue;
+    const int nc = (n + CHUNK - 1) / CHUNK;
+    if (c < nc) break;
+    c -= nc;
+  }
+  if (b == n_seqs) return;
+  const int t0 = seq_start[b] + c * CHUNK, nt = min(CHUNK, n - c * CHUNK);
+  float* const dst = chunks + ((size_t)blockIdx.x * n_heads + h) * chunk_floats(D, DVP);
+  for (int i = tid; i < CHUNK * (D / 4); i += CHUNK_THREADS) {
+    const int t = i / (D / 4), w = i % (D / 4) * 4;
+    float4 k = make_float4(0.f, 0.f, 0.f, 0.f), q = k;
+    if (t < nt) {
+      k = *reinterpret_cast<const float4*>(kn + ((size_t)(t0 + t) * n_kv_heads + hk) * D + w);
+      q = *reinterpret_cast<const float4*>(qn + ((size_t)(t0 + t) * n_kv_heads + hk) * D + w);
+    }
+    *reinterpret_cast<float4*>(&ks[t][w]) = k;
+    *reinterpret_cast<float4*>(&qs[t][w]) = q;
+  }
+  if (tid < CHUNK) {  // tokens beyond the sequence change nothing: no decay, no step
+    const float* r = rec + ((size_t)(t0 + tid) * n_heads + h) * 4;
+    gs[tid] = tid < nt ? r[0] : 1.f;
+    betas[tid] = tid < nt ? r[1] : 0.f;
+  }
+  __syncthreads();
+  if (tid <= CHUNK) {  // column tid of D; thread 32: the decays from the chunk's start
+    const int j = tid < CHUNK ? tid : -1;
+    float x = 1.f;
+    for (int i = j < 0 ? 0 : j; i < CHUNK; ++i) {
+      if (i > j) x *= gs[i];
+      if (j < 0) cs[i] = x;
+      else dm[i][j] = x;
+    }
+  }
+  __syncthreads();
+  {  // K K^T (the first half of the threads) and Q K^T: 4 x 4 places a thread, 8 apart
+    const bool of_q = tid >= 64;
+    const int ib = (tid & 63) >> 3, jb = tid & 7;
+    const float (*left)[SK] = of_q ? qs : ks;
+    float acc[4][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int f = 0; f < 4; ++f) acc[e][f] = 0.f;
+#pragma unroll 2
+    for (int w = 0; w < D; w += 4) {
+      float4 a[4], k[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        a[e] = *reinterpret_cast<const float4*>(&left[ib + 8 * e][w]);
+        k[e] = *reinterpret_cast<const float4*>(&ks[jb + 8 * e][w]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          acc[e][f] = fmaf(a[e].x, k[f].x, acc[e][f]);
+          acc[e][f] = fmaf(a[e].y, k[f].y, acc[e][f]);
+          acc[e][f] = fmaf(a[e].z, k[f].z, acc[e][f]);
+          acc[e][f] = fmaf(a[e].w, k[f].w, acc[e][f]);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        const int i = ib + 8 * e, j = jb + 8 * f;
+        if (of_q) dst[96 * D + i * CHUNK + j] = j <= i ? dm[i][j] * acc[e][f] : 0.f;
+        else at[j][i] = j < i ? betas[i] * dm[i][j] * acc[e][f] : 0.f;
+      }
+  }
+  __syncthreads();
+  for (int col = tid; col < D + DVP; col += CHUNK_THREADS) {
+    float x[CHUNK];
+    if (col < D) {
+#pragma unroll
+      for (int i = 0; i < CHUNK; i += 4) {
+        float kd[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float k = ks[i + e][col];
+          kd[e] = dm[CHUNK - 1][i + e] * k;
+          x[i + e] = betas[i + e] * cs[i + e] * k;
+          dst[32 * D + (i + e) * D + col] = cs[i + e] * qs[i + e][col];
+        }
+        *reinterpret_cast<float4*>(dst + 64 * D + col * CHUNK + i) = make_float4(kd[0], kd[1], kd[2], kd[3]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < CHUNK; ++i)
+        x[i] = i < nt ? betas[i] * vp[((size_t)(t0 + i) * n_heads + h) * DVP + col - D] : 0.f;
+    }
+#pragma unroll
+    for (int m = 0; m < CHUNK - 1; ++m) {
+#pragma unroll
+      for (int i = (m + 1) / 4 * 4; i < CHUNK; i += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(&at[m][i]);  // zero up to i = m
+        if (i > m) x[i] = fmaf(-a.x, x[m], x[i]);
+        if (i + 1 > m) x[i + 1] = fmaf(-a.y, x[m], x[i + 1]);
+        if (i + 2 > m) x[i + 2] = fmaf(-a.z, x[m], x[i + 2]);
+        x[i + 3] = fmaf(-a.w, x[m], x[i + 3]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < CHUNK; ++i) {
+      if (col < D) dst[i * D + col] = x[i];
+      else dst[96 * D + CHUNK * CHUNK + i * DVP + col - D] = x[i];
+    }
+  }
+  if (tid == 0) dst[96 * D + CHUNK * CHUNK + CHUNK * DVP] = cs[CHUNK - 1];
+}
+
+template <int D>
+struct ChunkWalk {
+  static constexpr int SW = D + 4, SK = CHUNK + 4;  // padded rows: eight lanes read eight bank groups
+  static constexpr int W = 0, Q = W + CHUNK * SW, K = Q + CHUNK * SW, A = K + D * SK, V = A + CHUNK * SK;
+  static constexpr int END = V + CHUNK * CHUNK_COLS, BUF = END + 4;
+  static constexpr size_t SMEM = sizeof(float) * (CHUNK_STAGES * BUF + CHUNK_COLS * (SW + SK));
+};
+
+__device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+
+template <int D>
+__global__ void __launch_bounds__(CHUNK_THREADS)
+delta_chunk_kernel(const float* __restrict__ chunks, float* __restrict__ out, long out_stride, float* __restrict__ state,
+                   long state_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_heads,
+                   int d, int dv, int DVP) {
+  using L = ChunkWalk<D>;
+  constexpr int ND = D / 32;
+  extern __shared__ __align__(16) float smem[];
+  float* const s_t = smem + CHUNK_STAGES * L::BUF;   // the state, a column a row: [COLS][SW]
+  float* const u_t = s_t + CHUNK_COLS * L::SW;       // U, a column a row: [COLS][SK]
+  const int b = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
+  int n;
+  if (!chunked_sequence(seq_slot, seq_start, b, n)) return;
+  int first = 0;  // the sequence's first chunk
+  for (int i = 0; i < b; ++i) {
+    int m;
+    if (chunked_sequence(seq_slot, seq_start, i, m)) first += (m + CHUNK - 1) / CHUNK;
+  }
+  const int start = seq_start[b], n_chunks = (n + CHUNK - 1) / CHUNK;
+  const int col0 = blockIdx.x * CHUNK_COLS;
+  const long REC = chunk_floats(D, DVP);
+
+  auto issue = [&](int c) {
+    const float* src = chunks + ((size_t)(first + c) * n_heads + h) * REC;
+    float* buf = smem + c % CHUNK_STAGES * L::BUF;
+    for (int i = tid; i < 2 * CHUNK * (D / 4); i += CHUNK_THREADS)  // W and c Q
+      delta_copy16(buf + i / (D / 4) * L::SW + i % (D / 4) * 4, src + i * 4, true);
+    for (int i = tid; i < (D + CHUNK) * (CHUNK / 4); i += CHUNK_THREADS)  // (D[C] o K)^T and D o Q K^T
+      delta_copy16(buf + L::K + i / (CHUNK / 4) * L::SK + i % (CHUNK / 4) * 4, src + 64 * D + i * 4, true);
+    if (tid < CHUNK * CHUNK_COLS / 4) {
+      const int r = tid / (CHUNK_COLS / 4), w = tid % (CHUNK_COLS / 4) * 4;
+      const bool ok = col0 + w < DVP;
+      delta_copy16(buf + L::V + r * CHUNK_COLS + w, src + 96 * D + CHUNK * CHUNK + r * DVP + (ok ? col0 + w : 0), ok);
+    }
+    if (tid == 64) delta_copy16(buf + L::END, src + 96 * D + CHUNK * CHUNK + CHUNK * DVP, true);
+  };
+#pragma unroll
+  for (int c = 0; c < CHUNK_STAGES - 1; ++c) {
+    if (c < n_chunks) issue(c);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  // a thread: row r of the chunk (or rows r + 32 i of the state) against two columns
+  const int r = tid >> 2, c0 = (tid & 3) * 2;
+  float* const st = state + (size_t)seq_slot[b] * state_stride + ((size_t)h * dv + col0) * d;
+  float s[ND][2];
+#pragma unroll
+  for (int i = 0; i < ND; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int row = r + 32 * i, col = c0 + e;
+      s[i][e] = (row < d && col0 + col < dv) ? st[(size_t)col * d + row] : 0.f;
+      s_t[col * L::SW + row] = s[i][e];
+    }
+  for (int c = 0; c < n_chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(CHUNK_STAGES - 2) : "memory");
+    __syncthreads();  // the chunk has landed, and the state of the chunk before stands in shared memory
+    if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const float* buf = smem + c % CHUNK_STAGES * L::BUF;
+    float w0 = 0.f, w1 = 0.f, q0 = 0.f, q1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < D; k += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(buf + L::W + r * L::SW + k);
+      const float4 q = *reinterpret_cast<const float4*>(buf + L::Q + r * L::SW + k);
+      const float4 a = *reinterpret_cast<const float4*>(s_t + c0 * L::SW + k);
+      const float4 e = *reinterpret_cast<const float4*>(s_t + (c0 + 1) * L::SW + k);
+      w0 = dot4(w, a, w0);
+      w1 = dot4(w, e, w1);
+      q0 = dot4(q, a, q0);
+      q1 = dot4(q, e, q1);
+    }
+    const float2 v = *reinterpret_cast<const float2*>(buf + L::V + r * CHUNK_COLS + c0);
+    u_t[c0 * L::SK + r] = v.x - w0;
+    u_t[(c0 + 1) * L::SK + r] = v.y - w1;
+    __syncthreads();
+    const float gc = buf[L::END];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+      s[i][0] *= gc;
+      s[i][1] *= gc;
+    }
+#pragma unroll
+    for (int k = 0; k < CHUNK; k += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(u_t + c0 * L::SK + k);
+      const float4 e = *reinterpret_cast<const float4*>(u_t + (c0 + 1) * L::SK + k);
+      const float4 m = *reinterpret_cast<const float4*>(buf + L::A + r * L::SK + k);
+      q0 = dot4(m, a, q0);
+      q1 = dot4(m, e, q1);
+#pragma unroll
+      for (int i = 0; i < ND; ++i) {
+        const float4 kd = *reinterpret_cast<const float4*>(buf + L::K + (r + 32 * i) * L::SK + k);
+        s[i][0] = dot4(kd, a, s[i][0]);
+        s[i][1] = dot4(kd, e, s[i][1]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+      s_t[c0 * L::SW + r + 32 * i] = s[i][0];
+      s_t[(c0 + 1) * L::SW + r + 32 * i] = s[i][1];
+    }
+    if (c * CHUNK + r < n) {
+      float* o = out + (size_t)(start + c * CHUNK + r) * out_stride + h * dv + col0 + c0;
+      if (col0 + c0 < dv) o[0] = q0;
+      if (col0 + c0 + 1 < dv) o[1] = q1;
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < ND; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int row = r + 32 * i, col = c0 + e;
+      if (row < d && col0 + col < dv) st[(size_t)col * d + row] = s[i][e];
+    }
+}
+
 // rows of the prepared arrays for key size d (the row count of the kernel that takes it)
 static int delta_rows(int d) { return d <= 32 ? 32 : d <= 64 ? 64 : d <= 128 ? 128 : 256; }
 
 template <bool HEAD>
 static int launch_scan(cudaStream_t stream, const float* qn, const float* kn, const float* rec, const float* vp,
                        float* out, long out_stride, float* state, long state_stride, const int* seq_slot,
-                       const int* seq_start, int n_seqs, int n_heads, int n_kv_heads, int d, int dv, int DVP) {
+                       const int* seq_start, int n_seqs, int n_heads, int n_kv_heads, int d, int dv, int DVP, int most) {
 #define CASE(LPC, RPL)                                                                                         \
   {                                                                                                            \
     constexpr int COLS = DELTA_WARPS * (32 / LPC);                                                             \
@@ -251,7 +533,7 @@ static int launch_scan(cudaStream_t stream, const float* qn, const float* kn, co
     }                                                                                                           \
     dim3 grid((dv + COLS - 1) / COLS, n_heads, n_seqs);                                                         \
     kern<<<grid, DELTA_THREADS, smem, stream>>>(qn, kn, rec, vp, out, out_stride, state, state_stride, seq_slot, \
-                                                seq_start, n_heads, n_kv_heads, d, dv, DVP);                    \
+                                                seq_start, n_heads, n_kv_heads, d, dv, DVP, most);              \
   }
   if (d <= 32) CASE(8, 4)
   else if (d <= 64) CASE(16, 4)
@@ -261,10 +543,23 @@ static int launch_scan(cudaStream_t stream, const float* qn, const float* kn, co
   return 0;
 }
 
+// Whether a step may hold sequences for delta_chunk_kernel: 16-bit serving, one decay a head, key sizes whose
+// rows are 64 or 128, and enough tokens for one such sequence.
+static bool chunks_apply(int n_tokens, int d, int dtype, int head_decay) {
+  return dtype == FG_BF16 && head_decay && d > 32 && d <= 128 && n_tokens >= CHUNK_MIN;
+}
+// most chunks of a step's sequences that have CHUNK_MIN tokens or more
+static long most_chunks(int n_tokens, int n_seqs) {
+  const int long_ones = n_tokens / CHUNK_MIN;
+  return n_tokens / CHUNK + (n_seqs < long_ones ? n_seqs : long_ones);
+}
+
 // floats of the scratch that fg_delta_scan needs for `n_tokens` tokens
-extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int n_heads, int n_kv_heads, int d, int dv) {
+extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int n_seqs, int n_heads, int n_kv_heads, int d, int dv, int dtype,
+                                             int head_decay) {
   const long DP = delta_rows(d), DVP = (dv + 3) / 4 * 4;
-  return (long)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
+  const long rows = (long)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
+  return rows + (chunks_apply(n_tokens, d, dtype, head_decay) ? most_chunks(n_tokens, n_seqs) * n_heads * chunk_floats((int)DP, (int)DVP) : 0);
 }
 
 // qkv: float32 [T, q (kv heads x d) | k (kv heads x d) | v (heads x dv)], the convolutions' outputs.
@@ -300,9 +595,30 @@ extern "C" int fg_delta_scan(const float* qkv, long qkv_stride, const void* a, l
   }
 #undef PREPARE
   FG_CHECK_LAUNCH("fg_delta_scan (prepare)");
+  int most = 0x7fffffff;  // tokens of the longest sequence that the token kernel takes
+  if (chunks_apply(n_tokens, d, dtype, head_decay)) {
+    most = CHUNK_MIN - 1;
+    float* chunks = scratch + (size_t)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
+    const dim3 wy_grid((unsigned)most_chunks(n_tokens, n_seqs), n_heads), grid((dv + CHUNK_COLS - 1) / CHUNK_COLS, n_heads, n_seqs);
+#define CHUNKS(D)                                                                                                       \
+  do {                                                                                                                  \
+    delta_wy_kernel<D><<<wy_grid, CHUNK_THREADS, 0, stream>>>(qn, kn, rec, vp, chunks, seq_slot, seq_start, n_seqs, n_heads, \
+                                                              n_kv_heads, DVP);                                         \
+    FG_CHECK_LAUNCH("fg_delta_scan (chunks)");                                                                          \
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
+                                         (int)ChunkWalk<D>::SMEM);                                                      \
+    FG_CHECK_ARG(e == cudaSuccess, "fg_delta_scan: shared memory: %s", cudaGetErrorString(e));                          \
+    delta_chunk_kernel<D><<<grid, CHUNK_THREADS, ChunkWalk<D>::SMEM, stream>>>(                                         \
+        chunks, out, out_stride, state, state_stride, seq_slot, seq_start, n_heads, d, dv, DVP);                        \
+    FG_CHECK_LAUNCH("fg_delta_scan (walk)");                                                                            \
+  } while (0)
+    if (DP == 64) CHUNKS(64);
+    else CHUNKS(128);
+#undef CHUNKS
+  }
   const auto scan = head_decay ? launch_scan<true> : launch_scan<false>;
   const int rc = scan(stream, qn, kn, rec, vp, out, out_stride, state, state_stride, seq_slot, seq_start, n_seqs,
-                      n_heads, n_kv_heads, d, dv, DVP);
+                      n_heads, n_kv_heads, d, dv, DVP, most);
   if (rc != 0) return rc;
   FG_CHECK_LAUNCH("fg_delta_scan");
   return 0;

@@ -201,7 +201,7 @@ def latent(rank: int, rot_dim: int):
 
 _DELTA_SIGNATURES = {
     "fg_delta_scan": [_P, _L, _P, _L, _P, _L, _I, _P, _P, _P, _L, _P, _L, _P, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P],
-    "fg_delta_scan_scratch_floats": [_I, _I, _I, _I, _I],
+    "fg_delta_scan_scratch_floats": [_I, _I, _I, _I, _I, _I, _I, _I],
     "fg_head_norm_gate": [_P, _L, _P, _L, _I, _P, _P, _L, _P, _I, _I, _I, _F, _I, _P],
 }
 _MOE_SIGNATURES = {
@@ -245,6 +245,7 @@ def delta_rule():
     if _delta is None:
         lib = build.delta_rule_library()
         _declare(lib, _DELTA_SIGNATURES)
+        lib.fg_delta_scan_scratch_floats.restype = ctypes.c_longlong
         _delta = lib
     return _delta
 
@@ -823,8 +824,9 @@ class Ops:
         assert a_log.dtype == torch.float32 and a_log.numel() == heads and a_log.is_contiguous()
         out = torch.empty((t, heads * dv), dtype=torch.float32, device=qkv.device)
         # the tokens as the recurrence reads them (unit vectors, decays, step sizes; padded rows)
-        scratch = torch.empty(lib.fg_delta_scan_scratch_floats(t, heads, kv_heads, d, dv), dtype=torch.float32,
-                              device=qkv.device)
+        # (and, where sequences of many tokens go chunk by chunk, what the chunks are alone)
+        scratch = torch.empty(lib.fg_delta_scan_scratch_floats(t, ctx.n_seqs, heads, kv_heads, d, dv, _code(a.dtype),
+                                                               int(head_decay)), dtype=torch.float32, device=qkv.device)
         _check(lib, lib.fg_delta_scan(
             _ptr(qkv), qkv.stride(0), _ptr(a), a.stride(0), _ptr(b), b.stride(0), _code(a.dtype), _ptr(dt_bias),
             _ptr(a_log), _ptr(out), out.stride(0), _ptr(state), state.stride(0), _ptr(ctx.seq_slot),

@@ -145,3 +145,51 @@ def _stream_norm(ops, h, w, out, delta, mix, out_coef, in_coef, bias, eps, rms, 
     _check(ops.lib, ops.lib.fg_stream_norm(_ptr(h), h.shape[1], _ptr(delta), _code(delta.dtype), _ptr(mix), _ptr(out_coef),
                                            _ptr(in_coef), _ptr(w), _ptr(bias), _ptr(out), _code(out.dtype), _ptr(rows), n,
                                            h.shape[2], eps, int(rms), _stream()))
+
+
+# -- recurrences, chunk by chunk ---------------------------------------------------------------------------
+
+LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0)]
+
+
+def _relative(got, ref):
+    return float((got.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("d,dv", [(64, 64), (40, 24), (128, 12), (100, 130)])
+@pytest.mark.parametrize("lengths,pad", LENGTHS)
+def test_delta_rule_with_one_decay_a_head(ops16, lengths, pad, d, dv):
+    heads, kv = 4, 2
+    slots = [1, 3, 0][: len(lengths)]
+    ctx = _sequences(lengths, pad, slots)
+    t = ctx.n_tokens
+    g = torch.Generator().manual_seed(sum(lengths) + d)
+    qkv = _randn(g, t, 2 * kv * d + heads * dv)
+    proj = _randn(g, t, 2 * heads).to(torch.bfloat16)
+    a, b = proj[:, :heads], proj[:, heads:]
+    dt_bias, a_log = torch.rand(heads, generator=g).to(DEV) * 3.5 - 3, torch.rand(heads, generator=g).to(DEV) * 2.5 - 2
+    state = _randn(g, 4, heads * d * dv + 8, scale=0.3)
+    before = state.clone()
+    out = ops16.delta_scan(qkv, a, b, dt_bias, a_log, state, ctx, heads, kv, d, dv, head_decay=True)
+    for i, (n, slot) in enumerate(zip(lengths, slots)):
+        o = int(ctx.seq_start[i])
+        rows = qkv[o : o + n].double()
+        q = rows[:, : kv * d].reshape(n, kv, d).repeat_interleave(heads // kv, 1)
+        k = rows[:, kv * d : 2 * kv * d].reshape(n, kv, d).repeat_interleave(heads // kv, 1)
+        v = rows[:, 2 * kv * d :].reshape(n, heads, dv)
+        q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * d ** -0.5
+        k = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+        gate = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(a[o : o + n].double() + dt_bias.double(), threshold=1e9))
+        beta = torch.sigmoid(b[o : o + n].double())
+        S = before[slot, : heads * d * dv].double().reshape(heads, dv, d).clone()
+        ref = torch.empty(n, heads, dv, dtype=torch.float64, device=DEV)
+        for s in range(n):
+            S = gate[s][:, None, None] * S
+            u = beta[s][:, None] * (v[s] - (S * k[s][:, None, :]).sum(-1))
+            S = S + u[:, :, None] * k[s][:, None, :]
+            ref[s] = (S * q[s][:, None, :]).sum(-1)
+        bound = (2 * d + 4 * 32 + 64) * EPS  # a row's sums, the chunk's triangular system and its decays
+        assert _relative(out[o : o + n], ref.reshape(n, heads * dv)) <= bound
+        assert _relative(state[slot, : heads * d * dv], S.reshape(-1)) <= bound
+    for slot in {0, 1, 2, 3} - set(slots):
+        assert torch.equal(state[slot], before[slot])
