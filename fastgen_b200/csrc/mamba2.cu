@@ -349,7 +349,7 @@ ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* _
                       const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                       const float* __restrict__ d_skip, float* __restrict__ y, long y_stride,
                       float* __restrict__ state, long state_stride, const int* __restrict__ seq_slot,
-                      const int* __restrict__ seq_start, int heads, int groups, int P) {
+                      const int* __restrict__ seq_start, int heads, int groups, int P, int most) {
   constexpr int N = 32 * NPT;
   constexpr int STAGE = 2 * SCAN_TOKENS * N + SCAN_TOKENS * SCAN_PB + 2 * SCAN_TOKENS;  // floats
   extern __shared__ __align__(16) float smem[];
@@ -361,7 +361,7 @@ ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* _
   const int slot = seq_slot[blockIdx.x];
   if (slot < 0) return;
   const int start = seq_start[blockIdx.x], n_tok = seq_start[blockIdx.x + 1] - start;
-  if (n_tok <= 0) return;
+  if (n_tok <= 0 || n_tok > most) return;  // (more than `most`: ssm_chunk_kernel's)
   const int h = blockIdx.y, g = h / (heads / groups);
   const int p0 = blockIdx.z * SCAN_PB;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -468,6 +468,292 @@ ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* _
 #pragma unroll
     for (int i = 0; i < NPT; ++i)
       if (pc + c < P) S[(size_t)(pc + c) * N + lane + 32 * i] = s[c][i];
+}
+
+// ---- sequences of many tokens, 16-bit serving: chunks ---------------------------------------------------
+// Token by token the recurrence takes about 390 cycles a token and reads its operands from shared memory once per
+// token.  Over a chunk of 32 tokens from state S0 it is also, with D[i][j] = a_{j+1} .. a_i (a product of the
+// tokens' decays), e_i = a_1 .. a_i and w_j = D[32][j] dt_j,
+//
+//     Y = e (C S0) + M X + D_skip X,  M[i][j] = (C_i . B_j) D[i][j] dt_j  (j <= i)
+//     S <- e_32 S0 + B^T (w X)
+//
+// 2,048 tokens of 64 heads, 128 x 64 states: 420 -> 187 us and 13 of preparing (the multiply-adds alone take 75; what
+// bounds the walk is shared memory: a 16-byte read a lane takes its 4 cycles whoever shares the address, and 4 x 4
+// numbers a thread want two such reads for 16 multiply-adds).
+//
+// ssm_chunk_prepare_kernel forms M, e and w for all chunks side by side (a block a (chunk, group): C B^T once for the
+// group's heads); ssm_chunk_kernel walks the chunks of one (sequence, head, 32 columns), a state of 4 x 4 numbers a
+// thread.  All float32 multiply-adds; the sums have another order than the token kernel's, so the float32 mode,
+// whose results do not depend on how a prompt is cut, keeps that one.
+constexpr int SC_TOKENS = 32;   // tokens a chunk
+constexpr int SC_COLS = 32;     // columns of P a block of the walk
+constexpr int SC_THREADS = 256;
+constexpr int SC_STAGES = 2;
+constexpr int SC_MIN = 64;      // fewest tokens of a sequence that takes this way (two chunks; single tokens are better off above)
+constexpr int SC_REC = SC_TOKENS * SC_TOKENS + 2 * SC_TOKENS;  // floats of a (chunk, head): M, e, w
+
+__device__ __forceinline__ bool sc_takes(const int* seq_slot, const int* seq_start, int b, int& n) {
+  n = seq_start[b + 1] - seq_start[b];
+  return seq_slot[b] >= 0 && n >= SC_MIN;
+}
+__device__ __forceinline__ void cp_async_16(float* dst, const float* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(ok ? 16 : 0)
+               : "memory");
+}
+
+template <typename T, int N>
+__global__ void __launch_bounds__(SC_THREADS)
+ssm_chunk_prepare_kernel(const float* __restrict__ xbc, long xbc_stride, const T* __restrict__ dt_raw, long dt_stride,
+                         const float* __restrict__ dt_bias, const float* __restrict__ a_log, float* __restrict__ chunks,
+                         const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs, int heads,
+                         int groups, int P) {
+  __shared__ __align__(16) float bs[SC_TOKENS][N + 4];
+  __shared__ __align__(16) float cs[SC_TOKENS][N + 4];
+  __shared__ float gram[SC_TOKENS][SC_TOKENS + 1];
+  __shared__ float decs[SC_THREADS / 32][SC_TOKENS];
+  const int g = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int c = blockIdx.x, b = 0, n = 0;
+  for (; b < n_seqs; ++b) {
+    if (!sc_takes(seq_slot, seq_start, b, n)) continue;
+    const int nc = (n + SC_TOKENS - 1) / SC_TOKENS;
+    if (c < nc) break;
+    c -= nc;
+  }
+  if (b == n_seqs) return;
+  const int t0 = seq_start[b] + c * SC_TOKENS, nt = min(SC_TOKENS, n - c * SC_TOKENS), inner = heads * P;
+  for (int i = tid; i < SC_TOKENS * (N / 4); i += SC_THREADS) {
+    const int t = i / (N / 4), w = i % (N / 4) * 4;
+    float4 bv = make_float4(0.f, 0.f, 0.f, 0.f), cv = bv;
+    if (t < nt) {
+      const float* row = xbc + (size_t)(t0 + t) * xbc_stride + inner + g * N + w;
+      bv = *reinterpret_cast<const float4*>(row);
+      cv = *reinterpret_cast<const float4*>(row + groups * N);
+    }
+    *reinterpret_cast<float4*>(&bs[t][w]) = bv;
+    *reinterpret_cast<float4*>(&cs[t][w]) = cv;
+  }
+  __syncthreads();
+  {
+    const int ib = tid >> 4, jb = tid & 15;
+    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+    for (int w = 0; w < N; w += 4) {
+      float4 cv[2], bv[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        cv[e] = *reinterpret_cast<const float4*>(&cs[ib + 16 * e][w]);
+        bv[e] = *reinterpret_cast<const float4*>(&bs[jb + 16 * e][w]);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+          acc[e][f] = fmaf(cv[e].x, bv[f].x, acc[e][f]);
+          acc[e][f] = fmaf(cv[e].y, bv[f].y, acc[e][f]);
+          acc[e][f] = fmaf(cv[e].z, bv[f].z, acc[e][f]);
+          acc[e][f] = fmaf(cv[e].w, bv[f].w, acc[e][f]);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int f = 0; f < 2; ++f) gram[ib + 16 * e][jb + 16 * f] = acc[e][f];
+  }
+  __syncthreads();
+  const int per = heads / groups;
+  for (int hh = warp; hh < per; hh += SC_THREADS / 32) {  // a warp a head, a lane a column j
+    const int h = g * per + hh;
+    float dt = 0.f, dec = 1.f;  // tokens beyond the sequence change nothing
+    if (lane < nt) {
+      const float v = to_f32<T>(dt_raw[(size_t)(t0 + lane) * dt_stride + h]) + dt_bias[h];
+      dt = v > 20.f ? v : log1pf(expf(v));
+      dec = expf(-expf(a_log[h]) * dt);
+    }
+    decs[warp][lane] = dec;
+    __syncwarp();
+    float* rec = chunks + ((size_t)blockIdx.x * heads + h) * SC_REC;
+    float d = 1.f, e = 1.f;
+    for (int i = 0; i < SC_TOKENS; ++i) {
+      const float ai = decs[warp][i];
+      e *= ai;
+      if (i > lane) d *= ai;
+      rec[i * SC_TOKENS + lane] = i >= lane ? gram[i][lane] * d * dt : 0.f;
+      if (lane == 0) rec[SC_TOKENS * SC_TOKENS + i] = e;
+    }
+    rec[SC_TOKENS * SC_TOKENS + SC_TOKENS + lane] = d * dt;
+    __syncwarp();
+  }
+}
+
+template <int N>
+struct ScanWalk {
+  static constexpr int SCN = N + 4, SM = SC_TOKENS + 4, SP = SC_COLS;
+  static constexpr int C = 0, B = C + SC_TOKENS * SCN, M = B + SC_TOKENS * N, X = M + SC_TOKENS * SM, E = X + SC_TOKENS * SP,
+                       W = E + SC_TOKENS, BUF = W + SC_TOKENS;
+  static constexpr int GROUPS = 4;  // groups of threads that share out the sums of C S0 and M X
+  static constexpr int S = SC_STAGES * BUF, XW = S + N * SP, PART = XW + SC_TOKENS * SP, SPART = SP + 4;
+  static constexpr size_t SMEM = sizeof(float) * (PART + GROUPS * SC_TOKENS * SPART);
+};
+
+template <int N>
+__global__ void __launch_bounds__(SC_THREADS)
+ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, const float* __restrict__ chunks,
+                 const float* __restrict__ d_skip, float* __restrict__ y, long y_stride, float* __restrict__ state,
+                 long state_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int heads,
+                 int groups, int P) {
+  using L = ScanWalk<N>;
+  constexpr int NROWS = N / 32;  // rows of the state a thread, side by side
+  extern __shared__ __align__(16) float smem[];
+  float *const s_s = smem + L::S, *const xw_s = smem + L::XW, *const part = smem + L::PART;
+  const int b = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * SC_COLS, tid = threadIdx.x;
+  int n;
+  if (!sc_takes(seq_slot, seq_start, b, n)) return;
+  int first = 0;  // the sequence's first chunk
+  for (int i = 0; i < b; ++i) {
+    int m;
+    if (sc_takes(seq_slot, seq_start, i, m)) first += (m + SC_TOKENS - 1) / SC_TOKENS;
+  }
+  const int start = seq_start[b], n_chunks = (n + SC_TOKENS - 1) / SC_TOKENS;
+  const int g = h / (heads / groups), inner = heads * P;
+  const float dsk = d_skip[h];
+
+  auto issue = [&](int c) {
+    float* buf = smem + c % SC_STAGES * L::BUF;
+    const int t0 = start + c * SC_TOKENS, nt = min(SC_TOKENS, n - c * SC_TOKENS);
+    for (int i = tid; i < SC_TOKENS * (N / 4); i += SC_THREADS) {
+      const int t = i / (N / 4), w = i % (N / 4) * 4;
+      const float* row = xbc + (size_t)(t < nt ? t0 + t : t0) * xbc_stride + inner + g * N + w;
+      cp_async_16(buf + L::B + t * N + w, row, t < nt);
+      cp_async_16(buf + L::C + t * L::SCN + w, row + groups * N, t < nt);
+    }
+    const float* rec = chunks + ((size_t)(first + c) * heads + h) * SC_REC;
+    {
+      const int t = tid / 8, w = tid % 8 * 4;  // 32 rows of 32 numbers: M and x
+      cp_async_16(buf + L::M + t * L::SM + w, rec + t * SC_TOKENS + w, true);
+      const bool ok = t < nt && p0 + w < P;
+      cp_async_16(buf + L::X + t * L::SP + w, ok ? xbc + (size_t)(t0 + t) * xbc_stride + h * P + p0 + w : xbc, ok);
+    }
+    if (tid < 2 * SC_TOKENS / 4) cp_async_16(buf + L::E + tid * 4, rec + SC_TOKENS * SC_TOKENS + tid * 4, true);
+  };
+  issue(0);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+
+  // the state: rows NROWS nb + r, columns 4 pb .. + 3
+  const int pb = tid & 7, nb = tid >> 3;
+  float* const st = state + (size_t)seq_slot[b] * state_stride + (size_t)h * N * P;
+  float s[NROWS][4];
+#pragma unroll
+  for (int r = 0; r < NROWS; ++r)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int p = p0 + 4 * pb + e;
+      s[r][e] = p < P ? st[(size_t)p * N + NROWS * nb + r] : 0.f;
+    }
+  // the sums of C S0 and M X: group q takes a quarter of the state's rows and of the tokens, a thread 4 x 4 places
+  const int q = tid >> 6, ib = (tid & 63) >> 3;
+  for (int c = 0; c < n_chunks; ++c) {
+    const float* buf = smem + c % SC_STAGES * L::BUF;
+#pragma unroll
+    for (int r = 0; r < NROWS; ++r)
+      *reinterpret_cast<float4*>(s_s + (NROWS * nb + r) * L::SP + 4 * pb) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // the chunk has landed, the state stands in shared memory, the buffer of the chunk before is free
+    if (c + 1 < n_chunks) issue(c + 1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    {  // w X for the state's update
+      const int t = tid / 8, w = tid % 8 * 4;
+      const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
+      const float wt = buf[L::W + t];
+      *reinterpret_cast<float4*>(xw_s + t * L::SP + w) = make_float4(x.x * wt, x.y * wt, x.z * wt, x.w * wt);
+    }
+    float acc[4][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int f = 0; f < 4; ++f) acc[e][f] = 0.f;
+    auto products = [&](const float* left, int left_stride, const float* right, int from, int count) {
+#pragma unroll 2
+      for (int k = from; k < from + count; k += 4) {
+        float4 a[4], v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          a[e] = *reinterpret_cast<const float4*>(left + (ib + 8 * e) * left_stride + k);
+          v[e] = *reinterpret_cast<const float4*>(right + (k + e) * L::SP + 4 * pb);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float ae[4] = {a[e].x, a[e].y, a[e].z, a[e].w};
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {
+            acc[e][0] = fmaf(ae[f], v[f].x, acc[e][0]);
+            acc[e][1] = fmaf(ae[f], v[f].y, acc[e][1]);
+            acc[e][2] = fmaf(ae[f], v[f].z, acc[e][2]);
+            acc[e][3] = fmaf(ae[f], v[f].w, acc[e][3]);
+          }
+        }
+      }
+    };
+    products(buf + L::C, L::SCN, s_s, q * (N / 4), N / 4);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float ei = buf[L::E + ib + 8 * e];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) acc[e][f] *= ei;
+    }
+    products(buf + L::M, L::SM, buf + L::X, q * (SC_TOKENS / 4), SC_TOKENS / 4);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      *reinterpret_cast<float4*>(part + (q * SC_TOKENS + ib + 8 * e) * L::SPART + 4 * pb) =
+          make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
+    __syncthreads();
+    {  // a token's four columns a thread: the groups' sums in order
+      const int t = tid / 8, w = tid % 8 * 4;
+      const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
+      float4 v = *reinterpret_cast<const float4*>(part + t * L::SPART + w);
+#pragma unroll
+      for (int i = 1; i < L::GROUPS; ++i) {
+        const float4 u = *reinterpret_cast<const float4*>(part + (i * SC_TOKENS + t) * L::SPART + w);
+        v.x += u.x;
+        v.y += u.y;
+        v.z += u.z;
+        v.w += u.w;
+      }
+      if (c * SC_TOKENS + t < n && p0 + w < P)
+        *reinterpret_cast<float4*>(y + (size_t)(start + c * SC_TOKENS + t) * y_stride + h * P + p0 + w) =
+            make_float4(fmaf(dsk, x.x, v.x), fmaf(dsk, x.y, v.y), fmaf(dsk, x.z, v.z), fmaf(dsk, x.w, v.w));
+    }
+    const float whole = buf[L::E + SC_TOKENS - 1];
+#pragma unroll
+    for (int r = 0; r < NROWS; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[r][e] *= whole;
+#pragma unroll 8
+    for (int t = 0; t < SC_TOKENS; ++t) {
+      const float4 x = *reinterpret_cast<const float4*>(xw_s + t * L::SP + 4 * pb);
+      __align__(16) float bt[NROWS];
+      if (NROWS == 4) *reinterpret_cast<float4*>(bt) = *reinterpret_cast<const float4*>(buf + L::B + t * N + 4 * nb);
+      else *reinterpret_cast<float2*>(bt) = *reinterpret_cast<const float2*>(buf + L::B + t * N + 2 * nb);
+#pragma unroll
+      for (int r = 0; r < NROWS; ++r) {
+        const float bv = bt[r];
+        s[r][0] = fmaf(bv, x.x, s[r][0]);
+        s[r][1] = fmaf(bv, x.y, s[r][1]);
+        s[r][2] = fmaf(bv, x.z, s[r][2]);
+        s[r][3] = fmaf(bv, x.w, s[r][3]);
+      }
+    }
+    // (the next chunk's state goes to shared memory at once: its readers are through since the barrier above;
+    // w X is written behind the next barrier)
+  }
+#pragma unroll
+  for (int r = 0; r < NROWS; ++r)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int p = p0 + 4 * pb + e;
+      if (p < P) st[(size_t)p * N + NROWS * nb + r] = s[r][e];
+    }
 }
 
 // ---- gate, then RMS norm in equal parts ---------------------------------------------------------
@@ -635,22 +921,57 @@ extern "C" int fg_mamba2_conv(const void* proj, long proj_stride, long xbc_offse
                       conv_offset, req, seq_slot, seq_start, n_tokens, n_seqs, channels, taps, 1, stream);
 }
 
+// Whether a step may hold sequences for ssm_chunk_kernel: 16-bit serving, states of 64 or 128 rows, rows in
+// whole groups of four, and enough tokens for one such sequence.
+static bool sc_apply(int n_tokens, int n_state, int head_dim, int dtype) {
+  return dtype == FG_BF16 && (n_state == 64 || n_state == 128) && head_dim % 4 == 0 && n_tokens >= SC_MIN;
+}
+// most chunks of a step's sequences that have SC_MIN tokens or more
+static long sc_most_chunks(int n_tokens, int n_seqs) {
+  const int long_ones = n_tokens / SC_MIN;
+  return n_tokens / SC_TOKENS + (n_seqs < long_ones ? n_seqs : long_ones);
+}
+
+// floats of the scratch that fg_mamba2_scan takes (0: none; without it every token goes through the token kernels)
+extern "C" long fg_mamba2_scan_scratch_floats(int n_tokens, int n_seqs, int heads, int n_state, int head_dim, int dtype) {
+  return sc_apply(n_tokens, n_state, head_dim, dtype) ? sc_most_chunks(n_tokens, n_seqs) * heads * SC_REC : 0;
+}
+
 template <typename T>
 static int launch_scan(const float* xbc, long xbc_stride, const T* dt_raw, long dt_stride, const float* dt_bias,
                        const float* a_log, const float* d_skip, float* y, long y_stride, float* state, long state_stride,
                        const int* seq_slot, const int* seq_start, int n_seqs, int heads, int groups, int N, int P,
-                       cudaStream_t stream) {
+                       int n_tokens, float* scratch, cudaStream_t stream) {
   const dim3 grid(n_seqs, heads, (P + SCAN_PB - 1) / SCAN_PB);
   const size_t smem = 2 * sizeof(float) * (size_t)(2 * SCAN_TOKENS * N + SCAN_TOKENS * SCAN_PB + 2 * SCAN_TOKENS);
   if (N == 64 || N == 128 || N == 256) {
     const size_t tsmem = 2 * sizeof(float) * (size_t)(2 * SCAN_TOKENS * N + SCAN_TOKENS * SCAN_PB + 2 * SCAN_TOKENS);
+    int most = 0x7fffffff;  // tokens of the longest sequence that the token kernel takes
+    if (scratch != nullptr) {
+      most = SC_MIN - 1;
+      const dim3 prepare((unsigned)sc_most_chunks(n_tokens, n_seqs), groups), walk(n_seqs, heads, (P + SC_COLS - 1) / SC_COLS);
+#define CHUNKS(NN)                                                                                                   \
+  do {                                                                                                               \
+    ssm_chunk_prepare_kernel<T, NN><<<prepare, SC_THREADS, 0, stream>>>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias,  \
+                                                                        a_log, scratch, seq_slot, seq_start, n_seqs, \
+                                                                        heads, groups, P);                           \
+    cudaFuncSetAttribute(ssm_chunk_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ScanWalk<NN>::SMEM); \
+    ssm_chunk_kernel<NN><<<walk, SC_THREADS, ScanWalk<NN>::SMEM, stream>>>(xbc, xbc_stride, scratch, d_skip, y,       \
+                                                                           y_stride, state, state_stride, seq_slot,  \
+                                                                           seq_start, heads, groups, P);             \
+  } while (0)
+      if (N == 64) CHUNKS(64);
+      else CHUNKS(128);
+#undef CHUNKS
+      FG_CHECK_LAUNCH("fg_mamba2_scan (chunks)");
+    }
 #define TILED(NPT)                                                                                              \
   do {                                                                                                          \
     auto kern = ssm_scan_tiled_kernel<T, NPT>;                                                                  \
     if (tsmem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem); \
     kern<<<grid, TS_THREADS, tsmem, stream>>>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, d_skip, y,    \
                                               y_stride, state, state_stride, seq_slot, seq_start, heads,        \
-                                              groups, P);                                                       \
+                                              groups, P, most);                                                 \
   } while (0)
     if (N == 64) TILED(2);
     else if (N == 128) TILED(4);
@@ -686,19 +1007,23 @@ extern "C" int fg_mamba2_scan(const float* xbc, long xbc_stride, const void* pro
                               int dtype, const float* dt_bias, const float* a_log, const float* d_skip, float* y,
                               long y_stride, float* state, long state_stride, const int* seq_slot,
                               const int* seq_start, int n_seqs, int heads, int groups, int N, int P,
-                              cudaStream_t stream) {
+                              int n_tokens, float* scratch, cudaStream_t stream) {
   if (n_seqs == 0) return 0;
   FG_CHECK_ARG(heads > 0 && groups > 0 && heads % groups == 0 && N > 0 && P > 0,
                "fg_mamba2_scan: bad sizes heads=%d groups=%d N=%d P=%d", heads, groups, N, P);
+  // the chunks' copies are of 16 bytes
+  if (!sc_apply(n_tokens, N, P, dtype) || xbc_stride % 4 != 0 || y_stride % 4 != 0 ||
+      (((uintptr_t)xbc | (uintptr_t)y | (uintptr_t)scratch) & 15) != 0)
+    scratch = nullptr;
   int rc;
   if (dtype == FG_F32)
     rc = launch_scan<float>(xbc, xbc_stride, (const float*)proj + dt_offset, proj_stride, dt_bias,
                             a_log, d_skip, y, y_stride, state, state_stride, seq_slot,
-                            seq_start, n_seqs, heads, groups, N, P, stream);
+                            seq_start, n_seqs, heads, groups, N, P, n_tokens, scratch, stream);
   else if (dtype == FG_BF16)
     rc = launch_scan<__nv_bfloat16>(xbc, xbc_stride, (const __nv_bfloat16*)proj + dt_offset, proj_stride,
                                     dt_bias, a_log, d_skip, y, y_stride, state, state_stride, seq_slot,
-                                    seq_start, n_seqs, heads, groups, N, P, stream);
+                                    seq_start, n_seqs, heads, groups, N, P, n_tokens, scratch, stream);
   else
     FG_CHECK_ARG(false, "fg_mamba2_scan: bad dtype %d", dtype);
   if (rc) return rc;

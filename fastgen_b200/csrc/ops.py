@@ -55,7 +55,8 @@ _CORE_SIGNATURES = {
     "fg_time_conv": [_P, _L, _L, _I, _P, _L, _I, _P, _P, _P, _L, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fg_head_gate": [_P, _L, _P, _L, _I, _P, _I, _I, _I, _P],
     "fg_qk_head_factors": [_P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P, _P, _P, _I, _P],
-    "fg_mamba2_scan": [_P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _I, _P],
+    "fg_mamba2_scan": [_P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+    "fg_mamba2_scan_scratch_floats": [_I, _I, _I, _I, _I, _I],
     "fg_gated_part_norm": [_P, _L, _P, _L, _I, _P, _P, _L, _P, _I, _I, _I, _F, _P],
     "fg_selective_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _P],
     "fg_layer_norm_pair": [_P, _P, _P, _I, _I, _P, _P, _F, _P, _P, _F, _P, _I, _P, _I, _I, _P],
@@ -265,6 +266,7 @@ def core():
     if _core is None:
         lib = build.core_library()
         _declare(lib, _CORE_SIGNATURES)
+        lib.fg_mamba2_scan_scratch_floats.restype = ctypes.c_longlong
         _core = lib
     return _core
 
@@ -440,10 +442,14 @@ class Ops:
         for v in (dt_bias, a_log, d_skip):
             assert v.dtype == torch.float32 and v.numel() == heads and v.is_contiguous()
         y = torch.empty((t, heads * head_dim), dtype=torch.float32, device=xbc.device)
+        # sequences of many tokens in 16-bit serving go chunk by chunk: what the chunks are alone
+        floats = self.lib.fg_mamba2_scan_scratch_floats(t, ctx.n_seqs, heads, n_state, head_dim, _code(proj.dtype))
+        scratch = torch.empty(floats, dtype=torch.float32, device=xbc.device) if floats else None
         _check(self.lib, self.lib.fg_mamba2_scan(
             _ptr(xbc), xbc.stride(0), _ptr(proj), proj.stride(0), int(dt_offset), _code(proj.dtype), _ptr(dt_bias),
             _ptr(a_log), _ptr(d_skip), _ptr(y), y.stride(0), _ptr(state), state.stride(0), _ptr(ctx.seq_slot),
-            _ptr(ctx.seq_start), ctx.n_seqs, heads, groups, n_state, head_dim, _stream()))
+            _ptr(ctx.seq_start), ctx.n_seqs, heads, groups, n_state, head_dim, t, _ptr(scratch), _stream()))
+        Ops.launches += 2 * int(scratch is not None)  # the chunks' two kernels
         return y
 
     def gated_part_norm(self, y, z, weight, parts: int, eps: float, ctx) -> torch.Tensor:

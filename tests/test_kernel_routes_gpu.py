@@ -156,6 +156,45 @@ def _relative(got, ref):
     return float((got.double() - ref).norm() / ref.norm())
 
 
+@pytest.mark.parametrize("n_state,p", [(128, 64), (64, 40), (128, 4)])
+@pytest.mark.parametrize("lengths,pad", LENGTHS)
+def test_state_space_recurrence(ops16, lengths, pad, n_state, p):
+    """Sequences on both sides of the length from which chunks are walked, in one step."""
+    heads, groups = 6, 2
+    slots = [3, 0, 2][: len(lengths)]
+    ctx = _sequences(lengths, pad, slots)
+    t = ctx.n_tokens
+    g = torch.Generator().manual_seed(sum(lengths) + p)
+    inner, bc = heads * p, groups * n_state
+    xbc = _randn(g, t, inner + 2 * bc, scale=0.5)
+    proj = _randn(g, t, 16 + heads).to(torch.bfloat16)
+    dt_bias, a_log = torch.rand(heads, generator=g).to(DEV) * 3.5 - 3, torch.rand(heads, generator=g).to(DEV) * 2.5 - 1
+    d = _randn(g, heads)
+    state = _randn(g, 5, heads * n_state * p + 12)
+    before = state.clone()
+    y = ops16.mamba2_scan(xbc, proj, 16, dt_bias, a_log, d, state, ctx, heads, groups, n_state, p)
+    per = heads // groups
+    for i, (n, slot) in enumerate(zip(lengths, slots)):
+        a = int(ctx.seq_start[i])
+        rows = xbc[a : a + n].double()
+        x = rows[:, :inner].reshape(n, heads, p)
+        b = rows[:, inner : inner + bc].reshape(n, groups, n_state).repeat_interleave(per, 1)
+        c = rows[:, inner + bc :].reshape(n, groups, n_state).repeat_interleave(per, 1)
+        dt = torch.nn.functional.softplus(proj[a : a + n, 16:].double() + dt_bias.double(), threshold=1e9)
+        decay = torch.exp(-torch.exp(a_log.double()) * dt)
+        S = before[slot, : heads * n_state * p].double().reshape(heads, p, n_state).clone()
+        ref = torch.empty(n, heads, p, dtype=torch.float64, device=DEV)
+        for s in range(n):
+            S = decay[s][:, None, None] * S + (dt[s][:, None] * x[s])[:, :, None] * b[s][:, None, :]
+            ref[s] = (S * c[s][:, None, :]).sum(-1) + d.double()[:, None] * x[s]
+        bound = (n_state + 2 * 32 + 64) * EPS  # the sums of a row and of a chunk, the decays of a chunk
+        assert _relative(y[a : a + n], ref.reshape(n, inner)) <= bound
+        assert _relative(state[slot, : heads * n_state * p], S.reshape(-1)) <= bound
+        assert torch.equal(state[slot, heads * n_state * p :], before[slot, heads * n_state * p :])
+    for slot in {0, 1, 2, 3, 4} - set(slots):
+        assert torch.equal(state[slot], before[slot])
+
+
 @pytest.mark.parametrize("d,dv", [(64, 64), (40, 24), (128, 12), (100, 130)])
 @pytest.mark.parametrize("lengths,pad", LENGTHS)
 def test_delta_rule_with_one_decay_a_head(ops16, lengths, pad, d, dv):
