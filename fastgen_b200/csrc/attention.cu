@@ -37,7 +37,17 @@ extern "C" int fg_attention_simt(const void* q, int q_stride, void* out, int out
   dim3 grid(n_tiles, n_kv_heads, (group + hpb - 1) / hpb);
   constexpr size_t smem = simt_smem_bytes<FG_HEAD_DIM>();
   cudaError_t e;
-  if (dtype == FG_F32) {
+  // pages whose rows start on 16 bytes (head sizes are multiples of 16 numbers): asynchronous copies
+  if (dtype == FG_F32 && (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
+    auto kern = attention_simt_f32_kernel<FG_HEAD_DIM>;
+    constexpr size_t bytes = SimtShape<FG_HEAD_DIM>::SMEM;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    FG_CHECK_ARG(e == cudaSuccess, "fg_attention_simt: shared memory: %s", cudaGetErrorString(e));
+    kern<<<grid, THREADS, bytes, stream>>>((const float*)q, q_stride, (float*)out, out_stride, (const float*)k_pages,
+                                           (const float*)v_pages, block_table, table_width, page_size, n_pages, pos,
+                                           tile_req, tile_tok0, tile_ntok, n_kv_heads, group, hpb, window, keep_first,
+                                           scale, status, softcap, sinks);
+  } else if (dtype == FG_F32) {
     auto kern = attention_simt_kernel<float, FG_HEAD_DIM>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     FG_CHECK_ARG(e == cudaSuccess, "fg_attention_simt: shared memory: %s", cudaGetErrorString(e));

@@ -55,6 +55,10 @@ def test_float32_product_routes(ops32, m, n, k):
     assert bool(((got.double() - ref).abs() <= bound + 1e-30).all())
 
 
+def _relative(got, ref):
+    return float((got.double() - ref).norm() / ref.norm())
+
+
 # -- convolution, gate and norms -----------------------------------------------------------------------
 
 def _sequences(lengths, pad=0, slots=None):
@@ -147,13 +151,55 @@ def _stream_norm(ops, h, w, out, delta, mix, out_coef, in_coef, bias, eps, rms, 
                                            h.shape[2], eps, int(rms), _stream()))
 
 
+# -- attention ----------------------------------------------------------------------------------------------
+
+def _attention_step(lengths, cached, page, heads, kv, hd, dtype, seed):
+    """Queries of sequences that bring ``lengths`` tokens behind ``cached`` ones, and pools that hold random entries."""
+    from fastgen_b200.engine.step import StepContext
+    g = torch.Generator().manual_seed(seed)
+    width = max(-(-(c + n) // page) for c, n in zip(cached, lengths))
+    n_pages = width * len(lengths) + 3
+    order = torch.randperm(n_pages, generator=g)[: width * len(lengths)].reshape(len(lengths), width)
+    ctx = StepContext(torch.device(DEV))
+    ctx.host_seq_slot, ctx.host_seq_cached = list(range(len(lengths))), list(cached)
+    ctx.host_seq_start = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    pos = [c + i for c, n in zip(cached, lengths) for i in range(n)]
+    ctx.pos = torch.tensor(pos, dtype=torch.int32, device=DEV)
+    ctx.n_tokens, ctx.n_seqs = len(pos), len(lengths)
+    q = _randn(g, len(pos), heads * hd).to(dtype)
+    pools = [_randn(g, n_pages, kv, page, hd).to(dtype) for _ in range(2)]
+    return ctx, q, pools, order.to(DEV, torch.int32)
+
+
+@pytest.mark.parametrize("hd,heads,kv", [(64, 8, 2), (16, 3, 3), (48, 20, 1)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (40, 0), (40, 5), (-37, 0)])
+def test_float32_attention_on_asynchronous_copies(ops32, hd, heads, kv, window, keep):
+    """The bits of the kernel that loads a number at a time (taken for pools that do not start on 16 bytes)."""
+    from fastgen_b200.csrc.ops import SIMT_ROWS, _check, _code, _ptr, _stream, attention_tiling, attn
+    ctx, q, pools, table = _attention_step([1, 33, 7], [130, 0, 31], 8, heads, kv, hd, torch.float32, hd + window)
+    sinks = torch.linspace(-1, 1, heads, device=DEV)
+    tiles = ctx.attention_tiles(attention_tiling(heads, kv, SIMT_ROWS), 1)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = []
+    for shift in (0, 1):
+        moved = []
+        for pool in pools:
+            room = torch.empty(pool.numel() + 4, device=DEV)
+            moved.append(room[shift : shift + pool.numel()].view(pool.shape))
+            moved[-1].copy_(pool)
+        out = torch.full_like(q, float("nan"))
+        lib = attn(hd)
+        _check(lib, lib.fg_attention_simt(
+            _ptr(q), q.stride(0), _ptr(out), out.stride(0), _code(q.dtype), _ptr(moved[0]), _ptr(moved[1]), _ptr(table),
+            table.shape[1], 8, pools[0].shape[0], _ptr(ctx.pos), _ptr(tiles.req), _ptr(tiles.tok0), _ptr(tiles.ntok), tiles.n,
+            heads, kv, hd, window, keep, hd ** -0.5, 3.0 if keep else 0.0, _ptr(sinks), _ptr(status), _stream()))
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all()) and int(status) == 0
+
+
 # -- recurrences, chunk by chunk ---------------------------------------------------------------------------
 
 LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0)]
-
-
-def _relative(got, ref):
-    return float((got.double() - ref).norm() / ref.norm())
 
 
 @pytest.mark.parametrize("n_state,p", [(128, 64), (64, 40), (128, 4)])
