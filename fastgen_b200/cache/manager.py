@@ -185,6 +185,7 @@ class CacheManager:
         device=None,
         tensor_map_factory=None,
         embedder_state: Optional[StateSpec] = None,
+        table_writer=None,
     ) -> None:
         if page_size <= 0:
             raise ValueError(f"page size must be positive, got {page_size}")
@@ -193,6 +194,9 @@ class CacheManager:
         self.max_length = max_length
         self.dtype = dtype
         self.device = device
+        #: ``table_writer(device table, places, values)`` carries changes of a table to the device; without
+        #: one they are copied (and the host waits for the copies)
+        self.table_writer = table_writer
         self.kv_from = list(kv_from)
         n_entries = len(cache_specs)
 
@@ -399,9 +403,12 @@ class CacheManager:
             # later writes to the same entry must win: keep the last of each index
             _, last = np.unique(flat[::-1], return_index=True)
             keep = len(flat) - 1 - last
-            idx = torch.from_numpy(flat[keep]).to(self.device, non_blocking=False)
-            val = torch.from_numpy(vals[keep]).to(self.device, non_blocking=False)
-            grp.device_table.view(-1).index_copy_(0, idx, val)
+            if self.table_writer is not None and grp.device_table.numel() < 1 << 31:
+                self.table_writer(grp.device_table, flat[keep], vals[keep])
+            else:
+                idx = torch.from_numpy(flat[keep]).to(self.device, non_blocking=False)
+                val = torch.from_numpy(vals[keep]).to(self.device, non_blocking=False)
+                grp.device_table.view(-1).index_copy_(0, idx, val)
             grp.dirty.clear()
 
     def memories(self) -> StepMemories:

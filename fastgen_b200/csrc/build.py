@@ -54,6 +54,7 @@ CORE_SOURCES = [
     "gemm_skinny.cu",
     "sampling.cu",
     "tensor_map.cu",
+    "table_entries.cu",
     "selftest.cu",
 ]
 

@@ -251,7 +251,9 @@ constexpr int CHUNK = 32;
 constexpr int CHUNK_THREADS = 128;
 constexpr int CHUNK_COLS = 8;    // columns of the state a block of the walk
 constexpr int CHUNK_STAGES = 3;  // chunks in its ring
-constexpr int CHUNK_MIN = 64;    // fewest tokens of a sequence that takes this way (64 tokens: 15 us above, about 20 here; 128: 30 and 22)
+// Fewest tokens of a sequence that takes this way: where the two meet.  One sequence of 63 tokens 20.8 us above, of
+// 64 here 19.7, of 128 23.4 (16 heads of 64, prepared and formed).
+constexpr int CHUNK_MIN = 64;
 
 // floats of a (chunk, head): W [32][D], c Q [32][D], (D[C] o K)^T [D][32], D o Q K^T [32][32], V' [32][DVP], c_C
 __host__ __device__ constexpr long chunk_floats(int D, int DVP) { return 96L * D + CHUNK * CHUNK + CHUNK * DVP + 4; }

@@ -14,6 +14,7 @@ import os
 from ctypes import c_float, c_int, c_ulonglong, c_void_p
 from typing import Optional
 
+import numpy as np
 import torch
 
 from . import build
@@ -87,6 +88,7 @@ _CORE_SIGNATURES = {
     "fg_sample": [_P, _I, _I, _I, _P, _F, c_ulonglong, _P, _P, _P, _P, _P, _P, _P],
     "fg_selftest_wait_timeout": [_I, _P, _P, _P],
     "fg_sample_uniform": [c_ulonglong, _P, _P, _P, _I, _P],
+    "fg_set_table_entries": [_P, _P, _P, _I, _P],
     "fg_make_kv_tensor_map": [_P, _P, _I, _I, _I, _I, _I, _I],
 }
 
@@ -1291,6 +1293,16 @@ class Ops:
         if buf is None:
             buf = self._scratch[size] = torch.empty(size, dtype=torch.float32, device=self.device)
         return buf
+
+    def set_table_entries(self, table: torch.Tensor, at, value) -> None:
+        """``table.view(-1)[at[i]] = value[i]`` for host arrays (numpy, integers) of places that all differ; the
+        entries travel in the launches' arguments, so the host waits for nothing."""
+        at, value = np.ascontiguousarray(at, dtype=np.int32), np.ascontiguousarray(value, dtype=np.int32)
+        assert table.dtype == torch.int32 and table.is_contiguous() and table.numel() < 1 << 31 and at.shape == value.shape
+        if at.size == 0:
+            return
+        assert 0 <= int(at.min()) and int(at.max()) < table.numel()
+        _check(self.lib, self.lib.fg_set_table_entries(_ptr(table), at.ctypes.data, value.ctypes.data, at.size, _stream()))
 
     def make_kv_tensor_maps(self, k_pool, v_pool, page_size: int):
         """Tensor maps of a key and a value pool [layers, pages, kv heads, page,

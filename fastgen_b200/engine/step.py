@@ -206,6 +206,7 @@ class Engine:
             device=self.device,
             tensor_map_factory=model.ops.make_kv_tensor_maps,
             embedder_state=model.embedder_state_spec(),
+            table_writer=model.ops.set_table_entries,
         )
         self.memories = self.cache.memories()
         self.last_h2d_bytes = 0

@@ -151,6 +151,20 @@ def _stream_norm(ops, h, w, out, delta, mix, out_coef, in_coef, bias, eps, rms, 
                                            h.shape[2], eps, int(rms), _stream()))
 
 
+# -- block tables ----------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("n", [1, 480, 481, 1300])
+def test_table_entries_in_launch_arguments(ops32, n):
+    g = torch.Generator().manual_seed(n)
+    table = torch.randint(0, 99, (7, 300), generator=g, dtype=torch.int32).to(DEV)
+    want = table.clone()
+    at = torch.randperm(table.numel(), generator=g)[:n]
+    value = torch.randint(-1, 1 << 20, (n,), generator=g, dtype=torch.int32)
+    want.view(-1)[at.to(DEV)] = value.to(DEV)
+    ops32.set_table_entries(table, at.numpy(), value.numpy())
+    assert torch.equal(table, want)
+
+
 # -- attention ----------------------------------------------------------------------------------------------
 
 def _attention_step(lengths, cached, page, heads, kv, hd, dtype, seed):
