@@ -110,7 +110,7 @@ _ATTN_SIGNATURES = {
     "fg_attention_prefill_tma_bf16": [_P, _I, _P, _I, _P, _P, _I, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I,
                                       _I, _F, _I, _P, _P],
     "fg_attention_prefill_tc5_bf16": [_P, _I, _P, _I, _P, _P, _I, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I,
-                                      _I, _F, _P, _P, _P, _I, _I, _P, _I, _F, _P, _P, _P],
+                                      _I, _F, _P, _P, _P, _I, _I, _P, _I, _F, _P, _I, _P, _P],
     "fg_attention_prefill_tc5_split_slots": [_I, _I, _I, _I, _I],
     "fg_attention_decode_tma_bf16": [_P, _I, _P, _I, _P, _P, _I, _P, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I,
                                      _F, _P, ctypes.c_longlong, _I, ctypes.c_longlong, _P, _P, _P, _P],
@@ -1378,15 +1378,15 @@ class Ops:
                 n_heads, n_kv_heads, head_dim, window, keep_first, float(scale), float(softcap or 0.0),
                 _ptr(sinks), _ptr(self.status), _stream()))
             return False
-        # windows that keep a sequence's first positions visible run on the mma.sync kernels (on TMA
-        # tiles for prompts where the pools have tensor maps), which walk the tiles of the kept
-        # positions before those of the window
+        # windows that keep a sequence's first positions visible: the kernels walk the tiles of the kept
+        # positions before those of the window (prompts: the tcgen05 kernel at head sizes 64 and 128 without a
+        # cap, else the mma.sync kernels)
         # capped scores: the cap lives in the tcgen05 kernel (head sizes 64 and 128) and in the
         # mma.sync kernels on cp.async tiles
         # sinks: in prompt portions a row starts its running maximum and sum from the sink, in the
         # tcgen05 kernel (head sizes 64 and 128) and in the mma.sync kernel on cp.async tiles; single
         # tokens keep their kernels (the sink joins where the splits are merged)
-        tc5 = head_dim in (64, 128) and self.use_tcgen05 and not keep_first
+        tc5 = head_dim in (64, 128) and self.use_tcgen05 and not (keep_first and softcap)
         use_tma = memory.tensor_maps is not None and (not softcap or tc5)
         prompt_tma = use_tma and (sinks is None or tc5)
         rows = PREFILL_TMA_ROWS if prompt_tma else PREFILL_ROWS
@@ -1407,7 +1407,8 @@ class Ops:
                 scratch, flags, room = self._split_buffers(head_dim, want)
                 _check(lib, lib.fg_attention_prefill_tc5_bf16(
                     *args, _ptr(self._work_counter), _ptr(scratch), _ptr(flags), room, max_keys,
-                    _ptr(tiles.count), nominal, float(softcap or 0.0), _ptr(sinks), _ptr(self.status), _stream()))
+                    _ptr(tiles.count), nominal, float(softcap or 0.0), _ptr(sinks), keep_first, _ptr(self.status),
+                    _stream()))
             else:
                 _check(lib, lib.fg_attention_prefill_tma_bf16(*args, keep_first, _ptr(self.status), _stream()))
         elif tiles.n:

@@ -211,6 +211,37 @@ def test_float32_attention_on_asynchronous_copies(ops32, hd, heads, kv, window, 
     assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all()) and int(status) == 0
 
 
+@pytest.mark.parametrize("page", [8, 64, 128])
+@pytest.mark.parametrize("keep,window", [(1, 64), (4, 100), (70, 130), (200, 65)])
+def test_kept_positions_in_the_tensor_memory_kernel(ops16, keep, window, page):
+    """Prompt portions against a float64 reference; pages between the kept positions and the window are given back."""
+    from fastgen_b200.cache.manager import LayerMemory
+    heads, kv, hd = 8, 2, 64
+    lengths, cached = [200, 3, 64], [0, 390, 130]
+    ctx, q, pools, table = _attention_step(lengths, cached, page, heads, kv, hd, torch.bfloat16, keep + page)
+    keys = []
+    for i, (n, c) in enumerate(zip(lengths, cached)):
+        rows = [torch.cat([p[int(t)] for t in table[i]], dim=1)[:, : c + n].double() for p in pools]  # [kv, keys, hd]
+        keys.append(rows)
+        first, kept = max(0, c - window + 1) // page, -(-keep // page)
+        table[i, kept:first] = -1
+    memory = LayerMemory(k_pages=pools[0], v_pages=pools[1], block_table=table, page_size=page,
+                         tensor_maps=ops16.make_kv_tensor_maps(pools[0][None], pools[1][None], page), layer_index=0)
+    out = torch.empty_like(q)
+    ops16.attention(q, out, memory, ctx, heads, kv, hd, window, hd ** -0.5, keep_first=keep)
+    ops16.check_status()
+    for i, (n, c) in enumerate(zip(lengths, cached)):
+        a = ctx.host_seq_start[i]
+        qq = q[a : a + n].double().reshape(n, heads, hd)
+        k, v = (r.repeat_interleave(heads // kv, 0) for r in keys[i])
+        s = torch.einsum("thd,hkd->htk", qq, k) * hd ** -0.5
+        p, j = torch.arange(c, c + n, device=DEV)[:, None], torch.arange(c + n, device=DEV)[None, :]
+        seen = (j <= p) & ((p - j < window) | (j < keep))
+        ref = torch.einsum("htk,hkd->thd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), v)
+        # probabilities and outputs are rounded to bfloat16 (2^-8 each)
+        assert _relative(out[a : a + n], ref.reshape(n, heads * hd)) <= 2.0 ** -7
+
+
 # -- recurrences, chunk by chunk ---------------------------------------------------------------------------
 
 LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0)]
