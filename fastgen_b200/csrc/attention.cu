@@ -174,21 +174,6 @@ extern "C" int fg_attention_sigmoid_decode_bf16(const void* q, int q_stride, voi
 // ---------------------------------------------------------------------------------
 #include "attention_mma.cuh"
 
-extern "C" int fg_attention_prefill_rows() { return fg_mma::PREFILL_ROWS; }
-extern "C" int fg_attention_decode_split() { return fg_mma::DECODE_SPLIT; }
-
-// Floats of scratch that fg_attention_decode_bf16 needs.
-// The scratch opens with FIRST_PAIR_INTS ints (for every request the number of (request,
-// split) pairs before it, written by the persistent kernel for the merge of the splits), then
-// the partials.  max_pairs bounds the pairs of a step (0: n_seqs * max_splits).
-constexpr int FIRST_PAIR_INTS = 1024;
-
-extern "C" long long fg_attention_decode_scratch_floats(int n_seqs, int max_splits, int n_heads, long long max_pairs) {
-  const long long all = (long long)n_seqs * max_splits;
-  if (max_pairs <= 0 || max_pairs > all) max_pairs = all;
-  return FIRST_PAIR_INTS + max_pairs * n_heads * fg_mma::part_stride<FG_HEAD_DIM>();
-}
-
 [[maybe_unused]] static int sm_count() {
   static int n_sms = 0;
   if (n_sms == 0) {
@@ -198,6 +183,33 @@ extern "C" long long fg_attention_decode_scratch_floats(int n_seqs, int max_spli
   }
   return n_sms;
 }
+
+// The merge of the splits for a launch of n_heads x n_seqs blocks: half the threads a block where full blocks (four an
+// SM) would be more than one round.
+struct Combine {
+  decltype(&fg_mma::attention_combine_kernel<FG_HEAD_DIM, false>) kernel;
+  int threads;
+};
+[[maybe_unused]] static Combine combine_for(int window, int n_heads, int n_seqs) {
+  using namespace fg_mma;
+  constexpr int HALF = COMBINE_THREADS / 2;
+  if ((long long)n_heads * n_seqs > 4ll * sm_count())
+    return {window < 0 ? attention_combine_kernel<FG_HEAD_DIM, true, HALF> : attention_combine_kernel<FG_HEAD_DIM, false, HALF>, HALF};
+  return {window < 0 ? attention_combine_kernel<FG_HEAD_DIM, true> : attention_combine_kernel<FG_HEAD_DIM, false>, COMBINE_THREADS};
+}
+
+extern "C" int fg_attention_prefill_rows() { return fg_mma::PREFILL_ROWS; }
+extern "C" int fg_attention_decode_split() { return fg_mma::DECODE_SPLIT; }
+
+// Floats of scratch (the splits' partials) that fg_attention_decode_bf16 needs.  max_pairs bounds the (request,
+// split) pairs of a step (0: n_seqs * max_splits).
+
+extern "C" long long fg_attention_decode_scratch_floats(int n_seqs, int max_splits, int n_heads, long long max_pairs) {
+  const long long all = (long long)n_seqs * max_splits;
+  if (max_pairs <= 0 || max_pairs > all) max_pairs = all;
+  return max_pairs * n_heads * fg_mma::part_stride<FG_HEAD_DIM>();
+}
+
 
 // Whether single tokens of these shapes go to the persistent kernel (whose launch does not
 // depend on the requests' lengths and whose partials are numbered by pairs).
@@ -311,7 +323,6 @@ extern "C" int fg_attention_decode_bf16(const void* q, int q_stride, void* out, 
     attr_set = true;
   }
   const float scale_log2 = scale * 1.4426950408889634f;
-  scratch += FIRST_PAIR_INTS;
   dim3 grid(max_splits, n_kv_heads, n_seqs);
   kern<<<grid, THREADS, smem, stream>>>((const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k_pages,
                                         (const __nv_bfloat16*)v_pages, block_table, table_width, page_size,
@@ -321,9 +332,9 @@ extern "C" int fg_attention_decode_bf16(const void* q, int q_stride, void* out, 
                                         softcap > 0.f ? scale / softcap : 0.f);
   FG_CHECK_LAUNCH("fg_attention_decode_bf16");
   dim3 cgrid(n_heads, n_seqs);
-  (window < 0 ? attention_combine_kernel<FG_HEAD_DIM, true>
-              : attention_combine_kernel<FG_HEAD_DIM, false>)<<<cgrid, COMBINE_THREADS, 0, stream>>>(
-      scratch, (__nv_bfloat16*)out, out_stride, pos, seq_req, seq_tok, n_heads, window, max_splits, nullptr, status,
+  const Combine c = combine_for(window, n_heads, n_seqs);
+  c.kernel<<<cgrid, c.threads, 0, stream>>>(
+      scratch, (__nv_bfloat16*)out, out_stride, pos, seq_req, seq_tok, n_heads, window, max_splits, false, status,
       out_freqs, keep_first, sinks);
   FG_CHECK_LAUNCH("fg_attention_combine");
   return 0;
@@ -364,9 +375,7 @@ extern "C" int fg_attention_decode_tma_bf16(const void* q, int q_stride, void* o
   CUtensorMap km, vm;
   memcpy(&km, k_map, sizeof(CUtensorMap));
   memcpy(&vm, v_map, sizeof(CUtensorMap));
-  int* first_pair = reinterpret_cast<int*>(scratch);
-  float* partials = scratch + FIRST_PAIR_INTS;
-  const int* combine_pairs = nullptr;
+  bool numbered = false;
   if (fg_attention_decode_is_persistent(n_seqs, n_heads, n_kv_heads, page_size)) {
     // Blocks that stay on their SM (a producer warp ahead of four consumer warps) walk the
     // (request, split, kv head) items that exist; the launch does not depend on the lengths.
@@ -386,8 +395,8 @@ extern "C" int fg_attention_decode_tma_bf16(const void* q, int q_stride, void* o
     fg_launch_pdl(pkern, dim3(ps_blocks_per_sm<FG_HEAD_DIM>() * sm_count()), dim3(PS_THREADS), psmem, stream, km, vm,
                   layer, (const __nv_bfloat16*)q, q_stride, block_table, table_width, page_size, n_pages, pos,
                   seq_req, seq_tok, n_seqs, n_heads, n_kv_heads, group, window, scale * 1.4426950408889634f,
-                  partials, first_pair, max_pairs, max_splits, status);
-    combine_pairs = first_pair;
+                  scratch, max_pairs, max_splits, status);
+    numbered = true;
   } else {
     // one block per (request, kv head, split): larger groups of heads, very many requests
     FG_CHECK_ARG(scratch_floats >= fg_attention_decode_scratch_floats(n_seqs, max_splits, n_heads, 0),
@@ -403,13 +412,14 @@ extern "C" int fg_attention_decode_tma_bf16(const void* q, int q_stride, void* o
     dim3 grid(max_splits, n_kv_heads, n_seqs);
     fg_launch_pdl(kern, grid, dim3(THREADS), smem, stream, km, vm, layer, (const __nv_bfloat16*)q, q_stride,
                   block_table, table_width, page_size, n_pages, pos, seq_req, seq_tok, n_heads, group, window,
-                  scale * 1.4426950408889634f, partials, max_splits, status);
+                  scale * 1.4426950408889634f, scratch, max_splits, status);
   }
   FG_CHECK_LAUNCH("fg_attention_decode_tma_bf16");
   dim3 cgrid(n_heads, n_seqs);
-  fg_launch_pdl(window < 0 ? fg_mma::attention_combine_kernel<FG_HEAD_DIM, true> : fg_mma::attention_combine_kernel<FG_HEAD_DIM, false>, cgrid, dim3(fg_mma::COMBINE_THREADS), 0, stream,
-                (const float*)partials, (__nv_bfloat16*)out, out_stride, pos, seq_req, seq_tok, n_heads, window,
-                max_splits, combine_pairs, status, out_freqs, 0, sinks);
+  const Combine c = combine_for(window, n_heads, n_seqs);
+  fg_launch_pdl(c.kernel, cgrid, dim3(c.threads), 0, stream,
+                (const float*)scratch, (__nv_bfloat16*)out, out_stride, pos, seq_req, seq_tok, n_heads, window,
+                max_splits, numbered, status, out_freqs, 0, sinks);
   FG_CHECK_LAUNCH("fg_attention_combine");
   return 0;
 }

@@ -623,14 +623,20 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
 // s_lo + w, s_lo + w + W, ... (a lane holds two neighbouring dimensions of every 64), then the
 // warps' sums are added in ascending warp order.  The order of the additions depends on the
 // request's own splits only, never on the batch.
-constexpr int COMBINE_THREADS = 256;
+//
+// The launch is a chain of latencies (its partials are a few MB), so a warp's first split is on its way while the
+// overall maximum is found and the others come eight at a time; a launch of more blocks than are resident at once
+// (four an SM) runs with half the threads a block, each warp in the place of two: the same sums.
+// (Two requests of 30,000 keys, 32 heads of 64: 11 -> 8 us behind the attention; 64 requests of 24 heads, 8 -> 5.)
+constexpr int COMBINE_WARPS = 8;
+constexpr int COMBINE_THREADS = COMBINE_WARPS * 32;
 
-template <int HD, bool CHUNKS>
-__global__ void __launch_bounds__(COMBINE_THREADS)
+template <int HD, bool CHUNKS, int BLOCK = COMBINE_THREADS>
+__global__ void __launch_bounds__(BLOCK)
 attention_combine_kernel(const float* scratch, __nv_bfloat16* __restrict__ out, int out_stride,
                          const int* __restrict__ pos, const int* __restrict__ seq_req,
                          const int* __restrict__ seq_tok, int n_heads, int window, int max_splits,
-                         const int* first_pair, int* status, const float* __restrict__ out_freqs,
+                         bool numbered, int* status, const float* __restrict__ out_freqs,
                          int keep_first, const float* __restrict__ sinks) {
   // sinks: null, or float32 per query head: exp(sink_h) joins the denominator once (it has no key and
   // no value, so no split holds it: it is added here, where the splits meet)
@@ -639,10 +645,11 @@ attention_combine_kernel(const float* scratch, __nv_bfloat16* __restrict__ out, 
   // out_freqs: null, or HD/2 frequencies by which the output's adjacent pairs are turned
   // (angle position * frequency) before they are stored: a model that caches values turned by
   // their positions turns the sum back here, with the negated table.
-  // first_pair (written by the kernel before, so no __restrict__): null, or for every
-  // request the number of (request, split) pairs before it; the partials are then
-  // numbered [pair][head] (only the splits that exist), else [request][head][split].
-  constexpr int WARPS = COMBINE_THREADS / 32;
+  // numbered: the partials are numbered [pair][head] by the (request, split) pairs that exist, request after
+  // request (each block counts those before its own from the positions), else [request][head][split].
+  constexpr int WARPS = COMBINE_WARPS;
+  constexpr int EACH = COMBINE_THREADS / BLOCK;  // places a warp takes
+  constexpr int FLIGHT = EACH == 1 ? 8 : 2;      // splits whose loads a warp has in flight together
   constexpr int NV = (HD + 63) / 64;  // float2 pieces a lane holds
   constexpr int PS = part_stride<HD>();
   static_assert(PS % 2 == 0, "partials are read as float2");
@@ -651,12 +658,21 @@ attention_combine_kernel(const float* scratch, __nv_bfloat16* __restrict__ out, 
   __shared__ float ll_s[WARPS];
   pdl_trigger();
   // the lists of sequences and positions are inputs of the step: read while the kernel before
-  // this one finishes; its partials (and first_pair) are touched after the wait
+  // this one finishes; its partials are touched after the wait
   const int seq = blockIdx.y, head = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tok = seq_tok[seq];
   const int request = seq_req[seq];
   const int p = request < 0 ? 0 : pos[tok];
+  int first_pair = 0;
+  if (numbered) {
+    for (int sq = lane; sq < seq; sq += 32) {
+      if (seq_req[sq] < 0) continue;
+      const int at = pos[seq_tok[sq]];
+      first_pair += min(at / DECODE_SPLIT, max_splits - 1) - first_visible<CHUNKS>(at, window) / DECODE_SPLIT + 1;
+    }
+    first_pair = __reduce_add_sync(0xffffffffu, first_pair);
+  }
   pdl_wait();
   __nv_bfloat16* dst = out + (size_t)tok * out_stride + head * HD;
   // a padding lane has no request: nothing is written for it (its token index may be any row,
@@ -670,53 +686,99 @@ attention_combine_kernel(const float* scratch, __nv_bfloat16* __restrict__ out, 
     s_hi = max_splits - 1;
   }
   // base[s * step]: the partial of split s
-  const size_t step = first_pair != nullptr ? (size_t)n_heads * PS : PS;
-  const float* base = first_pair != nullptr
-                          ? scratch + ((size_t)(first_pair[seq] - s_lo) * n_heads + head) * PS
+  const size_t step = numbered ? (size_t)n_heads * PS : PS;
+  const float* base = numbered
+                          ? scratch + ((long long)(first_pair - s_lo) * n_heads + head) * PS
                           : scratch + ((size_t)seq * n_heads + head) * max_splits * PS;
-  const int n_keep = (window > 0 && keep_first > 0 && first_pair == nullptr)
+  const int n_keep = (window > 0 && keep_first > 0 && !numbered)
                          ? min(s_lo, (keep_first + DECODE_SPLIT - 1) / DECODE_SPLIT)
                          : 0;
   const int n_parts = n_keep + (s_hi - s_lo + 1);
   auto split_of = [&](int i) { return i < n_keep ? i : s_lo + (i - n_keep); };
+  // the first split of each of this warp's places
+  float first_m[EACH], first_l[EACH];
+  float2 first_o[EACH][NV];
+#pragma unroll
+  for (int e = 0; e < EACH; ++e) {
+    const int at = warp + e * (BLOCK / 32);
+    first_m[e] = -INFINITY;
+    first_l[e] = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) first_o[e][i] = make_float2(0.f, 0.f);
+    if (at < n_parts) {
+      const float* part = base + (size_t)split_of(at) * step;
+      first_m[e] = part[HD];
+      first_l[e] = part[HD + 1];
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        if (i * 64 + lane * 2 < HD) first_o[e][i] = *reinterpret_cast<const float2*>(part + i * 64 + lane * 2);
+    }
+  }
   // the overall maximum
   float mm = -INFINITY;
-  for (int i = tid; i < n_parts; i += COMBINE_THREADS) mm = fmaxf(mm, base[(size_t)split_of(i) * step + HD]);
+  for (int i = tid; i < n_parts; i += BLOCK) mm = fmaxf(mm, base[(size_t)split_of(i) * step + HD]);
   mm = warp_max(mm);
   if (lane == 0) red[warp] = mm;
   __syncthreads();
   mm = red[0];
 #pragma unroll
-  for (int w = 1; w < WARPS; ++w) mm = fmaxf(mm, red[w]);
+  for (int w = 1; w < BLOCK / 32; ++w) mm = fmaxf(mm, red[w]);
   const float sink2 = sinks != nullptr ? sinks[head] * 1.4426950408889634f : -INFINITY;  // base 2, as the partials
   mm = fmaxf(mm, sink2);
-  // this warp's splits
-  float2 acc[NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) acc[i] = make_float2(0.f, 0.f);
-  float ll = 0.f;
-#pragma unroll 4
-  for (int i = warp; i < n_parts; i += WARPS) {
-    const float* part = base + (size_t)split_of(i) * step;
-    const float ms = part[HD];
-    const float wgt = (ms == -INFINITY) ? 0.f : exp2f(ms - mm);
-    ll += wgt * part[HD + 1];
+  for (int e = 0; e < EACH; ++e) {
+    const int at = warp + e * (BLOCK / 32);
+    float2 acc[NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int d = i * 64 + lane * 2;
-      if (d < HD) {
-        const float2 v = *reinterpret_cast<const float2*>(part + d);
-        acc[i].x += wgt * v.x;
-        acc[i].y += wgt * v.y;
+    for (int i = 0; i < NV; ++i) acc[i] = make_float2(0.f, 0.f);
+    float ll = 0.f;
+    if (at < n_parts) {
+      const float wgt = (first_m[e] == -INFINITY) ? 0.f : exp2f(first_m[e] - mm);
+      ll += wgt * first_l[e];
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        acc[i].x += wgt * first_o[e][i].x;
+        acc[i].y += wgt * first_o[e][i].y;
       }
     }
-  }
+    for (int i0 = at + WARPS; i0 < n_parts; i0 += FLIGHT * WARPS) {
+      float ms[FLIGHT], ls[FLIGHT];
+      float2 vs[FLIGHT][NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    acc_s[warp][i * 64 + lane * 2] = acc[i].x;
-    acc_s[warp][i * 64 + lane * 2 + 1] = acc[i].y;
+      for (int u = 0; u < FLIGHT; ++u) {
+        const int i = i0 + u * WARPS;
+        ms[u] = -INFINITY;
+        ls[u] = 0.f;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) vs[u][k] = make_float2(0.f, 0.f);
+        if (i < n_parts) {
+          const float* part = base + (size_t)split_of(i) * step;
+          ms[u] = part[HD];
+          ls[u] = part[HD + 1];
+#pragma unroll
+          for (int k = 0; k < NV; ++k)
+            if (k * 64 + lane * 2 < HD) vs[u][k] = *reinterpret_cast<const float2*>(part + k * 64 + lane * 2);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < FLIGHT; ++u) {
+        if (i0 + u * WARPS >= n_parts) break;
+        const float wgt = (ms[u] == -INFINITY) ? 0.f : exp2f(ms[u] - mm);
+        ll += wgt * ls[u];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+          acc[k].x += wgt * vs[u][k].x;
+          acc[k].y += wgt * vs[u][k].y;
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      acc_s[at][i * 64 + lane * 2] = acc[i].x;
+      acc_s[at][i * 64 + lane * 2 + 1] = acc[i].y;
+    }
+    if (lane == 0) ll_s[at] = ll;
   }
-  if (lane == 0) ll_s[warp] = ll;
   __syncthreads();
   float total = 0.f;
 #pragma unroll
@@ -724,7 +786,7 @@ attention_combine_kernel(const float* scratch, __nv_bfloat16* __restrict__ out, 
   if (sinks != nullptr) total += exp2f(sink2 - mm);
   const float inv = total > 0.f ? 1.f / total : 0.f;
   if (out_freqs != nullptr) {
-    for (int j = tid; j < HD / 2; j += COMBINE_THREADS) {
+    for (int j = tid; j < HD / 2; j += BLOCK) {
       float re = 0.f, im = 0.f;
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) {
@@ -739,7 +801,7 @@ attention_combine_kernel(const float* scratch, __nv_bfloat16* __restrict__ out, 
     }
     return;
   }
-  for (int d = tid; d < HD; d += COMBINE_THREADS) {
+  for (int d = tid; d < HD; d += BLOCK) {
     float a = 0.f;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) a += acc_s[w][d];

@@ -310,7 +310,7 @@ attention_decode_persistent_kernel(const __grid_constant__ CUtensorMap k_map,
                                    int n_pages, const int* __restrict__ pos, const int* __restrict__ seq_req,
                                    const int* __restrict__ seq_tok, int n_seqs, int n_heads, int n_kv_heads,
                                    int group, int window, float scale_log2, float* __restrict__ scratch,
-                                   int* __restrict__ first_pair_out, long long max_pairs, int max_splits,
+                                   long long max_pairs, int max_splits,
                                    int* status) {
   static_assert(HD % 64 == 0, "tiled loads take 64-element halves");
   constexpr int HALVES = HD / 64;
@@ -376,10 +376,7 @@ attention_decode_persistent_kernel(const __grid_constant__ CUtensorMap k_map,
 
   const int box_rows = min(page_size, SPLIT);
   const int n_boxes = SPLIT / box_rows;
-  // the (request, split) pairs also number the partials, [pair][head]: what the merge of the
-  // splits needs to find them goes to global memory
-  if (blockIdx.x == 0)
-    for (int sq = tid; sq <= n_seqs; sq += PS_THREADS) first_pair_out[sq] = s_cum[sq];
+  // the (request, split) pairs also number the partials, [pair][head] (the merge counts them likewise)
   int n_pairs = s_cum[n_seqs];
   if (n_pairs > max_pairs) {
     // the scratch was sized for fewer: report instead of writing past it
