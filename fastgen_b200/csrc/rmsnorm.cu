@@ -96,16 +96,23 @@ rmsnorm_vec_kernel(TH* h, const TD* delta, const void* __restrict__ w, int w_dty
   const size_t obase = (size_t)blockIdx.x * dim;
   const bool store_h = delta != nullptr && rows == nullptr;
   pdl_wait();
-  float4 v[ITEMS];
+  // all of the row's loads before the first store: a store to h keeps the loads behind it waiting (the compiler cannot
+  // know that they are of other columns), which made a row of 4,096 four round trips in a row
+  // (64 rows of 3,072 behind a library product: 4.2 -> 3.0 us)
+  float4 v[ITEMS], e_all[ITEMS];
+#pragma unroll
+  for (int it = 0; it < ITEMS; ++it) {
+    const int d = (it * VEC_THREADS + threadIdx.x) * 4;
+    v[it] = d < dim ? load4<TH>(h + base + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    e_all[it] = delta != nullptr && d < dim ? load4<TD>(delta + base + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float ss = 0.f;
 #pragma unroll
   for (int it = 0; it < ITEMS; ++it) {
     const int d = (it * VEC_THREADS + threadIdx.x) * 4;
-    v[it] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (d < dim) {
-      v[it] = load4<TH>(h + base + d);
       if (delta != nullptr) {
-        const float4 e = load4<TD>(delta + base + d);
+        const float4 e = e_all[it];
         v[it].x += e.x; v[it].y += e.y; v[it].z += e.z; v[it].w += e.w;
         // the stored sum is what is normed
         v[it].x = to_f32<TH>(from_f32<TH>(v[it].x)); v[it].y = to_f32<TH>(from_f32<TH>(v[it].y));
