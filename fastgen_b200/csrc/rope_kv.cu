@@ -127,18 +127,22 @@ rope_kv_kernel(T* __restrict__ q, int q_stride, const T* __restrict__ k, int k_s
 
 // bfloat16 with 16-byte accesses: a thread owns four adjacent pairs (8 elements) of one
 // token, computes their four angles once and walks the heads, several heads in flight.
-// Needs head_dim % 8 == 0 and 16-byte aligned rows.
+// Needs head_dim % 8 == 0 and 16-byte aligned rows.  Angles and pages are inputs of the step: they are worked out before the
+// wait for the kernel before this one, and the single-token attention behind it may start on the keys that
+// are cached already while this one runs (64 requests, 24 / 8 heads of 128, from the
+// projection to the end of the attention: 47.7 -> 46.2 us a layer).
 constexpr int ROPE_UNROLL = 4;
 
 __global__ void __launch_bounds__(ROPE_THREADS)
-rope_kv_bf16x8_kernel(__nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k, int k_stride,
-                      const __nv_bfloat16* __restrict__ v, int v_stride, const int* __restrict__ pos,
+rope_kv_bf16x8_kernel(__nv_bfloat16* q, int q_stride, const __nv_bfloat16* k, int k_stride,
+                      const __nv_bfloat16* v, int v_stride, const int* __restrict__ pos,
                       const int* __restrict__ req, const float* __restrict__ freqs,
                       const float* __restrict__ v_freqs, __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages,
                       const int* __restrict__ block_table, int table_width, int page_size, int n_pages,
                       int n_heads, int n_kv_heads, int head_dim, int* status, int heads_per_block,
                       const float* rstd, const float* __restrict__ qn_w, const float* __restrict__ kn_w,
                       int rstd_heads, float magnitude, int rot_pairs) {
+  pdl_trigger();
   const int t = blockIdx.x;
   const int r = req[t];
   if (r < 0) return;
@@ -174,6 +178,7 @@ rope_kv_bf16x8_kernel(__nv_bfloat16* __restrict__ q, int q_stride, const __nv_bf
     }
     slot = (size_t)page * n_kv_heads * page_size + (p - logical * page_size);
   }
+  pdl_wait();
   const float rq = rstd && !rstd_heads ? rstd[2 * t] : 1.f, rk = rstd && !rstd_heads ? rstd[2 * t + 1] : 1.f;
   // nw: the eight norm weights of this piece of the head (null: ones), r: the factor of the token
   // (or of this head of the token)
@@ -210,7 +215,7 @@ rope_kv_bf16x8_kernel(__nv_bfloat16* __restrict__ q, int q_stride, const __nv_bf
       if (h < n_heads) src = q + (size_t)t * q_stride + h * head_dim;
       else if (h < n_heads + n_kv) src = k + (size_t)t * k_stride + (h - n_heads) * head_dim;
       else src = v + (size_t)t * v_stride + (h - n_heads - n_kv) * head_dim;
-      raw[u] = *reinterpret_cast<const uint4*>(src + piece * 8);
+      raw[u] = ld_global_16(src + piece * 8);
     }
 #pragma unroll
     for (int u = 0; u < ROPE_UNROLL; ++u) {
@@ -414,7 +419,7 @@ extern "C" int fg_rope_kv_write(void* q, int q_stride, const void* k, int k_stri
   const auto ok16 = [&](const void* p, int stride) { return p == nullptr || (((uintptr_t)p & 15) == 0 && stride % 8 == 0); };
   if (dtype == FG_BF16 && head_dim % 8 == 0 && head_dim / 8 <= ROPE_THREADS && ok16(q, q_stride) && ok16(k, k_stride) &&
       ok16(v, v_stride) && ok16(k_pages, 0) && ok16(v_pages, 0)) {
-    rope_kv_bf16x8_kernel<<<grid, threads, 0, stream>>>(
+    fg_launch_pdl(rope_kv_bf16x8_kernel, grid, dim3(threads), 0, stream,
         (__nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)k, k_stride, (const __nv_bfloat16*)v, v_stride, pos, req,
         freqs, v_freqs, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, block_table, table_width, page_size,
         n_pages, n_heads, n_kv_heads, head_dim, status, ipt, rstd, qn_w, kn_w, rstd_heads, magnitude, rot_pairs);
