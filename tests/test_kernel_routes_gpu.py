@@ -323,3 +323,21 @@ def test_delta_rule_with_one_decay_a_head(ops16, lengths, pad, d, dv):
         assert _relative(state[slot, : heads * d * dv], S.reshape(-1)) <= bound
     for slot in {0, 1, 2, 3} - set(slots):
         assert torch.equal(state[slot], before[slot])
+
+
+# -- embedding --------------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim,copies", [(8, 1), (2040, 2), (2048, 1), (4104, 3), (8192, 1), (100, 2)])
+def test_embedding_rows(ops32, dtype, dim, copies):
+    from fastgen_b200.csrc.ops import _check, _code, _ptr, _stream
+    g = torch.Generator().manual_seed(dim)
+    table = _randn(g, 50, dim).to(dtype)
+    tokens = torch.tensor([49, 0, 7, 50, -1], dtype=torch.int32, device=DEV)  # the last two are no tokens
+    out = torch.full((5, copies, dim), float("nan"), device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    _check(ops32.lib, ops32.lib.fg_embedding(_ptr(table), _code(dtype), _ptr(tokens), _ptr(out), _code(torch.float32), 5, dim, 50,
+                                             0.7, copies, _ptr(status), _stream()))
+    want = torch.zeros(5, dim, device=DEV)
+    want[:3] = table[tokens[:3].long()].float() * torch.tensor(0.7, device=DEV)
+    assert torch.equal(out, want[:, None].expand(5, copies, dim)) and int(status) == 2  # STATUS_BAD_TOKEN
