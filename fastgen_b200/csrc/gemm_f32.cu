@@ -78,7 +78,7 @@ gemm_f32_nt_kernel(const TA* __restrict__ A, int lda, const float* __restrict__ 
 // this one is multiplied) into shared memory with k as the slow index: a thread's operands of one k are
 // four 16-byte reads for 64 multiply-adds, which is what the shared memory can deliver beside them (4 x 4
 // outputs a thread, as the last kernel of this file, need twice as much).  Two multiply-adds an instruction
-// (fma.rn.f32x2, each rounded as fmaf rounds).  777 x 128,256 x 2,048: 16.7 -> 8.6 ms (47 TFLOP/s).
+// (fma.rn.f32x2, each rounded as fmaf rounds).  777 x 128,256 x 2,048: 16.7 -> 8.1 ms (50 TFLOP/s).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
   unsigned long long r;
@@ -168,6 +168,8 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
 #pragma unroll
     for (int kk = 0; kk < KT; ++kk) {
       const int f = kk & 1;
+      // the next tile goes to the other buffer (free since the last barrier) while this one is multiplied
+      if (kk == KT * 3 / 4 && more) store(buf ^ 1);
       if (kk + 1 < KT) fetch(kk + 1, f ^ 1);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -180,7 +182,6 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
         fma2(acc[i][3], xx, b[f][1].y);
       }
     }
-    if (more) store(buf ^ 1);
     __syncthreads();
     buf ^= 1;
   }
