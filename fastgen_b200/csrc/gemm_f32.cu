@@ -115,6 +115,8 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 
+  // (of a tile's upper eight k, runs of eight rows change places with their neighbours: a warp's transposing stores are
+  // of four k and eight rows, and fall on 32 banks that way)
   float4 ra[S::LA], rw[S::LW];
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   auto load = [&](int k0) {
@@ -133,18 +135,18 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
 #pragma unroll
     for (int u = 0; u < S::LA; ++u) {
       const int i = tid + u * S::THREADS, row = i / (KT / 4), k = i % (KT / 4) * 4;
-      as[buf][k][row] = ra[u].x;
-      as[buf][k + 1][row] = ra[u].y;
-      as[buf][k + 2][row] = ra[u].z;
-      as[buf][k + 3][row] = ra[u].w;
+      as[buf][k][row ^ (k & 8)] = ra[u].x;
+      as[buf][k + 1][row ^ (k & 8)] = ra[u].y;
+      as[buf][k + 2][row ^ (k & 8)] = ra[u].z;
+      as[buf][k + 3][row ^ (k & 8)] = ra[u].w;
     }
 #pragma unroll
     for (int u = 0; u < S::LW; ++u) {
       const int i = tid + u * S::THREADS, row = i / (KT / 4), k = i % (KT / 4) * 4;
-      ws[buf][k][row] = rw[u].x;
-      ws[buf][k + 1][row] = rw[u].y;
-      ws[buf][k + 2][row] = rw[u].z;
-      ws[buf][k + 3][row] = rw[u].w;
+      ws[buf][k][row ^ (k & 8)] = rw[u].x;
+      ws[buf][k + 1][row ^ (k & 8)] = rw[u].y;
+      ws[buf][k + 2][row ^ (k & 8)] = rw[u].z;
+      ws[buf][k + 3][row ^ (k & 8)] = rw[u].w;
     }
   };
 
@@ -160,8 +162,8 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
     auto fetch = [&](int kk, int f) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        a[f][i] = *reinterpret_cast<const float4*>(&as[buf][kk][wm + 16 * i]);
-        b[f][i] = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][wn + 32 * i]);
+        a[f][i] = *reinterpret_cast<const float4*>(&as[buf][kk][(wm + 16 * i) ^ (kk & 8)]);
+        b[f][i] = *reinterpret_cast<const ulonglong2*>(&ws[buf][kk][(wn + 32 * i) ^ (kk & 8)]);
       }
     };
     fetch(0, 0);
