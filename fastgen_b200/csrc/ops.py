@@ -833,14 +833,17 @@ class Ops:
         out = torch.empty((t, heads * dv), dtype=torch.float32, device=qkv.device)
         # the tokens as the recurrence reads them (unit vectors, decays, step sizes; padded rows)
         # (and, where sequences of many tokens go chunk by chunk, what the chunks are alone)
-        scratch = torch.empty(lib.fg_delta_scan_scratch_floats(t, ctx.n_seqs, heads, kv_heads, d, dv, _code(a.dtype),
-                                                               int(head_decay)), dtype=torch.float32, device=qkv.device)
+        def room(dtype):
+            return lib.fg_delta_scan_scratch_floats(t, ctx.n_seqs, heads, kv_heads, d, dv, dtype, int(head_decay))
+
+        scratch = torch.empty(room(_code(a.dtype)), dtype=torch.float32, device=qkv.device)
         _check(lib, lib.fg_delta_scan(
             _ptr(qkv), qkv.stride(0), _ptr(a), a.stride(0), _ptr(b), b.stride(0), _code(a.dtype), _ptr(dt_bias),
             _ptr(a_log), _ptr(out), out.stride(0), _ptr(state), state.stride(0), _ptr(ctx.seq_slot),
             _ptr(ctx.seq_start), ctx.n_seqs, _ptr(ctx.req), t, _ptr(scratch), heads, kv_heads, d, dv,
             int(head_decay), _stream()))
-        Ops.launches += 1  # the kernel that prepares the tokens
+        # the kernel that prepares the tokens, and the chunks' two (float32 never has those)
+        Ops.launches += 1 + 2 * int(scratch.numel() > room(FG_F32))
         return out
 
     def head_norm_gate(self, o, z, weight, heads: int, dv: int, eps: float, ctx, act: str = "sigmoid") -> torch.Tensor:
