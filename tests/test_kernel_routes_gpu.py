@@ -242,6 +242,37 @@ def test_kept_positions_in_the_tensor_memory_kernel(ops16, keep, window, page):
         assert _relative(out[a : a + n], ref.reshape(n, heads * hd)) <= 2.0 ** -7
 
 
+@pytest.mark.parametrize("hd,length,cached,window,keep", [(64, 700, 0, 300, 4), (64, 90, 1500, 1024, 70), (128, 333, 200, 128, 64)])
+@pytest.mark.parametrize("deviation", [0.8, 3.0])
+def test_kept_positions_lose_no_precision(ops16, hd, length, cached, window, keep, deviation):
+    """Against float64, and no further from it than the mma.sync kernel on the same inputs (with sharp scores
+    a weight of almost one that is rounded on its own counts)."""
+    from fastgen_b200.cache.manager import LayerMemory
+    from fastgen_b200.csrc.ops import Ops
+    heads, kv, page = 16, 4, 64
+    other = Ops(torch.bfloat16, DEV)
+    other.use_tcgen05 = False
+    ctx, q, pools, table = _attention_step([length], [cached], page, heads, kv, hd, torch.bfloat16, hd + keep)
+    q = (q.float() * deviation).to(torch.bfloat16)
+    memory = LayerMemory(k_pages=pools[0], v_pages=pools[1], block_table=table, page_size=page,
+                         tensor_maps=ops16.make_kv_tensor_maps(pools[0][None], pools[1][None], page), layer_index=0)
+    k, v = (torch.cat([p[int(t)] for t in table[0]], dim=1)[:, : cached + length].double().repeat_interleave(heads // kv, 0)
+            for p in pools)
+    s = torch.einsum("thd,hkd->htk", q.double().reshape(length, heads, hd), k) * hd ** -0.5
+    p, j = torch.arange(cached, cached + length, device=DEV)[:, None], torch.arange(cached + length, device=DEV)[None, :]
+    seen = (j <= p) & ((p - j < window) | (j < keep))
+    ref = torch.einsum("htk,hkd->thd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), v).reshape(length, -1)
+    errors = []
+    for ops in (ops16, other):
+        out = torch.empty_like(q)
+        ops.attention(q, out, memory, ctx, heads, kv, hd, window, hd ** -0.5, keep_first=keep)
+        ops.check_status()
+        errors.append(_relative(out, ref))
+    # Both round the same weights and outputs: their errors are means over the same 90,000 or more values, equal to
+    # 1 % (a tile's maximum is found at other places of the walk).
+    assert errors[0] <= 1.01 * errors[1]
+
+
 # -- recurrences, chunk by chunk ---------------------------------------------------------------------------
 
 LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0)]
