@@ -478,13 +478,13 @@ ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* _
 //     Y = e (C S0) + M X + D_skip X,  M[i][j] = (C_i . B_j) D[i][j] dt_j  (j <= i)
 //     S <- e_32 S0 + B^T (w X)
 //
-// 2,048 tokens of 64 heads, 128 x 64 states: 420 -> 187 us and 13 of preparing (the multiply-adds alone take 75; what
+// 2,048 tokens of 64 heads, 128 x 64 states: 420 -> 197 us and 15 of preparing (the multiply-adds alone take 75; what
 // bounds the walk is shared memory: a 16-byte read a lane takes its 4 cycles whoever shares the address, and 4 x 4
 // numbers a thread want two such reads for 16 multiply-adds).
 //
 // ssm_chunk_prepare_kernel forms M, e and w for all chunks side by side (a block a (chunk, group): C B^T once for the
 // group's heads); ssm_chunk_kernel walks the chunks of one (sequence, head, 32 columns), a state of 4 x 4 numbers a
-// thread.  All float32 multiply-adds; the sums have another order than the token kernel's, so the float32 mode,
+// thread.  float32 multiply-adds (the decays and C B^T in 64 bits); the sums have another order than the token kernel's, so the float32 mode,
 // whose results do not depend on how a prompt is cut, keeps that one.
 constexpr int SC_TOKENS = 32;   // tokens a chunk
 constexpr int SC_COLS = 32;     // columns of P a block of the walk
@@ -493,6 +493,14 @@ constexpr int SC_STAGES = 2;
 // Fewest tokens of a sequence that takes this way (prepared and walked): where the two meet.  One sequence of 63
 // tokens 15.9 us above, of 64 here 16.7, of 96 19.9; four of 63 48 us, of 64 42.
 constexpr int SC_MIN = 64;
+// Products of the state that are summed by themselves before they join a token's sum: the token kernel's sums over N are
+// trees (a few products a lane, then exchanges), and one chain over N is twice as far from 64 bits as those
+// (1.9e-7 against 1.05e-7 at N = 128; with runs of 16 and C B^T summed in 64 bits 1.0e-7, for 5 % of the walk's time).
+constexpr int SC_RUN = 16;
+template <int V>
+struct Whole {
+  static constexpr int value = V;
+};
 constexpr int SC_REC = SC_TOKENS * SC_TOKENS + 2 * SC_TOKENS;  // floats of a (chunk, head): M, e, w
 
 __device__ __forceinline__ bool sc_takes(const int* seq_slot, const int* seq_start, int b, int& n) {
@@ -513,7 +521,7 @@ ssm_chunk_prepare_kernel(const float* __restrict__ xbc, long xbc_stride, const T
                          int groups, int P) {
   __shared__ __align__(16) float bs[SC_TOKENS][N + 4];
   __shared__ __align__(16) float cs[SC_TOKENS][N + 4];
-  __shared__ float gram[SC_TOKENS][SC_TOKENS + 1];
+  __shared__ double gram[SC_TOKENS][SC_TOKENS + 1];
   __shared__ float decs[SC_THREADS / 32][SC_TOKENS];
   const int g = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int c = blockIdx.x, b = 0, n = 0;
@@ -539,24 +547,37 @@ ssm_chunk_prepare_kernel(const float* __restrict__ xbc, long xbc_stride, const T
   __syncthreads();
   {
     const int ib = tid >> 4, jb = tid & 15;
-    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll 4
-    for (int w = 0; w < N; w += 4) {
-      float4 cv[2], bv[2];
+    // short chains: a sum over N in stretches of 16 that are four chains each, added up in 64 bits (see SC_RUN)
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 2
+    for (int w0 = 0; w0 < N; w0 += 16) {
+      float4 run[2][2];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        cv[e] = *reinterpret_cast<const float4*>(&cs[ib + 16 * e][w]);
-        bv[e] = *reinterpret_cast<const float4*>(&bs[jb + 16 * e][w]);
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int f = 0; f < 2; ++f) run[e][f] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = w0; w < w0 + 16; w += 4) {
+        float4 cv[2], bv[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          cv[e] = *reinterpret_cast<const float4*>(&cs[ib + 16 * e][w]);
+          bv[e] = *reinterpret_cast<const float4*>(&bs[jb + 16 * e][w]);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int f = 0; f < 2; ++f) {
+            run[e][f].x = fmaf(cv[e].x, bv[f].x, run[e][f].x);
+            run[e][f].y = fmaf(cv[e].y, bv[f].y, run[e][f].y);
+            run[e][f].z = fmaf(cv[e].z, bv[f].z, run[e][f].z);
+            run[e][f].w = fmaf(cv[e].w, bv[f].w, run[e][f].w);
+          }
       }
 #pragma unroll
       for (int e = 0; e < 2; ++e)
 #pragma unroll
-        for (int f = 0; f < 2; ++f) {
-          acc[e][f] = fmaf(cv[e].x, bv[f].x, acc[e][f]);
-          acc[e][f] = fmaf(cv[e].y, bv[f].y, acc[e][f]);
-          acc[e][f] = fmaf(cv[e].z, bv[f].z, acc[e][f]);
-          acc[e][f] = fmaf(cv[e].w, bv[f].w, acc[e][f]);
-        }
+        for (int f = 0; f < 2; ++f) acc[e][f] += (run[e][f].x + run[e][f].y) + (run[e][f].z + run[e][f].w);
     }
 #pragma unroll
     for (int e = 0; e < 2; ++e)
@@ -576,15 +597,16 @@ ssm_chunk_prepare_kernel(const float* __restrict__ xbc, long xbc_stride, const T
     decs[warp][lane] = dec;
     __syncwarp();
     float* rec = chunks + ((size_t)blockIdx.x * heads + h) * SC_REC;
-    float d = 1.f, e = 1.f;
+    // M is rounded once, from 64 bits: its error, unlike that of a state's numbers, is the same for all of P
+    double d = 1.0, e = 1.0;
     for (int i = 0; i < SC_TOKENS; ++i) {
-      const float ai = decs[warp][i];
+      const double ai = decs[warp][i];
       e *= ai;
       if (i > lane) d *= ai;
-      rec[i * SC_TOKENS + lane] = i >= lane ? gram[i][lane] * d * dt : 0.f;
-      if (lane == 0) rec[SC_TOKENS * SC_TOKENS + i] = e;
+      rec[i * SC_TOKENS + lane] = i >= lane ? (float)(gram[i][lane] * (d * dt)) : 0.f;
+      if (lane == 0) rec[SC_TOKENS * SC_TOKENS + i] = (float)e;
     }
-    rec[SC_TOKENS * SC_TOKENS + SC_TOKENS + lane] = d * dt;
+    rec[SC_TOKENS * SC_TOKENS + SC_TOKENS + lane] = (float)(d * dt);
     __syncwarp();
   }
 }
@@ -675,36 +697,49 @@ ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, const float* __
     for (int e = 0; e < 4; ++e)
 #pragma unroll
       for (int f = 0; f < 4; ++f) acc[e][f] = 0.f;
-    auto products = [&](const float* left, int left_stride, const float* right, int from, int count) {
+    auto products = [&](const float* left, int left_stride, const float* right, int from, auto count, auto run_length) {
+      constexpr int COUNT = decltype(count)::value, RUN = decltype(run_length)::value;
+#pragma unroll 1
+      for (int k0 = from; k0 < from + COUNT; k0 += RUN) {
+        float run[4][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int f = 0; f < 4; ++f) run[e][f] = 0.f;
 #pragma unroll 2
-      for (int k = from; k < from + count; k += 4) {
-        float4 a[4], v[4];
+        for (int k = k0; k < k0 + RUN; k += 4) {
+          float4 a[4], v[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          a[e] = *reinterpret_cast<const float4*>(left + (ib + 8 * e) * left_stride + k);
-          v[e] = *reinterpret_cast<const float4*>(right + (k + e) * L::SP + 4 * pb);
-        }
+          for (int e = 0; e < 4; ++e) {
+            a[e] = *reinterpret_cast<const float4*>(left + (ib + 8 * e) * left_stride + k);
+            v[e] = *reinterpret_cast<const float4*>(right + (k + e) * L::SP + 4 * pb);
+          }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float ae[4] = {a[e].x, a[e].y, a[e].z, a[e].w};
+          for (int e = 0; e < 4; ++e) {
+            const float ae[4] = {a[e].x, a[e].y, a[e].z, a[e].w};
 #pragma unroll
-          for (int f = 0; f < 4; ++f) {
-            acc[e][0] = fmaf(ae[f], v[f].x, acc[e][0]);
-            acc[e][1] = fmaf(ae[f], v[f].y, acc[e][1]);
-            acc[e][2] = fmaf(ae[f], v[f].z, acc[e][2]);
-            acc[e][3] = fmaf(ae[f], v[f].w, acc[e][3]);
+            for (int f = 0; f < 4; ++f) {
+              run[e][0] = fmaf(ae[f], v[f].x, run[e][0]);
+              run[e][1] = fmaf(ae[f], v[f].y, run[e][1]);
+              run[e][2] = fmaf(ae[f], v[f].z, run[e][2]);
+              run[e][3] = fmaf(ae[f], v[f].w, run[e][3]);
+            }
           }
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int f = 0; f < 4; ++f) acc[e][f] += run[e][f];
       }
     };
-    products(buf + L::C, L::SCN, s_s, q * (N / 4), N / 4);
+    products(buf + L::C, L::SCN, s_s, q * (N / 4), Whole<N / 4>(), Whole<SC_RUN>());
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float ei = buf[L::E + ib + 8 * e];
 #pragma unroll
       for (int f = 0; f < 4; ++f) acc[e][f] *= ei;
     }
-    products(buf + L::M, L::SM, buf + L::X, q * (SC_TOKENS / 4), SC_TOKENS / 4);
+    products(buf + L::M, L::SM, buf + L::X, q * (SC_TOKENS / 4), Whole<SC_TOKENS / 4>(), Whole<SC_TOKENS / 4>());
 #pragma unroll
     for (int e = 0; e < 4; ++e)
       *reinterpret_cast<float4*>(part + (q * SC_TOKENS + ib + 8 * e) * L::SPART + 4 * pb) =

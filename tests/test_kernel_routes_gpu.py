@@ -317,6 +317,42 @@ def test_state_space_recurrence(ops16, lengths, pad, n_state, p):
         assert torch.equal(state[slot], before[slot])
 
 
+def _portions(n, most=63):
+    """The cut of ``n`` tokens into portions that the token kernels take."""
+    return [(a, min(a + most, n)) for a in range(0, n, most)]
+
+
+@pytest.mark.parametrize("n_state,p", [(128, 64), (64, 64)])
+def test_state_space_chunks_lose_no_precision(ops16, n_state, p):
+    """One long sequence whole (chunks) and in portions of 63 tokens (the token kernel) against float64."""
+    heads, groups, n = 64, 8, 600
+    g = torch.Generator().manual_seed(n_state)
+    inner, bc = heads * p, groups * n_state
+    xbc = _randn(g, n, inner + 2 * bc, scale=0.5)
+    proj = _randn(g, n, 16 + heads).to(torch.bfloat16)
+    dt_bias, a_log = torch.rand(heads, generator=g).to(DEV) * 3.5 - 3, torch.rand(heads, generator=g).to(DEV) * 2.5 - 1
+    d, first = _randn(g, heads), _randn(g, 1, heads * n_state * p)
+    per, rows = heads // groups, xbc.double()
+    x = rows[:, :inner].reshape(n, heads, p)
+    b = rows[:, inner : inner + bc].reshape(n, groups, n_state).repeat_interleave(per, 1)
+    c = rows[:, inner + bc :].reshape(n, groups, n_state).repeat_interleave(per, 1)
+    dt = torch.nn.functional.softplus(proj[:, 16:].double() + dt_bias.double(), threshold=1e9)
+    decay = torch.exp(-torch.exp(a_log.double()) * dt)
+    S = first.double().reshape(heads, p, n_state).clone()
+    ref = torch.empty(n, heads, p, dtype=torch.float64, device=DEV)
+    for s in range(n):
+        S = decay[s][:, None, None] * S + (dt[s][:, None] * x[s])[:, :, None] * b[s][:, None, :]
+        ref[s] = (S * c[s][:, None, :]).sum(-1) + d.double()[:, None] * x[s]
+    errors = []
+    for cuts in ([(0, n)], _portions(n)):
+        state = first.clone()
+        y = torch.cat([ops16.mamba2_scan(xbc[a:z], proj[a:z], 16, dt_bias, a_log, d, state, _sequences([z - a]), heads, groups,
+                                         n_state, p) for a, z in cuts])
+        errors.append((_relative(y, ref.reshape(n, inner)), _relative(state, S.reshape(1, -1))))
+    # means over 64 heads, whose decays (rounded alike on both sides) differ: equal to a few per cent
+    assert errors[0][0] <= 1.05 * errors[1][0] and errors[0][1] <= 1.05 * errors[1][1], errors
+
+
 @pytest.mark.parametrize("d,dv", [(64, 64), (40, 24), (128, 12), (100, 130)])
 @pytest.mark.parametrize("lengths,pad", LENGTHS)
 def test_delta_rule_with_one_decay_a_head(ops16, lengths, pad, d, dv):
