@@ -244,10 +244,13 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 // (a block a (chunk, head); the triangular system by forward substitution, a thread a column):
 //     W = (I + A)^-1 beta c K,  V' = (I + A)^-1 beta V,  c Q,  (D[C] o K)^T,  D o Q K^T
 // and delta_chunk_kernel walks the chunks: U = V' - W S0, then O and the next state, two small products
-// and two barriers for 32 tokens.  1,501 tokens, 16 heads of 64: 347 -> 77 us and 24 of forming the chunks.
-// float32 throughout; the order of the sums is not the token kernel's, so the
-// float32 mode, whose results do not depend on how a prompt is cut, keeps the kernel above.
+// and two barriers for 32 tokens.  1,501 tokens, 16 heads of 64: 347 -> 78 us and 32 of forming the chunks.
+// float32, but for the products of decays, K K^T and Q K^T, which are added up in 64 bits.  (As single float32 chains these,
+// the substitution and the sums over the state's rows made the outputs 2.6e-7 off at key size 64 and 3.2e-7 at
+// 128, against 2.0e-7 and 2.3e-7 of the token kernel; with short chains 1.9e-7 and 2.1e-7.)  The order of the
+// sums is not the token kernel's, so the float32 mode, whose results do not depend on how a prompt is cut, keeps that.
 constexpr int CHUNK = 32;
+constexpr int CHUNK_RUN = 8;     // rows of the state that are summed by themselves
 constexpr int CHUNK_THREADS = 128;
 constexpr int CHUNK_COLS = 8;    // columns of the state a block of the walk
 constexpr int CHUNK_STAGES = 3;  // chunks in its ring
@@ -273,7 +276,7 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
   __shared__ __align__(16) float ks[CHUNK][SK];
   __shared__ __align__(16) float qs[CHUNK][SK];
   __shared__ __align__(16) float at[CHUNK][SA];  // A transposed: [m][i]
-  __shared__ float dm[CHUNK][CHUNK + 1];         // D[i][j], j <= i
+  __shared__ double dm[CHUNK][CHUNK + 1];        // D[i][j], j <= i
   __shared__ float gs[CHUNK], betas[CHUNK], cs[CHUNK];
   const int h = blockIdx.y, hk = h / (n_heads / n_kv_heads), tid = threadIdx.x;
   int c = blockIdx.x, b = 0, n = 0;
@@ -304,10 +307,10 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
   __syncthreads();
   if (tid <= CHUNK) {  // column tid of D; thread 32: the decays from the chunk's start
     const int j = tid < CHUNK ? tid : -1;
-    float x = 1.f;
+    double x = 1.0;
     for (int i = j < 0 ? 0 : j; i < CHUNK; ++i) {
       if (i > j) x *= gs[i];
-      if (j < 0) cs[i] = x;
+      if (j < 0) cs[i] = (float)x;
       else dm[i][j] = x;
     }
   }
@@ -316,36 +319,49 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
     const bool of_q = tid >= 64;
     const int ib = (tid & 63) >> 3, jb = tid & 7;
     const float (*left)[SK] = of_q ? qs : ks;
-    float acc[4][4];
+    // short chains: stretches of 16 products that are four chains each, added up in 64 bits
+    double acc[4][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e)
 #pragma unroll
-      for (int f = 0; f < 4; ++f) acc[e][f] = 0.f;
-#pragma unroll 2
-    for (int w = 0; w < D; w += 4) {
-      float4 a[4], k[4];
+      for (int f = 0; f < 4; ++f) acc[e][f] = 0.0;
+#pragma unroll 1
+    for (int w0 = 0; w0 < D; w0 += 16) {
+      float4 run[4][4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        a[e] = *reinterpret_cast<const float4*>(&left[ib + 8 * e][w]);
-        k[e] = *reinterpret_cast<const float4*>(&ks[jb + 8 * e][w]);
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) run[e][f] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = w0; w < w0 + 16; w += 4) {
+        float4 a[4], k[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          a[e] = *reinterpret_cast<const float4*>(&left[ib + 8 * e][w]);
+          k[e] = *reinterpret_cast<const float4*>(&ks[jb + 8 * e][w]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {
+            run[e][f].x = fmaf(a[e].x, k[f].x, run[e][f].x);
+            run[e][f].y = fmaf(a[e].y, k[f].y, run[e][f].y);
+            run[e][f].z = fmaf(a[e].z, k[f].z, run[e][f].z);
+            run[e][f].w = fmaf(a[e].w, k[f].w, run[e][f].w);
+          }
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e)
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          acc[e][f] = fmaf(a[e].x, k[f].x, acc[e][f]);
-          acc[e][f] = fmaf(a[e].y, k[f].y, acc[e][f]);
-          acc[e][f] = fmaf(a[e].z, k[f].z, acc[e][f]);
-          acc[e][f] = fmaf(a[e].w, k[f].w, acc[e][f]);
-        }
+        for (int f = 0; f < 4; ++f) acc[e][f] += (run[e][f].x + run[e][f].y) + (run[e][f].z + run[e][f].w);
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e)
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
         const int i = ib + 8 * e, j = jb + 8 * f;
-        if (of_q) dst[96 * D + i * CHUNK + j] = j <= i ? dm[i][j] * acc[e][f] : 0.f;
-        else at[j][i] = j < i ? betas[i] * dm[i][j] * acc[e][f] : 0.f;
+        if (of_q) dst[96 * D + i * CHUNK + j] = j <= i ? (float)(dm[i][j] * acc[e][f]) : 0.f;
+        else at[j][i] = j < i ? (float)(betas[i] * dm[i][j] * acc[e][f]) : 0.f;
       }
   }
   __syncthreads();
@@ -358,7 +374,7 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float k = ks[i + e][col];
-          kd[e] = dm[CHUNK - 1][i + e] * k;
+          kd[e] = (float)dm[CHUNK - 1][i + e] * k;
           x[i + e] = betas[i + e] * cs[i + e] * k;
           dst[32 * D + (i + e) * D + col] = cs[i + e] * qs[i + e][col];
         }
@@ -369,15 +385,20 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
       for (int i = 0; i < CHUNK; ++i)
         x[i] = i < nt ? betas[i] * vp[((size_t)(t0 + i) * n_heads + h) * DVP + col - D] : 0.f;
     }
+    // what the tokens before it take off a token is summed by itself: it is small beside the token's own number
+    float off[CHUNK];
 #pragma unroll
-    for (int m = 0; m < CHUNK - 1; ++m) {
+    for (int i = 0; i < CHUNK; ++i) off[i] = 0.f;
+#pragma unroll
+    for (int m = 0; m < CHUNK; ++m) {
+      x[m] -= off[m];
 #pragma unroll
       for (int i = (m + 1) / 4 * 4; i < CHUNK; i += 4) {
         const float4 a = *reinterpret_cast<const float4*>(&at[m][i]);  // zero up to i = m
-        if (i > m) x[i] = fmaf(-a.x, x[m], x[i]);
-        if (i + 1 > m) x[i + 1] = fmaf(-a.y, x[m], x[i + 1]);
-        if (i + 2 > m) x[i + 2] = fmaf(-a.z, x[m], x[i + 2]);
-        x[i + 3] = fmaf(-a.w, x[m], x[i + 3]);
+        if (i > m) off[i] = fmaf(a.x, x[m], off[i]);
+        if (i + 1 > m) off[i + 1] = fmaf(a.y, x[m], off[i + 1]);
+        if (i + 2 > m) off[i + 2] = fmaf(a.z, x[m], off[i + 2]);
+        off[i + 3] = fmaf(a.w, x[m], off[i + 3]);
       }
     }
 #pragma unroll
@@ -462,15 +483,23 @@ delta_chunk_kernel(const float* __restrict__ chunks, float* __restrict__ out, lo
     const float* buf = smem + c % CHUNK_STAGES * L::BUF;
     float w0 = 0.f, w1 = 0.f, q0 = 0.f, q1 = 0.f;
 #pragma unroll
-    for (int k = 0; k < D; k += 4) {
-      const float4 w = *reinterpret_cast<const float4*>(buf + L::W + r * L::SW + k);
-      const float4 q = *reinterpret_cast<const float4*>(buf + L::Q + r * L::SW + k);
-      const float4 a = *reinterpret_cast<const float4*>(s_t + c0 * L::SW + k);
-      const float4 e = *reinterpret_cast<const float4*>(s_t + (c0 + 1) * L::SW + k);
-      w0 = dot4(w, a, w0);
-      w1 = dot4(w, e, w1);
-      q0 = dot4(q, a, q0);
-      q1 = dot4(q, e, q1);
+    for (int k0 = 0; k0 < D; k0 += CHUNK_RUN) {
+      float rw0 = 0.f, rw1 = 0.f, rq0 = 0.f, rq1 = 0.f;
+#pragma unroll
+      for (int k = k0; k < k0 + CHUNK_RUN; k += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(buf + L::W + r * L::SW + k);
+        const float4 q = *reinterpret_cast<const float4*>(buf + L::Q + r * L::SW + k);
+        const float4 a = *reinterpret_cast<const float4*>(s_t + c0 * L::SW + k);
+        const float4 e = *reinterpret_cast<const float4*>(s_t + (c0 + 1) * L::SW + k);
+        rw0 = dot4(w, a, rw0);
+        rw1 = dot4(w, e, rw1);
+        rq0 = dot4(q, a, rq0);
+        rq1 = dot4(q, e, rq1);
+      }
+      w0 += rw0;
+      w1 += rw1;
+      q0 += rq0;
+      q1 += rq1;
     }
     const float2 v = *reinterpret_cast<const float2*>(buf + L::V + r * CHUNK_COLS + c0);
     u_t[c0 * L::SK + r] = v.x - w0;

@@ -392,6 +392,41 @@ def test_delta_rule_with_one_decay_a_head(ops16, lengths, pad, d, dv):
         assert torch.equal(state[slot], before[slot])
 
 
+@pytest.mark.parametrize("d", [64, 128])
+def test_delta_chunks_lose_no_precision(ops16, d):
+    """One long sequence whole (chunks) and in portions of 63 tokens (the token kernel) against float64."""
+    heads, kv, dv, n = 32, 8, 64, 600
+    g = torch.Generator().manual_seed(d)
+    qkv = _randn(g, n, 2 * kv * d + heads * dv)
+    proj = _randn(g, n, 2 * heads).to(torch.bfloat16)
+    a, b = proj[:, :heads], proj[:, heads:]
+    dt_bias, a_log = torch.rand(heads, generator=g).to(DEV) * 3.5 - 3, torch.rand(heads, generator=g).to(DEV) * 2.5 - 2
+    first = _randn(g, 1, heads * d * dv, scale=0.3)
+    rows = qkv.double()
+    q = rows[:, : kv * d].reshape(n, kv, d).repeat_interleave(heads // kv, 1)
+    k = rows[:, kv * d : 2 * kv * d].reshape(n, kv, d).repeat_interleave(heads // kv, 1)
+    v = rows[:, 2 * kv * d :].reshape(n, heads, dv)
+    q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * d ** -0.5
+    k = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    gate = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(a.double() + dt_bias.double(), threshold=1e9))
+    beta = torch.sigmoid(b.double())
+    S = first.double().reshape(heads, dv, d).clone()
+    ref = torch.empty(n, heads, dv, dtype=torch.float64, device=DEV)
+    for s in range(n):
+        S = gate[s][:, None, None] * S
+        u = beta[s][:, None] * (v[s] - (S * k[s][:, None, :]).sum(-1))
+        S = S + u[:, :, None] * k[s][:, None, :]
+        ref[s] = (S * q[s][:, None, :]).sum(-1)
+    errors = []
+    for cuts in ([(0, n)], _portions(n)):
+        state = first.clone()
+        out = torch.cat([ops16.delta_scan(qkv[y:z], a[y:z], b[y:z], dt_bias, a_log, state, _sequences([z - y]), heads, kv, d,
+                                          dv, head_decay=True) for y, z in cuts])
+        errors.append((_relative(out, ref.reshape(n, -1)), _relative(state, S.reshape(1, -1))))
+    # means over 32 heads, whose decays, unit vectors and step sizes are rounded alike on both sides: equal to a few per cent
+    assert errors[0][0] <= 1.05 * errors[1][0] and errors[0][1] <= 1.05 * errors[1][1], errors
+
+
 # -- embedding --------------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
