@@ -686,9 +686,11 @@ ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, const float* __
     __syncthreads();  // the chunk has landed, the state stands in shared memory, the buffer of the chunk before is free
     if (c + 1 < n_chunks) issue(c + 1);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
+    bool finite;
     {  // w X for the state's update
       const int t = tid / 8, w = tid % 8 * 4;
       const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
+      finite = isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(x.w);
       const float wt = buf[L::W + t];
       *reinterpret_cast<float4*>(xw_s + t * L::SP + w) = make_float4(x.x * wt, x.y * wt, x.z * wt, x.w * wt);
     }
@@ -744,7 +746,8 @@ ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, const float* __
     for (int e = 0; e < 4; ++e)
       *reinterpret_cast<float4*>(part + (q * SC_TOKENS + ib + 8 * e) * L::SPART + 4 * pb) =
           make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
-    __syncthreads();
+    // (an infinity or NaN in X would reach the tokens before its own through M's zeros)
+    const bool causal = __syncthreads_or(!finite) != 0;
     {  // a token's four columns a thread: the groups' sums in order
       const int t = tid / 8, w = tid % 8 * 4;
       const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
@@ -756,6 +759,18 @@ ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, const float* __
         v.y += u.y;
         v.z += u.z;
         v.w += u.w;
+      }
+      if (causal) {  // the token's sums once more, over the tokens up to it alone
+        v = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto add = [&](float a, const float* row) {
+          const float4 u = *reinterpret_cast<const float4*>(row + w);
+          v = make_float4(fmaf(a, u.x, v.x), fmaf(a, u.y, v.y), fmaf(a, u.z, v.z), fmaf(a, u.w, v.w));
+        };
+        for (int k = 0; k < N; ++k) add(buf[L::C + t * L::SCN + k], s_s + k * L::SP);
+        const float et = buf[L::E + t];
+        v = make_float4(v.x * et, v.y * et, v.z * et, v.w * et);
+        for (int k = 0; k <= t; ++k) add(buf[L::M + t * L::SM + k], buf + L::X + k * L::SP);
+        __syncthreads();  // the state in shared memory has been read
       }
       if (c * SC_TOKENS + t < n && p0 + w < P)
         *reinterpret_cast<float4*>(y + (size_t)(start + c * SC_TOKENS + t) * y_stride + h * P + p0 + w) =

@@ -317,6 +317,37 @@ def test_state_space_recurrence(ops16, lengths, pad, n_state, p):
         assert torch.equal(state[slot], before[slot])
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("at", [0, 31, 45, 64, 99])
+def test_state_space_chunks_are_causal(ops16, at, value):
+    """A number that is not finite changes nothing before its token, and no other column at all."""
+    heads, groups, n_state, p, n = 4, 2, 128, 40, 100
+    ctx = _sequences([n, 70], 2)
+    g = torch.Generator().manual_seed(at)
+    inner, bc = heads * p, groups * n_state
+    xbc = _randn(g, ctx.n_tokens, inner + 2 * bc, scale=0.5)
+    proj = _randn(g, ctx.n_tokens, 16 + heads).to(torch.bfloat16)
+    dt_bias, a_log, d = torch.rand(heads, generator=g).to(DEV) - 1, torch.rand(heads, generator=g).to(DEV) - 1, _randn(g, heads)
+    column = 2 * p + 35
+    outs, states = [], []
+    for x in (None, value):
+        rows, state = xbc.clone(), torch.zeros(2, heads * n_state * p, device=DEV)
+        if x is not None:
+            rows[at, column] = x
+        outs.append(ops16.mamba2_scan(rows, proj, 16, dt_bias, a_log, d, state, ctx, heads, groups, n_state, p))
+        states.append(state)
+    want, got = outs
+    other = torch.ones(inner, dtype=torch.bool, device=DEV)
+    other[column] = False
+    # (a chunk that holds such a number sums in another order)
+    assert torch.allclose(got[:n, other], want[:n, other], rtol=0, atol=2e-5)
+    assert torch.allclose(got[:at, column], want[:at, column], rtol=0, atol=2e-5)
+    assert not bool(torch.isfinite(got[at:n, column]).any())
+    assert torch.equal(got[n : n + 70], want[n : n + 70]) and torch.equal(states[0][1], states[1][1])
+    finite = torch.isfinite(states[1][0].view(heads * p, n_state)).all(1)
+    assert bool(finite[other].all()) and not bool(finite[column])
+
+
 def _portions(n, most=63):
     """The cut of ``n`` tokens into portions that the token kernels take."""
     return [(a, min(a + most, n)) for a in range(0, n, most)]
