@@ -24,6 +24,8 @@
 // The recurrence runs token by token, so prompt portions, single tokens and mixed batches take
 // these kernels and give the same numbers however a prompt is cut.  The state of a slot is
 // [heads][dv][d] float32 (a column's rows side by side), zero at admission.
+#include <type_traits>
+
 #include "common.cuh"
 
 constexpr int DELTA_WARPS = 8;
@@ -244,7 +246,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 // (a block a (chunk, head); the triangular system by forward substitution, a thread a column):
 //     W = (I + A)^-1 beta c K,  V' = (I + A)^-1 beta V,  c Q,  (D[C] o K)^T,  D o Q K^T
 // and delta_chunk_kernel walks the chunks: U = V' - W S0, then O and the next state, two small products
-// and two barriers for 32 tokens.  1,501 tokens, 16 heads of 64: 347 -> 78 us and 32 of forming the chunks.
+// and two barriers for 32 tokens.  1,501 tokens, 16 heads of 64: 347 -> 82 us and 32 of forming the chunks.
 // float32, but for the products of decays, K K^T and Q K^T, which are added up in 64 bits.  (As single float32 chains these,
 // the substitution and the sums over the state's rows made the outputs 2.6e-7 off at key size 64 and 3.2e-7 at
 // 128, against 2.0e-7 and 2.3e-7 of the token kernel; with short chains 1.9e-7 and 2.1e-7.)  The order of the
@@ -422,6 +424,11 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
 
+// v's numbers up to place n, zeros behind it
+__device__ __forceinline__ float4 up_to(float4 v, int n) {
+  return make_float4(n >= 0 ? v.x : 0.f, n >= 1 ? v.y : 0.f, n >= 2 ? v.z : 0.f, n >= 3 ? v.w : 0.f);
+}
+
 template <int D>
 __global__ void __launch_bounds__(CHUNK_THREADS)
 delta_chunk_kernel(const float* __restrict__ chunks, float* __restrict__ out, long out_stride, float* __restrict__ state,
@@ -458,92 +465,106 @@ delta_chunk_kernel(const float* __restrict__ chunks, float* __restrict__ out, lo
     }
     if (tid == 64) delta_copy16(buf + L::END, src + 96 * D + CHUNK * CHUNK + CHUNK * DVP, true);
   };
-#pragma unroll
-  for (int c = 0; c < CHUNK_STAGES - 1; ++c) {
-    if (c < n_chunks) issue(c);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  }
   // a thread: row r of the chunk (or rows r + 32 i of the state) against two columns
   const int r = tid >> 2, c0 = (tid & 3) * 2;
   float* const st = state + (size_t)seq_slot[b] * state_stride + ((size_t)h * dv + col0) * d;
-  float s[ND][2];
+  // An infinity or NaN in U reaches the tokens before its own through the zeros of D o Q K^T (0 * inf): where an output is
+  // not finite, the block walks once more with U cut off behind each token (CAUSAL; in the first walk the cuts,
+  // or a test in every chunk, cost 5 to 12 % of the time).  The state is stored at the walk's end, so that both start alike.
+  auto walk = [&](auto causal) {
+    constexpr bool CAUSAL = decltype(causal)::value;
 #pragma unroll
-  for (int i = 0; i < ND; ++i)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int row = r + 32 * i, col = c0 + e;
-      s[i][e] = (row < d && col0 + col < dv) ? st[(size_t)col * d + row] : 0.f;
-      s_t[col * L::SW + row] = s[i][e];
+    for (int c = 0; c < CHUNK_STAGES - 1; ++c) {
+      if (c < n_chunks) issue(c);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
-  for (int c = 0; c < n_chunks; ++c) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(CHUNK_STAGES - 2) : "memory");
-    __syncthreads();  // the chunk has landed, and the state of the chunk before stands in shared memory
-    if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    const float* buf = smem + c % CHUNK_STAGES * L::BUF;
-    float w0 = 0.f, w1 = 0.f, q0 = 0.f, q1 = 0.f;
+    float s[ND][2];
 #pragma unroll
-    for (int k0 = 0; k0 < D; k0 += CHUNK_RUN) {
-      float rw0 = 0.f, rw1 = 0.f, rq0 = 0.f, rq1 = 0.f;
+    for (int i = 0; i < ND; ++i)
 #pragma unroll
-      for (int k = k0; k < k0 + CHUNK_RUN; k += 4) {
-        const float4 w = *reinterpret_cast<const float4*>(buf + L::W + r * L::SW + k);
-        const float4 q = *reinterpret_cast<const float4*>(buf + L::Q + r * L::SW + k);
-        const float4 a = *reinterpret_cast<const float4*>(s_t + c0 * L::SW + k);
-        const float4 e = *reinterpret_cast<const float4*>(s_t + (c0 + 1) * L::SW + k);
-        rw0 = dot4(w, a, rw0);
-        rw1 = dot4(w, e, rw1);
-        rq0 = dot4(q, a, rq0);
-        rq1 = dot4(q, e, rq1);
+      for (int e = 0; e < 2; ++e) {
+        const int row = r + 32 * i, col = c0 + e;
+        s[i][e] = (row < d && col0 + col < dv) ? st[(size_t)col * d + row] : 0.f;
+        s_t[col * L::SW + row] = s[i][e];
       }
-      w0 += rw0;
-      w1 += rw1;
-      q0 += rq0;
-      q1 += rq1;
-    }
-    const float2 v = *reinterpret_cast<const float2*>(buf + L::V + r * CHUNK_COLS + c0);
-    u_t[c0 * L::SK + r] = v.x - w0;
-    u_t[(c0 + 1) * L::SK + r] = v.y - w1;
-    __syncthreads();
-    const float gc = buf[L::END];
+    float finite = 0.f;
+    for (int c = 0; c < n_chunks; ++c) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(CHUNK_STAGES - 2) : "memory");
+      __syncthreads();  // the chunk has landed, and the state of the chunk before stands in shared memory
+      if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      const float* buf = smem + c % CHUNK_STAGES * L::BUF;
+      float w0 = 0.f, w1 = 0.f, q0 = 0.f, q1 = 0.f;
 #pragma unroll
-    for (int i = 0; i < ND; ++i) {
-      s[i][0] *= gc;
-      s[i][1] *= gc;
-    }
+      for (int k0 = 0; k0 < D; k0 += CHUNK_RUN) {
+        float rw0 = 0.f, rw1 = 0.f, rq0 = 0.f, rq1 = 0.f;
 #pragma unroll
-    for (int k = 0; k < CHUNK; k += 4) {
-      const float4 a = *reinterpret_cast<const float4*>(u_t + c0 * L::SK + k);
-      const float4 e = *reinterpret_cast<const float4*>(u_t + (c0 + 1) * L::SK + k);
-      const float4 m = *reinterpret_cast<const float4*>(buf + L::A + r * L::SK + k);
-      q0 = dot4(m, a, q0);
-      q1 = dot4(m, e, q1);
+        for (int k = k0; k < k0 + CHUNK_RUN; k += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(buf + L::W + r * L::SW + k);
+          const float4 q = *reinterpret_cast<const float4*>(buf + L::Q + r * L::SW + k);
+          const float4 a = *reinterpret_cast<const float4*>(s_t + c0 * L::SW + k);
+          const float4 e = *reinterpret_cast<const float4*>(s_t + (c0 + 1) * L::SW + k);
+          rw0 = dot4(w, a, rw0);
+          rw1 = dot4(w, e, rw1);
+          rq0 = dot4(q, a, rq0);
+          rq1 = dot4(q, e, rq1);
+        }
+        w0 += rw0;
+        w1 += rw1;
+        q0 += rq0;
+        q1 += rq1;
+      }
+      const float2 v = *reinterpret_cast<const float2*>(buf + L::V + r * CHUNK_COLS + c0);
+      u_t[c0 * L::SK + r] = v.x - w0;
+      u_t[(c0 + 1) * L::SK + r] = v.y - w1;
+      __syncthreads();
+      const float gc = buf[L::END];
 #pragma unroll
       for (int i = 0; i < ND; ++i) {
-        const float4 kd = *reinterpret_cast<const float4*>(buf + L::K + (r + 32 * i) * L::SK + k);
-        s[i][0] = dot4(kd, a, s[i][0]);
-        s[i][1] = dot4(kd, e, s[i][1]);
+        s[i][0] *= gc;
+        s[i][1] *= gc;
+      }
+      float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+      for (int k = 0; k < CHUNK; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(u_t + c0 * L::SK + k);
+        const float4 e = *reinterpret_cast<const float4*>(u_t + (c0 + 1) * L::SK + k);
+        const float4 m = *reinterpret_cast<const float4*>(buf + L::A + r * L::SK + k);
+        m0 = dot4(m, CAUSAL ? up_to(a, r - k) : a, m0);
+        m1 = dot4(m, CAUSAL ? up_to(e, r - k) : e, m1);
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+          const float4 kd = *reinterpret_cast<const float4*>(buf + L::K + (r + 32 * i) * L::SK + k);
+          s[i][0] = dot4(kd, a, s[i][0]);
+          s[i][1] = dot4(kd, e, s[i][1]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < ND; ++i) {
+        s_t[c0 * L::SW + r + 32 * i] = s[i][0];
+        s_t[(c0 + 1) * L::SW + r + 32 * i] = s[i][1];
+      }
+      q0 += m0;
+      q1 += m1;
+      if (!CAUSAL) finite = fmaf(0.f, q0, fmaf(0.f, q1, finite));
+      if (c * CHUNK + r < n) {
+        float* o = out + (size_t)(start + c * CHUNK + r) * out_stride + h * dv + col0 + c0;
+        if (col0 + c0 < dv) o[0] = q0;
+        if (col0 + c0 + 1 < dv) o[1] = q1;
       }
     }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (!CAUSAL && __syncthreads_or(finite != 0.f)) return false;
 #pragma unroll
-    for (int i = 0; i < ND; ++i) {
-      s_t[c0 * L::SW + r + 32 * i] = s[i][0];
-      s_t[(c0 + 1) * L::SW + r + 32 * i] = s[i][1];
-    }
-    if (c * CHUNK + r < n) {
-      float* o = out + (size_t)(start + c * CHUNK + r) * out_stride + h * dv + col0 + c0;
-      if (col0 + c0 < dv) o[0] = q0;
-      if (col0 + c0 + 1 < dv) o[1] = q1;
-    }
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    for (int i = 0; i < ND; ++i)
 #pragma unroll
-  for (int i = 0; i < ND; ++i)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int row = r + 32 * i, col = c0 + e;
-      if (row < d && col0 + col < dv) st[(size_t)col * d + row] = s[i][e];
-    }
+      for (int e = 0; e < 2; ++e) {
+        const int row = r + 32 * i, col = c0 + e;
+        if (row < d && col0 + col < dv) st[(size_t)col * d + row] = s[i][e];
+      }
+    return true;
+  };
+  if (!walk(std::false_type())) walk(std::true_type());
 }
 
 // rows of the prepared arrays for key size d (the row count of the kernel that takes it)

@@ -423,6 +423,42 @@ def test_delta_rule_with_one_decay_a_head(ops16, lengths, pad, d, dv):
         assert torch.equal(state[slot], before[slot])
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("part", ["v", "k", "q"])
+@pytest.mark.parametrize("at", [0, 31, 45, 99])
+def test_delta_chunks_are_causal(ops16, at, part, value):
+    """A number that is not finite changes nothing before its token, and nothing of other columns (a value's) or heads."""
+    heads, kv, d, dv, n = 4, 2, 64, 40, 100
+    ctx = _sequences([n, 70], 2)
+    g = torch.Generator().manual_seed(at)
+    qkv = _randn(g, ctx.n_tokens, 2 * kv * d + heads * dv)
+    proj = _randn(g, ctx.n_tokens, 2 * heads).to(torch.bfloat16)
+    a, b = proj[:, :heads], proj[:, heads:]
+    dt_bias, a_log = torch.rand(heads, generator=g).to(DEV) - 1, torch.rand(heads, generator=g).to(DEV) - 1
+    # the second value head's 7th value, or the first key head's 5th key or query
+    column = {"v": 2 * kv * d + dv + 7, "k": kv * d + 5, "q": 5}[part]
+    hit = torch.zeros(heads, dv, dtype=torch.bool, device=DEV)
+    if part == "v":
+        hit[1, 7] = True
+    else:
+        hit[:2] = True
+    hit = hit.view(-1)
+    outs = []
+    for x in (None, value):
+        rows, state = qkv.clone(), torch.zeros(2, heads * d * dv, device=DEV)
+        if x is not None:
+            rows[at, column] = x
+        outs.append(ops16.delta_scan(rows, a, b, dt_bias, a_log, state, ctx, heads, kv, d, dv, head_decay=True))
+    want, got = outs
+    assert torch.allclose(got[:n, ~hit], want[:n, ~hit], rtol=0, atol=2e-6)
+    assert torch.allclose(got[:at, hit], want[:at, hit], rtol=0, atol=2e-6)
+    bad = got[at:n, hit] if part != "q" else got[at, hit]
+    assert not bool(torch.isfinite(bad).any())
+    if part == "q":
+        assert torch.allclose(got[at + 1 : n, hit], want[at + 1 : n, hit], rtol=0, atol=2e-6)
+    assert torch.equal(got[n : n + 70], want[n : n + 70])
+
+
 @pytest.mark.parametrize("d", [64, 128])
 def test_delta_chunks_lose_no_precision(ops16, d):
     """One long sequence whole (chunks) and in portions of 63 tokens (the token kernel) against float64."""
