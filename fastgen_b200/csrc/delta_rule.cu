@@ -596,9 +596,9 @@ static int launch_scan(cudaStream_t stream, const float* qn, const float* kn, co
 }
 
 // Whether a step may hold sequences for delta_chunk_kernel: 16-bit serving, one decay a head, key sizes whose
-// rows are 64 or 128, and enough tokens for one such sequence.
-static bool chunks_apply(int n_tokens, int d, int dtype, int head_decay) {
-  return dtype == FG_BF16 && head_decay && d > 32 && d <= 128 && n_tokens >= CHUNK_MIN;
+// rows are 64 or 128, and enough tokens (`longest`: the most that one of its sequences can bring).
+static bool chunks_apply(int longest, int d, int dtype, int head_decay) {
+  return dtype == FG_BF16 && head_decay && d > 32 && d <= 128 && longest >= CHUNK_MIN;
 }
 // most chunks of a step's sequences that have CHUNK_MIN tokens or more
 static long most_chunks(int n_tokens, int n_seqs) {
@@ -607,11 +607,11 @@ static long most_chunks(int n_tokens, int n_seqs) {
 }
 
 // floats of the scratch that fg_delta_scan needs for `n_tokens` tokens
-extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int n_seqs, int n_heads, int n_kv_heads, int d, int dv, int dtype,
-                                             int head_decay) {
+extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int longest, int n_seqs, int n_heads, int n_kv_heads, int d, int dv,
+                                             int dtype, int head_decay) {
   const long DP = delta_rows(d), DVP = (dv + 3) / 4 * 4;
   const long rows = (long)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
-  return rows + (chunks_apply(n_tokens, d, dtype, head_decay) ? most_chunks(n_tokens, n_seqs) * n_heads * chunk_floats((int)DP, (int)DVP) : 0);
+  return rows + (chunks_apply(longest, d, dtype, head_decay) ? most_chunks(n_tokens, n_seqs) * n_heads * chunk_floats((int)DP, (int)DVP) : 0);
 }
 
 // qkv: float32 [T, q (kv heads x d) | k (kv heads x d) | v (heads x dv)], the convolutions' outputs.
@@ -621,7 +621,7 @@ extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int n_seqs, int n_hea
 extern "C" int fg_delta_scan(const float* qkv, long qkv_stride, const void* a, long a_stride, const void* b,
                              long b_stride, int dtype, const float* dt_bias, const float* a_log, float* out,
                              long out_stride, float* state, long state_stride, const int* seq_slot,
-                             const int* seq_start, int n_seqs, const int* req, int n_tokens, float* scratch,
+                             const int* seq_start, int n_seqs, const int* req, int n_tokens, int longest, float* scratch,
                              int n_heads, int n_kv_heads, int d, int dv, int head_decay, cudaStream_t stream) {
   if (n_seqs == 0 || n_tokens == 0) return 0;
   FG_CHECK_ARG(n_heads > 0 && n_kv_heads > 0 && n_heads % n_kv_heads == 0, "fg_delta_scan: %d heads over %d key heads",
@@ -648,7 +648,7 @@ extern "C" int fg_delta_scan(const float* qkv, long qkv_stride, const void* a, l
 #undef PREPARE
   FG_CHECK_LAUNCH("fg_delta_scan (prepare)");
   int most = 0x7fffffff;  // tokens of the longest sequence that the token kernel takes
-  if (chunks_apply(n_tokens, d, dtype, head_decay)) {
+  if (chunks_apply(longest, d, dtype, head_decay)) {
     most = CHUNK_MIN - 1;
     float* chunks = scratch + (size_t)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
     const dim3 wy_grid((unsigned)most_chunks(n_tokens, n_seqs), n_heads), grid((dv + CHUNK_COLS - 1) / CHUNK_COLS, n_heads, n_seqs);

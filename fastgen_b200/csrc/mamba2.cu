@@ -984,9 +984,11 @@ static long sc_most_chunks(int n_tokens, int n_seqs) {
   return n_tokens / SC_TOKENS + (n_seqs < long_ones ? n_seqs : long_ones);
 }
 
-// floats of the scratch that fg_mamba2_scan takes (0: none; without it every token goes through the token kernels)
-extern "C" long fg_mamba2_scan_scratch_floats(int n_tokens, int n_seqs, int heads, int n_state, int head_dim, int dtype) {
-  return sc_apply(n_tokens, n_state, head_dim, dtype) ? sc_most_chunks(n_tokens, n_seqs) * heads * SC_REC : 0;
+// floats of the scratch that fg_mamba2_scan takes (0: none; without it every token goes through the token kernels, as
+// it does where no sequence of the step brings more than `longest` tokens and those are too few)
+extern "C" long fg_mamba2_scan_scratch_floats(int n_tokens, int longest, int n_seqs, int heads, int n_state, int head_dim,
+                                              int dtype) {
+  return sc_apply(longest, n_state, head_dim, dtype) ? sc_most_chunks(n_tokens, n_seqs) * heads * SC_REC : 0;
 }
 
 template <typename T>

@@ -57,7 +57,7 @@ _CORE_SIGNATURES = {
     "fg_head_gate": [_P, _L, _P, _L, _I, _P, _I, _I, _I, _P],
     "fg_qk_head_factors": [_P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P, _P, _P, _I, _P],
     "fg_mamba2_scan": [_P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
-    "fg_mamba2_scan_scratch_floats": [_I, _I, _I, _I, _I, _I],
+    "fg_mamba2_scan_scratch_floats": [_I, _I, _I, _I, _I, _I, _I],
     "fg_gated_part_norm": [_P, _L, _P, _L, _I, _P, _P, _L, _P, _I, _I, _I, _F, _P],
     "fg_selective_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _P],
     "fg_layer_norm_pair": [_P, _P, _P, _I, _I, _P, _P, _F, _P, _P, _F, _P, _I, _P, _I, _I, _P],
@@ -203,8 +203,8 @@ def latent(rank: int, rot_dim: int):
 
 
 _DELTA_SIGNATURES = {
-    "fg_delta_scan": [_P, _L, _P, _L, _P, _L, _I, _P, _P, _P, _L, _P, _L, _P, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P],
-    "fg_delta_scan_scratch_floats": [_I, _I, _I, _I, _I, _I, _I, _I],
+    "fg_delta_scan": [_P, _L, _P, _L, _P, _L, _I, _P, _P, _P, _L, _P, _L, _P, _P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _P],
+    "fg_delta_scan_scratch_floats": [_I, _I, _I, _I, _I, _I, _I, _I, _I],
     "fg_head_norm_gate": [_P, _L, _P, _L, _I, _P, _P, _L, _P, _I, _I, _I, _F, _I, _P],
 }
 _MOE_SIGNATURES = {
@@ -316,6 +316,12 @@ def attention_tiling(n_heads: int, n_kv_heads: int, rows: int = SIMT_ROWS) -> in
     query rows (see attention.cu)."""
     group = n_heads // n_kv_heads
     return max(1, rows // min(group, rows))
+
+
+def _longest(ctx, n_tokens: int) -> int:
+    """A bound on the tokens that one sequence of the step brings."""
+    longest = getattr(ctx, "longest", None)
+    return n_tokens if longest is None else min(longest, n_tokens)
 
 
 class Ops:
@@ -445,7 +451,8 @@ class Ops:
             assert v.dtype == torch.float32 and v.numel() == heads and v.is_contiguous()
         y = torch.empty((t, heads * head_dim), dtype=torch.float32, device=xbc.device)
         # sequences of many tokens in 16-bit serving go chunk by chunk: what the chunks are alone
-        floats = self.lib.fg_mamba2_scan_scratch_floats(t, ctx.n_seqs, heads, n_state, head_dim, _code(proj.dtype))
+        floats = self.lib.fg_mamba2_scan_scratch_floats(t, _longest(ctx, t), ctx.n_seqs, heads, n_state, head_dim,
+                                                        _code(proj.dtype))
         scratch = torch.empty(floats, dtype=torch.float32, device=xbc.device) if floats else None
         _check(self.lib, self.lib.fg_mamba2_scan(
             _ptr(xbc), xbc.stride(0), _ptr(proj), proj.stride(0), int(dt_offset), _code(proj.dtype), _ptr(dt_bias),
@@ -831,16 +838,17 @@ class Ops:
         assert dt_bias.dtype == torch.float32 and dt_bias.numel() == decays and dt_bias.is_contiguous()
         assert a_log.dtype == torch.float32 and a_log.numel() == heads and a_log.is_contiguous()
         out = torch.empty((t, heads * dv), dtype=torch.float32, device=qkv.device)
+        longest = _longest(ctx, t)
         # the tokens as the recurrence reads them (unit vectors, decays, step sizes; padded rows)
         # (and, where sequences of many tokens go chunk by chunk, what the chunks are alone)
         def room(dtype):
-            return lib.fg_delta_scan_scratch_floats(t, ctx.n_seqs, heads, kv_heads, d, dv, dtype, int(head_decay))
+            return lib.fg_delta_scan_scratch_floats(t, longest, ctx.n_seqs, heads, kv_heads, d, dv, dtype, int(head_decay))
 
         scratch = torch.empty(room(_code(a.dtype)), dtype=torch.float32, device=qkv.device)
         _check(lib, lib.fg_delta_scan(
             _ptr(qkv), qkv.stride(0), _ptr(a), a.stride(0), _ptr(b), b.stride(0), _code(a.dtype), _ptr(dt_bias),
             _ptr(a_log), _ptr(out), out.stride(0), _ptr(state), state.stride(0), _ptr(ctx.seq_slot),
-            _ptr(ctx.seq_start), ctx.n_seqs, _ptr(ctx.req), t, _ptr(scratch), heads, kv_heads, d, dv,
+            _ptr(ctx.seq_start), ctx.n_seqs, _ptr(ctx.req), t, longest, _ptr(scratch), heads, kv_heads, d, dv,
             int(head_decay), _stream()))
         # the kernel that prepares the tokens, and the chunks' two (float32 never has those)
         Ops.launches += 1 + 2 * int(scratch.numel() > room(FG_F32))

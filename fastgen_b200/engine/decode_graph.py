@@ -61,6 +61,7 @@ class _Bucket:
         # every sequence is its one token: slot and cached tokens are the token's slot and position
         ctx.seq_slot, ctx.seq_start, ctx.seq_cached = ctx.req, self.seq_start, ctx.pos
         ctx.n_tokens = ctx.n_seqs = ctx.n_want = n
+        ctx.longest = 1
         # every sequence is one token: one-token tiles for kernels that tile all
         # sequences, none for kernels that only take longer ones
         tiles = AttentionTiles(ctx.req, self.dev[3 * n : 4 * n], self.dev[4 * n :], n)

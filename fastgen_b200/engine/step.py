@@ -104,6 +104,8 @@ class StepContext:
         self.n_tokens = 0
         self.n_seqs = 0
         self.n_want = 0
+        #: the most tokens one sequence of the step can bring (None: any number of the step's)
+        self.longest: Optional[int] = None
         self.tokens = self.pos = self.req = self.want_rows = None
         self.seq_slot = self.seq_start = self.seq_cached = None
         self.host_seq_slot: List[int] = []
@@ -304,6 +306,7 @@ class Engine:
         ctx.seq_start, o = dev[o : o + b + 1], o + b + 1
         ctx.seq_cached, o = dev[o : o + b], o + b
         ctx.n_tokens, ctx.n_seqs, ctx.n_want = t, b, nw
+        ctx.longest = max(len(e.tokens) for e in entries)
         return ctx
 
     @torch.inference_mode()

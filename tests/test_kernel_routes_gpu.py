@@ -494,6 +494,32 @@ def test_delta_chunks_lose_no_precision(ops16, d):
     assert errors[0][0] <= 1.05 * errors[1][0] and errors[0][1] <= 1.05 * errors[1][1], errors
 
 
+def test_decode_buckets_launch_no_chunks(ops16):
+    """A captured step of 64 and more single tokens runs the token kernels alone."""
+    from fastgen_b200.csrc.ops import Ops
+    from fastgen_b200.engine.decode_graph import _Bucket
+    g = torch.Generator().manual_seed(5)
+    heads, groups, n_state, p, d = 4, 2, 64, 32, 64
+
+    def launches(n, longest):
+        ctx = _Bucket(n, 100, 1000, DEV).context(torch.device(DEV))
+        assert ctx.longest == 1
+        ctx.longest = longest
+        ctx.seq_slot.copy_(torch.arange(n, dtype=torch.int32, device=DEV))
+        proj = _randn(g, n, 2 * heads).to(torch.bfloat16)
+        vec = torch.zeros(heads, device=DEV)
+        before = Ops.launches
+        ops16.mamba2_scan(_randn(g, n, heads * p + 2 * groups * n_state), proj, 0, vec, vec, vec,
+                          torch.zeros(n, heads * n_state * p, device=DEV), ctx, heads, groups, n_state, p)
+        between = Ops.launches
+        ops16.delta_scan(_randn(g, n, 2 * groups * d + heads * p), proj[:, :heads], proj[:, heads:], vec, vec,
+                         torch.zeros(n, heads * d * p, device=DEV), ctx, heads, groups, d, p, head_decay=True)
+        return between - before, Ops.launches - between
+
+    assert launches(64, 1) == launches(63, None) == (1, 2)
+    assert launches(64, None) == (3, 4)
+
+
 # -- embedding --------------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
