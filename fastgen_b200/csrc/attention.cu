@@ -174,16 +174,6 @@ extern "C" int fg_attention_sigmoid_decode_bf16(const void* q, int q_stride, voi
 // ---------------------------------------------------------------------------------
 #include "attention_mma.cuh"
 
-[[maybe_unused]] static int sm_count() {
-  static int n_sms = 0;
-  if (n_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return n_sms;
-}
-
 // The merge of the splits for a launch of n_heads x n_seqs blocks: half the threads a block where full blocks (four an
 // SM) would be more than one round.
 struct Combine {
@@ -193,7 +183,7 @@ struct Combine {
 [[maybe_unused]] static Combine combine_for(int window, int n_heads, int n_seqs) {
   using namespace fg_mma;
   constexpr int HALF = COMBINE_THREADS / 2;
-  if ((long long)n_heads * n_seqs > 4ll * sm_count())
+  if ((long long)n_heads * n_seqs > 4ll * fg_sm_count())
     return {window < 0 ? attention_combine_kernel<FG_HEAD_DIM, true, HALF> : attention_combine_kernel<FG_HEAD_DIM, false, HALF>, HALF};
   return {window < 0 ? attention_combine_kernel<FG_HEAD_DIM, true> : attention_combine_kernel<FG_HEAD_DIM, false>, COMBINE_THREADS};
 }
@@ -392,7 +382,7 @@ extern "C" int fg_attention_decode_tma_bf16(const void* q, int q_stride, void* o
       FG_CHECK_ARG(e == cudaSuccess, "fg_attention_decode_tma_bf16: shared memory: %s", cudaGetErrorString(e));
       pattr_set = psmem;
     }
-    fg_launch_pdl(pkern, dim3(ps_blocks_per_sm<FG_HEAD_DIM>() * sm_count()), dim3(PS_THREADS), psmem, stream, km, vm,
+    fg_launch_pdl(pkern, dim3(ps_blocks_per_sm<FG_HEAD_DIM>() * fg_sm_count()), dim3(PS_THREADS), psmem, stream, km, vm,
                   layer, (const __nv_bfloat16*)q, q_stride, block_table, table_width, page_size, n_pages, pos,
                   seq_req, seq_tok, n_seqs, n_heads, n_kv_heads, group, window, scale * 1.4426950408889634f,
                   scratch, max_pairs, max_splits, status);
@@ -507,7 +497,7 @@ static long long tc5_items(int n_tiles, int n_heads, int n_kv_heads) {
 }
 
 static int tc5_parts(long long items) {
-  const long long parts = 2ll * sm_count() / (items > 0 ? items : 1);
+  const long long parts = 2ll * fg_sm_count() / (items > 0 ? items : 1);
   return (int)(parts < 1 ? 1 : parts > fg_tc5::MAX_PARTS ? fg_tc5::MAX_PARTS : parts);
 }
 
@@ -518,7 +508,7 @@ extern "C" int fg_attention_prefill_tc5_split_slots(int n_tiles, int n_heads, in
   if (max_keys >= 0 && max_keys <= (2 * fg_tc5::SPLIT_MIN_TILES - 1) * fg_tc5::KEYS) return 0;
   // (with padding in the list: the instantiation that can split, unless a step whose tokens
   // are all prompt tokens, `nominal_tiles` tiles, would fill the launch's blocks anyway)
-  if (nominal_tiles > 0) return tc5_items(nominal_tiles, n_heads, n_kv_heads) < 2ll * sm_count() ? 2 * sm_count() : 0;
+  if (nominal_tiles > 0) return tc5_items(nominal_tiles, n_heads, n_kv_heads) < 2ll * fg_sm_count() ? 2 * fg_sm_count() : 0;
   const long long items = tc5_items(n_tiles, n_heads, n_kv_heads);
   const int parts = tc5_parts(items);
   return parts > 1 ? (int)(items * parts) : 0;
@@ -574,7 +564,7 @@ extern "C" int fg_attention_prefill_tc5_bf16(const void* q, int q_stride, void* 
   FG_CHECK_ARG(items < (1ll << 30), "fg_attention_prefill_tc5_bf16: %lld work items in one call", items);
   const int want = fg_attention_prefill_tc5_split_slots(n_tiles, n_heads, n_kv_heads, max_keys,
                                                         real_tiles ? (nominal_tiles > 0 ? nominal_tiles : 1) : 0);
-  const long long resident = 2ll * sm_count();
+  const long long resident = 2ll * fg_sm_count();
   const bool split = want > 0 && split_scratch && split_flags && want <= split_slots;
   const int parts = split && !real_tiles ? tc5_parts(items) : 1;
   const long long total = items * parts;
@@ -628,7 +618,7 @@ extern "C" int fg_attention_sigmoid_prefill_tc5_bf16(const void* q, int q_stride
   }
   const long long items = tc5_items(n_tiles, n_heads, n_kv_heads);
   FG_CHECK_ARG(items < (1ll << 30), "fg_attention_sigmoid_prefill_tc5_bf16: %lld work items in one call", items);
-  const long long resident = 2ll * sm_count();
+  const long long resident = 2ll * fg_sm_count();
   const int grid = (int)(items < resident ? items : resident);
   kern<<<grid, fg_tc5::THREADS, smem, stream>>>(
       km, vm, layer, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, block_table, table_width,

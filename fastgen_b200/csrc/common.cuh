@@ -72,6 +72,22 @@ __device__ __forceinline__ uint32_t ld_global_4(const void* p) {
 
 bool fg_pdl_enabled();
 
+// the device's multiprocessors
+inline int fg_sm_count() {
+  static const int n = [] {
+    int dev = 0, count = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    return count;
+  }();
+  return n;
+}
+// blocks of `threads` threads and `smem` bytes that an SM holds, as far as those go
+inline int fg_blocks_per_sm(int threads, size_t smem) {
+  const int by_smem = (int)(228 * 1024 / (smem + 1024)), by_threads = 2048 / threads;
+  return by_smem < by_threads ? (by_smem < 1 ? 1 : by_smem) : by_threads;
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t fg_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                  Args... args) {

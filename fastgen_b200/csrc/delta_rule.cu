@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "long_sequences.cuh"
 
 constexpr int DELTA_WARPS = 8;
 constexpr int DELTA_TOKENS = 8;  // tokens a stage
@@ -246,7 +247,7 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 // (a block a (chunk, head); the triangular system by forward substitution, a thread a column):
 //     W = (I + A)^-1 beta c K,  V' = (I + A)^-1 beta V,  c Q,  (D[C] o K)^T,  D o Q K^T
 // and delta_chunk_kernel walks the chunks: U = V' - W S0, then O and the next state, two small products
-// and two barriers for 32 tokens.  1,501 tokens, 16 heads of 64: 347 -> 82 us and 32 of forming the chunks.
+// and two barriers for 32 tokens.  1,501 tokens, 16 heads of 64: 347 -> 63 us and 28 of forming the chunks.
 // float32, but for the products of decays, K K^T and Q K^T, which are added up in 64 bits.  (As single float32 chains these,
 // the substitution and the sums over the state's rows made the outputs 2.6e-7 off at key size 64 and 3.2e-7 at
 // 128, against 2.0e-7 and 2.3e-7 of the token kernel; with short chains 1.9e-7 and 2.1e-7.)  The order of the
@@ -263,17 +264,11 @@ constexpr int CHUNK_MIN = 64;
 // floats of a (chunk, head): W [32][D], c Q [32][D], (D[C] o K)^T [D][32], D o Q K^T [32][32], V' [32][DVP], c_C
 __host__ __device__ constexpr long chunk_floats(int D, int DVP) { return 96L * D + CHUNK * CHUNK + CHUNK * DVP + 4; }
 
-// Sequence b's tokens take the chunks (else the token kernel).
-__device__ __forceinline__ bool chunked_sequence(const int* seq_slot, const int* seq_start, int b, int& n) {
-  n = seq_start[b + 1] - seq_start[b];
-  return seq_slot[b] >= 0 && n >= CHUNK_MIN;
-}
-
 template <int D>
 __global__ void __launch_bounds__(CHUNK_THREADS)
 delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ rec,
-                const float* __restrict__ vp, float* __restrict__ chunks, const int* __restrict__ seq_slot,
-                const int* __restrict__ seq_start, int n_seqs, int n_heads, int n_kv_heads, int DVP) {
+                const float* __restrict__ vp, long_seq::Head* list, float* __restrict__ chunks,
+                const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs, int n_heads, int n_kv_heads, int DVP) {
   constexpr int SK = D + 4, SA = CHUNK + 4;
   __shared__ __align__(16) float ks[CHUNK][SK];
   __shared__ __align__(16) float qs[CHUNK][SK];
@@ -281,15 +276,11 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
   __shared__ double dm[CHUNK][CHUNK + 1];        // D[i][j], j <= i
   __shared__ float gs[CHUNK], betas[CHUNK], cs[CHUNK];
   const int h = blockIdx.y, hk = h / (n_heads / n_kv_heads), tid = threadIdx.x;
-  int c = blockIdx.x, b = 0, n = 0;
-  for (; b < n_seqs; ++b) {
-    if (!chunked_sequence(seq_slot, seq_start, b, n)) continue;
-    const int nc = (n + CHUNK - 1) / CHUNK;
-    if (c < nc) break;
-    c -= nc;
-  }
-  if (b == n_seqs) return;
-  const int t0 = seq_start[b] + c * CHUNK, nt = min(CHUNK, n - c * CHUNK);
+  const auto found = long_seq::find_chunk<CHUNK_MIN, CHUNK, CHUNK_THREADS>(seq_slot, seq_start, n_seqs, blockIdx.x,
+                                                                           blockIdx.x + h == 0 ? list : nullptr);
+  if (found.seq < 0) return;
+  const int c = blockIdx.x - found.first_chunk;
+  const int t0 = seq_start[found.seq] + c * CHUNK, nt = min(CHUNK, found.tokens - c * CHUNK);
   float* const dst = chunks + ((size_t)blockIdx.x * n_heads + h) * chunk_floats(D, DVP);
   for (int i = tid; i < CHUNK * (D / 4); i += CHUNK_THREADS) {
     const int t = i / (D / 4), w = i % (D / 4) * 4;
@@ -429,9 +420,11 @@ __device__ __forceinline__ float4 up_to(float4 v, int n) {
   return make_float4(n >= 0 ? v.x : 0.f, n >= 1 ? v.y : 0.f, n >= 2 ? v.z : 0.f, n >= 3 ? v.w : 0.f);
 }
 
+// (Two blocks an SM said outright, which is what the ring leaves room for at key size 64: the registers of a chunk's operands
+// stay in flight; left to itself the compiler keeps to 72 and the walk takes 82 us instead of 63.)
 template <int D>
-__global__ void __launch_bounds__(CHUNK_THREADS)
-delta_chunk_kernel(const float* __restrict__ chunks, float* __restrict__ out, long out_stride, float* __restrict__ state,
+__global__ void __launch_bounds__(CHUNK_THREADS, 2)
+delta_chunk_kernel(long_seq::Head* list, const float* __restrict__ chunks, float* __restrict__ out, long out_stride, float* __restrict__ state,
                    long state_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_heads,
                    int d, int dv, int DVP) {
   using L = ChunkWalk<D>;
@@ -439,132 +432,130 @@ delta_chunk_kernel(const float* __restrict__ chunks, float* __restrict__ out, lo
   extern __shared__ __align__(16) float smem[];
   float* const s_t = smem + CHUNK_STAGES * L::BUF;   // the state, a column a row: [COLS][SW]
   float* const u_t = s_t + CHUNK_COLS * L::SW;       // U, a column a row: [COLS][SK]
-  const int b = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
-  int n;
-  if (!chunked_sequence(seq_slot, seq_start, b, n)) return;
-  int first = 0;  // the sequence's first chunk
-  for (int i = 0; i < b; ++i) {
-    int m;
-    if (chunked_sequence(seq_slot, seq_start, i, m)) first += (m + CHUNK - 1) / CHUNK;
-  }
-  const int start = seq_start[b], n_chunks = (n + CHUNK - 1) / CHUNK;
-  const int col0 = blockIdx.x * CHUNK_COLS;
-  const long REC = chunk_floats(D, DVP);
-
-  auto issue = [&](int c) {
-    const float* src = chunks + ((size_t)(first + c) * n_heads + h) * REC;
-    float* buf = smem + c % CHUNK_STAGES * L::BUF;
-    for (int i = tid; i < 2 * CHUNK * (D / 4); i += CHUNK_THREADS)  // W and c Q
-      delta_copy16(buf + i / (D / 4) * L::SW + i % (D / 4) * 4, src + i * 4, true);
-    for (int i = tid; i < (D + CHUNK) * (CHUNK / 4); i += CHUNK_THREADS)  // (D[C] o K)^T and D o Q K^T
-      delta_copy16(buf + L::K + i / (CHUNK / 4) * L::SK + i % (CHUNK / 4) * 4, src + 64 * D + i * 4, true);
-    if (tid < CHUNK * CHUNK_COLS / 4) {
-      const int r = tid / (CHUNK_COLS / 4), w = tid % (CHUNK_COLS / 4) * 4;
-      const bool ok = col0 + w < DVP;
-      delta_copy16(buf + L::V + r * CHUNK_COLS + w, src + 96 * D + CHUNK * CHUNK + r * DVP + (ok ? col0 + w : 0), ok);
-    }
-    if (tid == 64) delta_copy16(buf + L::END, src + 96 * D + CHUNK * CHUNK + CHUNK * DVP, true);
-  };
-  // a thread: row r of the chunk (or rows r + 32 i of the state) against two columns
+  const int tid = threadIdx.x;
   const int r = tid >> 2, c0 = (tid & 3) * 2;
-  float* const st = state + (size_t)seq_slot[b] * state_stride + ((size_t)h * dv + col0) * d;
-  // An infinity or NaN in U reaches the tokens before its own through the zeros of D o Q K^T (0 * inf): where an output is
-  // not finite, the block walks once more with U cut off behind each token (CAUSAL; in the first walk the cuts,
-  // or a test in every chunk, cost 5 to 12 % of the time).  The state is stored at the walk's end, so that both start alike.
-  auto walk = [&](auto causal) {
-    constexpr bool CAUSAL = decltype(causal)::value;
-#pragma unroll
-    for (int c = 0; c < CHUNK_STAGES - 1; ++c) {
-      if (c < n_chunks) issue(c);
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    float s[ND][2];
-#pragma unroll
-    for (int i = 0; i < ND; ++i)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int row = r + 32 * i, col = c0 + e;
-        s[i][e] = (row < d && col0 + col < dv) ? st[(size_t)col * d + row] : 0.f;
-        s_t[col * L::SW + row] = s[i][e];
+  const int columns = (dv + CHUNK_COLS - 1) / CHUNK_COLS;
+  const long REC = chunk_floats(D, DVP);
+  for (long_seq::Items items(list, n_heads * columns); items.more(); items.draw()) {
+    const auto sequence = items.sequence();
+    const int h = items.part() / columns, col0 = items.part() % columns * CHUNK_COLS;
+    const int n = sequence.tokens, first = sequence.first_chunk, start = seq_start[sequence.seq];
+    const int n_chunks = (n + CHUNK - 1) / CHUNK;
+
+    auto issue = [&](int c) {
+      const float* src = chunks + ((size_t)(first + c) * n_heads + h) * REC;
+      float* buf = smem + c % CHUNK_STAGES * L::BUF;
+      for (int i = tid; i < 2 * CHUNK * (D / 4); i += CHUNK_THREADS)  // W and c Q
+        delta_copy16(buf + i / (D / 4) * L::SW + i % (D / 4) * 4, src + i * 4, true);
+      for (int i = tid; i < (D + CHUNK) * (CHUNK / 4); i += CHUNK_THREADS)  // (D[C] o K)^T and D o Q K^T
+        delta_copy16(buf + L::K + i / (CHUNK / 4) * L::SK + i % (CHUNK / 4) * 4, src + 64 * D + i * 4, true);
+      if (tid < CHUNK * CHUNK_COLS / 4) {
+        const int r = tid / (CHUNK_COLS / 4), w = tid % (CHUNK_COLS / 4) * 4;
+        const bool ok = col0 + w < DVP;
+        delta_copy16(buf + L::V + r * CHUNK_COLS + w, src + 96 * D + CHUNK * CHUNK + r * DVP + (ok ? col0 + w : 0), ok);
       }
-    float finite = 0.f;
-    for (int c = 0; c < n_chunks; ++c) {
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(CHUNK_STAGES - 2) : "memory");
-      __syncthreads();  // the chunk has landed, and the state of the chunk before stands in shared memory
-      if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-      const float* buf = smem + c % CHUNK_STAGES * L::BUF;
-      float w0 = 0.f, w1 = 0.f, q0 = 0.f, q1 = 0.f;
+      if (tid == 64) delta_copy16(buf + L::END, src + 96 * D + CHUNK * CHUNK + CHUNK * DVP, true);
+    };
+    // a thread: row r of the chunk (or rows r + 32 i of the state) against two columns
+    float* const st = state + (size_t)seq_slot[sequence.seq] * state_stride + ((size_t)h * dv + col0) * d;
+    // An infinity or NaN in U reaches the tokens before its own through the zeros of D o Q K^T (0 * inf): where an output is
+    // not finite, the block walks once more with U cut off behind each token (CAUSAL; in the first walk the cuts,
+    // or a test in every chunk, cost 5 to 12 % of the time).  The state is stored at the walk's end, so that both start alike.
+    auto walk = [&](auto causal) {
+      constexpr bool CAUSAL = decltype(causal)::value;
 #pragma unroll
-      for (int k0 = 0; k0 < D; k0 += CHUNK_RUN) {
-        float rw0 = 0.f, rw1 = 0.f, rq0 = 0.f, rq1 = 0.f;
+      for (int c = 0; c < CHUNK_STAGES - 1; ++c) {
+        if (c < n_chunks) issue(c);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+      }
+      float s[ND][2];
 #pragma unroll
-        for (int k = k0; k < k0 + CHUNK_RUN; k += 4) {
-          const float4 w = *reinterpret_cast<const float4*>(buf + L::W + r * L::SW + k);
-          const float4 q = *reinterpret_cast<const float4*>(buf + L::Q + r * L::SW + k);
-          const float4 a = *reinterpret_cast<const float4*>(s_t + c0 * L::SW + k);
-          const float4 e = *reinterpret_cast<const float4*>(s_t + (c0 + 1) * L::SW + k);
-          rw0 = dot4(w, a, rw0);
-          rw1 = dot4(w, e, rw1);
-          rq0 = dot4(q, a, rq0);
-          rq1 = dot4(q, e, rq1);
+      for (int i = 0; i < ND; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int row = r + 32 * i, col = c0 + e;
+          s[i][e] = (row < d && col0 + col < dv) ? st[(size_t)col * d + row] : 0.f;
+          s_t[col * L::SW + row] = s[i][e];
         }
-        w0 += rw0;
-        w1 += rw1;
-        q0 += rq0;
-        q1 += rq1;
-      }
-      const float2 v = *reinterpret_cast<const float2*>(buf + L::V + r * CHUNK_COLS + c0);
-      u_t[c0 * L::SK + r] = v.x - w0;
-      u_t[(c0 + 1) * L::SK + r] = v.y - w1;
-      __syncthreads();
-      const float gc = buf[L::END];
+      float finite = 0.f;
+      for (int c = 0; c < n_chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(CHUNK_STAGES - 2) : "memory");
+        __syncthreads();  // the chunk has landed, and the state of the chunk before stands in shared memory
+        if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const float* buf = smem + c % CHUNK_STAGES * L::BUF;
+        float w0 = 0.f, w1 = 0.f, q0 = 0.f, q1 = 0.f;
 #pragma unroll
-      for (int i = 0; i < ND; ++i) {
-        s[i][0] *= gc;
-        s[i][1] *= gc;
-      }
-      float m0 = 0.f, m1 = 0.f;
+        for (int k0 = 0; k0 < D; k0 += CHUNK_RUN) {
+          float rw0 = 0.f, rw1 = 0.f, rq0 = 0.f, rq1 = 0.f;
 #pragma unroll
-      for (int k = 0; k < CHUNK; k += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(u_t + c0 * L::SK + k);
-        const float4 e = *reinterpret_cast<const float4*>(u_t + (c0 + 1) * L::SK + k);
-        const float4 m = *reinterpret_cast<const float4*>(buf + L::A + r * L::SK + k);
-        m0 = dot4(m, CAUSAL ? up_to(a, r - k) : a, m0);
-        m1 = dot4(m, CAUSAL ? up_to(e, r - k) : e, m1);
+          for (int k = k0; k < k0 + CHUNK_RUN; k += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(buf + L::W + r * L::SW + k);
+            const float4 q = *reinterpret_cast<const float4*>(buf + L::Q + r * L::SW + k);
+            const float4 a = *reinterpret_cast<const float4*>(s_t + c0 * L::SW + k);
+            const float4 e = *reinterpret_cast<const float4*>(s_t + (c0 + 1) * L::SW + k);
+            rw0 = dot4(w, a, rw0);
+            rw1 = dot4(w, e, rw1);
+            rq0 = dot4(q, a, rq0);
+            rq1 = dot4(q, e, rq1);
+          }
+          w0 += rw0;
+          w1 += rw1;
+          q0 += rq0;
+          q1 += rq1;
+        }
+        const float2 v = *reinterpret_cast<const float2*>(buf + L::V + r * CHUNK_COLS + c0);
+        u_t[c0 * L::SK + r] = v.x - w0;
+        u_t[(c0 + 1) * L::SK + r] = v.y - w1;
+        __syncthreads();
+        const float gc = buf[L::END];
 #pragma unroll
         for (int i = 0; i < ND; ++i) {
-          const float4 kd = *reinterpret_cast<const float4*>(buf + L::K + (r + 32 * i) * L::SK + k);
-          s[i][0] = dot4(kd, a, s[i][0]);
-          s[i][1] = dot4(kd, e, s[i][1]);
+          s[i][0] *= gc;
+          s[i][1] *= gc;
+        }
+        float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+        for (int k = 0; k < CHUNK; k += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(u_t + c0 * L::SK + k);
+          const float4 e = *reinterpret_cast<const float4*>(u_t + (c0 + 1) * L::SK + k);
+          const float4 m = *reinterpret_cast<const float4*>(buf + L::A + r * L::SK + k);
+          m0 = dot4(m, CAUSAL ? up_to(a, r - k) : a, m0);
+          m1 = dot4(m, CAUSAL ? up_to(e, r - k) : e, m1);
+#pragma unroll
+          for (int i = 0; i < ND; ++i) {
+            const float4 kd = *reinterpret_cast<const float4*>(buf + L::K + (r + 32 * i) * L::SK + k);
+            s[i][0] = dot4(kd, a, s[i][0]);
+            s[i][1] = dot4(kd, e, s[i][1]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+          s_t[c0 * L::SW + r + 32 * i] = s[i][0];
+          s_t[(c0 + 1) * L::SW + r + 32 * i] = s[i][1];
+        }
+        q0 += m0;
+        q1 += m1;
+        if (!CAUSAL) finite = fmaf(0.f, q0, fmaf(0.f, q1, finite));
+        if (c * CHUNK + r < n) {
+          float* o = out + (size_t)(start + c * CHUNK + r) * out_stride + h * dv + col0 + c0;
+          if (col0 + c0 < dv) o[0] = q0;
+          if (col0 + c0 + 1 < dv) o[1] = q1;
         }
       }
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      if (!CAUSAL && __syncthreads_or(finite != 0.f)) return false;
 #pragma unroll
-      for (int i = 0; i < ND; ++i) {
-        s_t[c0 * L::SW + r + 32 * i] = s[i][0];
-        s_t[(c0 + 1) * L::SW + r + 32 * i] = s[i][1];
-      }
-      q0 += m0;
-      q1 += m1;
-      if (!CAUSAL) finite = fmaf(0.f, q0, fmaf(0.f, q1, finite));
-      if (c * CHUNK + r < n) {
-        float* o = out + (size_t)(start + c * CHUNK + r) * out_stride + h * dv + col0 + c0;
-        if (col0 + c0 < dv) o[0] = q0;
-        if (col0 + c0 + 1 < dv) o[1] = q1;
-      }
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    if (!CAUSAL && __syncthreads_or(finite != 0.f)) return false;
+      for (int i = 0; i < ND; ++i)
 #pragma unroll
-    for (int i = 0; i < ND; ++i)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int row = r + 32 * i, col = c0 + e;
-        if (row < d && col0 + col < dv) st[(size_t)col * d + row] = s[i][e];
-      }
-    return true;
-  };
-  if (!walk(std::false_type())) walk(std::true_type());
+        for (int e = 0; e < 2; ++e) {
+          const int row = r + 32 * i, col = c0 + e;
+          if (row < d && col0 + col < dv) st[(size_t)col * d + row] = s[i][e];
+        }
+      return true;
+    };
+    if (!walk(std::false_type())) walk(std::true_type());
+  }
 }
 
 // rows of the prepared arrays for key size d (the row count of the kernel that takes it)
@@ -600,18 +591,14 @@ static int launch_scan(cudaStream_t stream, const float* qn, const float* kn, co
 static bool chunks_apply(int longest, int d, int dtype, int head_decay) {
   return dtype == FG_BF16 && head_decay && d > 32 && d <= 128 && longest >= CHUNK_MIN;
 }
-// most chunks of a step's sequences that have CHUNK_MIN tokens or more
-static long most_chunks(int n_tokens, int n_seqs) {
-  const int long_ones = n_tokens / CHUNK_MIN;
-  return n_tokens / CHUNK + (n_seqs < long_ones ? n_seqs : long_ones);
-}
-
 // floats of the scratch that fg_delta_scan needs for `n_tokens` tokens
 extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int longest, int n_seqs, int n_heads, int n_kv_heads, int d, int dv,
                                              int dtype, int head_decay) {
   const long DP = delta_rows(d), DVP = (dv + 3) / 4 * 4;
   const long rows = (long)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
-  return rows + (chunks_apply(longest, d, dtype, head_decay) ? most_chunks(n_tokens, n_seqs) * n_heads * chunk_floats((int)DP, (int)DVP) : 0);
+  if (!chunks_apply(longest, d, dtype, head_decay)) return rows;
+  return rows + long_seq::list_floats(n_tokens, n_seqs, CHUNK_MIN) +
+         long_seq::most_chunks(n_tokens, n_seqs, CHUNK_MIN, CHUNK) * n_heads * chunk_floats((int)DP, (int)DVP);
 }
 
 // qkv: float32 [T, q (kv heads x d) | k (kv heads x d) | v (heads x dv)], the convolutions' outputs.
@@ -650,18 +637,22 @@ extern "C" int fg_delta_scan(const float* qkv, long qkv_stride, const void* a, l
   int most = 0x7fffffff;  // tokens of the longest sequence that the token kernel takes
   if (chunks_apply(longest, d, dtype, head_decay)) {
     most = CHUNK_MIN - 1;
-    float* chunks = scratch + (size_t)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
-    const dim3 wy_grid((unsigned)most_chunks(n_tokens, n_seqs), n_heads), grid((dv + CHUNK_COLS - 1) / CHUNK_COLS, n_heads, n_seqs);
+    float* const behind = scratch + (size_t)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
+    long_seq::Head* const list = reinterpret_cast<long_seq::Head*>(behind);
+    float* const chunks = behind + long_seq::list_floats(n_tokens, n_seqs, CHUNK_MIN);
+    const dim3 wy_grid((unsigned)long_seq::most_chunks(n_tokens, n_seqs, CHUNK_MIN, CHUNK), n_heads);
+    const long items = long_seq::most_sequences(n_tokens, n_seqs, CHUNK_MIN) * n_heads * ((dv + CHUNK_COLS - 1) / CHUNK_COLS);
 #define CHUNKS(D)                                                                                                       \
   do {                                                                                                                  \
-    delta_wy_kernel<D><<<wy_grid, CHUNK_THREADS, 0, stream>>>(qn, kn, rec, vp, chunks, seq_slot, seq_start, n_seqs, n_heads, \
-                                                              n_kv_heads, DVP);                                         \
+    delta_wy_kernel<D><<<wy_grid, CHUNK_THREADS, 0, stream>>>(qn, kn, rec, vp, list, chunks, seq_slot, seq_start, n_seqs, \
+                                                              n_heads, n_kv_heads, DVP);                                \
     FG_CHECK_LAUNCH("fg_delta_scan (chunks)");                                                                          \
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
                                          (int)ChunkWalk<D>::SMEM);                                                      \
     FG_CHECK_ARG(e == cudaSuccess, "fg_delta_scan: shared memory: %s", cudaGetErrorString(e));                          \
-    delta_chunk_kernel<D><<<grid, CHUNK_THREADS, ChunkWalk<D>::SMEM, stream>>>(                                         \
-        chunks, out, out_stride, state, state_stride, seq_slot, seq_start, n_heads, d, dv, DVP);                        \
+    const long resident = (long)fg_sm_count() * fg_blocks_per_sm(CHUNK_THREADS, ChunkWalk<D>::SMEM);                    \
+    delta_chunk_kernel<D><<<(unsigned)(items < resident ? items : resident), CHUNK_THREADS, ChunkWalk<D>::SMEM, stream>>>( \
+        list, chunks, out, out_stride, state, state_stride, seq_slot, seq_start, n_heads, d, dv, DVP);                  \
     FG_CHECK_LAUNCH("fg_delta_scan (walk)");                                                                            \
   } while (0)
     if (DP == 64) CHUNKS(64);

@@ -19,6 +19,7 @@
 // The recurrence runs token by token, so its sums do not depend on how a prompt was cut or
 // what else is in the batch.
 #include "common.cuh"
+#include "long_sequences.cuh"
 
 // ---- convolution + SiLU ---------------------------------------------------------------------
 // out[t, c] = silu(bias[c] + sum_k w[c, k] * in[t - (taps-1-k), c]); inputs before the step's
@@ -478,7 +479,7 @@ ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* _
 //     Y = e (C S0) + M X + D_skip X,  M[i][j] = (C_i . B_j) D[i][j] dt_j  (j <= i)
 //     S <- e_32 S0 + B^T (w X)
 //
-// 2,048 tokens of 64 heads, 128 x 64 states: 420 -> 197 us and 15 of preparing (the multiply-adds alone take 75; what
+// 2,048 tokens of 64 heads, 128 x 64 states: 420 -> 202 us and 17 of preparing (the multiply-adds alone take 75; what
 // bounds the walk is shared memory: a 16-byte read a lane takes its 4 cycles whoever shares the address, and 4 x 4
 // numbers a thread want two such reads for 16 multiply-adds).
 //
@@ -503,10 +504,6 @@ struct Whole {
 };
 constexpr int SC_REC = SC_TOKENS * SC_TOKENS + 2 * SC_TOKENS;  // floats of a (chunk, head): M, e, w
 
-__device__ __forceinline__ bool sc_takes(const int* seq_slot, const int* seq_start, int b, int& n) {
-  n = seq_start[b + 1] - seq_start[b];
-  return seq_slot[b] >= 0 && n >= SC_MIN;
-}
 __device__ __forceinline__ void cp_async_16(float* dst, const float* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
                "r"(ok ? 16 : 0)
@@ -516,23 +513,19 @@ __device__ __forceinline__ void cp_async_16(float* dst, const float* src, bool o
 template <typename T, int N>
 __global__ void __launch_bounds__(SC_THREADS)
 ssm_chunk_prepare_kernel(const float* __restrict__ xbc, long xbc_stride, const T* __restrict__ dt_raw, long dt_stride,
-                         const float* __restrict__ dt_bias, const float* __restrict__ a_log, float* __restrict__ chunks,
-                         const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs, int heads,
+                         const float* __restrict__ dt_bias, const float* __restrict__ a_log, long_seq::Head* list,
+                         float* __restrict__ chunks, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs, int heads,
                          int groups, int P) {
   __shared__ __align__(16) float bs[SC_TOKENS][N + 4];
   __shared__ __align__(16) float cs[SC_TOKENS][N + 4];
   __shared__ double gram[SC_TOKENS][SC_TOKENS + 1];
   __shared__ float decs[SC_THREADS / 32][SC_TOKENS];
   const int g = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int c = blockIdx.x, b = 0, n = 0;
-  for (; b < n_seqs; ++b) {
-    if (!sc_takes(seq_slot, seq_start, b, n)) continue;
-    const int nc = (n + SC_TOKENS - 1) / SC_TOKENS;
-    if (c < nc) break;
-    c -= nc;
-  }
-  if (b == n_seqs) return;
-  const int t0 = seq_start[b] + c * SC_TOKENS, nt = min(SC_TOKENS, n - c * SC_TOKENS), inner = heads * P;
+  const auto found = long_seq::find_chunk<SC_MIN, SC_TOKENS, SC_THREADS>(seq_slot, seq_start, n_seqs, blockIdx.x,
+                                                                         blockIdx.x + g == 0 ? list : nullptr);
+  if (found.seq < 0) return;
+  const int c = blockIdx.x - found.first_chunk;
+  const int t0 = seq_start[found.seq] + c * SC_TOKENS, nt = min(SC_TOKENS, found.tokens - c * SC_TOKENS), inner = heads * P;
   for (int i = tid; i < SC_TOKENS * (N / 4); i += SC_THREADS) {
     const int t = i / (N / 4), w = i % (N / 4) * 4;
     float4 bv = make_float4(0.f, 0.f, 0.f, 0.f), cv = bv;
@@ -622,8 +615,8 @@ struct ScanWalk {
 };
 
 template <int N>
-__global__ void __launch_bounds__(SC_THREADS)
-ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, const float* __restrict__ chunks,
+__global__ void __launch_bounds__(SC_THREADS, 1)
+ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, long_seq::Head* list, const float* __restrict__ chunks,
                  const float* __restrict__ d_skip, float* __restrict__ y, long y_stride, float* __restrict__ state,
                  long state_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int heads,
                  int groups, int P) {
@@ -631,181 +624,178 @@ ssm_chunk_kernel(const float* __restrict__ xbc, long xbc_stride, const float* __
   constexpr int NROWS = N / 32;  // rows of the state a thread, side by side
   extern __shared__ __align__(16) float smem[];
   float *const s_s = smem + L::S, *const xw_s = smem + L::XW, *const part = smem + L::PART;
-  const int b = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * SC_COLS, tid = threadIdx.x;
-  int n;
-  if (!sc_takes(seq_slot, seq_start, b, n)) return;
-  int first = 0;  // the sequence's first chunk
-  for (int i = 0; i < b; ++i) {
-    int m;
-    if (sc_takes(seq_slot, seq_start, i, m)) first += (m + SC_TOKENS - 1) / SC_TOKENS;
-  }
-  const int start = seq_start[b], n_chunks = (n + SC_TOKENS - 1) / SC_TOKENS;
-  const int g = h / (heads / groups), inner = heads * P;
-  const float dsk = d_skip[h];
+  const int tid = threadIdx.x, pb = tid & 7, nb = tid >> 3;
+  const int columns = (P + SC_COLS - 1) / SC_COLS, inner = heads * P;
+  for (long_seq::Items items(list, heads * columns); items.more(); items.draw()) {
+    const auto sequence = items.sequence();
+    const int h = items.part() / columns, p0 = items.part() % columns * SC_COLS, g = h / (heads / groups);
+    const int n = sequence.tokens, first = sequence.first_chunk, start = seq_start[sequence.seq];
+    const int n_chunks = (n + SC_TOKENS - 1) / SC_TOKENS;
+    const float dsk = d_skip[h];
 
-  auto issue = [&](int c) {
-    float* buf = smem + c % SC_STAGES * L::BUF;
-    const int t0 = start + c * SC_TOKENS, nt = min(SC_TOKENS, n - c * SC_TOKENS);
-    for (int i = tid; i < SC_TOKENS * (N / 4); i += SC_THREADS) {
-      const int t = i / (N / 4), w = i % (N / 4) * 4;
-      const float* row = xbc + (size_t)(t < nt ? t0 + t : t0) * xbc_stride + inner + g * N + w;
-      cp_async_16(buf + L::B + t * N + w, row, t < nt);
-      cp_async_16(buf + L::C + t * L::SCN + w, row + groups * N, t < nt);
-    }
-    const float* rec = chunks + ((size_t)(first + c) * heads + h) * SC_REC;
-    {
-      const int t = tid / 8, w = tid % 8 * 4;  // 32 rows of 32 numbers: M and x
-      cp_async_16(buf + L::M + t * L::SM + w, rec + t * SC_TOKENS + w, true);
-      const bool ok = t < nt && p0 + w < P;
-      cp_async_16(buf + L::X + t * L::SP + w, ok ? xbc + (size_t)(t0 + t) * xbc_stride + h * P + p0 + w : xbc, ok);
-    }
-    if (tid < 2 * SC_TOKENS / 4) cp_async_16(buf + L::E + tid * 4, rec + SC_TOKENS * SC_TOKENS + tid * 4, true);
-  };
-  issue(0);
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
+    auto issue = [&](int c) {
+      float* buf = smem + c % SC_STAGES * L::BUF;
+      const int t0 = start + c * SC_TOKENS, nt = min(SC_TOKENS, n - c * SC_TOKENS);
+      for (int i = tid; i < SC_TOKENS * (N / 4); i += SC_THREADS) {
+        const int t = i / (N / 4), w = i % (N / 4) * 4;
+        const float* row = xbc + (size_t)(t < nt ? t0 + t : t0) * xbc_stride + inner + g * N + w;
+        cp_async_16(buf + L::B + t * N + w, row, t < nt);
+        cp_async_16(buf + L::C + t * L::SCN + w, row + groups * N, t < nt);
+      }
+      const float* rec = chunks + ((size_t)(first + c) * heads + h) * SC_REC;
+      {
+        const int t = tid / 8, w = tid % 8 * 4;  // 32 rows of 32 numbers: M and x
+        cp_async_16(buf + L::M + t * L::SM + w, rec + t * SC_TOKENS + w, true);
+        const bool ok = t < nt && p0 + w < P;
+        cp_async_16(buf + L::X + t * L::SP + w, ok ? xbc + (size_t)(t0 + t) * xbc_stride + h * P + p0 + w : xbc, ok);
+      }
+      if (tid < 2 * SC_TOKENS / 4) cp_async_16(buf + L::E + tid * 4, rec + SC_TOKENS * SC_TOKENS + tid * 4, true);
+    };
+    issue(0);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
 
-  // the state: rows NROWS nb + r, columns 4 pb .. + 3
-  const int pb = tid & 7, nb = tid >> 3;
-  float* const st = state + (size_t)seq_slot[b] * state_stride + (size_t)h * N * P;
-  float s[NROWS][4];
-#pragma unroll
-  for (int r = 0; r < NROWS; ++r)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int p = p0 + 4 * pb + e;
-      s[r][e] = p < P ? st[(size_t)p * N + NROWS * nb + r] : 0.f;
-    }
-  // the sums of C S0 and M X: group q takes a quarter of the state's rows and of the tokens, a thread 4 x 4 places
-  const int q = tid >> 6, ib = (tid & 63) >> 3;
-  for (int c = 0; c < n_chunks; ++c) {
-    const float* buf = smem + c % SC_STAGES * L::BUF;
+    // the state: rows NROWS nb + r, columns 4 pb .. + 3
+    float* const st = state + (size_t)seq_slot[sequence.seq] * state_stride + (size_t)h * N * P;
+    float s[NROWS][4];
 #pragma unroll
     for (int r = 0; r < NROWS; ++r)
-      *reinterpret_cast<float4*>(s_s + (NROWS * nb + r) * L::SP + 4 * pb) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();  // the chunk has landed, the state stands in shared memory, the buffer of the chunk before is free
-    if (c + 1 < n_chunks) issue(c + 1);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    bool finite;
-    {  // w X for the state's update
-      const int t = tid / 8, w = tid % 8 * 4;
-      const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
-      finite = isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(x.w);
-      const float wt = buf[L::W + t];
-      *reinterpret_cast<float4*>(xw_s + t * L::SP + w) = make_float4(x.x * wt, x.y * wt, x.z * wt, x.w * wt);
-    }
-    float acc[4][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+      for (int e = 0; e < 4; ++e) {
+        const int p = p0 + 4 * pb + e;
+        s[r][e] = p < P ? st[(size_t)p * N + NROWS * nb + r] : 0.f;
+      }
+    // the sums of C S0 and M X: group q takes a quarter of the state's rows and of the tokens, a thread 4 x 4 places
+    const int q = tid >> 6, ib = (tid & 63) >> 3;
+    for (int c = 0; c < n_chunks; ++c) {
+      const float* buf = smem + c % SC_STAGES * L::BUF;
 #pragma unroll
-      for (int f = 0; f < 4; ++f) acc[e][f] = 0.f;
-    auto products = [&](const float* left, int left_stride, const float* right, int from, auto count, auto run_length) {
-      constexpr int COUNT = decltype(count)::value, RUN = decltype(run_length)::value;
+      for (int r = 0; r < NROWS; ++r)
+        *reinterpret_cast<float4*>(s_s + (NROWS * nb + r) * L::SP + 4 * pb) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      __syncthreads();  // the chunk has landed, the state stands in shared memory, the buffer of the chunk before is free
+      if (c + 1 < n_chunks) issue(c + 1);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      bool finite;
+      {  // w X for the state's update
+        const int t = tid / 8, w = tid % 8 * 4;
+        const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
+        finite = isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(x.w);
+        const float wt = buf[L::W + t];
+        *reinterpret_cast<float4*>(xw_s + t * L::SP + w) = make_float4(x.x * wt, x.y * wt, x.z * wt, x.w * wt);
+      }
+      float acc[4][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) acc[e][f] = 0.f;
+      auto products = [&](const float* left, int left_stride, const float* right, int from, auto count, auto run_length) {
+        constexpr int COUNT = decltype(count)::value, RUN = decltype(run_length)::value;
 #pragma unroll 1
-      for (int k0 = from; k0 < from + COUNT; k0 += RUN) {
-        float run[4][4];
+        for (int k0 = from; k0 < from + COUNT; k0 += RUN) {
+          float run[4][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+          for (int e = 0; e < 4; ++e)
 #pragma unroll
-          for (int f = 0; f < 4; ++f) run[e][f] = 0.f;
+            for (int f = 0; f < 4; ++f) run[e][f] = 0.f;
 #pragma unroll 2
-        for (int k = k0; k < k0 + RUN; k += 4) {
-          float4 a[4], v[4];
+          for (int k = k0; k < k0 + RUN; k += 4) {
+            float4 a[4], v[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            a[e] = *reinterpret_cast<const float4*>(left + (ib + 8 * e) * left_stride + k);
-            v[e] = *reinterpret_cast<const float4*>(right + (k + e) * L::SP + 4 * pb);
-          }
+            for (int e = 0; e < 4; ++e) {
+              a[e] = *reinterpret_cast<const float4*>(left + (ib + 8 * e) * left_stride + k);
+              v[e] = *reinterpret_cast<const float4*>(right + (k + e) * L::SP + 4 * pb);
+            }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float ae[4] = {a[e].x, a[e].y, a[e].z, a[e].w};
+            for (int e = 0; e < 4; ++e) {
+              const float ae[4] = {a[e].x, a[e].y, a[e].z, a[e].w};
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-              run[e][0] = fmaf(ae[f], v[f].x, run[e][0]);
-              run[e][1] = fmaf(ae[f], v[f].y, run[e][1]);
-              run[e][2] = fmaf(ae[f], v[f].z, run[e][2]);
-              run[e][3] = fmaf(ae[f], v[f].w, run[e][3]);
+              for (int f = 0; f < 4; ++f) {
+                run[e][0] = fmaf(ae[f], v[f].x, run[e][0]);
+                run[e][1] = fmaf(ae[f], v[f].y, run[e][1]);
+                run[e][2] = fmaf(ae[f], v[f].z, run[e][2]);
+                run[e][3] = fmaf(ae[f], v[f].w, run[e][3]);
+              }
             }
           }
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int f = 0; f < 4; ++f) acc[e][f] += run[e][f];
         }
+      };
+      products(buf + L::C, L::SCN, s_s, q * (N / 4), Whole<N / 4>(), Whole<SC_RUN>());
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+      for (int e = 0; e < 4; ++e) {
+        const float ei = buf[L::E + ib + 8 * e];
 #pragma unroll
-          for (int f = 0; f < 4; ++f) acc[e][f] += run[e][f];
+        for (int f = 0; f < 4; ++f) acc[e][f] *= ei;
       }
-    };
-    products(buf + L::C, L::SCN, s_s, q * (N / 4), Whole<N / 4>(), Whole<SC_RUN>());
+      products(buf + L::M, L::SM, buf + L::X, q * (SC_TOKENS / 4), Whole<SC_TOKENS / 4>(), Whole<SC_TOKENS / 4>());
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float ei = buf[L::E + ib + 8 * e];
+      for (int e = 0; e < 4; ++e)
+        *reinterpret_cast<float4*>(part + (q * SC_TOKENS + ib + 8 * e) * L::SPART + 4 * pb) =
+            make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
+      // (an infinity or NaN in X would reach the tokens before its own through M's zeros)
+      const bool causal = __syncthreads_or(!finite) != 0;
+      {  // a token's four columns a thread: the groups' sums in order
+        const int t = tid / 8, w = tid % 8 * 4;
+        const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
+        float4 v = *reinterpret_cast<const float4*>(part + t * L::SPART + w);
 #pragma unroll
-      for (int f = 0; f < 4; ++f) acc[e][f] *= ei;
+        for (int i = 1; i < L::GROUPS; ++i) {
+          const float4 u = *reinterpret_cast<const float4*>(part + (i * SC_TOKENS + t) * L::SPART + w);
+          v.x += u.x;
+          v.y += u.y;
+          v.z += u.z;
+          v.w += u.w;
+        }
+        if (causal) {  // the token's sums once more, over the tokens up to it alone
+          v = make_float4(0.f, 0.f, 0.f, 0.f);
+          auto add = [&](float a, const float* row) {
+            const float4 u = *reinterpret_cast<const float4*>(row + w);
+            v = make_float4(fmaf(a, u.x, v.x), fmaf(a, u.y, v.y), fmaf(a, u.z, v.z), fmaf(a, u.w, v.w));
+          };
+          for (int k = 0; k < N; ++k) add(buf[L::C + t * L::SCN + k], s_s + k * L::SP);
+          const float et = buf[L::E + t];
+          v = make_float4(v.x * et, v.y * et, v.z * et, v.w * et);
+          for (int k = 0; k <= t; ++k) add(buf[L::M + t * L::SM + k], buf + L::X + k * L::SP);
+          __syncthreads();  // the state in shared memory has been read
+        }
+        if (c * SC_TOKENS + t < n && p0 + w < P)
+          *reinterpret_cast<float4*>(y + (size_t)(start + c * SC_TOKENS + t) * y_stride + h * P + p0 + w) =
+              make_float4(fmaf(dsk, x.x, v.x), fmaf(dsk, x.y, v.y), fmaf(dsk, x.z, v.z), fmaf(dsk, x.w, v.w));
+      }
+      const float whole = buf[L::E + SC_TOKENS - 1];
+#pragma unroll
+      for (int r = 0; r < NROWS; ++r)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[r][e] *= whole;
+#pragma unroll 8
+      for (int t = 0; t < SC_TOKENS; ++t) {
+        const float4 x = *reinterpret_cast<const float4*>(xw_s + t * L::SP + 4 * pb);
+        __align__(16) float bt[NROWS];
+        if (NROWS == 4) *reinterpret_cast<float4*>(bt) = *reinterpret_cast<const float4*>(buf + L::B + t * N + 4 * nb);
+        else *reinterpret_cast<float2*>(bt) = *reinterpret_cast<const float2*>(buf + L::B + t * N + 2 * nb);
+#pragma unroll
+        for (int r = 0; r < NROWS; ++r) {
+          const float bv = bt[r];
+          s[r][0] = fmaf(bv, x.x, s[r][0]);
+          s[r][1] = fmaf(bv, x.y, s[r][1]);
+          s[r][2] = fmaf(bv, x.z, s[r][2]);
+          s[r][3] = fmaf(bv, x.w, s[r][3]);
+        }
+      }
+      // (the next chunk's state goes to shared memory at once: its readers are through since the barrier above;
+      // w X is written behind the next barrier)
     }
-    products(buf + L::M, L::SM, buf + L::X, q * (SC_TOKENS / 4), Whole<SC_TOKENS / 4>(), Whole<SC_TOKENS / 4>());
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      *reinterpret_cast<float4*>(part + (q * SC_TOKENS + ib + 8 * e) * L::SPART + 4 * pb) =
-          make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
-    // (an infinity or NaN in X would reach the tokens before its own through M's zeros)
-    const bool causal = __syncthreads_or(!finite) != 0;
-    {  // a token's four columns a thread: the groups' sums in order
-      const int t = tid / 8, w = tid % 8 * 4;
-      const float4 x = *reinterpret_cast<const float4*>(buf + L::X + t * L::SP + w);
-      float4 v = *reinterpret_cast<const float4*>(part + t * L::SPART + w);
-#pragma unroll
-      for (int i = 1; i < L::GROUPS; ++i) {
-        const float4 u = *reinterpret_cast<const float4*>(part + (i * SC_TOKENS + t) * L::SPART + w);
-        v.x += u.x;
-        v.y += u.y;
-        v.z += u.z;
-        v.w += u.w;
-      }
-      if (causal) {  // the token's sums once more, over the tokens up to it alone
-        v = make_float4(0.f, 0.f, 0.f, 0.f);
-        auto add = [&](float a, const float* row) {
-          const float4 u = *reinterpret_cast<const float4*>(row + w);
-          v = make_float4(fmaf(a, u.x, v.x), fmaf(a, u.y, v.y), fmaf(a, u.z, v.z), fmaf(a, u.w, v.w));
-        };
-        for (int k = 0; k < N; ++k) add(buf[L::C + t * L::SCN + k], s_s + k * L::SP);
-        const float et = buf[L::E + t];
-        v = make_float4(v.x * et, v.y * et, v.z * et, v.w * et);
-        for (int k = 0; k <= t; ++k) add(buf[L::M + t * L::SM + k], buf + L::X + k * L::SP);
-        __syncthreads();  // the state in shared memory has been read
-      }
-      if (c * SC_TOKENS + t < n && p0 + w < P)
-        *reinterpret_cast<float4*>(y + (size_t)(start + c * SC_TOKENS + t) * y_stride + h * P + p0 + w) =
-            make_float4(fmaf(dsk, x.x, v.x), fmaf(dsk, x.y, v.y), fmaf(dsk, x.z, v.z), fmaf(dsk, x.w, v.w));
-    }
-    const float whole = buf[L::E + SC_TOKENS - 1];
 #pragma unroll
     for (int r = 0; r < NROWS; ++r)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s[r][e] *= whole;
-#pragma unroll 8
-    for (int t = 0; t < SC_TOKENS; ++t) {
-      const float4 x = *reinterpret_cast<const float4*>(xw_s + t * L::SP + 4 * pb);
-      __align__(16) float bt[NROWS];
-      if (NROWS == 4) *reinterpret_cast<float4*>(bt) = *reinterpret_cast<const float4*>(buf + L::B + t * N + 4 * nb);
-      else *reinterpret_cast<float2*>(bt) = *reinterpret_cast<const float2*>(buf + L::B + t * N + 2 * nb);
-#pragma unroll
-      for (int r = 0; r < NROWS; ++r) {
-        const float bv = bt[r];
-        s[r][0] = fmaf(bv, x.x, s[r][0]);
-        s[r][1] = fmaf(bv, x.y, s[r][1]);
-        s[r][2] = fmaf(bv, x.z, s[r][2]);
-        s[r][3] = fmaf(bv, x.w, s[r][3]);
+      for (int e = 0; e < 4; ++e) {
+        const int p = p0 + 4 * pb + e;
+        if (p < P) st[(size_t)p * N + NROWS * nb + r] = s[r][e];
       }
-    }
-    // (the next chunk's state goes to shared memory at once: its readers are through since the barrier above;
-    // w X is written behind the next barrier)
   }
-#pragma unroll
-  for (int r = 0; r < NROWS; ++r)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int p = p0 + 4 * pb + e;
-      if (p < P) st[(size_t)p * N + NROWS * nb + r] = s[r][e];
-    }
 }
 
 // ---- gate, then RMS norm in equal parts ---------------------------------------------------------
@@ -978,17 +968,13 @@ extern "C" int fg_mamba2_conv(const void* proj, long proj_stride, long xbc_offse
 static bool sc_apply(int n_tokens, int n_state, int head_dim, int dtype) {
   return dtype == FG_BF16 && (n_state == 64 || n_state == 128) && head_dim % 4 == 0 && n_tokens >= SC_MIN;
 }
-// most chunks of a step's sequences that have SC_MIN tokens or more
-static long sc_most_chunks(int n_tokens, int n_seqs) {
-  const int long_ones = n_tokens / SC_MIN;
-  return n_tokens / SC_TOKENS + (n_seqs < long_ones ? n_seqs : long_ones);
-}
-
 // floats of the scratch that fg_mamba2_scan takes (0: none; without it every token goes through the token kernels, as
 // it does where no sequence of the step brings more than `longest` tokens and those are too few)
 extern "C" long fg_mamba2_scan_scratch_floats(int n_tokens, int longest, int n_seqs, int heads, int n_state, int head_dim,
                                               int dtype) {
-  return sc_apply(longest, n_state, head_dim, dtype) ? sc_most_chunks(n_tokens, n_seqs) * heads * SC_REC : 0;
+  return sc_apply(longest, n_state, head_dim, dtype)
+             ? long_seq::list_floats(n_tokens, n_seqs, SC_MIN) + long_seq::most_chunks(n_tokens, n_seqs, SC_MIN, SC_TOKENS) * heads * SC_REC
+             : 0;
 }
 
 template <typename T>
@@ -1003,16 +989,19 @@ static int launch_scan(const float* xbc, long xbc_stride, const T* dt_raw, long 
     int most = 0x7fffffff;  // tokens of the longest sequence that the token kernel takes
     if (scratch != nullptr) {
       most = SC_MIN - 1;
-      const dim3 prepare((unsigned)sc_most_chunks(n_tokens, n_seqs), groups), walk(n_seqs, heads, (P + SC_COLS - 1) / SC_COLS);
-#define CHUNKS(NN)                                                                                                   \
-  do {                                                                                                               \
-    ssm_chunk_prepare_kernel<T, NN><<<prepare, SC_THREADS, 0, stream>>>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias,  \
-                                                                        a_log, scratch, seq_slot, seq_start, n_seqs, \
-                                                                        heads, groups, P);                           \
-    cudaFuncSetAttribute(ssm_chunk_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ScanWalk<NN>::SMEM); \
-    ssm_chunk_kernel<NN><<<walk, SC_THREADS, ScanWalk<NN>::SMEM, stream>>>(xbc, xbc_stride, scratch, d_skip, y,       \
-                                                                           y_stride, state, state_stride, seq_slot,  \
-                                                                           seq_start, heads, groups, P);             \
+      long_seq::Head* const list = reinterpret_cast<long_seq::Head*>(scratch);
+      float* const chunks = scratch + long_seq::list_floats(n_tokens, n_seqs, SC_MIN);
+      const dim3 prepare((unsigned)long_seq::most_chunks(n_tokens, n_seqs, SC_MIN, SC_TOKENS), groups);
+      const long items = long_seq::most_sequences(n_tokens, n_seqs, SC_MIN) * heads * ((P + SC_COLS - 1) / SC_COLS);
+#define CHUNKS(NN)                                                                                                     \
+  do {                                                                                                                 \
+    ssm_chunk_prepare_kernel<T, NN><<<prepare, SC_THREADS, 0, stream>>>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias,    \
+                                                                        a_log, list, chunks, seq_slot, seq_start,      \
+                                                                        n_seqs, heads, groups, P);                     \
+    cudaFuncSetAttribute(ssm_chunk_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ScanWalk<NN>::SMEM);   \
+    const long resident = (long)fg_sm_count() * fg_blocks_per_sm(SC_THREADS, ScanWalk<NN>::SMEM);                      \
+    ssm_chunk_kernel<NN><<<(unsigned)(items < resident ? items : resident), SC_THREADS, ScanWalk<NN>::SMEM, stream>>>(  \
+        xbc, xbc_stride, list, chunks, d_skip, y, y_stride, state, state_stride, seq_slot, seq_start, heads, groups, P); \
   } while (0)
       if (N == 64) CHUNKS(64);
       else CHUNKS(128);

@@ -494,6 +494,45 @@ def test_delta_chunks_lose_no_precision(ops16, d):
     assert errors[0][0] <= 1.05 * errors[1][0] and errors[0][1] <= 1.05 * errors[1][1], errors
 
 
+@pytest.mark.parametrize("places,lengths", [(1, [130]), (300, [64]), (300, [63, 200, 0, 65, 1]), (300, [64 + i % 9 for i in range(90)])])
+def test_chunks_of_sequences_among_empty_places(ops16, places, lengths):
+    """A captured step has a place for every request: sequences behind one another or with empty places between
+    them, fewer and more (sequence, part) items than blocks, against each sequence by itself, bit for bit."""
+    heads, groups, n_state, p, kv, d, dv = 6, 2, 128, 40, 2, 64, 20
+    g = torch.Generator().manual_seed(places + len(lengths))
+    t = sum(lengths) + 3
+    slots = torch.randperm(len(lengths), generator=g).tolist()
+    ctx = _sequences(lengths, 3, slots)
+    at, step = [], max(1, places // len(lengths) - 1) if places > 1 else 1
+    slot_of, start = [-1] * max(places, len(lengths)), []
+    for i in range(len(slot_of)):
+        if i % step == 0 and len(at) < len(lengths):
+            slot_of[i] = slots[len(at)]
+            at.append(i)
+    for i in range(len(slot_of) + 1):  # a place without a sequence has no tokens
+        start.append(sum(n for n, place in zip(lengths, at) if place < i))
+    ctx.seq_slot, ctx.seq_start = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in (slot_of, start))
+    ctx.n_seqs = len(slot_of)
+    xbc, proj = _randn(g, t, heads * p + 2 * groups * n_state, scale=0.5), _randn(g, t, 2 * heads).to(torch.bfloat16)
+    qkv, vec = _randn(g, t, 2 * kv * d + heads * dv), _randn(g, heads, scale=0.5)
+    states = [_randn(g, len(lengths), heads * n_state * p), _randn(g, len(lengths), heads * d * dv)]
+
+    def run(ctx, rows, first, second):
+        return (ops16.mamba2_scan(xbc[rows], proj[rows], 0, vec, vec, vec, first, ctx, heads, groups, n_state, p),
+                ops16.delta_scan(qkv[rows], proj[rows, :heads], proj[rows, heads:], vec, vec, second, ctx, heads, kv, d, dv,
+                                 head_decay=True))
+
+    together, alone = [s.clone() for s in states], [s.clone() for s in states]
+    outs = run(ctx, slice(0, t), *together)
+    begin = 0
+    for n, slot in zip(lengths, slots):
+        if n:
+            one = run(_sequences([n], 0, [slot]), slice(begin, begin + n), *alone)
+            assert all(torch.equal(a[begin : begin + n], b) for a, b in zip(outs, one))
+        begin += n
+    assert all(torch.equal(a, b) for a, b in zip(together, alone))
+
+
 def test_decode_buckets_launch_no_chunks(ops16):
     """A captured step of 64 and more single tokens runs the token kernels alone."""
     from fastgen_b200.csrc.ops import Ops
