@@ -258,8 +258,13 @@ constexpr int CHUNK_THREADS = 128;
 constexpr int CHUNK_COLS = 8;    // columns of the state a block of the walk
 constexpr int CHUNK_STAGES = 3;  // chunks in its ring
 // Fewest tokens of a sequence that takes this way: where the two meet.  One sequence of 63 tokens 20.8 us above, of
-// 64 here 19.7, of 128 23.4 (16 heads of 64, prepared and formed).
+// 64 here 16.8 (16 heads of 64; 11.4 of them forming the chunks).
 constexpr int CHUNK_MIN = 64;
+
+// Chunks formed and walked at a time: a step of more goes in stretches, through the same room (at 32 heads of 128 a chunk
+// takes 2.2 MB, and 16,384 tokens of 256 requests would take 1.7 GB).  One sequence of 8,192
+// tokens, 16 heads of 64: walked in 328 us either way; 16 of 512: 251 instead of 227.
+constexpr int CHUNK_ROOM = 128;
 
 // floats of a (chunk, head): W [32][D], c Q [32][D], (D[C] o K)^T [D][32], D o Q K^T [32][32], V' [32][DVP], c_C
 __host__ __device__ constexpr long chunk_floats(int D, int DVP) { return 96L * D + CHUNK * CHUNK + CHUNK * DVP + 4; }
@@ -268,7 +273,8 @@ template <int D>
 __global__ void __launch_bounds__(CHUNK_THREADS)
 delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ rec,
                 const float* __restrict__ vp, long_seq::Head* list, float* __restrict__ chunks,
-                const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs, int n_heads, int n_kv_heads, int DVP) {
+                const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs, int n_heads, int n_kv_heads,
+                int DVP, int base) {
   constexpr int SK = D + 4, SA = CHUNK + 4;
   __shared__ __align__(16) float ks[CHUNK][SK];
   __shared__ __align__(16) float qs[CHUNK][SK];
@@ -276,10 +282,10 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
   __shared__ double dm[CHUNK][CHUNK + 1];        // D[i][j], j <= i
   __shared__ float gs[CHUNK], betas[CHUNK], cs[CHUNK];
   const int h = blockIdx.y, hk = h / (n_heads / n_kv_heads), tid = threadIdx.x;
-  const auto found = long_seq::find_chunk<CHUNK_MIN, CHUNK, CHUNK_THREADS>(seq_slot, seq_start, n_seqs, blockIdx.x,
+  const auto found = long_seq::find_chunk<CHUNK_MIN, CHUNK, CHUNK_THREADS>(seq_slot, seq_start, n_seqs, base + blockIdx.x,
                                                                            blockIdx.x + h == 0 ? list : nullptr);
   if (found.seq < 0) return;
-  const int c = blockIdx.x - found.first_chunk;
+  const int c = base + blockIdx.x - found.first_chunk;
   const int t0 = seq_start[found.seq] + c * CHUNK, nt = min(CHUNK, found.tokens - c * CHUNK);
   float* const dst = chunks + ((size_t)blockIdx.x * n_heads + h) * chunk_floats(D, DVP);
   for (int i = tid; i < CHUNK * (D / 4); i += CHUNK_THREADS) {
@@ -426,7 +432,7 @@ template <int D>
 __global__ void __launch_bounds__(CHUNK_THREADS, 2)
 delta_chunk_kernel(long_seq::Head* list, const float* __restrict__ chunks, float* __restrict__ out, long out_stride, float* __restrict__ state,
                    long state_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_heads,
-                   int d, int dv, int DVP) {
+                   int d, int dv, int DVP, int base) {
   using L = ChunkWalk<D>;
   constexpr int ND = D / 32;
   extern __shared__ __align__(16) float smem[];
@@ -439,8 +445,10 @@ delta_chunk_kernel(long_seq::Head* list, const float* __restrict__ chunks, float
   for (long_seq::Items items(list, n_heads * columns); items.more(); items.draw()) {
     const auto sequence = items.sequence();
     const int h = items.part() / columns, col0 = items.part() % columns * CHUNK_COLS;
-    const int n = sequence.tokens, first = sequence.first_chunk, start = seq_start[sequence.seq];
-    const int n_chunks = (n + CHUNK - 1) / CHUNK;
+    const int n = sequence.tokens, first = sequence.first_chunk - base, start = seq_start[sequence.seq];
+    // the sequence's chunks of this stretch
+    const int c_lo = max(0, -first), c_hi = min((n + CHUNK - 1) / CHUNK, CHUNK_ROOM - first);
+    if (c_lo >= c_hi) continue;
 
     auto issue = [&](int c) {
       const float* src = chunks + ((size_t)(first + c) * n_heads + h) * REC;
@@ -464,8 +472,8 @@ delta_chunk_kernel(long_seq::Head* list, const float* __restrict__ chunks, float
     auto walk = [&](auto causal) {
       constexpr bool CAUSAL = decltype(causal)::value;
 #pragma unroll
-      for (int c = 0; c < CHUNK_STAGES - 1; ++c) {
-        if (c < n_chunks) issue(c);
+      for (int c = c_lo; c < c_lo + CHUNK_STAGES - 1; ++c) {
+        if (c < c_hi) issue(c);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
       }
       float s[ND][2];
@@ -478,10 +486,10 @@ delta_chunk_kernel(long_seq::Head* list, const float* __restrict__ chunks, float
           s_t[col * L::SW + row] = s[i][e];
         }
       float finite = 0.f;
-      for (int c = 0; c < n_chunks; ++c) {
+      for (int c = c_lo; c < c_hi; ++c) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(CHUNK_STAGES - 2) : "memory");
         __syncthreads();  // the chunk has landed, and the state of the chunk before stands in shared memory
-        if (c + CHUNK_STAGES - 1 < n_chunks) issue(c + CHUNK_STAGES - 1);
+        if (c + CHUNK_STAGES - 1 < c_hi) issue(c + CHUNK_STAGES - 1);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         const float* buf = smem + c % CHUNK_STAGES * L::BUF;
         float w0 = 0.f, w1 = 0.f, q0 = 0.f, q1 = 0.f;
@@ -591,14 +599,22 @@ static int launch_scan(cudaStream_t stream, const float* qn, const float* kn, co
 static bool chunks_apply(int longest, int d, int dtype, int head_decay) {
   return dtype == FG_BF16 && head_decay && d > 32 && d <= 128 && longest >= CHUNK_MIN;
 }
+static long most_chunks(int n_tokens, int n_seqs) { return long_seq::most_chunks(n_tokens, n_seqs, CHUNK_MIN, CHUNK); }
+
+// kernels that fg_delta_scan launches
+extern "C" int fg_delta_scan_launches(int n_tokens, int longest, int n_seqs, int d, int dtype, int head_decay) {
+  return 2 + (chunks_apply(longest, d, dtype, head_decay) ? 2 * (int)((most_chunks(n_tokens, n_seqs) + CHUNK_ROOM - 1) / CHUNK_ROOM) : 0);
+}
+
 // floats of the scratch that fg_delta_scan needs for `n_tokens` tokens
 extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int longest, int n_seqs, int n_heads, int n_kv_heads, int d, int dv,
                                              int dtype, int head_decay) {
   const long DP = delta_rows(d), DVP = (dv + 3) / 4 * 4;
   const long rows = (long)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
   if (!chunks_apply(longest, d, dtype, head_decay)) return rows;
+  const long most = most_chunks(n_tokens, n_seqs);
   return rows + long_seq::list_floats(n_tokens, n_seqs, CHUNK_MIN) +
-         long_seq::most_chunks(n_tokens, n_seqs, CHUNK_MIN, CHUNK) * n_heads * chunk_floats((int)DP, (int)DVP);
+         (most < CHUNK_ROOM ? most : CHUNK_ROOM) * n_heads * chunk_floats((int)DP, (int)DVP);
 }
 
 // qkv: float32 [T, q (kv heads x d) | k (kv heads x d) | v (heads x dv)], the convolutions' outputs.
@@ -640,23 +656,27 @@ extern "C" int fg_delta_scan(const float* qkv, long qkv_stride, const void* a, l
     float* const behind = scratch + (size_t)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
     long_seq::Head* const list = reinterpret_cast<long_seq::Head*>(behind);
     float* const chunks = behind + long_seq::list_floats(n_tokens, n_seqs, CHUNK_MIN);
-    const dim3 wy_grid((unsigned)long_seq::most_chunks(n_tokens, n_seqs, CHUNK_MIN, CHUNK), n_heads);
+    const int all = (int)most_chunks(n_tokens, n_seqs);
     const long items = long_seq::most_sequences(n_tokens, n_seqs, CHUNK_MIN) * n_heads * ((dv + CHUNK_COLS - 1) / CHUNK_COLS);
 #define CHUNKS(D)                                                                                                       \
-  do {                                                                                                                  \
+  for (int base = 0; base < all; base += CHUNK_ROOM) {                                                                  \
+    const dim3 wy_grid(all - base < CHUNK_ROOM ? all - base : CHUNK_ROOM, n_heads);                                     \
     delta_wy_kernel<D><<<wy_grid, CHUNK_THREADS, 0, stream>>>(qn, kn, rec, vp, list, chunks, seq_slot, seq_start, n_seqs, \
-                                                              n_heads, n_kv_heads, DVP);                                \
+                                                              n_heads, n_kv_heads, DVP, base);                          \
     FG_CHECK_LAUNCH("fg_delta_scan (chunks)");                                                                          \
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
                                          (int)ChunkWalk<D>::SMEM);                                                      \
     FG_CHECK_ARG(e == cudaSuccess, "fg_delta_scan: shared memory: %s", cudaGetErrorString(e));                          \
     const long resident = (long)fg_sm_count() * fg_blocks_per_sm(CHUNK_THREADS, ChunkWalk<D>::SMEM);                    \
     delta_chunk_kernel<D><<<(unsigned)(items < resident ? items : resident), CHUNK_THREADS, ChunkWalk<D>::SMEM, stream>>>( \
-        list, chunks, out, out_stride, state, state_stride, seq_slot, seq_start, n_heads, d, dv, DVP);                  \
+        list, chunks, out, out_stride, state, state_stride, seq_slot, seq_start, n_heads, d, dv, DVP, base);            \
     FG_CHECK_LAUNCH("fg_delta_scan (walk)");                                                                            \
-  } while (0)
-    if (DP == 64) CHUNKS(64);
-    else CHUNKS(128);
+  }
+    if (DP == 64) {
+      CHUNKS(64)
+    } else {
+      CHUNKS(128)
+    }
 #undef CHUNKS
   }
   const auto scan = head_decay ? launch_scan<true> : launch_scan<false>;

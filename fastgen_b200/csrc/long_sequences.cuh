@@ -97,7 +97,7 @@ __device__ __forceinline__ Found find_chunk(const int* __restrict__ seq_slot, co
 // The blocks of a walk take the items (list.n_seqs sequences of `parts` parts) in order, each the next one when it is
 // through; draw() is called by all threads, between two items.  A launch may have more blocks than there are
 // items, and two neighbours may come up on one SM while others have none: a block that finds as many on its SM as each
-// would have items waits a few microseconds before it draws.
+// would have items waits a microsecond or two before it draws.
 struct Items {
   Head* list;
   int parts, total, item;
@@ -110,8 +110,7 @@ struct Items {
       asm volatile("mov.u32 %0, %%nsmid;\n" : "=r"(sms));
       take([&] {
         if (sm < SMS && atomicAdd(&list->on_sm[sm], 1) * (int)sms >= total) {
-#pragma unroll 1
-          for (int i = 0; i < 4; ++i) __nanosleep(1000);
+          __nanosleep(1500);
         }
         return atomicAdd(&list->drawn, 1);
       });

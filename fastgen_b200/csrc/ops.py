@@ -204,6 +204,7 @@ def latent(rank: int, rot_dim: int):
 
 _DELTA_SIGNATURES = {
     "fg_delta_scan": [_P, _L, _P, _L, _P, _L, _I, _P, _P, _P, _L, _P, _L, _P, _P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _P],
+    "fg_delta_scan_launches": [_I, _I, _I, _I, _I, _I],
     "fg_delta_scan_scratch_floats": [_I, _I, _I, _I, _I, _I, _I, _I, _I],
     "fg_head_norm_gate": [_P, _L, _P, _L, _I, _P, _P, _L, _P, _I, _I, _I, _F, _I, _P],
 }
@@ -841,17 +842,15 @@ class Ops:
         longest = _longest(ctx, t)
         # the tokens as the recurrence reads them (unit vectors, decays, step sizes; padded rows)
         # (and, where sequences of many tokens go chunk by chunk, what the chunks are alone)
-        def room(dtype):
-            return lib.fg_delta_scan_scratch_floats(t, longest, ctx.n_seqs, heads, kv_heads, d, dv, dtype, int(head_decay))
-
-        scratch = torch.empty(room(_code(a.dtype)), dtype=torch.float32, device=qkv.device)
+        scratch = torch.empty(lib.fg_delta_scan_scratch_floats(t, longest, ctx.n_seqs, heads, kv_heads, d, dv, _code(a.dtype),
+                                                               int(head_decay)), dtype=torch.float32, device=qkv.device)
         _check(lib, lib.fg_delta_scan(
             _ptr(qkv), qkv.stride(0), _ptr(a), a.stride(0), _ptr(b), b.stride(0), _code(a.dtype), _ptr(dt_bias),
             _ptr(a_log), _ptr(out), out.stride(0), _ptr(state), state.stride(0), _ptr(ctx.seq_slot),
             _ptr(ctx.seq_start), ctx.n_seqs, _ptr(ctx.req), t, longest, _ptr(scratch), heads, kv_heads, d, dv,
             int(head_decay), _stream()))
-        # the kernel that prepares the tokens, and the chunks' two (float32 never has those)
-        Ops.launches += 1 + 2 * int(scratch.numel() > room(FG_F32))
+        # (_check counts one)
+        Ops.launches += lib.fg_delta_scan_launches(t, longest, ctx.n_seqs, d, _code(a.dtype), int(head_decay)) - 1
         return out
 
     def head_norm_gate(self, o, z, weight, heads: int, dv: int, eps: float, ctx, act: str = "sigmoid") -> torch.Tensor:

@@ -533,6 +533,42 @@ def test_chunks_of_sequences_among_empty_places(ops16, places, lengths):
     assert all(torch.equal(a, b) for a, b in zip(together, alone))
 
 
+@pytest.mark.parametrize("lengths", [[4097], [4200, 64, 63, 4000], [130] * 40])
+def test_delta_chunks_in_stretches(ops16, lengths):
+    """More chunks than there is room for: the room does not grow with them, and the bits are those of each sequence in
+    portions of whole chunks that need one stretch."""
+    from fastgen_b200.csrc.ops import FG_BF16, delta_rule
+    heads, kv, d, dv = 3, 1, 64, 24
+    slots = list(range(len(lengths)))
+    ctx = _sequences(lengths, 0, slots)
+    t = ctx.n_tokens
+    g = torch.Generator().manual_seed(t)
+    qkv, proj = _randn(g, t, 2 * kv * d + heads * dv), _randn(g, t, 2 * heads).to(torch.bfloat16)
+    vec = _randn(g, heads, scale=0.5)
+    state = _randn(g, len(lengths), heads * d * dv)
+    alone = state.clone()
+
+    def run(a, z, ctx, state):
+        return ops16.delta_scan(qkv[a:z], proj[a:z, :heads], proj[a:z, heads:], vec, vec, state, ctx, heads, kv, d, dv,
+                                head_decay=True)
+
+    out = run(0, t, ctx, state)
+    at = 0
+    for n, slot in zip(lengths, slots):
+        for a in range(0, n, 2048):
+            z = min(a + 2048, n)
+            if z - a < 64:  # (the token kernel's)
+                assert _relative(out[at + a : at + z], run(at + a, at + z, _sequences([z - a], 0, [slot]), alone).double()) < 1e-5
+            else:
+                assert torch.equal(out[at + a : at + z], run(at + a, at + z, _sequences([z - a], 0, [slot]), alone))
+        at += n
+    assert _relative(state, alone.double()) < 1e-5
+    sizes = [delta_rule().fg_delta_scan_scratch_floats(n, n, 256, 32, 32, 128, 128, FG_BF16, 1) -
+             delta_rule().fg_delta_scan_scratch_floats(n, n, 256, 32, 32, 128, 128, FG_BF16, 0) for n in (8192, 16384)]
+    # beside what the tokens take: 128 chunks of 2.2 MB
+    assert all(4 * x < 300e6 for x in sizes)
+
+
 def test_decode_buckets_launch_no_chunks(ops16):
     """A captured step of 64 and more single tokens runs the token kernels alone."""
     from fastgen_b200.csrc.ops import Ops
