@@ -257,9 +257,10 @@ constexpr int CHUNK_RUN = 8;     // rows of the state that are summed by themsel
 constexpr int CHUNK_THREADS = 128;
 constexpr int CHUNK_COLS = 8;    // columns of the state a block of the walk
 constexpr int CHUNK_STAGES = 3;  // chunks in its ring
-// Fewest tokens of a sequence that takes this way: where the two meet.  One sequence of 63 tokens 20.8 us above, of
-// 64 here 16.8 (16 heads of 64; 11.4 of them forming the chunks).
-constexpr int CHUNK_MIN = 64;
+// Fewest tokens of a sequence that takes this way: from where no number of sequences is slower (16 heads of 64).  Chunks,
+// formed and walked, against tokens, us at 96 / 128 tokens: one sequence 19.7 / 21.0 against 24.4 / 31.8, four
+// 33.1 / 39.4 against 30.1 / 39.2, eight 49.5 / 66.7 against 46.7 / 66.9.  (At 64: 18.0 against 17.0, 29 against 21.)
+constexpr int CHUNK_MIN = 128;
 
 // Chunks formed and walked at a time: a step of more goes in stretches, through the same room (at 32 heads of 128 a chunk
 // takes 2.2 MB, and 16,384 tokens of 256 requests would take 1.7 GB).  One sequence of 8,192

@@ -491,9 +491,10 @@ constexpr int SC_TOKENS = 32;   // tokens a chunk
 constexpr int SC_COLS = 32;     // columns of P a block of the walk
 constexpr int SC_THREADS = 256;
 constexpr int SC_STAGES = 2;
-// Fewest tokens of a sequence that takes this way (prepared and walked): where the two meet.  One sequence of 63
-// tokens 15.9 us above, of 64 here 16.7, of 96 19.9; four of 63 48 us, of 64 42.
-constexpr int SC_MIN = 64;
+// Fewest tokens of a sequence that takes this way (prepared and walked): where the two meet.  Chunks against tokens, us at
+// 96 / 112 / 128 tokens: one sequence 22.8 / 25.8 / 25.8 against 22.0 / 25.3 / 28.6, four 60 / 75 / 75 against
+// 64 / 74 / 84, eight 101 / 125 / 125 against 121 / 143 / 165.  (At 64: 19.3 against 15.5, 47 against 44, 79 against 83.)
+constexpr int SC_MIN = 112;
 // Products of the state that are summed by themselves before they join a token's sum: the token kernel's sums over N are
 // trees (a few products a lane, then exchanges), and one chain over N is twice as far from 64 bits as those
 // (1.9e-7 against 1.05e-7 at N = 128; with runs of 16 and C B^T summed in 64 bits 1.0e-7, for 5 % of the walk's time).

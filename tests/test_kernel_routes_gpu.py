@@ -275,7 +275,8 @@ def test_kept_positions_lose_no_precision(ops16, hd, length, cached, window, kee
 
 # -- recurrences, chunk by chunk ---------------------------------------------------------------------------
 
-LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0)]
+LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0),
+           ([111, 112, 113], 0), ([127, 128, 129], 1)]
 
 
 @pytest.mark.parametrize("n_state,p", [(128, 64), (64, 40), (128, 4)])
@@ -321,8 +322,8 @@ def test_state_space_recurrence(ops16, lengths, pad, n_state, p):
 @pytest.mark.parametrize("at", [0, 31, 45, 64, 99])
 def test_state_space_chunks_are_causal(ops16, at, value):
     """A number that is not finite changes nothing before its token, and no other column at all."""
-    heads, groups, n_state, p, n = 4, 2, 128, 40, 100
-    ctx = _sequences([n, 70], 2)
+    heads, groups, n_state, p, n = 4, 2, 128, 40, 150
+    ctx = _sequences([n, 130], 2)
     g = torch.Generator().manual_seed(at)
     inner, bc = heads * p, groups * n_state
     xbc = _randn(g, ctx.n_tokens, inner + 2 * bc, scale=0.5)
@@ -343,7 +344,7 @@ def test_state_space_chunks_are_causal(ops16, at, value):
     assert torch.allclose(got[:n, other], want[:n, other], rtol=0, atol=2e-5)
     assert torch.allclose(got[:at, column], want[:at, column], rtol=0, atol=2e-5)
     assert not bool(torch.isfinite(got[at:n, column]).any())
-    assert torch.equal(got[n : n + 70], want[n : n + 70]) and torch.equal(states[0][1], states[1][1])
+    assert torch.equal(got[n : n + 130], want[n : n + 130]) and torch.equal(states[0][1], states[1][1])
     finite = torch.isfinite(states[1][0].view(heads * p, n_state)).all(1)
     assert bool(finite[other].all()) and not bool(finite[column])
 
@@ -428,8 +429,8 @@ def test_delta_rule_with_one_decay_a_head(ops16, lengths, pad, d, dv):
 @pytest.mark.parametrize("at", [0, 31, 45, 99])
 def test_delta_chunks_are_causal(ops16, at, part, value):
     """A number that is not finite changes nothing before its token, and nothing of other columns (a value's) or heads."""
-    heads, kv, d, dv, n = 4, 2, 64, 40, 100
-    ctx = _sequences([n, 70], 2)
+    heads, kv, d, dv, n = 4, 2, 64, 40, 150
+    ctx = _sequences([n, 130], 2)
     g = torch.Generator().manual_seed(at)
     qkv = _randn(g, ctx.n_tokens, 2 * kv * d + heads * dv)
     proj = _randn(g, ctx.n_tokens, 2 * heads).to(torch.bfloat16)
@@ -456,7 +457,7 @@ def test_delta_chunks_are_causal(ops16, at, part, value):
     assert not bool(torch.isfinite(bad).any())
     if part == "q":
         assert torch.allclose(got[at + 1 : n, hit], want[at + 1 : n, hit], rtol=0, atol=2e-6)
-    assert torch.equal(got[n : n + 70], want[n : n + 70])
+    assert torch.equal(got[n : n + 130], want[n : n + 130])
 
 
 @pytest.mark.parametrize("d", [64, 128])
@@ -494,7 +495,7 @@ def test_delta_chunks_lose_no_precision(ops16, d):
     assert errors[0][0] <= 1.05 * errors[1][0] and errors[0][1] <= 1.05 * errors[1][1], errors
 
 
-@pytest.mark.parametrize("places,lengths", [(1, [130]), (300, [64]), (300, [63, 200, 0, 65, 1]), (300, [64 + i % 9 for i in range(90)])])
+@pytest.mark.parametrize("places,lengths", [(1, [130]), (300, [128]), (300, [63, 200, 0, 129, 1]), (300, [128 + i % 9 for i in range(90)])])
 def test_chunks_of_sequences_among_empty_places(ops16, places, lengths):
     """A captured step has a place for every request: sequences behind one another or with empty places between
     them, fewer and more (sequence, part) items than blocks, against each sequence by itself, bit for bit."""
@@ -533,7 +534,7 @@ def test_chunks_of_sequences_among_empty_places(ops16, places, lengths):
     assert all(torch.equal(a, b) for a, b in zip(together, alone))
 
 
-@pytest.mark.parametrize("lengths", [[4097], [4200, 64, 63, 4000], [130] * 40])
+@pytest.mark.parametrize("lengths", [[4097], [4200, 128, 63, 4000], [130] * 40])
 def test_delta_chunks_in_stretches(ops16, lengths):
     """More chunks than there is room for: the room does not grow with them, and the bits are those of each sequence in
     portions of whole chunks that need one stretch."""
@@ -557,7 +558,7 @@ def test_delta_chunks_in_stretches(ops16, lengths):
     for n, slot in zip(lengths, slots):
         for a in range(0, n, 2048):
             z = min(a + 2048, n)
-            if z - a < 64:  # (the token kernel's)
+            if z - a < 128:  # (the token kernel's)
                 assert _relative(out[at + a : at + z], run(at + a, at + z, _sequences([z - a], 0, [slot]), alone).double()) < 1e-5
             else:
                 assert torch.equal(out[at + a : at + z], run(at + a, at + z, _sequences([z - a], 0, [slot]), alone))
@@ -570,7 +571,7 @@ def test_delta_chunks_in_stretches(ops16, lengths):
 
 
 def test_decode_buckets_launch_no_chunks(ops16):
-    """A captured step of 64 and more single tokens runs the token kernels alone."""
+    """A captured step of many single tokens runs the token kernels alone."""
     from fastgen_b200.csrc.ops import Ops
     from fastgen_b200.engine.decode_graph import _Bucket
     g = torch.Generator().manual_seed(5)
@@ -591,8 +592,8 @@ def test_decode_buckets_launch_no_chunks(ops16):
                          torch.zeros(n, heads * d * p, device=DEV), ctx, heads, groups, d, p, head_decay=True)
         return between - before, Ops.launches - between
 
-    assert launches(64, 1) == launches(63, None) == (1, 2)
-    assert launches(64, None) == (3, 4)
+    assert launches(128, 1) == launches(63, None) == (1, 2)
+    assert launches(128, None) == (3, 4)
 
 
 # -- embedding --------------------------------------------------------------------------------------------
