@@ -424,12 +424,8 @@ int launch_block(int warps, const float* A, int lda, const float* W, int ldw, fl
   using S = BlockShape<TOK, NC, STAGES, BLOCKS, MAX_WARPS>;
   auto kern = gemm_f32_block_kernel<S>;
   auto bytes = [](int w) { return (int)(sizeof(float) * S::STAGES * (S::NT + w * TOK) * S::COLS); };
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(MAX_WARPS));
-    FG_CHECK_ARG(e == cudaSuccess, "fg_gemm_f32_nt: shared memory: %s", cudaGetErrorString(e));
-    attr_set = true;
-  }
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(MAX_WARPS));
+  FG_CHECK_ARG(e == cudaSuccess, "fg_gemm_f32_nt: shared memory: %s", cudaGetErrorString(e));
   const dim3 grid((M + warps * TOK - 1) / (warps * TOK), (N + S::NT - 1) / S::NT);
   FG_CHECK_ARG(grid.y <= 65535, "fg_gemm_f32_nt: N=%d too large", N);
   kern<<<grid, warps * 32, bytes(warps), stream>>>(A, lda, W, ldw, C, ldc, M, N, K, bias);
@@ -441,12 +437,8 @@ int launch_rows(const float* A, int lda, const float* W, int ldw, float* C, int 
                 cudaStream_t stream) {
   using S = RowsShape<TOK, COLS, STAGES>;
   auto kern = gemm_f32_rows_kernel<S>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    FG_CHECK_ARG(e == cudaSuccess, "fg_gemm_f32_nt: shared memory: %s", cudaGetErrorString(e));
-    attr_set = true;
-  }
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+  FG_CHECK_ARG(e == cudaSuccess, "fg_gemm_f32_nt: shared memory: %s", cudaGetErrorString(e));
   const dim3 grid((N + S::ROWS - 1) / S::ROWS, (M + S::A_ROWS - 1) / S::A_ROWS);
   kern<<<grid, S::THREADS, S::SMEM, stream>>>(A, lda, W, ldw, C, ldc, M, N, K, bias);
   return 0;
