@@ -77,7 +77,7 @@ gemm_f32_nt_kernel(const TA* __restrict__ A, int lda, const float* __restrict__ 
 // of them.  Tiles of 16 columns of k go through registers (16-byte loads of the next tile are on their way while
 // this one is multiplied) into shared memory with k as the slow index: a thread's operands of one k are
 // four 16-byte reads for 64 multiply-adds, which is what the shared memory can deliver beside them (4 x 4
-// outputs a thread, as the last kernel of this file, need twice as much).  Two multiply-adds an instruction
+// outputs a thread, as in the kernel above, need twice as much).  Two multiply-adds an instruction
 // (fma.rn.f32x2, each rounded as fmaf rounds).  777 x 128,256 x 2,048: 16.7 -> 8.1 ms (50 TFLOP/s).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
@@ -455,25 +455,26 @@ extern "C" int fg_gemm_f32_nt(const float* A, int lda, const float* W, int ldw, 
     //  * up to 8 rows the kernel of few rows with a row of A a lane; up to 64 rows with four rows a lane while its
     //    blocks of 16 columns are not more than about two an SM (48 rows: 2,048 x 2,048 30 against 62 of the next
     //    one, 5,120 x 3,072 101 against 133; but 16,384 x 2,048 181 against 134);
-    //  * two 64 x 128 tiles an SM or more: the tile kernel (160 rows, 16,384 x 2,048: 358 against 369);
+    //  * two 64 x 128 tiles an SM or more (296 on 148 SMs): the tile kernel (160 rows, 16,384 x 2,048: 358 against 369);
     //  * between them the small block while it is about two an SM (300 rows, 2,048 x 2,048: 124 against 136), else
     //    128 columns by as many rows as divide the launch best.
     auto up = [](long a, long b) { return (a + b - 1) / b; };
+    const long two_an_sm = 2 * fg_sm_count(), about_two = two_an_sm + two_an_sm / 12;  // (296 and 320)
     int rc = 0;
     if (M <= 8) rc = launch_rows<1, 128, 4>(A, lda, W, ldw, C, ldc, M, N, K, bias, stream);
-    else if (M <= 64 && up(N, 16) <= 320) rc = launch_rows<4, 128, 4>(A, lda, W, ldw, C, ldc, M, N, K, bias, stream);
-    else if (M > 32 && up(M, 64) * up(N, 128) >= 296) {
+    else if (M <= 64 && up(N, 16) <= about_two) rc = launch_rows<4, 128, 4>(A, lda, W, ldw, C, ldc, M, N, K, bias, stream);
+    else if (M > 32 && up(M, 64) * up(N, 128) >= two_an_sm) {
       const dim3 grid((unsigned)up(M, TileShape::MT), (unsigned)up(N, TileShape::NT));
       FG_CHECK_ARG(grid.y <= 65535, "fg_gemm_f32_nt: N=%d too large", N);
       gemm_f32_tile_kernel<<<grid, TileShape::THREADS, 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K, bias);
-    } else if (M <= 32 || up(M, 32) * up(N, 64) <= 320) {
-      rc = launch_block<8, 2, 4, 4, 4>(M <= 8 ? 1 : M <= 16 ? 2 : M <= 24 ? 3 : 4, A, lda, W, ldw, C, ldc, M, N, K, bias, stream);
+    } else if (M <= 32 || up(M, 32) * up(N, 64) <= about_two) {
+      rc = launch_block<8, 2, 4, 4, 4>(M <= 16 ? 2 : M <= 24 ? 3 : 4, A, lda, W, ldw, C, ldc, M, N, K, bias, stream);
     } else {
       // warps of 8 rows: the fewest rounds of two blocks an SM, and of those the fewest rows
       int warps = 8;
       long best = 1l << 40;
       for (int w = 8; w >= 3; --w) {
-        const long cost = up(up(M, 8 * w) * up(N, 128), 296) * (w + 1);
+        const long cost = up(up(M, 8 * w) * up(N, 128), two_an_sm) * (w + 1);
         if (cost < best) {
           best = cost;
           warps = w;

@@ -32,9 +32,10 @@ def _randn(gen, *shape, scale=1.0):
 @pytest.mark.parametrize("m,n,k", [
     (1, 16, 4), (7, 17, 132), (8, 2051, 128), (8, 40, 1028),           # few rows, a row a lane
     (9, 33, 100), (31, 200, 2048), (33, 5120, 36), (64, 15, 260),      # few rows, four a lane
-    (9, 5200, 36), (24, 5300, 68), (32, 9001, 32),                     # small blocks of 1 to 4 warps
-    (65, 64, 4), (97, 65, 100), (160, 2047, 64), (321, 63, 33 * 4),    # small blocks
-    (64, 9000, 36), (65, 7001, 32), (200, 5121, 40), (777, 2050, 28),  # 128 columns by 3 to 8 warps
+    (9, 5200, 36), (24, 5300, 68), (32, 9001, 32),                     # small blocks of 2, 3 and 4 warps
+    (65, 64, 4), (97, 65, 100), (160, 2047, 64), (321, 63, 33 * 4), (64, 9000, 36),  # small blocks of 4
+    (65, 7001, 32), (200, 5121, 40), (777, 2050, 28),                  # 128 columns by 3, 4 and 6 warps
+    (33, 28672, 36), (49, 28672, 36), (57, 28672, 36),                 # ... by 5, 7 and 8
     (33, 37889, 16), (65, 19201, 20), (777, 3100, 36),                 # 64 x 128 tiles
 ])
 def test_float32_product_routes(ops32, m, n, k):
