@@ -274,6 +274,149 @@ def test_kept_positions_lose_no_precision(ops16, hd, length, cached, window, kee
     assert errors[0] <= 1.01 * errors[1]
 
 
+def _attention_reference(q, pools, table, heads, kv, hd, cached, seen, sinks=None):
+    """One sequence's queries in float64; ``seen`` [queries, keys]."""
+    n, keys = seen.shape
+    k, v = (torch.cat([p[int(t)] for t in table], dim=1)[:, :keys].double().repeat_interleave(heads // kv, 0) for p in pools)
+    s = (torch.einsum("thd,hkd->htk", q.double().reshape(n, heads, hd), k) * hd ** -0.5).masked_fill(~seen, float("-inf"))
+    if sinks is not None:
+        s = torch.cat([s, sinks.double()[:, None, None].expand(heads, n, 1)], -1)
+    w = torch.softmax(s, -1)[..., :keys]
+    return torch.einsum("htk,hkd->thd", w, v).reshape(n, heads * hd)
+
+
+# tiles of 64 keys, the kept ones, then the window's, in parts of equal length of eight tiles or more
+@pytest.mark.parametrize("keep,window,length", [
+    (4, 1100, 40),     # 1 + 19 tiles in two parts
+    (600, 1100, 40),   # 10 + 19 in three parts of ten: the second begins at the seam
+    (640, 600, 30),    # 10 + 11 in two parts: the seam lies inside the first
+    (1250, 400, 7),    # 20 + 7 in three parts: inside the last
+])
+@pytest.mark.parametrize("hd,page,with_sinks", [(64, 16, False), (64, 128, True), (128, 64, True), (128, 128, False)])
+def test_kept_positions_of_items_in_parts(ops16, hd, page, with_sinks, keep, window, length):
+    """A few tokens on a long context: their items are worked on in parts, which start at any of their tiles."""
+    from fastgen_b200.cache.manager import LayerMemory
+    heads, kv, cached = 4, 2, 3000
+    ctx, q, pools, table = _attention_step([length], [cached], page, heads, kv, hd, torch.bfloat16, keep + hd)
+    whole = table.clone()
+    table[0, -(-keep // page) : (cached - window + 1) // page] = -1
+    sinks = torch.linspace(0, 6, heads, device=DEV) if with_sinks else None
+    memory = LayerMemory(k_pages=pools[0], v_pages=pools[1], block_table=table, page_size=page,
+                         tensor_maps=ops16.make_kv_tensor_maps(pools[0][None], pools[1][None], page), layer_index=0)
+    ops16._split.pop(hd, None)  # so that the flags hold nothing of an earlier launch
+    out = torch.empty_like(q)
+    ops16.attention(q, out, memory, ctx, heads, kv, hd, window, hd ** -0.5, keep_first=keep, sinks=sinks)
+    ops16.check_status()
+    flags = ops16._split[hd][1].view(-1, 2)
+    assert int(flags[:, 1].max()) >= 2 and not bool(flags[:, 0].any())  # parts of an item; all of them counted
+    p, j = torch.arange(cached, cached + length, device=DEV)[:, None], torch.arange(cached + length, device=DEV)[None, :]
+    seen = (j <= p) & ((p - j < window) | (j < keep))
+    ref = _attention_reference(q, pools, whole[0], heads, kv, hd, cached, seen, sinks)
+    # probabilities and outputs are rounded to bfloat16 (2^-8 each)
+    assert _relative(out, ref) <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("hd,heads,kv,page", [(64, 20, 4, 64), (128, 24, 8, 16), (48, 20, 5, 8)])
+@pytest.mark.parametrize("form", ["whole", "window", "kept", "chunk", "sinks", "turned"])
+def test_merge_of_splits_in_half_blocks(ops16, hd, heads, kv, page, form):
+    """Single tokens of more heads x requests than full blocks are resident at once: the bits of the same requests a few
+    at a time, and padding lanes between them stay untouched."""
+    from fastgen_b200.cache.manager import LayerMemory
+    from fastgen_b200.engine.step import SingleTokens
+    n = 42
+    g = torch.Generator().manual_seed(hd)
+    cached = [int(x) for x in torch.randint(0, 1400, (n,), generator=g)]
+    cached[:6] = [0, 127, 128, 255, 256, 1399]  # on both sides of where splits of 128 keys begin
+    ctx, q, pools, table = _attention_step([1] * n, cached, page, heads, kv, hd, torch.bfloat16, hd + 1)
+    memory = LayerMemory(k_pages=pools[0], v_pages=pools[1], block_table=table, page_size=page,
+                         tensor_maps=ops16.make_kv_tensor_maps(pools[0][None], pools[1][None], page), layer_index=0)
+    kw = dict(window=dict(window=300), kept=dict(window=300, keep_first=5), chunk=dict(window=None, chunk=500),
+              sinks=dict(window=None, sinks=torch.linspace(-2, 4, heads, device=DEV)),
+              turned=dict(window=None, out_freqs=torch.linspace(0.01, 1, hd // 2, device=DEV)), whole=dict(window=None))[form]
+
+    def run(lanes):
+        """Outputs of the requests in ``lanes`` (None: a padding lane, whose token index is any row's)."""
+        out = torch.full_like(q, 7.0)
+        to = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        singles = SingleTokens(to([-1 if i is None else i for i in lanes]), to([0 if i is None else i for i in lanes]),
+                               len(lanes), 1400, None, n * 1400)
+        ctx.single_tokens = lambda: singles
+        ops16.attention(q, out, memory, ctx, heads, kv, hd, scale=hd ** -0.5, **kw)
+        ops16.check_status()
+        return out
+
+    lanes = [i for k in range(n) for i in ((None, k) if k % 5 == 2 else (k,))]
+    assert heads * len(lanes) > 592 and heads * 6 < 592
+    together = run(lanes)
+    for a in range(0, n, 6):
+        few = run(list(range(a, a + 6)))
+        assert torch.equal(together[a : a + 6], few[a : a + 6])
+        assert bool((few[a + 6 :] == 7.0).all()) and bool((few[:a] == 7.0).all())
+    assert bool((run(lanes[:20])[20:] == 7.0).all())
+    if form in ("whole", "window", "sinks"):
+        for i in (0, 1, 5, 30):
+            c = cached[i]
+            seen = torch.arange(c + 1, device=DEV)[None, :] > c - kw["window"] if kw["window"] else torch.ones(1, c + 1, dtype=torch.bool, device=DEV)
+            ref = _attention_reference(q[i : i + 1], pools, table[i], heads, kv, hd, c, seen, kw.get("sinks"))
+            assert _relative(together[i : i + 1], ref) <= 2.0 ** -7
+
+
+def test_rotation_and_attention_start_early(ops16):
+    """Projection, rotation with the page write, and single-token attention as programmatic launches behind one another in
+    a graph, where splits that end before the new position are read while the rotation runs: the bits of the same
+    launches with a wait after each.  New positions at both ends of splits of 128 keys and of pages."""
+    from fastgen_b200.cache.manager import LayerMemory
+    from fastgen_b200.engine.step import SingleTokens
+    heads, kv, hd, page, n, dim = 8, 2, 64, 64, 8, 512
+    first = [0, 63, 64, 127, 128, 129, 255, 511]
+    steps = 3
+    ctx, _, pools, table = _attention_step([steps] * n, first, page, heads, kv, hd, torch.bfloat16, 3)
+    g = torch.Generator().manual_seed(4)
+    w = _randn(g, (heads + 2 * kv) * hd, dim, scale=dim ** -0.5).to(torch.bfloat16)
+    xs = [_randn(g, n + 1, dim).to(torch.bfloat16) for _ in range(steps)]
+    freqs = torch.linspace(1, 0.01, hd // 2, device=DEV)
+    to = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    req = to(list(range(n)) + [-1])  # (the last token is padding)
+    singles = SingleTokens(req, to(list(range(n + 1))), n + 1, 1024, None, n * 1024)
+    ctx.single_tokens = lambda: singles
+    ctx.attention_tiles = lambda tpt, least=1: SimpleNamespace(n=0)
+
+    def layer(x, out, pos, pool, wait):
+        ctx.pos = pos
+        memory = LayerMemory(k_pages=pool[0], v_pages=pool[1], block_table=table, page_size=page,
+                             tensor_maps=ops16.make_kv_tensor_maps(pool[0][None], pool[1][None], page), layer_index=0)
+        qkv = ops16.linear(x, w)
+        wait()
+        q, k, v = qkv[:, : heads * hd], qkv[:, heads * hd : (heads + kv) * hd], qkv[:, (heads + kv) * hd :]
+        ops16.rope_kv_write(q, k, v, pos, req, freqs, pool[0], pool[1], table, page, heads, kv, hd)
+        wait()
+        ops16.attention(q, out, memory, ctx, heads, kv, hd, None, hd ** -0.5)
+        wait()
+
+    results = []
+    for graph in (False, True):
+        pool = [p.clone() for p in pools]
+        x, out, pos = xs[0].clone(), torch.zeros(n + 1, heads * hd, dtype=torch.bfloat16, device=DEV), to(first + [0])
+        if graph:
+            layer(x, out, to([c for c in first] + [0]), [p.clone() for p in pool], lambda: None)  # loads and sizes
+            stream, replay = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                replay.capture_begin()
+                layer(x, out, pos, pool, lambda: None)
+                replay.capture_end()
+            torch.cuda.current_stream().wait_stream(stream)
+        got = []
+        for s in range(steps):
+            x.copy_(xs[s])
+            pos.copy_(to([c + s for c in first] + [0]))
+            replay.replay() if graph else layer(x, out, pos, pool, torch.cuda.synchronize)
+            got.append(out[:n].clone())
+        ops16.check_status()
+        results.append(got + pool)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 # -- recurrences, chunk by chunk ---------------------------------------------------------------------------
 
 LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0),
