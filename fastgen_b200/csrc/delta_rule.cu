@@ -21,8 +21,9 @@
 // (Measured at key size 64, 2,048 tokens: 16 lanes x 4 rows 536 us, 32 x 4 591 us, 8 x 8 601 us, 2 x 32 669 us.)
 // Tokens arrive eight at a time through a ring of cp.async buffers, several stages ahead; whole
 // stages run unrolled, so that a token's operands are read while the one before it is reduced.
-// The recurrence runs token by token, so prompt portions, single tokens and mixed batches take
-// these kernels and give the same numbers however a prompt is cut.  The state of a slot is
+// The recurrence runs token by token, so prompt portions, single tokens and mixed batches take these kernels and give the
+// same numbers however a prompt is cut; the exception is 16-bit serving with one decay a head, where sequences that bring
+// many tokens (CHUNK_MIN and more) go chunk by chunk, with sums of another order.  The state of a slot is
 // [heads][dv][d] float32 (a column's rows side by side), zero at admission.
 #include <type_traits>
 
@@ -252,6 +253,8 @@ delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
 // the substitution and the sums over the state's rows made the outputs 2.6e-7 off at key size 64 and 3.2e-7 at
 // 128, against 2.0e-7 and 2.3e-7 of the token kernel; with short chains 1.9e-7 and 2.1e-7.)  The order of the
 // sums is not the token kernel's, so the float32 mode, whose results do not depend on how a prompt is cut, keeps that.
+// (The chunked form is published, for instance in Yang et al., "Parallelizing Linear Transformers with the Delta
+// Rule over Sequence Length", 2024.)
 constexpr int CHUNK = 32;
 constexpr int CHUNK_RUN = 8;     // rows of the state that are summed by themselves
 constexpr int CHUNK_THREADS = 128;

@@ -16,8 +16,9 @@
 // sequence any number of tokens; sequences are consecutive runs of tokens with one slot, and
 // tokens of slot < 0 are padding that touches nothing.
 //
-// The recurrence runs token by token, so its sums do not depend on how a prompt was cut or
-// what else is in the batch.
+// No sum depends on what else is in the batch.  The recurrence runs token by token, so that its sums do not depend on how
+// a prompt was cut either, except in 16-bit serving for sequences that bring many tokens (SC_MIN and more): those go
+// chunk by chunk, with float32 sums of another order that are as close to 64 bits.
 #include "common.cuh"
 #include "long_sequences.cuh"
 
@@ -485,8 +486,9 @@ ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* _
 //
 // ssm_chunk_prepare_kernel forms M, e and w for all chunks side by side (a block a (chunk, group): C B^T once for the
 // group's heads); ssm_chunk_kernel walks the chunks of one (sequence, head, 32 columns), a state of 4 x 4 numbers a
-// thread.  float32 multiply-adds (the decays and C B^T in 64 bits); the sums have another order than the token kernel's, so the float32 mode,
-// whose results do not depend on how a prompt is cut, keeps that one.
+// thread.  float32 multiply-adds (the decays and C B^T in 64 bits); the sums have another order than the token kernel's,
+// so the float32 mode, whose results do not depend on how a prompt is cut, keeps that one.  (The chunked form is
+// published, for instance in Dao and Gu, "Transformers are SSMs", 2024.)
 constexpr int SC_TOKENS = 32;   // tokens a chunk
 constexpr int SC_COLS = 32;     // columns of P a block of the walk
 constexpr int SC_THREADS = 256;

@@ -442,9 +442,9 @@ class Ops:
 
     def mamba2_scan(self, xbc, proj, dt_offset: int, dt_bias, a_log, d_skip, state, ctx, heads: int, groups: int,
                     n_state: int, head_dim: int) -> torch.Tensor:
-        """The recurrence ``S <- exp(-exp(A) dt) S + dt B x^T; y = S^T C + D x`` per (sequence, head),
-        token by token in float32, from and into ``state`` [slots, .] (its first
-        ``heads * n_state * head_dim`` numbers).  ``xbc`` [T, x | B | C] float32; the raw step sizes are
+        """The recurrence ``S <- exp(-exp(A) dt) S + dt B x^T; y = S^T C + D x`` per (sequence, head) in
+        float32, token by token (in 16-bit serving long sequences chunk by chunk), from and into ``state``
+        [slots, .] (its first ``heads * n_state * head_dim`` numbers).  ``xbc`` [T, x | B | C] float32; the raw step sizes are
         the columns ``dt_offset .. + heads`` of ``proj``.  Returns y [T, heads * head_dim] float32."""
         t = xbc.shape[0]
         assert xbc.dtype == torch.float32 and xbc.stride(1) == 1 and proj.stride(1) == 1
@@ -822,8 +822,8 @@ class Ops:
 
     def delta_scan(self, qkv, a, b, dt_bias, a_log, state, ctx, heads: int, kv_heads: int, d: int, dv: int,
                    head_decay: bool = False):
-        """The gated delta rule per (sequence, head), token by token in float32, from and into ``state``
-        [slots, .] (a slot's first ``heads * dv * d`` numbers, laid out [heads][dv][d]):
+        """The gated delta rule per (sequence, head) in float32, token by token (in 16-bit serving with one decay
+        a head, long sequences chunk by chunk), from and into ``state`` [slots, .] (a slot's first ``heads * dv * d`` numbers, laid out [heads][dv][d]):
         ``S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q`` with q, k made unit vectors
         (q also times ``d ** -0.5``), ``g = exp(-exp(a_log) softplus(a + dt_bias))``, ``beta =
         sigmoid(b)``.  With ``head_decay`` there is one decay per head: ``a`` [T, heads], ``dt_bias`` [heads].

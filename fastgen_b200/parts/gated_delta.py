@@ -39,8 +39,10 @@ class GatedDeltaRule(Mixer):
     every part padded to a multiple of 8 rows, so that the views handed on are aligned).  The request's state is
     fixed-size: S of every head ([heads][v_head_dim][head_dim]) and the convolutions' last
     ``conv - 1`` inputs, one float32 row per slot that the cache manager zeroes on admission.  The
-    recurrence runs token by token in float32, so prompt portions, single tokens and mixed batches
-    take the same kernels and give the same numbers however a prompt is cut.
+    recurrence runs in float32.  Serving in float32, one decay a key channel, and sequences that bring few
+    tokens walk it token by token: prompt portions, single tokens and mixed batches give the same numbers
+    however a prompt is cut.  With one decay a head, 16-bit serving walks sequences that bring 128 tokens or
+    more in chunks of 32 (key sizes of 33 to 128), whose sums have another order.
     """
 
     params: GatedDeltaParams

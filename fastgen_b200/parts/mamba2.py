@@ -23,8 +23,10 @@ class Mamba2(Mixer):
     ``y * silu(z)`` is RMS-normed in ``norm_groups`` equal parts of its columns and multiplied by
     ``norm``.  The request's state is fixed-size: S of every head and the convolution's last
     ``conv - 1`` inputs, one float32 row per slot that the cache manager zeroes on admission.
-    The recurrence runs token by token in float32, so prompt portions, single tokens and mixed
-    batches take the same kernels and give the same numbers however a prompt is cut.
+    The recurrence runs in float32.  Serving in float32, and sequences that bring few tokens, walk it token
+    by token: prompt portions, single tokens and mixed batches give the same numbers however a prompt is cut.
+    In 16-bit serving sequences that bring 112 tokens or more are walked in chunks of 32 (states of 64 or 128
+    rows), whose sums have another order.
     """
 
     params: Mamba2Params
