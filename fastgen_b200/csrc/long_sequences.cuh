@@ -104,7 +104,7 @@ struct Items {
   __device__ __forceinline__ Items(Head* l, int parts_) : list(l), parts(parts_) {
     total = l->n_seqs * parts;
     item = blockIdx.x;
-    if (total < (int)gridDim.x) {
+    if (total > 0 && total < (int)gridDim.x) {
       unsigned sm, sms;
       asm volatile("mov.u32 %0, %%smid;\n" : "=r"(sm));
       asm volatile("mov.u32 %0, %%nsmid;\n" : "=r"(sms));
