@@ -23,7 +23,8 @@
 // stages run unrolled, so that a token's operands are read while the one before it is reduced.
 // The recurrence runs token by token, so prompt portions, single tokens and mixed batches take these kernels and give the
 // same numbers however a prompt is cut; the exception is 16-bit serving with one decay a head, where sequences that bring
-// many tokens (CHUNK_MIN and more) go chunk by chunk, with sums of another order.  The state of a slot is
+// many tokens (chunk_min() and more, which looks at the step's tokens too) go chunk by chunk, with sums of another
+// order.  The state of a slot is
 // [heads][dv][d] float32 (a column's rows side by side), zero at admission.
 #include <type_traits>
 
@@ -260,10 +261,11 @@ constexpr int CHUNK_RUN = 8;     // rows of the state that are summed by themsel
 constexpr int CHUNK_THREADS = 128;
 constexpr int CHUNK_COLS = 8;    // columns of the state a block of the walk
 constexpr int CHUNK_STAGES = 3;  // chunks in its ring
-// Fewest tokens of a sequence that takes this way: from where no number of sequences is slower (16 heads of 64).  Chunks,
-// formed and walked, against tokens, us at 96 / 128 tokens: one sequence 19.7 / 21.0 against 24.4 / 31.8, four
-// 33.1 / 39.4 against 30.1 / 39.2, eight 49.5 / 66.7 against 46.7 / 66.9.  (At 64: 18.0 against 17.0, 29 against 21.)
-constexpr int CHUNK_MIN = 128;
+// Fewest tokens of a sequence that takes this way: where the two meet, which depends on how many such sequences the
+// step's tokens leave room for (16 heads of 64).  Chunks, formed and walked, against tokens, us: one sequence of 80 / 96 / 128
+// 19.5 / 19.7 / 21.0 against 20.7 / 24.4 / 31.8 (of 64: 18.0 against 17.0), two of 96 / 128 23.2 / 26.6 against 24.6 / 32.2,
+// four 33.1 / 39.4 against 30.1 / 39.2, eight 49.5 / 66.7 against 46.7 / 66.9.
+inline int chunk_min(int n_tokens) { return n_tokens < 2 * 80 ? 80 : n_tokens < 3 * 96 ? 96 : 128; }
 
 // Chunks formed and walked at a time: a step of more goes in stretches, through the same room (at 32 heads of 128 a chunk
 // takes 2.2 MB, and 16,384 tokens of 256 requests would take 1.7 GB).  One sequence of 8,192
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS)
 delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ rec,
                 const float* __restrict__ vp, long_seq::Head* list, float* __restrict__ chunks,
                 const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs, int n_heads, int n_kv_heads,
-                int DVP, int base) {
+                int DVP, int min_tokens, int base) {
   constexpr int SK = D + 4, SA = CHUNK + 4;
   __shared__ __align__(16) float ks[CHUNK][SK];
   __shared__ __align__(16) float qs[CHUNK][SK];
@@ -286,8 +288,8 @@ delta_wy_kernel(const float* __restrict__ qn, const float* __restrict__ kn, cons
   __shared__ double dm[CHUNK][CHUNK + 1];        // D[i][j], j <= i
   __shared__ float gs[CHUNK], betas[CHUNK], cs[CHUNK];
   const int h = blockIdx.y, hk = h / (n_heads / n_kv_heads), tid = threadIdx.x;
-  const auto found = long_seq::find_chunk<CHUNK_MIN, CHUNK, CHUNK_THREADS>(seq_slot, seq_start, n_seqs, base + blockIdx.x,
-                                                                           blockIdx.x + h == 0 ? list : nullptr);
+  const auto found = long_seq::find_chunk<CHUNK, CHUNK_THREADS>(seq_slot, seq_start, n_seqs, min_tokens, base + blockIdx.x,
+                                                                blockIdx.x + h == 0 ? list : nullptr);
   if (found.seq < 0) return;
   const int c = base + blockIdx.x - found.first_chunk;
   const int t0 = seq_start[found.seq] + c * CHUNK, nt = min(CHUNK, found.tokens - c * CHUNK);
@@ -600,14 +602,14 @@ static int launch_scan(cudaStream_t stream, const float* qn, const float* kn, co
 
 // Whether a step may hold sequences for delta_chunk_kernel: 16-bit serving, one decay a head, key sizes whose
 // rows are 64 or 128, and enough tokens (`longest`: the most that one of its sequences can bring).
-static bool chunks_apply(int longest, int d, int dtype, int head_decay) {
-  return dtype == FG_BF16 && head_decay && d > 32 && d <= 128 && longest >= CHUNK_MIN;
+static bool chunks_apply(int n_tokens, int longest, int d, int dtype, int head_decay) {
+  return dtype == FG_BF16 && head_decay && d > 32 && d <= 128 && longest >= chunk_min(n_tokens);
 }
-static long most_chunks(int n_tokens, int n_seqs) { return long_seq::most_chunks(n_tokens, n_seqs, CHUNK_MIN, CHUNK); }
+static long most_chunks(int n_tokens, int n_seqs) { return long_seq::most_chunks(n_tokens, n_seqs, chunk_min(n_tokens), CHUNK); }
 
 // kernels that fg_delta_scan launches
 extern "C" int fg_delta_scan_launches(int n_tokens, int longest, int n_seqs, int d, int dtype, int head_decay) {
-  return 2 + (chunks_apply(longest, d, dtype, head_decay) ? 2 * (int)((most_chunks(n_tokens, n_seqs) + CHUNK_ROOM - 1) / CHUNK_ROOM) : 0);
+  return 2 + (chunks_apply(n_tokens, longest, d, dtype, head_decay) ? 2 * (int)((most_chunks(n_tokens, n_seqs) + CHUNK_ROOM - 1) / CHUNK_ROOM) : 0);
 }
 
 // floats of the scratch that fg_delta_scan needs for `n_tokens` tokens
@@ -615,9 +617,9 @@ extern "C" long fg_delta_scan_scratch_floats(int n_tokens, int longest, int n_se
                                              int dtype, int head_decay) {
   const long DP = delta_rows(d), DVP = (dv + 3) / 4 * 4;
   const long rows = (long)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
-  if (!chunks_apply(longest, d, dtype, head_decay)) return rows;
+  if (!chunks_apply(n_tokens, longest, d, dtype, head_decay)) return rows;
   const long most = most_chunks(n_tokens, n_seqs);
-  return rows + long_seq::list_floats(n_tokens, n_seqs, CHUNK_MIN) +
+  return rows + long_seq::list_floats(n_tokens, n_seqs, chunk_min(n_tokens)) +
          (most < CHUNK_ROOM ? most : CHUNK_ROOM) * n_heads * chunk_floats((int)DP, (int)DVP);
 }
 
@@ -655,18 +657,18 @@ extern "C" int fg_delta_scan(const float* qkv, long qkv_stride, const void* a, l
 #undef PREPARE
   FG_CHECK_LAUNCH("fg_delta_scan (prepare)");
   int most = 0x7fffffff;  // tokens of the longest sequence that the token kernel takes
-  if (chunks_apply(longest, d, dtype, head_decay)) {
-    most = CHUNK_MIN - 1;
+  if (chunks_apply(n_tokens, longest, d, dtype, head_decay)) {
+    most = chunk_min(n_tokens) - 1;
     float* const behind = scratch + (size_t)n_tokens * (2 * n_kv_heads * DP + n_heads * (DP + 4) + n_heads * DVP);
     long_seq::Head* const list = reinterpret_cast<long_seq::Head*>(behind);
-    float* const chunks = behind + long_seq::list_floats(n_tokens, n_seqs, CHUNK_MIN);
+    float* const chunks = behind + long_seq::list_floats(n_tokens, n_seqs, chunk_min(n_tokens));
     const int all = (int)most_chunks(n_tokens, n_seqs);
-    const long items = long_seq::most_sequences(n_tokens, n_seqs, CHUNK_MIN) * n_heads * ((dv + CHUNK_COLS - 1) / CHUNK_COLS);
+    const long items = long_seq::most_sequences(n_tokens, n_seqs, chunk_min(n_tokens)) * n_heads * ((dv + CHUNK_COLS - 1) / CHUNK_COLS);
 #define CHUNKS(D)                                                                                                       \
   for (int base = 0; base < all; base += CHUNK_ROOM) {                                                                  \
     const dim3 wy_grid(all - base < CHUNK_ROOM ? all - base : CHUNK_ROOM, n_heads);                                     \
     delta_wy_kernel<D><<<wy_grid, CHUNK_THREADS, 0, stream>>>(qn, kn, rec, vp, list, chunks, seq_slot, seq_start, n_seqs, \
-                                                              n_heads, n_kv_heads, DVP, base);                          \
+                                                              n_heads, n_kv_heads, DVP, most + 1, base);                \
     FG_CHECK_LAUNCH("fg_delta_scan (chunks)");                                                                          \
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
                                          (int)ChunkWalk<D>::SMEM);                                                      \

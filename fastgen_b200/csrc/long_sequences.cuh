@@ -1,4 +1,4 @@
-// The sequences of a step that the recurrences walk chunk by chunk: those of MIN tokens and more.
+// The sequences of a step that the recurrences walk chunk by chunk: those of `min_tokens` tokens and more.
 //
 // A captured step holds a place for every request the engine admits (256 by default), most of them empty, so nothing
 // may be launched by places.  The blocks that prepare the chunks are launched for the most chunks the step's tokens
@@ -26,7 +26,7 @@ struct Head {
 struct Entry {
   int seq, tokens, first_chunk, pad;
 };
-// most sequences of MIN tokens in a step, most chunks of them, and the floats of head and list
+// most sequences of `min_tokens` tokens in a step, most chunks of them, and the floats of head and list
 inline long most_sequences(int n_tokens, int n_seqs, int min_tokens) {
   return n_seqs < n_tokens / min_tokens ? n_seqs : n_tokens / min_tokens;
 }
@@ -39,9 +39,9 @@ inline long list_floats(int n_tokens, int n_seqs, int min_tokens) {
 
 // The sequence that holds chunk `target` (the long sequences' chunks are numbered one after another).  With `list`,
 // the whole list is written too.  For all threads of a block, THREADS of them; places are read THREADS at a time.
-template <int MIN, int CHUNK, int THREADS>
+template <int CHUNK, int THREADS>
 __device__ __forceinline__ Found find_chunk(const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int n_seqs,
-                                            int target, Head* list) {
+                                            int min_tokens, int target, Head* list) {
   constexpr int WARPS = THREADS / 32;
   __shared__ int seqs_s[WARPS], chunks_s[WARPS];
   __shared__ Found found_s;
@@ -52,7 +52,7 @@ __device__ __forceinline__ Found find_chunk(const int* __restrict__ seq_slot, co
     const int i = base + tid;
     int n = 0;
     if (i < n_seqs && seq_slot[i] >= 0) n = seq_start[i + 1] - seq_start[i];
-    const bool is_long = n >= MIN;
+    const bool is_long = n >= min_tokens;
     const int own = is_long ? (n + CHUNK - 1) / CHUNK : 0;
     const unsigned longs = __ballot_sync(0xffffffffu, is_long);
     int upto = own;

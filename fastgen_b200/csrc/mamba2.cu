@@ -524,8 +524,8 @@ ssm_chunk_prepare_kernel(const float* __restrict__ xbc, long xbc_stride, const T
   __shared__ double gram[SC_TOKENS][SC_TOKENS + 1];
   __shared__ float decs[SC_THREADS / 32][SC_TOKENS];
   const int g = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const auto found = long_seq::find_chunk<SC_MIN, SC_TOKENS, SC_THREADS>(seq_slot, seq_start, n_seqs, blockIdx.x,
-                                                                         blockIdx.x + g == 0 ? list : nullptr);
+  const auto found = long_seq::find_chunk<SC_TOKENS, SC_THREADS>(seq_slot, seq_start, n_seqs, SC_MIN, blockIdx.x,
+                                                                 blockIdx.x + g == 0 ? list : nullptr);
   if (found.seq < 0) return;
   const int c = blockIdx.x - found.first_chunk;
   const int t0 = seq_start[found.seq] + c * SC_TOKENS, nt = min(SC_TOKENS, found.tokens - c * SC_TOKENS), inner = heads * P;

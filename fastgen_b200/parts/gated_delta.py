@@ -41,8 +41,8 @@ class GatedDeltaRule(Mixer):
     ``conv - 1`` inputs, one float32 row per slot that the cache manager zeroes on admission.  The
     recurrence runs in float32.  Serving in float32, one decay a key channel, and sequences that bring few
     tokens walk it token by token: prompt portions, single tokens and mixed batches give the same numbers
-    however a prompt is cut.  With one decay a head, 16-bit serving walks sequences that bring 128 tokens or
-    more in chunks of 32 (key sizes of 33 to 128), whose sums have another order.
+    however a prompt is cut.  With one decay a head, 16-bit serving walks sequences that bring many tokens
+    (80 to 128 and more, by the step's size) in chunks of 32 (key sizes of 33 to 128), whose sums have another order.
     """
 
     params: GatedDeltaParams

@@ -420,7 +420,7 @@ def test_rotation_and_attention_start_early(ops16):
 # -- recurrences, chunk by chunk ---------------------------------------------------------------------------
 
 LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0),
-           ([111, 112, 113], 0), ([127, 128, 129], 1)]
+           ([111, 112, 113], 0), ([127, 128, 129], 1), ([79], 80), ([80], 79), ([95, 96], 96)]
 
 
 @pytest.mark.parametrize("n_state,p", [(128, 64), (64, 40), (128, 4)])
