@@ -225,8 +225,18 @@ extern "C" int fg_stream_norm(float* h, int n_streams, const void* delta, int de
     fg_launch_pdl(kern, dim3(n_rows), dim3(SN_THREADS), smem, stream, h, n_streams, (const TD*)delta, mix,   \
                   out_coef, in_coef, w, b, (TO*)out, rows, dim, eps, kind);                                  \
   } while (0)
-  // rows that fit the registers: at most 16 columns a thread, streams as the instantiations below have them
-  const int cols = n_streams <= 4 && dim <= 16 * SN_THREADS ? (dim <= 8 * SN_THREADS ? 8 : 16) : 0;
+  // Rows in registers (up to 16 columns a thread, up to four streams) or in shared memory, by what was measured over 1 to
+  // 2,048 rows of 256 to 4,096 columns (us, shared memory against registers; launches back to back):
+  //  * a row or less an SM is a matter of latency, and registers win once there are enough columns (64 rows: 4 streams of
+  //    1,024 0.88 and of 4,096 0.55 of the time, 2 of 4,096 0.47; but 4 of 512 1.18; one row of one stream of 1,280 1.10);
+  //  * of many rows, registers keep blocks off the SM, and pay only where a thread's columns are nearly all
+  //    there (2,048 rows: 2 streams of 2,048 0.80, of 4,096 0.99, 4 of 2,048 0.81; but 1 of 4,096 32 against 51, 2 of
+  //    2,560 28 against 37, 3 of 2,048 27 against 30, 3 of 2,560 50 against 96, 4 of 512 14 against 21).
+  int cols = n_streams <= 4 && dim <= 16 * SN_THREADS ? (dim <= 8 * SN_THREADS ? 8 : 16) : 0;
+  const bool pays = n_rows <= fg_sm_count() ? dim >= (n_streams == 1 ? 1536 : 1024)
+                    : n_streams == 2        ? dim >= 1280 && (cols == 8 || dim > 14 * SN_THREADS)
+                                            : n_streams == 4 && cols == 8 && dim > 7 * SN_THREADS;
+  if (!pays) cols = 0;
 #define LAUNCH_R(TD, TO, S, COLS)                                                                                       \
   fg_launch_pdl(stream_norm_reg_kernel<TD, TO, S, COLS>, dim3(n_rows), dim3(SN_THREADS), 0, stream, h, (const TD*)delta, \
                 mix, out_coef, in_coef, w, b, (TO*)out, rows, dim, eps, kind)

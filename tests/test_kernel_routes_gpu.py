@@ -144,6 +144,22 @@ def test_stream_norm_rows_in_registers(ops32, streams, dim, kind):
     assert torch.equal(some, out[rows.long()])
 
 
+@pytest.mark.parametrize("streams,dim", [(1, 1535), (1, 1536), (2, 1023), (2, 1280), (2, 2560), (2, 3585), (3, 1024), (4, 1793), (4, 2049)])
+def test_stream_norm_routes_by_rows(ops32, streams, dim):
+    """Few rows and many take different kernels at these sizes: the same bits for a row."""
+    g = torch.Generator().manual_seed(dim + streams)
+    n = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    h, delta = _randn(g, n, streams, dim), _randn(g, n, dim).to(torch.bfloat16)
+    mix, oc, ic = torch.rand(streams, streams, generator=g).to(DEV), torch.rand(streams, generator=g).to(DEV), torch.rand(streams, generator=g).to(DEV)
+    w, b = 1 + _randn(g, dim, scale=0.1), _randn(g, dim, scale=0.1)
+    args = dict(mix=mix, out_coef=oc, in_coef=ic, bias=b, eps=1e-5, rms=False)
+    many, few = h.clone(), h[:7].clone()
+    outs = [torch.empty(x.shape[0], dim, dtype=torch.float32, device=DEV) for x in (many, few)]
+    for x, out in zip((many, few), outs):
+        _stream_norm(ops32, x, w, out, delta=delta[: x.shape[0]], **args)
+    assert torch.equal(outs[0][:7], outs[1]) and torch.equal(many[:7], few)
+
+
 def _stream_norm(ops, h, w, out, delta, mix, out_coef, in_coef, bias, eps, rms, rows=None):
     from fastgen_b200.csrc.ops import _check, _code, _ptr, _stream
     n = out.shape[0]
