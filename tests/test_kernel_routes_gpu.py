@@ -759,7 +759,7 @@ def test_decode_buckets_launch_no_chunks(ops16):
 # -- embedding --------------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("dim,copies", [(8, 1), (2040, 2), (2048, 1), (4104, 3), (8192, 1), (100, 2)])
+@pytest.mark.parametrize("dim,copies", [(8, 1), (504, 2), (512, 1), (1016, 1), (1024, 2), (2040, 2), (2048, 1), (4104, 3), (8192, 1), (100, 2)])
 def test_embedding_rows(ops32, dtype, dim, copies):
     from fastgen_b200.csrc.ops import _check, _code, _ptr, _stream
     g = torch.Generator().manual_seed(dim)
