@@ -51,6 +51,7 @@ CORE_SOURCES = [
     "rope_kv.cu",
     "silu_gate.cu",
     "gemm_f32.cu",
+    "gemm_f32_split.cu",
     "gemm_skinny.cu",
     "sampling.cu",
     "tensor_map.cu",

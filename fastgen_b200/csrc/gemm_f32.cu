@@ -1,7 +1,7 @@
 // True 32-bit matrix product  C[M, N] = A[M, K] * W[N, K]^T  on the CUDA cores.
 //
-// This is the GEMM of the float32 path: IEEE float32 fused multiply-adds, no
-// tensor cores and no reduced-precision mode.  Every output element is the sum
+// This is the GEMM of the float32 path for small weights (N or K below 1,024) and for rows that do not lie on 16 bytes
+// (gemm_f32_split.cu has the others): IEEE float32 fused multiply-adds, no tensor cores.  Every output element is the sum
 // over k = 0 .. K-1 in ascending order in a single accumulator, so its value
 // does not depend on M, on the tile it falls in, on which of the kernels below
 // computes it, or on what else is in the batch.

@@ -81,6 +81,9 @@ _CORE_SIGNATURES = {
     "fg_part_norm": [_P, _I, _P, _I, _P, _P, _P, _I, _P, _I, _I, _I, _F, _P],
     "fg_gemm_f32_nt_from": [_P, _I, _I, _P, _I, _P, _I, _I, _I, _I, _P],
     "fg_gemm_f32_nt": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P, _P],
+    "fg_gemm_f32_split": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P, _P, _P, _P],
+    "fg_gemm_f32_split_takes": [_P, _I, _P, _I, _I, _I],
+    "fg_gemm_f32_split_scratch": [_I, _I],
     "fg_gemm_skinny_bf16": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _P],
     "fg_gemm_skinny_swiglu_bf16": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P],
     "fg_gemm_skinny_qkv_bf16": [_P, _I, _P, _I, _P, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I,
@@ -270,6 +273,7 @@ def core():
         lib = build.core_library()
         _declare(lib, _CORE_SIGNATURES)
         lib.fg_mamba2_scan_scratch_floats.restype = ctypes.c_longlong
+        lib.fg_gemm_f32_split_scratch.restype = ctypes.c_longlong
         _core = lib
     return _core
 
@@ -1028,9 +1032,18 @@ class Ops:
             if out is None:
                 out = torch.empty((m, n), dtype=torch.float32, device=x.device)
             assert out.dtype == torch.float32 and out.stride(1) == 1
-            _check(self.lib, self.lib.fg_gemm_f32_nt(
-                _ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0),
-                m, n, k, _ptr(bias), _stream()))
+            if self.lib.fg_gemm_f32_split_takes(_ptr(x), x.stride(0), _ptr(w), w.stride(0), n, k):
+                # weights of some size: tensor cores, float32 operands in three bfloat16 parts
+                need = self.lib.fg_gemm_f32_split_scratch(m, k)
+                parts = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
+                _check(self.lib, self.lib.fg_gemm_f32_split(
+                    _ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0),
+                    m, n, k, _ptr(bias), _ptr(parts), _ptr(self.status), _stream()))
+                Ops.launches += need > 0
+            else:
+                _check(self.lib, self.lib.fg_gemm_f32_nt(
+                    _ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0),
+                    m, n, k, _ptr(bias), _stream()))
             if code:
                 assert out.is_contiguous()
                 self.bias_act(out, act)

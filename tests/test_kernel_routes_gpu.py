@@ -56,6 +56,43 @@ def test_float32_product_routes(ops32, m, n, k):
     assert bool(((got.double() - ref).abs() <= bound + 1e-30).all())
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (1, 1024, 1024), (16, 1025, 1028), (5, 2100, 8192),                  # one tile of 16 rows, shared by 8, 8 and 4 blocks
+    (9, 9000, 1024), (3, 37889, 1024),                                   # ... by 2, and a tile to a block
+    (17, 2050, 1100), (32, 10241, 1024), (32, 60000, 1024),              # a tile of 32
+    (33, 1024, 1024), (64, 19000, 1088),                                 # of 64
+    (65, 1024, 2052), (113, 1500, 1028), (225, 9600, 1024),              # of 112
+    (160, 19000, 1028), (400, 5121, 1024),                               # of 160
+])
+def test_float32_product_on_tensor_cores(ops32, m, n, k):
+    """Weights from 1,024 x 1,024 on: no further from float64 than the multiply-adds of the general kernel, the same bits for
+    a row whatever is beside it (other rows, other tiles, other numbers of blocks), and its infinities and NaNs."""
+    g = torch.Generator().manual_seed(m * 5 + n)
+    x, w, bias = _randn(g, m, k), _randn(g, n, k), _randn(g, n)
+    odd_x = torch.empty(m, k + 1, device=DEV)[:, :k]  # rows off 16 bytes: the general kernel
+    odd_x.copy_(x)
+    got, other = ops32.linear(x, w), ops32.linear(odd_x, w)
+    ref = x.double() @ w.double().T
+    assert bool(((got.double() - ref).abs() <= k * EPS * (x.double().abs() @ w.double().abs().T)).all())
+    assert _relative(got, ref) <= _relative(other, ref)
+    for row in (0, m // 2, m - 1):
+        assert torch.equal(ops32.linear(x[row : row + 1], w)[0], got[row])
+    assert torch.equal(ops32.linear(x[: min(m, 40)], w), got[:40])
+    assert torch.equal(ops32.linear(x, w, bias=bias), got + bias)
+    wide = torch.full((m, n + 5), 3.0, device=DEV)
+    ops32.linear(x, w, out=wide[:, :n])
+    assert torch.equal(wide[:, :n], got) and bool((wide[:, n:] == 3.0).all())
+    x[0, 3], x[m // 2, 1], w[n - 1, k - 1], w[7, 5] = float("inf"), float("nan"), -float("inf"), 3e38
+    x[m - 1, :] *= 2.0
+    odd_x.copy_(x)
+    got, other = ops32.linear(x, w), ops32.linear(odd_x, w)
+    finite = torch.isfinite(other)
+    assert torch.equal(torch.isnan(got), torch.isnan(other)) and torch.equal(torch.isposinf(got), torch.isposinf(other))
+    assert torch.equal(torch.isfinite(got), finite) and int(ops32.status.flatten()[0]) == 0
+    bound = 2 * k * EPS * (x.double().abs() @ w.double().abs().T)
+    assert bool(((got.double() - other.double()).abs() <= bound)[finite].all())
+
+
 def _relative(got, ref):
     return float((got.double() - ref).norm() / ref.norm())
 
