@@ -246,7 +246,7 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __
   constexpr int PAGE_STAGE = 256;
   __shared__ int box_pages[PAGE_STAGE];
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const bool softmax_thread = tid < SOFTMAX_THREADS;
 
   // Tensor memory first: while a block holds the allocation permit no other block of the
@@ -276,7 +276,7 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
 
   // Work = (query tile, key/value head, slice of the group's heads).  The blocks of the
   // launch (two an SM) take the first items by their index and draw the rest from a
@@ -439,7 +439,7 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __
             const int page = box_pages[staged];
             const int gt = base + t, stage = gt & 1;
             if (page >= 0) {
-              if (lane == 0) {
+              if (elect_one()) {
                 const int slot = tile_pos(t) & (page_size - 1);
                 unsigned char* kb = Ks + stage * STAGE_BYTES;
                 unsigned char* vb = Vs + stage * STAGE_BYTES;
@@ -480,7 +480,7 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __
         // One thread issues everything; products run in the order of issue, so the S
         // that overwrites the columns of the S / P two tiles back follows that tile's O
         // by itself.
-        if (lane == 0) {
+        if (elect_one()) {
           const uint64_t q_desc = smem_desc(Qs, 16), k_desc = smem_desc(Ks, 16), v_desc = smem_desc(Vs, KV_HALF);
           auto issue_s = [&](int t) {
             const int gt = base + t, stage = gt & 1;

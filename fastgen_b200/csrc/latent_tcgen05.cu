@@ -100,7 +100,7 @@ latent_attention_tc5_kernel(const __grid_constant__ CUtensorMap map, const __nv_
   __shared__ uint32_t tmem_base_s;
   __shared__ int gave_up;  // set by a wait that ran out: the waits after it return at once (see mbar_wait)
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   // the tiles are in ascending order of work and are handed out from the list's end
   const int slices = (n_heads + heads_per_block - 1) / heads_per_block * NSPLIT;
   const int tile = n_tiles_total - 1 - (int)blockIdx.x / slices;
@@ -141,7 +141,7 @@ latent_attention_tc5_kernel(const __grid_constant__ CUtensorMap map, const __nv_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
   const int k_end = pos[tok0] + ntok;  // tokens of a tile are consecutive positions
   const int n_tiles = (k_end + TILE_KEYS - 1) / TILE_KEYS;
 
@@ -232,7 +232,7 @@ latent_attention_tc5_kernel(const __grid_constant__ CUtensorMap map, const __nv_
       // ================================ MMA warp ================================
       // One thread issues everything; products run in the order of issue, so the S that overwrites the
       // columns of the S / P two tiles back follows that tile's P C by itself.
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_S = instr_desc(TILE_KEYS, false), IDESC_O = instr_desc(RO, true);
         const uint64_t q_desc = smem_desc(Qs, 16), k_desc = smem_desc(Ks, 16);
         const uint64_t c_desc = smem_desc(Ks + half * (RO / 64) * K_GROUP, K_GROUP);
