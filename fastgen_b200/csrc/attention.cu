@@ -3,7 +3,7 @@
 // size a model needs.
 #include <string.h>
 
-#include "attention_simt.cuh"
+#include "attention_f32.cuh"
 
 #ifndef FG_HEAD_DIM
 #error "compile with -DFG_HEAD_DIM=<head size>"
@@ -68,6 +68,69 @@ extern "C" int fg_attention_simt(const void* q, int q_stride, void* out, int out
     FG_CHECK_ARG(false, "fg_attention_simt: bad dtype %d", dtype);
   }
   FG_CHECK_LAUNCH("fg_attention_simt");
+  return 0;
+}
+
+// The rows of a block of fg_attention_f32_prompt: tiles hold max(1, rows / min(group, rows)) tokens.  16: that entry is not
+// there for this head size (its tiles would not fit shared memory), fg_attention_simt takes such prompts.
+extern "C" int fg_attention_f32_prompt_rows() { return FG_HEAD_DIM <= 128 ? fg_attn::P_ROWS : fg_attn::ROWS; }
+
+// Prompt tiles in float32; pools start on 16 bytes.  Entries of request -1 or without tokens are padding.
+extern "C" int fg_attention_f32_prompt(const float* q, int q_stride, float* out, int out_stride, const float* k_pages,
+                                       const float* v_pages, const int* block_table, int table_width, int page_size,
+                                       int n_pages, const int* pos, const int* tile_req, const int* tile_tok0,
+                                       const int* tile_ntok, int n_tiles, int n_heads, int n_kv_heads, int head_dim,
+                                       int window, int keep_first, float scale, float softcap, const float* sinks,
+                                       int* status, cudaStream_t stream) {
+  using namespace fg_attn;
+  if (n_tiles == 0) return 0;
+  FG_CHECK_ARG(head_dim == FG_HEAD_DIM && head_dim <= 128, "fg_attention_f32_prompt: library built for head size %d, got %d",
+               FG_HEAD_DIM, head_dim);
+  FG_CHECK_ARG(n_kv_heads > 0 && n_heads % n_kv_heads == 0 && n_kv_heads <= 65535,
+               "fg_attention_f32_prompt: %d heads over %d kv heads", n_heads, n_kv_heads);
+  FG_CHECK_ARG((((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0, "fg_attention_f32_prompt: pools off 16 bytes");
+#if FG_HEAD_DIM <= 128
+  const int group = n_heads / n_kv_heads, hpb = group < P_ROWS ? group : P_ROWS;
+  auto kern = attention_prompt_f32_kernel<FG_HEAD_DIM>;
+  constexpr size_t bytes = PromptShape<FG_HEAD_DIM>::SMEM;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  FG_CHECK_ARG(e == cudaSuccess, "fg_attention_f32_prompt: shared memory: %s", cudaGetErrorString(e));
+  const int slices = (group + hpb - 1) / hpb;
+  const long items = (long)n_tiles * n_kv_heads * slices;
+  FG_CHECK_ARG(items < (1l << 31), "fg_attention_f32_prompt: %d tiles are too many", n_tiles);
+  kern<<<(unsigned)items, 128, bytes, stream>>>(q, q_stride, out, out_stride, k_pages, v_pages, block_table, table_width,
+                                                page_size, n_pages, pos, tile_req, tile_tok0, tile_ntok, n_kv_heads, group, hpb,
+                                                window, keep_first, scale, status, softcap, sinks, n_tiles, slices,
+                                                fg_sm_count());
+  FG_CHECK_LAUNCH("fg_attention_f32_prompt");
+#endif
+  return 0;
+}
+
+// Single tokens in float32; pools start on 16 bytes.  `req_of`: the slot of every token of the step (negative: none); the
+// rows of such a token in the list are zeroed.
+extern "C" int fg_attention_f32_singles(const float* q, int q_stride, float* out, int out_stride, const float* k_pages,
+                                        const float* v_pages, const int* block_table, int table_width, int page_size,
+                                        int n_pages, const int* pos, const int* req_of, const int* single_req,
+                                        const int* single_tok, int n_singles, int n_heads, int n_kv_heads, int head_dim,
+                                        int window, int keep_first, float scale, float softcap, const float* sinks,
+                                        int* status, cudaStream_t stream) {
+  using namespace fg_attn;
+  if (n_singles == 0) return 0;
+  FG_CHECK_ARG(head_dim == FG_HEAD_DIM, "fg_attention_f32_singles: library built for head size %d, got %d", FG_HEAD_DIM,
+               head_dim);
+  FG_CHECK_ARG(n_kv_heads > 0 && n_heads % n_kv_heads == 0 && n_kv_heads <= 65535,
+               "fg_attention_f32_singles: %d heads over %d kv heads", n_heads, n_kv_heads);
+  FG_CHECK_ARG((((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0, "fg_attention_f32_singles: pools off 16 bytes");
+  const int group = n_heads / n_kv_heads;
+  auto kern = attention_single_f32_kernel<FG_HEAD_DIM>;
+  constexpr size_t bytes = SingleShape<FG_HEAD_DIM>::SMEM;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  FG_CHECK_ARG(e == cudaSuccess, "fg_attention_f32_singles: shared memory: %s", cudaGetErrorString(e));
+  fg_launch_pdl(kern, dim3(n_singles, n_kv_heads, (group + S_ROWS - 1) / S_ROWS), dim3(S_THREADS), bytes, stream, q, q_stride,
+                out, out_stride, k_pages, v_pages, block_table, table_width, page_size, n_pages, pos, req_of, single_req,
+                single_tok, n_kv_heads, group, window, keep_first, scale, status, softcap, sinks);
+  FG_CHECK_LAUNCH("fg_attention_f32_singles");
   return 0;
 }
 

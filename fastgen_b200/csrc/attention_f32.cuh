@@ -1,0 +1,483 @@
+// Paged causal attention in float32 for prompts in tiles of 64 rows, and for single tokens.  Every score, weight and output
+// is the sum of attention_simt.cuh in the same order (tiles of 32 keys from position 0, running maximum and sum a tile,
+// keys in ascending order), bit for bit: a token's result does not depend on which of the kernels computes it.
+// A key that a row does not see contributes nothing to it here, whatever its value holds.
+//
+// Pools start on 16 bytes (head sizes are multiples of 16 numbers, so that all rows do).
+#pragma once
+
+#include "attention_simt.cuh"
+
+namespace fg_attn {
+
+__device__ __forceinline__ void cp_async_row16(float* dst, const float* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(ok ? 16 : 0)
+               : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Prompts: a block holds 64 rows (tokens x heads of a group), a thread the scores of 4 rows x 4 keys and the outputs of the
+// same 4 rows x HD / 8 columns, so that only keys and values meet at a barrier (one a tile; the next tile's arrive by
+// asynchronous copies meanwhile).  What bounds it is shared memory: 8 reads of 16 bytes for 64 multiply-adds.
+// 777 tokens, 32 / 8 heads of 64: 16 rows a block (attention_simt.cuh) 250 us, here FIXME.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int P_ROWS = 64;
+
+template <int HD>
+struct PromptShape {
+  static constexpr int HP = HD + 4, PP = KEYS + 4;
+  static constexpr size_t SMEM = sizeof(float) * ((P_ROWS + 4 * KEYS) * HP + P_ROWS * PP);
+};
+
+template <int HD>
+__global__ void __launch_bounds__(128)
+attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, int out_stride,
+                            const float* __restrict__ k_pages, const float* __restrict__ v_pages,
+                            const int* __restrict__ block_table, int table_width, int page_size, int n_pages,
+                            const int* __restrict__ pos, const int* __restrict__ tile_req,
+                            const int* __restrict__ tile_tok0, const int* __restrict__ tile_ntok, int n_kv_heads,
+                            int group, int heads_per_block, int window, int keep_first, float scale, int* status,
+                            float softcap, const float* __restrict__ sinks, int n_tiles, int slices, int wave) {
+  constexpr int HP = PromptShape<HD>::HP, PP = PromptShape<HD>::PP;
+  extern __shared__ __align__(16) float smem_f[];
+  float* const Qs = smem_f;                 // [P_ROWS][HP]
+  float* const Ks = Qs + P_ROWS * HP;       // [2][KEYS][HP]
+  float* const Vs = Ks + 2 * KEYS * HP;     // [2][KEYS][HP]
+  float* const Ps = Vs + 2 * KEYS * HP;     // [P_ROWS][PP]; -1: a key that the row does not see
+  __shared__ int key_ok[2][KEYS];
+
+  // The list is in ascending order of keys: the longest tiles first.  The launch's blocks are mostly on the chip at once,
+  // `wave` of them side by side: every second such run goes backwards, or the SM with the longest block of one had the
+  // longest of all (777 tokens: 183 us instead of FIXME2).
+  const int run = blockIdx.x / wave, in_run = blockIdx.x % wave;
+  const int item = (run & 1) && (run + 1) * wave <= gridDim.x ? run * wave + wave - 1 - in_run : blockIdx.x;
+  const int tile = n_tiles - 1 - item / (n_kv_heads * slices), g = item % n_kv_heads, sub = item / n_kv_heads % slices;
+  const int b = tile_req[tile], tok0 = tile_tok0[tile], ntok = tile_ntok[tile];
+  if (b < 0 || ntok <= 0) return;  // padding of a captured list
+  const int tid = threadIdx.x;
+  auto row_token = [&](int r) { return r / heads_per_block; };
+  auto row_head = [&](int r) { return sub * heads_per_block + (r % heads_per_block); };
+  auto row_valid = [&](int r) { return row_token(r) < ntok && row_head(r) < group; };
+  for (int i = tid; i < P_ROWS * HD; i += 128) {
+    const int r = i / HD, d = i - r * HD;
+    Qs[r * HP + d] = row_valid(r) ? q[(size_t)(tok0 + row_token(r)) * q_stride + (g * group + row_head(r)) * HD + d] : 0.f;
+  }
+  // the tokens of a tile are consecutive positions of one request
+  const int min_pos = pos[tok0], max_pos = min_pos + ntok - 1;
+  const int lo_min = first_visible(min_pos, window);
+  int k_win = 0, k_keep_end = 0;  // tiles between the kept positions and the window are skipped
+  if (window != 0) {
+    k_win = lo_min / KEYS * KEYS;
+    k_keep_end = min(k_win, (max(keep_first, 0) + KEYS - 1) / KEYS * KEYS);
+  }
+  auto settle = [&](int k0) { return k0 >= k_keep_end && k0 < k_win ? k_win : k0; };
+
+  // a thread copies a quarter of one key's row (and of its value's)
+  const int ck = tid >> 2, cp = tid & 3;
+  auto page_of = [&](int k0) {
+    const int j = k0 + ck;
+    if (j > max_pos) return -1;
+    const int logical = j / page_size;
+    return logical < table_width ? block_table[(size_t)b * table_width + logical] : -1;
+  };
+  auto issue = [&](int k0, int page, int buf) {
+    const int j = k0 + ck;
+    const bool ok = j <= max_pos && page >= 0 && page < n_pages;
+    // a key some row must see has no page
+    if (!ok && j <= max_pos && (j >= lo_min || j < keep_first) && cp == 0 && status) atomicOr(status, FG_STATUS_BAD_PAGE);
+    const size_t base = ok ? (((size_t)page * n_kv_heads + g) * page_size + j % page_size) * HD : 0;
+#pragma unroll
+    for (int i = cp; i < HD / 4; i += 4) {
+      cp_async_row16(Ks + (buf * KEYS + ck) * HP + i * 4, k_pages + base + i * 4, ok);
+      cp_async_row16(Vs + (buf * KEYS + ck) * HP + i * 4, v_pages + base + i * 4, ok);
+    }
+    if (cp == 0) key_ok[buf][ck] = ok;
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+
+  // this thread's rows rg + 16 i, keys kg + 8 j of a tile, columns 32 c + 4 kg (and two of the last 16 of an odd HD / 16)
+  const int rg = tid >> 3, kg = tid & 7;
+  constexpr int QUADS = HD / 32, REST = HD % 32 != 0 ? 2 : 0;
+  float m_run[4], l_run[4];
+  int p_row[4], lo_row[4];
+  float4 o4[4][QUADS > 0 ? QUADS : 1];
+  float2 o2[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = rg + 16 * i;
+    p_row[i] = row_valid(r) ? min_pos + row_token(r) : -1;
+    lo_row[i] = first_visible(p_row[i], window);
+    m_run[i] = -INFINITY;
+    l_run[i] = 0.f;
+    if (sinks != nullptr && row_head(r) < group) {
+      m_run[i] = sinks[g * group + row_head(r)];
+      l_run[i] = 1.f;
+    }
+#pragma unroll
+    for (int c = 0; c < QUADS; ++c) o4[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    o2[i] = make_float2(0.f, 0.f);
+  }
+
+  int k0 = settle(0), buf = 0;
+  issue(k0, page_of(k0), 0);
+  int next = settle(k0 + KEYS);
+  int next_page = page_of(next);
+  while (k0 <= max_pos) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // the tile has landed for all, and the other buffer is read by nobody
+    if (next <= max_pos) issue(next, next_page, buf ^ 1);
+    const int after = settle(next + KEYS);
+    next_page = page_of(after);
+    // whether some row does not see some key of the tile (rows without a query are computed and not stored)
+    const bool masked = k0 + KEYS - 1 > min_pos || (window != 0 && k0 < first_visible(max_pos, window));
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+    const float* kt = Ks + buf * KEYS * HP;
+#pragma unroll 2
+    for (int d = 0; d < HD; d += 4) {
+      float4 kv[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const float4*>(kt + (kg + 8 * j) * HP + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 qv = *reinterpret_cast<const float4*>(Qs + (rg + 16 * i) * HP + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(qv.x, kv[j].x, s[i][j]);
+          s[i][j] = fmaf(qv.y, kv[j].y, s[i][j]);
+          s[i][j] = fmaf(qv.z, kv[j].z, s[i][j]);
+          s[i][j] = fmaf(qv.w, kv[j].w, s[i][j]);
+        }
+      }
+    }
+    float al[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      bool visible[4];
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = k0 + kg + 8 * j;
+        visible[j] = key_ok[buf][kg + 8 * j] != 0 && key <= p_row[i] && (key >= lo_row[i] || key < keep_first);
+        float sc = s[i][j] * scale;
+        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+        s[i][j] = visible[j] ? sc : -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const float m_new = fmaxf(m_run[i], mx);
+      float pr[4] = {0.f, 0.f, 0.f, 0.f};
+      al[i] = 1.f;
+      if (m_new != -INFINITY) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) pr[j] = visible[j] ? expf(s[i][j] - m_new) : 0.f;
+        al[i] = m_run[i] == -INFINITY ? 0.f : expf(m_run[i] - m_new);
+      }
+      // the tree of a warp's sum over 32 keys: distances 16, 8, 4, 2, 1
+      float sum = (pr[0] + pr[2]) + (pr[1] + pr[3]);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l_run[i] = l_run[i] * al[i] + sum;
+      m_run[i] = m_new;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) Ps[(rg + 16 * i) * PP + kg + 8 * j] = visible[j] || !masked ? pr[j] : -1.f;
+    }
+    __syncwarp();  // a row's weights are written and read by the same eight lanes
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int c = 0; c < QUADS; ++c)
+        o4[i][c] = make_float4(o4[i][c].x * al[i], o4[i][c].y * al[i], o4[i][c].z * al[i], o4[i][c].w * al[i]);
+      o2[i] = make_float2(o2[i].x * al[i], o2[i].y * al[i]);
+    }
+    const float* vt = Vs + buf * KEYS * HP;
+    auto add = [&](bool guarded) {
+#pragma unroll 1
+      for (int c = 0; c < KEYS; c += 4) {
+        float4 p4[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p4[i] = *reinterpret_cast<const float4*>(Ps + (rg + 16 * i) * PP + c);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float4 v[QUADS > 0 ? QUADS : 1];
+          float2 vr = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int n = 0; n < QUADS; ++n) v[n] = *reinterpret_cast<const float4*>(vt + (c + e) * HP + 32 * n + 4 * kg);
+          if (REST) vr = *reinterpret_cast<const float2*>(vt + (c + e) * HP + 32 * QUADS + 2 * kg);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float pr = e == 0 ? p4[i].x : e == 1 ? p4[i].y : e == 2 ? p4[i].z : p4[i].w;
+            if (guarded && pr < 0.f) continue;
+#pragma unroll
+            for (int n = 0; n < QUADS; ++n) {
+              o4[i][n].x = fmaf(pr, v[n].x, o4[i][n].x);
+              o4[i][n].y = fmaf(pr, v[n].y, o4[i][n].y);
+              o4[i][n].z = fmaf(pr, v[n].z, o4[i][n].z);
+              o4[i][n].w = fmaf(pr, v[n].w, o4[i][n].w);
+            }
+            if (REST) {
+              o2[i].x = fmaf(pr, vr.x, o2[i].x);
+              o2[i].y = fmaf(pr, vr.y, o2[i].y);
+            }
+          }
+        }
+      }
+    };
+    if (masked)
+      add(true);
+    else
+      add(false);
+    k0 = next;
+    next = after;
+    buf ^= 1;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = rg + 16 * i;
+    if (!row_valid(r)) continue;
+    const float inv = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
+    float* o = out + (size_t)(tok0 + row_token(r)) * out_stride + (g * group + row_head(r)) * HD;
+#pragma unroll
+    for (int c = 0; c < QUADS; ++c) {
+      float* at = o + 32 * c + 4 * kg;
+      at[0] = o4[i][c].x * inv;
+      at[1] = o4[i][c].y * inv;
+      at[2] = o4[i][c].z * inv;
+      at[3] = o4[i][c].w * inv;
+    }
+    if (REST) {
+      o[32 * QUADS + 2 * kg] = o2[i].x * inv;
+      o[32 * QUADS + 2 * kg + 1] = o2[i].y * inv;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Single tokens: a block holds one token and up to S_ROWS heads of a group.  The walk over the keys is a chain only in the
+// outputs' sums: eight tiles of 32 keys are scored at once, a warp each (a lane a key), their maxima meet in shared memory,
+// every warp finds the running maximum that its tile starts from, and only then the outputs walk the 256 keys, four rows a
+// thread side by side.  The next tiles' keys come by asynchronous copies during that walk, their values behind it.
+// 5 tokens on 100 to 500 keys, 32 / 8 heads of 64: tile after tile (attention_simt.cuh) 34 us, here FIXME.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int S_ROWS = 8, S_TILES = 8, S_KEYS = S_TILES * KEYS, S_THREADS = 256;
+
+template <int HD>
+struct SingleShape {
+  static constexpr int TILES = HD <= 80 ? S_TILES : HD <= 160 ? S_TILES / 2 : S_TILES / 4;  // what shared memory holds
+  static constexpr int CHUNK = TILES * KEYS, KP = HD + 4;  // padded rows of keys: eight lanes read eight bank groups
+  static constexpr size_t SMEM = sizeof(float) * (CHUNK * (HD + KP) + S_ROWS * HD + CHUNK * S_ROWS);
+};
+
+template <int HD>
+__global__ void __launch_bounds__(S_THREADS)
+attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_stride, const float* k_pages,
+                            const float* v_pages, const int* __restrict__ block_table, int table_width, int page_size,
+                            int n_pages, const int* __restrict__ pos, const int* __restrict__ req_of,
+                            const int* __restrict__ single_req, const int* __restrict__ single_tok, int n_kv_heads,
+                            int group, int window, int keep_first, float scale, int* status, float softcap,
+                            const float* __restrict__ sinks) {
+  constexpr int TILES = SingleShape<HD>::TILES, CHUNK = SingleShape<HD>::CHUNK, KP = SingleShape<HD>::KP;
+  extern __shared__ __align__(16) float smem_f[];
+  float* const Vs = smem_f;                 // [CHUNK][HD]
+  float* const Ks = Vs + CHUNK * HD;        // [CHUNK][KP]
+  float* const Qs = Ks + CHUNK * KP;        // [S_ROWS][HD]
+  float* const Ps = Qs + S_ROWS * HD;       // [CHUNK][S_ROWS]; -1: a key that is not seen
+  __shared__ __align__(16) float max_s[TILES][S_ROWS], sum_s[TILES][S_ROWS], al_s[TILES][S_ROWS], l_s[S_ROWS];
+  __shared__ unsigned row_s[2][CHUNK];  // the keys' rows in the pools, of this run of tiles and of the next
+
+  const int g = blockIdx.y, head0 = blockIdx.z * S_ROWS, rows = min(S_ROWS, group - head0);
+  const int b = single_req[blockIdx.x], tok = single_tok[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float* const o = out + (size_t)tok * out_stride + (size_t)(g * group + head0) * HD;
+  pdl_trigger();
+  pdl_wait();
+  if (b < 0) {
+    // padding of a fixed-size batch: no request; the rows of a token that belongs to none are zeroed
+    if (req_of[tok] < 0)
+      for (int i = tid; i < rows * HD; i += S_THREADS) o[i] = 0.f;
+    return;
+  }
+  const int p = pos[tok], lo = first_visible(p, window);
+  int k_win = 0, kept = 0;  // tiles: those of the kept positions, then the window's
+  if (window != 0) {
+    k_win = lo / KEYS;
+    kept = min(k_win, (max(keep_first, 0) + KEYS - 1) / KEYS);
+  }
+  const int n_tiles = kept + p / KEYS - k_win + 1;
+  auto tile_pos = [&](int t) { return (t < kept ? t : t - kept + k_win) * KEYS; };
+  // the walk's last tile and the window's edges hold keys that are not seen: the same ones for all rows
+  auto masked = [&](int t) {
+    const int first = tile_pos(t);
+    return first + KEYS - 1 > p || (first < lo && first + KEYS > keep_first);
+  };
+  // the row of a key in the pools
+  constexpr unsigned NONE = 0xffffffffu;
+  auto key_row = [&](int t, int key) -> unsigned {
+    const int j = tile_pos(t) + key;
+    if (t >= n_tiles || j > p) return NONE;
+    const int logical = j / page_size;
+    const int page = logical < table_width ? block_table[(size_t)b * table_width + logical] : -1;
+    if (page < 0 || page >= n_pages) {
+      if ((j >= lo || j < keep_first) && status) atomicOr(status, FG_STATUS_BAD_PAGE);
+      return NONE;
+    }
+    return ((unsigned)page * n_kv_heads + g) * page_size + j % page_size;
+  };
+  for (int i = tid; i < S_ROWS * HD; i += S_THREADS)
+    Qs[i] = i < rows * HD ? q[(size_t)tok * q_stride + (size_t)(g * group + head0) * HD + i] : 0.f;
+
+  // every thread keeps the running maxima; the sums' and outputs' state: thread -> column, four rows
+  float m_run[S_ROWS];
+#pragma unroll
+  for (int r = 0; r < S_ROWS; ++r) m_run[r] = sinks != nullptr && r < rows ? sinks[g * group + head0 + r] : -INFINITY;
+  float l_run = sinks != nullptr ? 1.f : 0.f;  // of row `tid` (tid < S_ROWS)
+  constexpr int SLOTS = (2 * HD + S_THREADS - 1) / S_THREADS;  // (column, four rows) pairs a thread
+  float acc[SLOTS][4];
+#pragma unroll
+  for (int u = 0; u < SLOTS; ++u)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[u][r] = 0.f;
+
+  auto look_up = [&](int t0, int buf) {
+    for (int i = tid; i < CHUNK; i += S_THREADS) row_s[buf][i] = key_row(t0 + i / KEYS, i % KEYS);
+  };
+  auto copy = [&](float* dst, int stride, const float* pool, int buf, int tiles) {
+    for (int i = tid; i < tiles * KEYS * (HD / 4); i += S_THREADS) {
+      const int key = i / (HD / 4), c = i % (HD / 4) * 4;
+      const unsigned row = row_s[buf][key];
+      cp_async_row16(dst + key * stride + c, pool + (row != NONE ? (size_t)row * HD + c : 0), row != NONE);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  int buf = 0;
+  look_up(0, 0);
+  __syncthreads();  // (and the queries)
+  copy(Ks, KP, k_pages, 0, min(TILES, n_tiles));
+  for (int t0 = 0; t0 < n_tiles; t0 += TILES, buf ^= 1) {
+    const int tiles = min(TILES, n_tiles - t0), t = t0 + warp;
+    copy(Vs, HD, v_pages, buf, tiles);
+    if (t0 + TILES < n_tiles) look_up(t0 + TILES, buf ^ 1);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // the keys have landed for all
+    float s[S_ROWS];
+    bool visible = false;
+    if (warp < tiles) {
+#pragma unroll
+      for (int r = 0; r < S_ROWS; ++r) s[r] = 0.f;
+      const float* kr = Ks + (warp * KEYS + lane) * KP;
+#pragma unroll 4
+      for (int d = 0; d < HD; d += 4) {
+        const float4 kv = *reinterpret_cast<const float4*>(kr + d);
+#pragma unroll
+        for (int r = 0; r < S_ROWS; ++r) {
+          if (r >= rows) break;
+          const float4 qv = *reinterpret_cast<const float4*>(Qs + r * HD + d);
+          s[r] = fmaf(qv.x, kv.x, s[r]);
+          s[r] = fmaf(qv.y, kv.y, s[r]);
+          s[r] = fmaf(qv.z, kv.z, s[r]);
+          s[r] = fmaf(qv.w, kv.w, s[r]);
+        }
+      }
+      const int j = tile_pos(t) + lane;
+      visible = row_s[buf][warp * KEYS + lane] != NONE && j <= p && (j >= lo || j < keep_first);
+#pragma unroll
+      for (int r = 0; r < S_ROWS; ++r) {
+        if (r >= rows) break;
+        float sc = s[r] * scale;
+        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+        s[r] = visible ? sc : -INFINITY;
+        const float mx = warp_max(s[r]);
+        if (lane == 0) max_s[warp][r] = mx;
+      }
+    }
+    __syncthreads();
+    // the keys are read: the next ones are on their way during the rest (an empty group keeps the count where there are none)
+    if (t0 + TILES < n_tiles)
+      copy(Ks, KP, k_pages, buf ^ 1, min(TILES, n_tiles - t0 - TILES));
+    else
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < S_ROWS; ++r) {
+      if (r >= rows) break;
+      float m = m_run[r], before = m, here = m;  // the running maximum before and with this warp's tile
+      for (int u = 0; u < tiles; ++u) {
+        if (u == warp) before = m;
+        m = fmaxf(m, max_s[u][r]);
+        if (u == warp) here = m;
+      }
+      m_run[r] = m;
+      if (warp < tiles) {
+        float pr = 0.f, al = 1.f;
+        if (here != -INFINITY) {
+          pr = visible ? expf(s[r] - here) : 0.f;
+          al = before == -INFINITY ? 0.f : expf(before - here);
+        }
+        const float sum = warp_sum(pr);
+        Ps[(warp * KEYS + lane) * S_ROWS + r] = visible || !masked(t) ? pr : -1.f;
+        if (lane == 0) {
+          sum_s[warp][r] = sum;
+          al_s[warp][r] = al;
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // the values have landed, the weights are written
+    if (tid < rows)
+      for (int u = 0; u < tiles; ++u) l_run = l_run * al_s[u][tid] + sum_s[u][tid];
+#pragma unroll
+    for (int u = 0; u < SLOTS; ++u) {
+      const int at = tid + u * S_THREADS, col = at % HD, r0 = at / HD * 4;
+      if (r0 >= rows) continue;
+      for (int n = 0; n < tiles; ++n) {
+        const float4 al = *reinterpret_cast<const float4*>(&al_s[n][r0]);
+        acc[u][0] *= al.x;
+        acc[u][1] *= al.y;
+        acc[u][2] *= al.z;
+        acc[u][3] *= al.w;
+        const float* vt = Vs + n * KEYS * HD + col;
+        const float* pt = Ps + n * KEYS * S_ROWS + r0;
+        if (masked(t0 + n)) {
+          for (int k = 0; k < KEYS; ++k) {
+            const float4 pr = *reinterpret_cast<const float4*>(pt + k * S_ROWS);
+            if (pr.x < 0.f) continue;
+            const float v = vt[k * HD];
+            acc[u][0] = fmaf(pr.x, v, acc[u][0]);
+            acc[u][1] = fmaf(pr.y, v, acc[u][1]);
+            acc[u][2] = fmaf(pr.z, v, acc[u][2]);
+            acc[u][3] = fmaf(pr.w, v, acc[u][3]);
+          }
+        } else {
+#pragma unroll 16
+          for (int k = 0; k < KEYS; ++k) {
+            const float4 pr = *reinterpret_cast<const float4*>(pt + k * S_ROWS);
+            const float v = vt[k * HD];
+            acc[u][0] = fmaf(pr.x, v, acc[u][0]);
+            acc[u][1] = fmaf(pr.y, v, acc[u][1]);
+            acc[u][2] = fmaf(pr.z, v, acc[u][2]);
+            acc[u][3] = fmaf(pr.w, v, acc[u][3]);
+          }
+        }
+      }
+    }
+    __syncthreads();  // values, weights and maxima are free
+  }
+  if (tid < S_ROWS) l_s[tid] = l_run;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < SLOTS; ++u) {
+    const int at = tid + u * S_THREADS, col = at % HD, r0 = at / HD * 4;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (r0 + r < rows) {
+        const float l = l_s[r0 + r];
+        o[(r0 + r) * HD + col] = acc[u][r] * (l > 0.f ? 1.f / l : 0.f);
+      }
+  }
+}
+
+}  // namespace fg_attn

@@ -98,6 +98,11 @@ _CORE_SIGNATURES = {
 _ATTN_SIGNATURES = {
     "fg_attention_simt": [_P, _I, _P, _I, _I, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F,
                           _P, _P, _P],
+    "fg_attention_f32_prompt_rows": [],
+    "fg_attention_f32_prompt": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P,
+                                _P],
+    "fg_attention_f32_singles": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P,
+                                 _P],
     "fg_attention_sigmoid": [_P, _I, _P, _I, _I, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F,
                              _P, _P, _P, _P, _P],
     "fg_attention_sigmoid_prefill_tc5_bf16": [_P, _I, _P, _I, _P, _P, _I, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I,
@@ -1394,12 +1399,25 @@ class Ops:
                   k_pages.shape[0], _ptr(ctx.pos))
         keep_first = int(keep_first) if window > 0 else 0
         if q.dtype == torch.float32:
-            tiles = ctx.attention_tiles(attention_tiling(n_heads, n_kv_heads, SIMT_ROWS), 1)
-            _check(lib, lib.fg_attention_simt(
-                _ptr(q), q.stride(0), _ptr(out), out.stride(0), _code(q.dtype), *common,
-                _ptr(tiles.req), _ptr(tiles.tok0), _ptr(tiles.ntok), tiles.n,
-                n_heads, n_kv_heads, head_dim, window, keep_first, float(scale), float(softcap or 0.0),
-                _ptr(sinks), _ptr(self.status), _stream()))
+            rest = (n_heads, n_kv_heads, head_dim, window, keep_first, float(scale), float(softcap or 0.0), _ptr(sinks),
+                    _ptr(self.status), _stream())
+            rows, least = lib.fg_attention_f32_prompt_rows(), 2
+            if (k_pages.data_ptr() | v_pages.data_ptr()) % 16:
+                rows, least = SIMT_ROWS, 1  # numbers one by one, whatever the tokens
+            tiles = ctx.attention_tiles(attention_tiling(n_heads, n_kv_heads, rows), least)
+            if tiles.n and rows == SIMT_ROWS:
+                _check(lib, lib.fg_attention_simt(
+                    _ptr(q), q.stride(0), _ptr(out), out.stride(0), _code(q.dtype), *common,
+                    _ptr(tiles.req), _ptr(tiles.tok0), _ptr(tiles.ntok), tiles.n, *rest))
+            elif tiles.n:
+                _check(lib, lib.fg_attention_f32_prompt(
+                    _ptr(q), q.stride(0), _ptr(out), out.stride(0), *common,
+                    _ptr(tiles.req), _ptr(tiles.tok0), _ptr(tiles.ntok), tiles.n, *rest))
+            singles = ctx.single_tokens() if least == 2 else None
+            if singles is not None and singles.n:
+                _check(lib, lib.fg_attention_f32_singles(
+                    _ptr(q), q.stride(0), _ptr(out), out.stride(0), *common, _ptr(ctx.req),
+                    _ptr(singles.req), _ptr(singles.tok), singles.n, *rest))
             return False
         # windows that keep a sequence's first positions visible: the kernels walk the tiles of the kept
         # positions before those of the window (prompts: the tcgen05 kernel at head sizes 64 and 128 without a

@@ -265,6 +265,43 @@ def test_float32_attention_on_asynchronous_copies(ops32, hd, heads, kv, window, 
     assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all()) and int(status) == 0
 
 
+@pytest.mark.parametrize("hd,heads,kv", [(64, 8, 2), (16, 3, 3), (48, 20, 1), (128, 9, 3), (256, 4, 2), (80, 1, 1)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (40, 0), (40, 5), (300, 70), (-37, 0)])
+def test_float32_attention_by_tokens(ops32, hd, heads, kv, window, keep):
+    """Prompts in tiles of 64 rows and single tokens eight tiles at a time, beside each other: the bits of the kernel that
+    walks 16 rows (taken for pools off 16 bytes), and what lies behind a row's keys never reaches it."""
+    from types import SimpleNamespace
+    ctx, q, pools, table = _attention_step([1, 130, 1, 7, 1, 1, 2], [0, 0, 700, 31, 255, 31, 330], 16, heads, kv, hd,
+                                           torch.float32, hd + window)
+    slots = [s for s, n in zip(ctx.host_seq_slot, torch.tensor(ctx.host_seq_start).diff().tolist()) for _ in range(n)]
+    ctx.req = torch.tensor(slots, dtype=torch.int32, device=DEV)
+    how = dict(window=max(window, 0) or None, scale=hd ** -0.5, keep_first=keep, softcap=3.0 if keep == 5 else None,
+               sinks=torch.linspace(-1, 1, heads, device=DEV) if window else None, chunk=-window if window < 0 else None)
+    outs = []
+    for shift in (0, 1):
+        moved = []
+        for pool in pools:
+            room = torch.empty(pool.numel() + 4, device=DEV)
+            moved.append(room[shift : shift + pool.numel()].view(pool.shape))
+            moved[-1].copy_(pool)
+        memory = SimpleNamespace(k_pages=moved[0], v_pages=moved[1], block_table=table, page_size=16)
+        out = torch.full_like(q, float("nan"))
+        ops32.attention(q, out, memory, ctx, heads, kv, hd, **how)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all()) and int(ops32.status) == 0
+    if hd > 128:
+        return  # (such prompts stay on the kernel of 16 rows)
+    # the entry of position 129 of the request of 130 tokens: only its last token sees it
+    moved[0][int(table[1, 8]), :, 1], moved[1][int(table[1, 8]), :, 1] = float("nan"), float("inf")
+    aligned = [p.clone() for p in moved]
+    memory = SimpleNamespace(k_pages=aligned[0], v_pages=aligned[1], block_table=table, page_size=16)
+    again = torch.empty_like(q)
+    ops32.attention(q, again, memory, ctx, heads, kv, hd, **how)
+    keepers = torch.ones(q.shape[0], dtype=torch.bool, device=DEV)
+    keepers[130] = False
+    assert torch.equal(again[keepers], outs[0][keepers]) and not bool(torch.isfinite(again[130]).all())
+
+
 @pytest.mark.parametrize("page", [8, 64, 128])
 @pytest.mark.parametrize("keep,window", [(1, 64), (4, 100), (70, 130), (200, 65)])
 def test_kept_positions_in_the_tensor_memory_kernel(ops16, keep, window, page):
