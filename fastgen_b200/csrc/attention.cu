@@ -123,13 +123,18 @@ extern "C" int fg_attention_f32_singles(const float* q, int q_stride, float* out
                "fg_attention_f32_singles: %d heads over %d kv heads", n_heads, n_kv_heads);
   FG_CHECK_ARG((((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0, "fg_attention_f32_singles: pools off 16 bytes");
   const int group = n_heads / n_kv_heads;
-  auto kern = attention_single_f32_kernel<FG_HEAD_DIM>;
-  constexpr size_t bytes = SingleShape<FG_HEAD_DIM>::SMEM;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  FG_CHECK_ARG(e == cudaSuccess, "fg_attention_f32_singles: shared memory: %s", cudaGetErrorString(e));
-  fg_launch_pdl(kern, dim3(n_singles, n_kv_heads, (group + S_ROWS - 1) / S_ROWS), dim3(S_THREADS), bytes, stream, q, q_stride,
-                out, out_stride, k_pages, v_pages, block_table, table_width, page_size, n_pages, pos, req_of, single_req,
-                single_tok, n_kv_heads, group, window, keep_first, scale, status, softcap, sinks);
+  auto launch = [&](auto kern, int rows, size_t bytes) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    FG_CHECK_ARG(e == cudaSuccess, "fg_attention_f32_singles: shared memory: %s", cudaGetErrorString(e));
+    fg_launch_pdl(kern, dim3(n_singles, n_kv_heads, (group + rows - 1) / rows), dim3(S_THREADS), bytes, stream, q, q_stride,
+                  out, out_stride, k_pages, v_pages, block_table, table_width, page_size, n_pages, pos, req_of, single_req,
+                  single_tok, n_kv_heads, group, window, keep_first, scale, status, softcap, sinks);
+    return 0;
+  };
+  // groups of up to 4 heads without the work of 8
+  const int rc = group <= 4 ? launch(attention_single_f32_kernel<FG_HEAD_DIM, 4>, 4, SingleShape<FG_HEAD_DIM, 4>::SMEM)
+                            : launch(attention_single_f32_kernel<FG_HEAD_DIM, 8>, 8, SingleShape<FG_HEAD_DIM, 8>::SMEM);
+  if (rc) return rc;
   FG_CHECK_LAUNCH("fg_attention_f32_singles");
   return 0;
 }

@@ -20,7 +20,7 @@ __device__ __forceinline__ void cp_async_row16(float* dst, const float* src, boo
 // Prompts: a block holds 64 rows (tokens x heads of a group), a thread the scores of 4 rows x 4 keys and the outputs of the
 // same 4 rows x HD / 8 columns, so that only keys and values meet at a barrier (one a tile; the next tile's arrive by
 // asynchronous copies meanwhile).  What bounds it is shared memory: 8 reads of 16 bytes for 64 multiply-adds.
-// 777 tokens, 32 / 8 heads of 64: 16 rows a block (attention_simt.cuh) 250 us, here FIXME.
+// 777 tokens, 32 / 8 heads of 64: 16 rows a block (attention_simt.cuh) 245 us, here 145; 300 tokens 61 and 42, 60 tokens 11 and 11.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int P_ROWS = 64;
 
@@ -31,7 +31,7 @@ struct PromptShape {
 };
 
 template <int HD>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 3)
 attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, int out_stride,
                             const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                             const int* __restrict__ block_table, int table_width, int page_size, int n_pages,
@@ -49,7 +49,7 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
 
   // The list is in ascending order of keys: the longest tiles first.  The launch's blocks are mostly on the chip at once,
   // `wave` of them side by side: every second such run goes backwards, or the SM with the longest block of one had the
-  // longest of all (777 tokens: 183 us instead of FIXME2).
+  // longest of all (777 tokens: 183 us instead of 165 when this was measured).
   const int run = blockIdx.x / wave, in_run = blockIdx.x % wave;
   const int item = (run & 1) && (run + 1) * wave <= gridDim.x ? run * wave + wave - 1 - in_run : blockIdx.x;
   const int tile = n_tiles - 1 - item / (n_kv_heads * slices), g = item % n_kv_heads, sub = item / n_kv_heads % slices;
@@ -59,9 +59,18 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
   auto row_token = [&](int r) { return r / heads_per_block; };
   auto row_head = [&](int r) { return sub * heads_per_block + (r % heads_per_block); };
   auto row_valid = [&](int r) { return row_token(r) < ntok && row_head(r) < group; };
-  for (int i = tid; i < P_ROWS * HD; i += 128) {
-    const int r = i / HD, d = i - r * HD;
-    Qs[r * HP + d] = row_valid(r) ? q[(size_t)(tok0 + row_token(r)) * q_stride + (g * group + row_head(r)) * HD + d] : 0.f;
+  // two threads a row: copies of 16 bytes where the queries lie on them (waited for with the first tile), else one by one
+  {
+    const int r = tid >> 1;
+    const bool ok = row_valid(r);
+    const float* src = ok ? q + (size_t)(tok0 + row_token(r)) * q_stride + (size_t)(g * group + row_head(r)) * HD : q;
+    if (q_stride % 4 == 0 && ((uintptr_t)q & 15) == 0) {
+#pragma unroll
+      for (int d = (tid & 1) * 4; d < HD; d += 8) cp_async_row16(Qs + r * HP + d, ok ? src + d : q, ok);
+    } else {
+#pragma unroll 8
+      for (int d = tid & 1; d < HD; d += 2) Qs[r * HP + d] = ok ? src[d] : 0.f;
+    }
   }
   // the tokens of a tile are consecutive positions of one request
   const int min_pos = pos[tok0], max_pos = min_pos + ntok - 1;
@@ -73,26 +82,31 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
   }
   auto settle = [&](int k0) { return k0 >= k_keep_end && k0 < k_win ? k_win : k0; };
 
-  // a thread copies a quarter of one key's row (and of its value's)
+  // a thread copies a quarter of one key's row (and of its value's); where that row lies is looked up a tile ahead
+  constexpr unsigned NONE = 0xffffffffu;
   const int ck = tid >> 2, cp = tid & 3;
-  auto page_of = [&](int k0) {
+  auto row_of = [&](int k0) {
     const int j = k0 + ck;
-    if (j > max_pos) return -1;
+    if (j > max_pos) return NONE;
     const int logical = j / page_size;
-    return logical < table_width ? block_table[(size_t)b * table_width + logical] : -1;
-  };
-  auto issue = [&](int k0, int page, int buf) {
-    const int j = k0 + ck;
-    const bool ok = j <= max_pos && page >= 0 && page < n_pages;
-    // a key some row must see has no page
-    if (!ok && j <= max_pos && (j >= lo_min || j < keep_first) && cp == 0 && status) atomicOr(status, FG_STATUS_BAD_PAGE);
-    const size_t base = ok ? (((size_t)page * n_kv_heads + g) * page_size + j % page_size) * HD : 0;
-#pragma unroll
-    for (int i = cp; i < HD / 4; i += 4) {
-      cp_async_row16(Ks + (buf * KEYS + ck) * HP + i * 4, k_pages + base + i * 4, ok);
-      cp_async_row16(Vs + (buf * KEYS + ck) * HP + i * 4, v_pages + base + i * 4, ok);
+    const int page = logical < table_width ? block_table[(size_t)b * table_width + logical] : -1;
+    if (page < 0 || page >= n_pages) {
+      // a key some row must see has no page
+      if ((j >= lo_min || j < keep_first) && cp == 0 && status) atomicOr(status, FG_STATUS_BAD_PAGE);
+      return NONE;
     }
-    if (cp == 0) key_ok[buf][ck] = ok;
+    return ((unsigned)page * n_kv_heads + g) * page_size + (j - logical * page_size);
+  };
+  float* const k_dst = Ks + ck * HP + cp * 4;
+  float* const v_dst = Vs + ck * HP + cp * 4;
+  auto issue = [&](unsigned row, int buf) {
+    const size_t base = row != NONE ? (size_t)row * HD + cp * 4 : 0;
+#pragma unroll
+    for (int i = 0; i < HD / 16; ++i) {
+      cp_async_row16(k_dst + buf * KEYS * HP + i * 16, k_pages + base + i * 16, row != NONE);
+      cp_async_row16(v_dst + buf * KEYS * HP + i * 16, v_pages + base + i * 16, row != NONE);
+    }
+    if (cp == 0) key_ok[buf][ck] = row != NONE;
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
 
@@ -120,15 +134,15 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
   }
 
   int k0 = settle(0), buf = 0;
-  issue(k0, page_of(k0), 0);
+  issue(row_of(k0), 0);
   int next = settle(k0 + KEYS);
-  int next_page = page_of(next);
+  unsigned next_row = row_of(next);
   while (k0 <= max_pos) {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();  // the tile has landed for all, and the other buffer is read by nobody
-    if (next <= max_pos) issue(next, next_page, buf ^ 1);
+    if (next <= max_pos) issue(next_row, buf ^ 1);
     const int after = settle(next + KEYS);
-    next_page = page_of(after);
+    next_row = row_of(after);
     // whether some row does not see some key of the tile (rows without a query are computed and not stored)
     const bool masked = k0 + KEYS - 1 > min_pos || (window != 0 && k0 < first_visible(max_pos, window));
     float s[4][4];
@@ -154,39 +168,53 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
         }
       }
     }
-    float al[4];
+    // (no branches but the cap's, the same for all: the four rows' exponentials and exchanges run side by side)
+    unsigned visible = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool ok = key_ok[buf][kg + 8 * j] != 0;
+      const int key = k0 + kg + 8 * j;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        s[i][j] *= scale;
+        if (ok && key <= p_row[i] && (key >= lo_row[i] || key < keep_first)) visible |= 1u << (4 * i + j);
+      }
+    }
+    if (softcap > 0.f)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) s[i / 4][i % 4] = softcap * tanhf(s[i / 4][i % 4] / softcap);
+    float mx[4], al[4], sum[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      bool visible[4];
-      float mx = -INFINITY;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int key = k0 + kg + 8 * j;
-        visible[j] = key_ok[buf][kg + 8 * j] != 0 && key <= p_row[i] && (key >= lo_row[i] || key < keep_first);
-        float sc = s[i][j] * scale;
-        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
-        s[i][j] = visible[j] ? sc : -INFINITY;
-        mx = fmaxf(mx, s[i][j]);
-      }
+      for (int j = 0; j < 4; ++j)
+        if (!(visible >> (4 * i + j) & 1)) s[i][j] = -INFINITY;
+      mx[i] = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+    }
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float m_new = fmaxf(m_run[i], mx);
-      float pr[4] = {0.f, 0.f, 0.f, 0.f};
-      al[i] = 1.f;
-      if (m_new != -INFINITY) {
+    for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) pr[j] = visible[j] ? expf(s[i][j] - m_new) : 0.f;
-        al[i] = m_run[i] == -INFINITY ? 0.f : expf(m_run[i] - m_new);
-      }
-      // the tree of a warp's sum over 32 keys: distances 16, 8, 4, 2, 1
-      float sum = (pr[0] + pr[2]) + (pr[1] + pr[3]);
+      for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], o));
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      l_run[i] = l_run[i] * al[i] + sum;
+    for (int i = 0; i < 4; ++i) {
+      const float m_new = fmaxf(m_run[i], mx[i]), base = m_new == -INFINITY ? 0.f : m_new;  // (-inf: no key so far)
+      al[i] = m_run[i] == -INFINITY ? (m_new == -INFINITY ? 1.f : 0.f) : expf(m_run[i] - base);
       m_run[i] = m_new;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) Ps[(rg + 16 * i) * PP + kg + 8 * j] = visible[j] || !masked ? pr[j] : -1.f;
+      for (int j = 0; j < 4; ++j) {
+        const bool seen = visible >> (4 * i + j) & 1;
+        s[i][j] = seen ? expf(s[i][j] - base) : 0.f;
+        Ps[(rg + 16 * i) * PP + kg + 8 * j] = seen || !masked ? s[i][j] : -1.f;
+      }
+      // the tree of a warp's sum over 32 keys: distances 16, 8, 4, 2, 1
+      sum[i] = (s[i][0] + s[i][2]) + (s[i][1] + s[i][3]);
     }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) l_run[i] = l_run[i] * al[i] + sum[i];
     __syncwarp();  // a row's weights are written and read by the same eight lanes
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -212,17 +240,17 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float pr = e == 0 ? p4[i].x : e == 1 ? p4[i].y : e == 2 ? p4[i].z : p4[i].w;
-            if (guarded && pr < 0.f) continue;
+            auto sum_up = [&](float value, float& o) { o = guarded && pr < 0.f ? o : fmaf(pr, value, o); };
 #pragma unroll
             for (int n = 0; n < QUADS; ++n) {
-              o4[i][n].x = fmaf(pr, v[n].x, o4[i][n].x);
-              o4[i][n].y = fmaf(pr, v[n].y, o4[i][n].y);
-              o4[i][n].z = fmaf(pr, v[n].z, o4[i][n].z);
-              o4[i][n].w = fmaf(pr, v[n].w, o4[i][n].w);
+              sum_up(v[n].x, o4[i][n].x);
+              sum_up(v[n].y, o4[i][n].y);
+              sum_up(v[n].z, o4[i][n].z);
+              sum_up(v[n].w, o4[i][n].w);
             }
             if (REST) {
-              o2[i].x = fmaf(pr, vr.x, o2[i].x);
-              o2[i].y = fmaf(pr, vr.y, o2[i].y);
+              sum_up(vr.x, o2[i].x);
+              sum_up(vr.y, o2[i].y);
             }
           }
         }
@@ -258,39 +286,40 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Single tokens: a block holds one token and up to S_ROWS heads of a group.  The walk over the keys is a chain only in the
-// outputs' sums: eight tiles of 32 keys are scored at once, a warp each (a lane a key), their maxima meet in shared memory,
+// Single tokens: a block holds one token and R heads of a group (as many as there are, rounded up to 4 or 8).  The walk over the keys is a chain only in the
+// outputs' sums: eight tiles of 32 keys are scored at once, two a warp, their maxima meet in shared memory,
 // every warp finds the running maximum that its tile starts from, and only then the outputs walk the 256 keys, four rows a
 // thread side by side.  The next tiles' keys come by asynchronous copies during that walk, their values behind it.
-// 5 tokens on 100 to 500 keys, 32 / 8 heads of 64: tile after tile (attention_simt.cuh) 34 us, here FIXME.
+// 5 tokens on 100 to 500 keys, 32 / 8 heads of 64: tile after tile (attention_simt.cuh) 38 us, here 16; one on 700 keys
+// 50 and 23, one on 20 5.6 and 5.5, 16 on 600 44 and 21.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int S_ROWS = 8, S_TILES = 8, S_KEYS = S_TILES * KEYS, S_THREADS = 256;
+constexpr int S_MAX_ROWS = 8, S_TILES = 8, S_THREADS = 256;
 
-template <int HD>
+template <int HD, int R>
 struct SingleShape {
   static constexpr int TILES = HD <= 80 ? S_TILES : HD <= 160 ? S_TILES / 2 : S_TILES / 4;  // what shared memory holds
   static constexpr int CHUNK = TILES * KEYS, KP = HD + 4;  // padded rows of keys: eight lanes read eight bank groups
-  static constexpr size_t SMEM = sizeof(float) * (CHUNK * (HD + KP) + S_ROWS * HD + CHUNK * S_ROWS);
+  static constexpr size_t SMEM = sizeof(float) * (CHUNK * (HD + KP) + R * HD + CHUNK * R);
 };
 
-template <int HD>
-__global__ void __launch_bounds__(S_THREADS)
+template <int HD, int R>
+__global__ void __launch_bounds__(S_THREADS, 1)
 attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_stride, const float* k_pages,
                             const float* v_pages, const int* __restrict__ block_table, int table_width, int page_size,
                             int n_pages, const int* __restrict__ pos, const int* __restrict__ req_of,
                             const int* __restrict__ single_req, const int* __restrict__ single_tok, int n_kv_heads,
                             int group, int window, int keep_first, float scale, int* status, float softcap,
                             const float* __restrict__ sinks) {
-  constexpr int TILES = SingleShape<HD>::TILES, CHUNK = SingleShape<HD>::CHUNK, KP = SingleShape<HD>::KP;
+  constexpr int TILES = SingleShape<HD, R>::TILES, CHUNK = SingleShape<HD, R>::CHUNK, KP = SingleShape<HD, R>::KP;
   extern __shared__ __align__(16) float smem_f[];
   float* const Vs = smem_f;                 // [CHUNK][HD]
   float* const Ks = Vs + CHUNK * HD;        // [CHUNK][KP]
-  float* const Qs = Ks + CHUNK * KP;        // [S_ROWS][HD]
-  float* const Ps = Qs + S_ROWS * HD;       // [CHUNK][S_ROWS]; -1: a key that is not seen
-  __shared__ __align__(16) float max_s[TILES][S_ROWS], sum_s[TILES][S_ROWS], al_s[TILES][S_ROWS], l_s[S_ROWS];
+  float* const Qs = Ks + CHUNK * KP;        // [R][HD]
+  float* const Ps = Qs + R * HD;       // [CHUNK][R]; -1: a key that is not seen
+  __shared__ __align__(16) float max_s[TILES][R], sum_s[TILES][R], al_s[TILES][R], l_s[R];
   __shared__ unsigned row_s[2][CHUNK];  // the keys' rows in the pools, of this run of tiles and of the next
 
-  const int g = blockIdx.y, head0 = blockIdx.z * S_ROWS, rows = min(S_ROWS, group - head0);
+  const int g = blockIdx.y, head0 = blockIdx.z * R, rows = min(R, group - head0);
   const int b = single_req[blockIdx.x], tok = single_tok[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* const o = out + (size_t)tok * out_stride + (size_t)(g * group + head0) * HD;
@@ -328,27 +357,29 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
     }
     return ((unsigned)page * n_kv_heads + g) * page_size + j % page_size;
   };
-  for (int i = tid; i < S_ROWS * HD; i += S_THREADS)
+  for (int i = tid; i < R * HD; i += S_THREADS)
     Qs[i] = i < rows * HD ? q[(size_t)tok * q_stride + (size_t)(g * group + head0) * HD + i] : 0.f;
 
   // every thread keeps the running maxima; the sums' and outputs' state: thread -> column, four rows
-  float m_run[S_ROWS];
+  float m_run[R];
 #pragma unroll
-  for (int r = 0; r < S_ROWS; ++r) m_run[r] = sinks != nullptr && r < rows ? sinks[g * group + head0 + r] : -INFINITY;
-  float l_run = sinks != nullptr ? 1.f : 0.f;  // of row `tid` (tid < S_ROWS)
-  constexpr int SLOTS = (2 * HD + S_THREADS - 1) / S_THREADS;  // (column, four rows) pairs a thread
-  float acc[SLOTS][4];
+  for (int r = 0; r < R; ++r) m_run[r] = sinks != nullptr && r < rows ? sinks[g * group + head0 + r] : -INFINITY;
+  float l_run = sinks != nullptr ? 1.f : 0.f;  // of row `tid` (tid < R)
+  constexpr int SLOTS = (R / 4 * (HD / 2) + S_THREADS - 1) / S_THREADS;  // (two columns, four rows) a thread
+  float2 acc[SLOTS][4];
 #pragma unroll
   for (int u = 0; u < SLOTS; ++u)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) acc[u][r] = 0.f;
+    for (int r = 0; r < 4; ++r) acc[u][r] = make_float2(0.f, 0.f);
 
   auto look_up = [&](int t0, int buf) {
     for (int i = tid; i < CHUNK; i += S_THREADS) row_s[buf][i] = key_row(t0 + i / KEYS, i % KEYS);
   };
   auto copy = [&](float* dst, int stride, const float* pool, int buf, int tiles) {
-    for (int i = tid; i < tiles * KEYS * (HD / 4); i += S_THREADS) {
-      const int key = i / (HD / 4), c = i % (HD / 4) * 4;
+#pragma unroll 4
+    for (int u = 0; u < CHUNK * (HD / 4) / S_THREADS; ++u) {
+      const int i = tid + u * S_THREADS, key = i / (HD / 4), c = i % (HD / 4) * 4;
+      if (key >= tiles * KEYS) break;
       const unsigned row = row_s[buf][key];
       cp_async_row16(dst + key * stride + c, pool + (row != NONE ? (size_t)row * HD + c : 0), row != NONE);
     }
@@ -359,41 +390,54 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
   __syncthreads();  // (and the queries)
   copy(Ks, KP, k_pages, 0, min(TILES, n_tiles));
   for (int t0 = 0; t0 < n_tiles; t0 += TILES, buf ^= 1) {
-    const int tiles = min(TILES, n_tiles - t0), t = t0 + warp;
+    const int tiles = min(TILES, n_tiles - t0);
     copy(Vs, HD, v_pages, buf, tiles);
     if (t0 + TILES < n_tiles) look_up(t0 + TILES, buf ^ 1);
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();  // the keys have landed for all
-    float s[S_ROWS];
-    bool visible = false;
-    if (warp < tiles) {
+    // a warp two tiles, a lane a key of each: a read of the queries serves both
+    const int w0 = warp * 2;
+    float s[2][R];
+    bool visible[2] = {false, false};
+    if (w0 < tiles) {
 #pragma unroll
-      for (int r = 0; r < S_ROWS; ++r) s[r] = 0.f;
-      const float* kr = Ks + (warp * KEYS + lane) * KP;
+      for (int r = 0; r < R; ++r) s[0][r] = s[1][r] = 0.f;
+      const float* kr = Ks + (w0 * KEYS + lane) * KP;
 #pragma unroll 4
       for (int d = 0; d < HD; d += 4) {
-        const float4 kv = *reinterpret_cast<const float4*>(kr + d);
+        const float4 ka = *reinterpret_cast<const float4*>(kr + d), kb = *reinterpret_cast<const float4*>(kr + KEYS * KP + d);
 #pragma unroll
-        for (int r = 0; r < S_ROWS; ++r) {
-          if (r >= rows) break;
+        for (int r = 0; r < R; ++r) {
           const float4 qv = *reinterpret_cast<const float4*>(Qs + r * HD + d);
-          s[r] = fmaf(qv.x, kv.x, s[r]);
-          s[r] = fmaf(qv.y, kv.y, s[r]);
-          s[r] = fmaf(qv.z, kv.z, s[r]);
-          s[r] = fmaf(qv.w, kv.w, s[r]);
+          s[0][r] = fmaf(qv.x, ka.x, s[0][r]);
+          s[1][r] = fmaf(qv.x, kb.x, s[1][r]);
+          s[0][r] = fmaf(qv.y, ka.y, s[0][r]);
+          s[1][r] = fmaf(qv.y, kb.y, s[1][r]);
+          s[0][r] = fmaf(qv.z, ka.z, s[0][r]);
+          s[1][r] = fmaf(qv.z, kb.z, s[1][r]);
+          s[0][r] = fmaf(qv.w, ka.w, s[0][r]);
+          s[1][r] = fmaf(qv.w, kb.w, s[1][r]);
         }
       }
-      const int j = tile_pos(t) + lane;
-      visible = row_s[buf][warp * KEYS + lane] != NONE && j <= p && (j >= lo || j < keep_first);
+      float mx[2][R];
 #pragma unroll
-      for (int r = 0; r < S_ROWS; ++r) {
-        if (r >= rows) break;
-        float sc = s[r] * scale;
-        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
-        s[r] = visible ? sc : -INFINITY;
-        const float mx = warp_max(s[r]);
-        if (lane == 0) max_s[warp][r] = mx;
+      for (int h = 0; h < 2; ++h) {
+        const int j = tile_pos(t0 + w0 + h) + lane;
+        visible[h] = w0 + h < tiles && row_s[buf][(w0 + h) * KEYS + lane] != NONE && j <= p && (j >= lo || j < keep_first);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          s[h][r] *= scale;
+          if (softcap > 0.f) s[h][r] = softcap * tanhf(s[h][r] / softcap);
+          mx[h][r] = s[h][r] = visible[h] ? s[h][r] : -INFINITY;
+        }
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 2 * R; ++r) mx[r / R][r % R] = fmaxf(mx[r / R][r % R], __shfl_xor_sync(0xffffffffu, mx[r / R][r % R], o));
+      if (lane == 0)
+#pragma unroll
+        for (int r = 0; r < 2 * R; ++r) max_s[w0 + r / R][r % R] = mx[r / R][r % R];
     }
     __syncthreads();
     // the keys are read: the next ones are on their way during the rest (an empty group keeps the count where there are none)
@@ -401,81 +445,92 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
       copy(Ks, KP, k_pages, buf ^ 1, min(TILES, n_tiles - t0 - TILES));
     else
       asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if (w0 < tiles) {
+      float before[2][R], sum[2][R];
 #pragma unroll
-    for (int r = 0; r < S_ROWS; ++r) {
-      if (r >= rows) break;
-      float m = m_run[r], before = m, here = m;  // the running maximum before and with this warp's tile
-      for (int u = 0; u < tiles; ++u) {
-        if (u == warp) before = m;
-        m = fmaxf(m, max_s[u][r]);
-        if (u == warp) here = m;
+      for (int r = 0; r < R; ++r) {
+        float m = m_run[r];
+#pragma unroll
+        for (int u = 0; u < TILES - 2; ++u) m = fmaxf(m, u < w0 ? max_s[u][r] : -INFINITY);
+        before[0][r] = m;
+        before[1][r] = fmaxf(m, max_s[w0][r]);
       }
-      m_run[r] = m;
-      if (warp < tiles) {
-        float pr = 0.f, al = 1.f;
-        if (here != -INFINITY) {
-          pr = visible ? expf(s[r] - here) : 0.f;
-          al = before == -INFINITY ? 0.f : expf(before - here);
-        }
-        const float sum = warp_sum(pr);
-        Ps[(warp * KEYS + lane) * S_ROWS + r] = visible || !masked(t) ? pr : -1.f;
-        if (lane == 0) {
-          sum_s[warp][r] = sum;
-          al_s[warp][r] = al;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const bool hide = w0 + h < tiles && masked(t0 + w0 + h);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float here = fmaxf(before[h][r], max_s[w0 + h][r]), base = here == -INFINITY ? 0.f : here;
+          const float pr = visible[h] ? expf(s[h][r] - base) : 0.f;
+          sum[h][r] = pr;
+          Ps[((w0 + h) * KEYS + lane) * R + r] = visible[h] || !hide ? pr : -1.f;
+          if (lane == 0)
+            al_s[w0 + h][r] = before[h][r] == -INFINITY ? (here == -INFINITY ? 1.f : 0.f) : expf(before[h][r] - base);
         }
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 2 * R; ++r) sum[r / R][r % R] += __shfl_xor_sync(0xffffffffu, sum[r / R][r % R], o);
+      if (lane == 0)
+#pragma unroll
+        for (int r = 0; r < 2 * R; ++r) sum_s[w0 + r / R][r % R] = sum[r / R][r % R];
     }
+#pragma unroll
+    for (int u = 0; u < TILES; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r) m_run[r] = fmaxf(m_run[r], u < tiles ? max_s[u][r] : -INFINITY);
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();  // the values have landed, the weights are written
-    if (tid < rows)
+    if (tid < R)
       for (int u = 0; u < tiles; ++u) l_run = l_run * al_s[u][tid] + sum_s[u][tid];
 #pragma unroll
     for (int u = 0; u < SLOTS; ++u) {
-      const int at = tid + u * S_THREADS, col = at % HD, r0 = at / HD * 4;
-      if (r0 >= rows) continue;
+      const int at = tid + u * S_THREADS, col = at % (HD / 2) * 2, r0 = at / (HD / 2) * 4;
+      if (r0 >= R) continue;
+      auto one_tile = [&](int n, bool guarded) {
+        const float* vt = Vs + n * KEYS * HD + col;
+        const float* pt = Ps + n * KEYS * R + r0;
+#pragma unroll 16
+        for (int k = 0; k < KEYS; ++k) {
+          const float4 pr = *reinterpret_cast<const float4*>(pt + k * R);
+          const float2 v = *reinterpret_cast<const float2*>(vt + k * HD);
+          if (guarded && pr.x < 0.f) continue;  // (the same for the whole block)
+          acc[u][0].x = fmaf(pr.x, v.x, acc[u][0].x);
+          acc[u][0].y = fmaf(pr.x, v.y, acc[u][0].y);
+          acc[u][1].x = fmaf(pr.y, v.x, acc[u][1].x);
+          acc[u][1].y = fmaf(pr.y, v.y, acc[u][1].y);
+          acc[u][2].x = fmaf(pr.z, v.x, acc[u][2].x);
+          acc[u][2].y = fmaf(pr.z, v.y, acc[u][2].y);
+          acc[u][3].x = fmaf(pr.w, v.x, acc[u][3].x);
+          acc[u][3].y = fmaf(pr.w, v.y, acc[u][3].y);
+        }
+      };
       for (int n = 0; n < tiles; ++n) {
         const float4 al = *reinterpret_cast<const float4*>(&al_s[n][r0]);
-        acc[u][0] *= al.x;
-        acc[u][1] *= al.y;
-        acc[u][2] *= al.z;
-        acc[u][3] *= al.w;
-        const float* vt = Vs + n * KEYS * HD + col;
-        const float* pt = Ps + n * KEYS * S_ROWS + r0;
-        if (masked(t0 + n)) {
-          for (int k = 0; k < KEYS; ++k) {
-            const float4 pr = *reinterpret_cast<const float4*>(pt + k * S_ROWS);
-            if (pr.x < 0.f) continue;
-            const float v = vt[k * HD];
-            acc[u][0] = fmaf(pr.x, v, acc[u][0]);
-            acc[u][1] = fmaf(pr.y, v, acc[u][1]);
-            acc[u][2] = fmaf(pr.z, v, acc[u][2]);
-            acc[u][3] = fmaf(pr.w, v, acc[u][3]);
-          }
-        } else {
-#pragma unroll 16
-          for (int k = 0; k < KEYS; ++k) {
-            const float4 pr = *reinterpret_cast<const float4*>(pt + k * S_ROWS);
-            const float v = vt[k * HD];
-            acc[u][0] = fmaf(pr.x, v, acc[u][0]);
-            acc[u][1] = fmaf(pr.y, v, acc[u][1]);
-            acc[u][2] = fmaf(pr.z, v, acc[u][2]);
-            acc[u][3] = fmaf(pr.w, v, acc[u][3]);
-          }
-        }
+        acc[u][0] = make_float2(acc[u][0].x * al.x, acc[u][0].y * al.x);
+        acc[u][1] = make_float2(acc[u][1].x * al.y, acc[u][1].y * al.y);
+        acc[u][2] = make_float2(acc[u][2].x * al.z, acc[u][2].y * al.z);
+        acc[u][3] = make_float2(acc[u][3].x * al.w, acc[u][3].y * al.w);
+        if (masked(t0 + n))
+          one_tile(n, true);
+        else
+          one_tile(n, false);
       }
     }
     __syncthreads();  // values, weights and maxima are free
   }
-  if (tid < S_ROWS) l_s[tid] = l_run;
+  if (tid < R) l_s[tid] = l_run;
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < SLOTS; ++u) {
-    const int at = tid + u * S_THREADS, col = at % HD, r0 = at / HD * 4;
+    const int at = tid + u * S_THREADS, col = at % (HD / 2) * 2, r0 = at / (HD / 2) * 4;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
       if (r0 + r < rows) {
-        const float l = l_s[r0 + r];
-        o[(r0 + r) * HD + col] = acc[u][r] * (l > 0.f ? 1.f / l : 0.f);
+        const float l = l_s[r0 + r], inv = l > 0.f ? 1.f / l : 0.f;
+        o[(r0 + r) * HD + col] = acc[u][r].x * inv;
+        o[(r0 + r) * HD + col + 1] = acc[u][r].y * inv;
       }
   }
 }
