@@ -198,34 +198,37 @@ latent_attention_tc5_kernel(const __grid_constant__ CUtensorMap map, const __nv_
       }
     }
   } else {
-    // the other warps bring the queries into the K-major operand layout (16-byte pieces, swizzled); rows
-    // without a query and columns from D on hold zeros
-    constexpr int PIECES = KSTEPS * 2;
-    const int first = warp == ISSUER ? tid - 32 : tid;  // 160 threads, without the load warp
-#pragma unroll 4
-    for (int i = first; i < TILE_ROWS * PIECES; i += N_THREADS - 32) {
-      const int r = i / PIECES, c = i - r * PIECES;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (row_valid(r)) {
-        const size_t tk = tok0 + row_token(r), hh = row_head(r);
-        if (c < R / 8) {
-          v = *reinterpret_cast<const uint4*>(qa + tk * qa_ts + hh * qa_hs + c * 8);
+    // The other warps bring the queries into the K-major operand layout (16-byte pieces, swizzled), a row at a time, all copies
+    // in flight at once; rows without a query and columns from D on hold zeros.  (A piece a thread at a time, each with its
+    // row's divisions, held a block up for 24,000 cycles: as long as 15 tiles of keys.  2,048 tokens, 32 heads, latents
+    // of 256 + 32: 125 -> 108 us.)
+    constexpr int PIECES = KSTEPS * 2, Q_WARPS = N_THREADS / 32 - 1;
+#pragma unroll 2
+    for (int r = warp == ISSUER ? LOADER : warp; r < TILE_ROWS; r += Q_WARPS) {
+      const bool ok = row_valid(r);
+      const size_t tk = ok ? tok0 + row_token(r) : 0, hh = ok ? row_head(r) : 0;
+      const __nv_bfloat16* const src_a = qa + tk * qa_ts + hh * qa_hs;
+      const __nv_bfloat16* const src_t = qt + tk * qt_ts + hh * qt_hs;
+      for (int c = lane; c < PIECES; c += 32) {
+        unsigned char* const dst = Qs + (c / 8) * Q_GROUP + swz(r, c % 8);
+        const int d0 = c * 8 - R;
+        if (d0 < 0) {
+          cp_async_16(dst, src_a + c * 8, ok);
+        } else if (qt_vec && d0 + 8 <= ROT) {
+          cp_async_16(dst, src_t + d0, ok);
         } else {
-          const __nv_bfloat16* src = qt + tk * qt_ts + hh * qt_hs;
-          const int d0 = c * 8 - R;
-          if (qt_vec && d0 + 8 <= ROT) {
-            v = *reinterpret_cast<const uint4*>(src + d0);
-          } else {
-            __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&v);
+          uint4 v = make_uint4(0u, 0u, 0u, 0u);
+          __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&v);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              if (d0 + k < ROT) e[k] = src[d0 + k];
-          }
+          for (int k = 0; k < 8; ++k)
+            if (ok && d0 + k < ROT) e[k] = src_t[d0 + k];
+          *reinterpret_cast<uint4*>(dst) = v;
         }
       }
-      *reinterpret_cast<uint4*>(Qs + (c / 8) * Q_GROUP + swz(r, c % 8)) = v;
     }
-    fence_async_smem();  // written by ordinary stores, read by the tensor core
+    cp_async_commit();
+    cp_async_wait<0>();
+    fence_async_smem();  // written by threads, read by the tensor core
     asm volatile("bar.sync 1, %0;\n" ::"n"(N_THREADS - 32) : "memory");
 
     if (warp == ISSUER) {
