@@ -145,8 +145,11 @@ __global__ void __launch_bounds__(128)
 rotate_part_kernel(T* x, long stride, const int* __restrict__ pos, const int* __restrict__ req,
                    const float* __restrict__ freqs, float magnitude, int n_heads, int head_size, int offset,
                    int rot_dims) {
+  pdl_trigger();
   const int t = blockIdx.x;
-  if (req[t] < 0) return;
+  const int slot = req[t];
+  pdl_wait();  // (every block: one that left before would let the next kernel pass the one before this)
+  if (slot < 0) return;
   turn_heads<T>(x + (size_t)t * stride, (float)pos[t], freqs, magnitude, n_heads, head_size, offset, rot_dims);
 }
 
@@ -195,8 +198,10 @@ latent_prepare_kernel(const T* src, long src_stride, const float* __restrict__ n
                       const float* __restrict__ q_norm, T* q_out, long q_out_stride, int q_dim, int n_heads,
                       int head_size) {
   __shared__ float scratch[32];
+  pdl_trigger();
   const int t = blockIdx.x;
   const int slot = req[t];
+  pdl_wait();  // (every block)
   if (slot < 0) return;
   if (blockIdx.y == 0)
     write_entry<T>(src + (size_t)t * src_stride, slot, pos[t], norm_w, eps, freqs, magnitude, pages, place, R, r, E, scratch);
@@ -357,11 +362,11 @@ extern "C" int fg_rotate_part(void* x, long stride, int dtype, const int* pos, c
   FG_CHECK_ARG(rot_dims % 2 == 0 && offset >= 0 && offset + rot_dims <= head_size,
                "fg_rotate_part: %d rotated dimensions at %d do not fit a head of %d", rot_dims, offset, head_size);
   if (dtype == FG_F32)
-    rotate_part_kernel<float><<<n_tokens, 128, 0, stream>>>((float*)x, stride, pos, req, freqs, magnitude, n_heads,
-                                                            head_size, offset, rot_dims);
+    fg_launch_pdl(rotate_part_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, (float*)x, stride, pos, req, freqs,
+                  magnitude, n_heads, head_size, offset, rot_dims);
   else if (dtype == FG_BF16)
-    rotate_part_kernel<__nv_bfloat16><<<n_tokens, 128, 0, stream>>>((__nv_bfloat16*)x, stride, pos, req, freqs,
-                                                                    magnitude, n_heads, head_size, offset, rot_dims);
+    fg_launch_pdl(rotate_part_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(128), 0, stream, (__nv_bfloat16*)x, stride, pos, req,
+                  freqs, magnitude, n_heads, head_size, offset, rot_dims);
   else
     FG_CHECK_ARG(false, "fg_rotate_part: bad dtype %d", dtype);
   FG_CHECK_LAUNCH("fg_rotate_part");
@@ -404,12 +409,12 @@ extern "C" int fg_latent_prepare(const void* src, long src_stride, int dtype, co
   const EntryPlace place{block_table, table_width, page_size, n_pages, status};
   const dim3 grid(n_tokens, 2);
   if (dtype == FG_F32)
-    latent_prepare_kernel<float><<<grid, 128, 0, stream>>>(
-        (const float*)src, src_stride, norm_w, eps, freqs, magnitude, (float*)pages, place, pos, req, R, r, E, (float*)q,
+    fg_launch_pdl(
+        latent_prepare_kernel<float>, grid, dim3(128), 0, stream, (const float*)src, src_stride, norm_w, eps, freqs, magnitude, (float*)pages, place, pos, req, R, r, E, (float*)q,
         q_stride, q_norm, (float*)q_out, q_out_stride, q_dim, n_heads, head_size);
   else if (dtype == FG_BF16)
-    latent_prepare_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>(
-        (const __nv_bfloat16*)src, src_stride, norm_w, eps, freqs, magnitude, (__nv_bfloat16*)pages, place, pos, req, R, r,
+    fg_launch_pdl(
+        latent_prepare_kernel<__nv_bfloat16>, grid, dim3(128), 0, stream, (const __nv_bfloat16*)src, src_stride, norm_w, eps, freqs, magnitude, (__nv_bfloat16*)pages, place, pos, req, R, r,
         E, (__nv_bfloat16*)q, q_stride, q_norm, (__nv_bfloat16*)q_out, q_out_stride, q_dim, n_heads, head_size);
   else
     FG_CHECK_ARG(false, "fg_latent_prepare: bad dtype %d", dtype);

@@ -48,15 +48,14 @@ static_assert(RW % 16 == 0, "a warp's output columns come in sixteens");
 constexpr size_t smem_bytes() { return sizeof(__nv_bfloat16) * (size_t)LD * (ROWS + 2 * KEYS); }
 
 __global__ void __launch_bounds__(NTHREADS)
-latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, long qa_ts, long qa_hs,
-                            const __nv_bfloat16* __restrict__ qt, long qt_ts, long qt_hs,
-                            __nv_bfloat16* __restrict__ out, long out_ts, long out_hs,
-                            const __nv_bfloat16* __restrict__ gate, long gate_ts,
-                            const __nv_bfloat16* __restrict__ pages, const int* __restrict__ block_table,
+latent_attention_mma_kernel(const __nv_bfloat16* qa, long qa_ts, long qa_hs, const __nv_bfloat16* qt, long qt_ts,
+                            long qt_hs, __nv_bfloat16* out, long out_ts, long out_hs, const __nv_bfloat16* gate,
+                            long gate_ts, const __nv_bfloat16* pages, const int* __restrict__ block_table,
                             int table_width, int page_size, int n_pages, const int* __restrict__ pos,
                             const int* __restrict__ tile_req, const int* __restrict__ tile_tok0,
                             const int* __restrict__ tile_ntok, int n_heads, int heads_per_block, float scale_log2,
-                            int n_splits, int keys_per_split, float* __restrict__ scratch, int* status) {
+                            int n_splits, int keys_per_split, float* scratch, int* status) {
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   __nv_bfloat16* Ks = Qs + ROWS * LD;  // 2 stages
@@ -73,6 +72,7 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, long qa_ts, lo
   auto row_valid = [&](int r) { return row_token(r) < ntok && row_head(r) < n_heads; };
   float* part_base = scratch + ((size_t)(tile * gridDim.y + sub) * ROWS) * n_splits * PART;
 
+  pdl_wait();
   if (b < 0) {
     // a tile of no request (padding of a captured step): its rows, if it names any, are zeroed
     if (n_splits == 1)
@@ -85,23 +85,33 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, long qa_ts, lo
     return;
   }
   if (tid < ROWS) row_pos[tid] = row_valid(tid) ? pos[tok0 + row_token(tid)] : -1;
-  // queries -> shared memory: [qa | qt | zeros], zero rows where the tile is not full; asynchronous
-  // 4-byte copies, all in flight at once (a tile of single tokens is mostly this load)
-  for (int i = tid; i < ROWS * (D16 / 2); i += NTHREADS) {
-    const int r = i / (D16 / 2), col = 2 * (i - r * (D16 / 2));
-    const bool ok = row_valid(r) && col < D;
-    const __nv_bfloat16* src = qa;
-    if (ok) {
-      const size_t tk = tok0 + row_token(r), hh = row_head(r);
-      src = col < R ? qa + tk * qa_ts + hh * qa_hs + col : qt + tk * qt_ts + hh * qt_hs + (col - R);
-    }
-    const int bytes = ok ? 4 : 0;  // 0: zero-filled, nothing is read
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(Qs + r * LD + col)), "l"(src), "r"(bytes)
-                 : "memory");
+  // queries -> shared memory: [qa | qt | zeros], zero rows where the tile is not full: a warp a row, asynchronous copies of
+  // 16 bytes where the rows lie on them (else of 4), all in flight at once beside the first keys'.  (A piece a thread at a
+  // time, each with its row's divisions, was two thirds of a launch of single tokens: 4 tokens on 210 keys, 32 heads,
+  // latents of 256 + 32: 17 -> 11 us.)
+  const bool a_vec = (qa_ts | qa_hs) % 8 == 0 && ((uintptr_t)qa & 15) == 0;
+  const bool t_vec = ROT % 8 == 0 && (qt_ts | qt_hs) % 8 == 0 && ((uintptr_t)qt & 15) == 0;
+  auto copy_4 = [&](__nv_bfloat16* dst, const __nv_bfloat16* src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 4 : 0) : "memory");
+  };
+  for (int r = warp; r < ROWS; r += NTHREADS / 32) {
+    const bool ok = row_valid(r);
+    const size_t tk = ok ? tok0 + row_token(r) : 0, hh = ok ? row_head(r) : 0;
+    const __nv_bfloat16* const src_a = qa + tk * qa_ts + hh * qa_hs;
+    const __nv_bfloat16* const src_t = qt + tk * qt_ts + hh * qt_hs;
+    __nv_bfloat16* const dst = Qs + r * LD;
+    if (a_vec)
+      for (int c = lane * 8; c < R; c += 256) cp_async_16(dst + c, ok ? src_a + c : qa, ok);
+    else
+      for (int c = lane * 2; c < R; c += 64) copy_4(dst + c, ok ? src_a + c : qa, ok);
+    if (t_vec)
+      for (int c = lane * 8; c < ROT; c += 256) cp_async_16(dst + R + c, ok ? src_t + c : qt, ok);
+    else
+      for (int c = lane * 2; c < ROT; c += 64) copy_4(dst + R + c, ok ? src_t + c : qt, ok);
+    for (int c = lane * 2; c < D16 - D; c += 64) copy_4(dst + D + c, qa, false);
   }
   cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
+  __syncthreads();  // (the rows' positions)
   int max_pos = -1;
   for (int r = 0; r < ROWS; r += heads_per_block) max_pos = max(max_pos, row_pos[r]);  // rows are ordered by token
   const int k_first = split * keys_per_split;
@@ -130,6 +140,8 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, long qa_ts, lo
     __syncthreads();
     issue(0);
     if (n_tiles > 1) offsets(1);
+  } else {
+    cp_async_wait<0>();  // (a stretch without keys: nothing of this block's is in flight when it leaves)
   }
   __syncthreads();  // tile 1's offsets are read by every thread when its copies are issued
 
@@ -236,15 +248,17 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, long qa_ts, lo
 // The stretches of a row, merged in ascending order: out = sum_s o_s 2^(m_s - m) / sum_s l_s 2^(m_s - m),
 // times the gate.  One block a (tile, head slice, row).
 __global__ void __launch_bounds__(128)
-latent_merge_kernel(const float* __restrict__ scratch, __nv_bfloat16* __restrict__ out, long out_ts, long out_hs,
-                    const __nv_bfloat16* __restrict__ gate, long gate_ts, const int* __restrict__ tile_req,
+latent_merge_kernel(const float* scratch, __nv_bfloat16* out, long out_ts, long out_hs, const __nv_bfloat16* gate, long gate_ts, const int* __restrict__ tile_req,
                     const int* __restrict__ tile_tok0, const int* __restrict__ tile_ntok, int n_heads,
                     int heads_per_block, int n_splits, int n_subs) {
   const int r = blockIdx.x % ROWS;
   const int ts = blockIdx.x / ROWS;  // tile * n_subs + sub
   const int tile = ts / n_subs, sub = ts - tile * n_subs;
   const int tok = r / heads_per_block, head = sub * heads_per_block + r % heads_per_block;
-  if (tok >= tile_ntok[tile] || head >= n_heads) return;
+  pdl_trigger();
+  const bool mine = tok < tile_ntok[tile] && head < n_heads;
+  pdl_wait();  // (every block: one that left before would let the next kernel pass the one before this)
+  if (!mine) return;
   const size_t tk = tile_tok0[tile] + tok;
   __nv_bfloat16* dst = out + tk * out_ts + (size_t)head * out_hs;
   if (tile_req[tile] < 0) {
@@ -327,16 +341,14 @@ extern "C" int fg_latent_attention_mma(const void* qa, long qa_ts, long qa_hs, c
     attr_set = true;
   }
   dim3 grid(n_tiles, subs, n_splits);
-  latent_attention_mma_kernel<<<grid, NTHREADS, smem, stream>>>(
-      (const __nv_bfloat16*)qa, qa_ts, qa_hs, (const __nv_bfloat16*)qt, qt_ts, qt_hs, (__nv_bfloat16*)out, out_ts,
-      out_hs, (const __nv_bfloat16*)gate, gate_ts, (const __nv_bfloat16*)pages, block_table, table_width, page_size,
-      n_pages, pos, tile_req, tile_tok0, tile_ntok, n_heads, hpb, scale * 1.4426950408889634f, n_splits,
-      keys_per_split, scratch, status);
+  fg_launch_pdl(latent_attention_mma_kernel, grid, dim3(NTHREADS), smem, stream, (const __nv_bfloat16*)qa, qa_ts, qa_hs,
+                (const __nv_bfloat16*)qt, qt_ts, qt_hs, (__nv_bfloat16*)out, out_ts, out_hs, (const __nv_bfloat16*)gate, gate_ts,
+                (const __nv_bfloat16*)pages, block_table, table_width, page_size, n_pages, pos, tile_req, tile_tok0, tile_ntok,
+                n_heads, hpb, scale * 1.4426950408889634f, n_splits, keys_per_split, scratch, status);
   FG_CHECK_LAUNCH("fg_latent_attention_mma");
   if (n_splits > 1) {
-    latent_merge_kernel<<<n_tiles * subs * ROWS, 128, 0, stream>>>(scratch, (__nv_bfloat16*)out, out_ts, out_hs,
-                                                                   (const __nv_bfloat16*)gate, gate_ts, tile_req,
-                                                                   tile_tok0, tile_ntok, n_heads, hpb, n_splits, subs);
+    fg_launch_pdl(latent_merge_kernel, dim3(n_tiles * subs * ROWS), dim3(128), 0, stream, scratch, (__nv_bfloat16*)out, out_ts,
+                  out_hs, (const __nv_bfloat16*)gate, gate_ts, tile_req, tile_tok0, tile_ntok, n_heads, hpb, n_splits, subs);
     FG_CHECK_LAUNCH("fg_latent_merge");
   }
   return 0;

@@ -117,11 +117,12 @@ __device__ __forceinline__ void conv_store4(__nv_bfloat16* p, float4 v) {
 
 template <typename T, typename TO, bool SILU>
 __global__ void __launch_bounds__(CONV_THREADS)
-conv4_silu_kernel(const T* __restrict__ in, long in_stride, TO* __restrict__ out, long out_stride,
-                  const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ state,
+conv4_silu_kernel(const T* in, long in_stride, TO* out, long out_stride, const float* __restrict__ w,
+                  const float* __restrict__ bias, const float* state,
                   long state_stride, long conv_offset, const int* __restrict__ req, int n_tokens, int channels) {
   constexpr int TAPS = 4, BACK = TAPS - 1;
   const int c = (blockIdx.y * CONV_THREADS + threadIdx.x) * 4;
+  pdl_trigger();
   if (c >= channels) return;
   const int t0 = blockIdx.x * CONV_RUN;
   int rq[CONV_RUN + BACK];  // rq[j]: the slot of token t0 - BACK + j
@@ -138,6 +139,7 @@ conv4_silu_kernel(const T* __restrict__ in, long in_stride, TO* __restrict__ out
   for (int e = 0; e < 4; ++e)
     *reinterpret_cast<float4*>(wk[e]) = *reinterpret_cast<const float4*>(w + (size_t)(c + e) * TAPS);
   const float4 bc = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  pdl_wait();  // (the weights and the slots are the step's from its start)
   auto emit = [&](int t, const float4& v0, const float4& v1, const float4& v2, const float4& v3) {
     float r[4] = {bc.x, bc.y, bc.z, bc.w};
     const float x[TAPS][4] = {{v0.x, v0.y, v0.z, v0.w}, {v1.x, v1.y, v1.z, v1.w}, {v2.x, v2.y, v2.z, v2.w}, {v3.x, v3.y, v3.z, v3.w}};
@@ -180,11 +182,13 @@ conv4_silu_kernel(const T* __restrict__ in, long in_stride, TO* __restrict__ out
 // The state's convolution inputs after the step: the last taps-1 of (old inputs, new inputs).
 template <typename T>
 __global__ void __launch_bounds__(CONV_THREADS)
-conv_state_kernel(const T* __restrict__ in, long in_stride, float* __restrict__ state, long state_stride,
+conv_state_kernel(const T* in, long in_stride, float* state, long state_stride,
                   long conv_offset, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                   int channels, int taps) {
   const int c = blockIdx.y * CONV_THREADS + threadIdx.x;
+  pdl_trigger();
   const int slot = seq_slot[blockIdx.x];
+  pdl_wait();  // (every block)
   if (c >= channels || slot < 0) return;
   const int start = seq_start[blockIdx.x], n = seq_start[blockIdx.x + 1] - start;
   float* st = state + (size_t)slot * state_stride + conv_offset;
@@ -347,11 +351,12 @@ constexpr int TS_THREADS = 32 * TS_WARPS;
 
 template <typename T, int NPT>
 __global__ void __launch_bounds__(TS_THREADS)
-ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* __restrict__ dt_raw, long dt_stride,
+ssm_scan_tiled_kernel(const float* xbc, long xbc_stride, const T* dt_raw, long dt_stride,
                       const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-                      const float* __restrict__ d_skip, float* __restrict__ y, long y_stride,
-                      float* __restrict__ state, long state_stride, const int* __restrict__ seq_slot,
+                      const float* __restrict__ d_skip, float* y, long y_stride,
+                      float* state, long state_stride, const int* __restrict__ seq_slot,
                       const int* __restrict__ seq_start, int heads, int groups, int P, int most) {
+  pdl_trigger();
   constexpr int N = 32 * NPT;
   constexpr int STAGE = 2 * SCAN_TOKENS * N + SCAN_TOKENS * SCAN_PB + 2 * SCAN_TOKENS;  // floats
   extern __shared__ __align__(16) float smem[];
@@ -361,6 +366,7 @@ ssm_scan_tiled_kernel(const float* __restrict__ xbc, long xbc_stride, const T* _
   auto decs = [&](int buf) { return dts(buf) + SCAN_TOKENS; };
 
   const int slot = seq_slot[blockIdx.x];
+  pdl_wait();  // (every block: one that left before would let the next kernel pass the one before this)
   if (slot < 0) return;
   const int start = seq_start[blockIdx.x], n_tok = seq_start[blockIdx.x + 1] - start;
   if (n_tok <= 0 || n_tok > most) return;  // (more than `most`: ssm_chunk_kernel's)
@@ -873,12 +879,14 @@ gated_part_norm_warp_kernel(const float* __restrict__ y, long y_stride, const T*
 // its 67 MB take 10).
 template <typename T, int ITEMS>
 __global__ void __launch_bounds__(GW_WARPS * 32)
-gated_part_norm_whole_kernel(const float* __restrict__ y, long y_stride, const T* __restrict__ z, long z_stride,
-                             const float* __restrict__ w, T* __restrict__ out, long out_stride,
+gated_part_norm_whole_kernel(const float* y, long y_stride, const T* z, long z_stride,
+                             const float* __restrict__ w, T* out, long out_stride,
                              const int* __restrict__ req, int n_tokens, int parts, float eps) {
   constexpr int PART = ITEMS * 32;
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const long item = (long)blockIdx.x * GW_WARPS + (threadIdx.x >> 5);
+  pdl_wait();
   if (item >= (long)n_tokens * parts) return;
   const int t = item / parts, c0 = (int)(item - (long)t * parts) * PART;
   if (req[t] < 0) return;
@@ -920,11 +928,11 @@ static int launch_time_conv(const T* in, long proj_stride, TO* out, long out_str
                      (((uintptr_t)w | (uintptr_t)bias | (uintptr_t)state) & 15) == 0;
   const dim3 fgrid((n_tokens + CONV_RUN - 1) / CONV_RUN, (channels / 4 + CONV_THREADS - 1) / CONV_THREADS);
   if (fours && act)
-    conv4_silu_kernel<T, TO, true><<<fgrid, CONV_THREADS, 0, stream>>>(in, proj_stride, out, out_stride, w, bias, state,
-                                                                       state_stride, conv_offset, req, n_tokens, channels);
+    fg_launch_pdl(conv4_silu_kernel<T, TO, true>, fgrid, dim3(CONV_THREADS), 0, stream, in, proj_stride, out, out_stride, w,
+                  bias, state, state_stride, conv_offset, req, n_tokens, channels);
   else if (fours)
-    conv4_silu_kernel<T, TO, false><<<fgrid, CONV_THREADS, 0, stream>>>(in, proj_stride, out, out_stride, w, bias, state,
-                                                                        state_stride, conv_offset, req, n_tokens, channels);
+    fg_launch_pdl(conv4_silu_kernel<T, TO, false>, fgrid, dim3(CONV_THREADS), 0, stream, in, proj_stride, out, out_stride, w,
+                  bias, state, state_stride, conv_offset, req, n_tokens, channels);
   else if (act)
     conv_silu_kernel<T, TO, true><<<grid, CONV_THREADS, 0, stream>>>(in, proj_stride, out, out_stride, w, bias, state,
                                                                      state_stride, conv_offset, req, n_tokens, channels,
@@ -935,8 +943,8 @@ static int launch_time_conv(const T* in, long proj_stride, TO* out, long out_str
                                                                       channels, taps);
   FG_CHECK_LAUNCH("fg_time_conv");
   if (taps > 1)
-    conv_state_kernel<T><<<sgrid, CONV_THREADS, 0, stream>>>(in, proj_stride, state, state_stride, conv_offset, seq_slot,
-                                                             seq_start, channels, taps);
+    fg_launch_pdl(conv_state_kernel<T>, sgrid, dim3(CONV_THREADS), 0, stream, in, proj_stride, state, state_stride, conv_offset,
+                  seq_slot, seq_start, channels, taps);
   FG_CHECK_LAUNCH("fg_time_conv (state)");
   return 0;
 }
@@ -1015,9 +1023,8 @@ static int launch_scan(const float* xbc, long xbc_stride, const T* dt_raw, long 
   do {                                                                                                          \
     auto kern = ssm_scan_tiled_kernel<T, NPT>;                                                                  \
     if (tsmem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem); \
-    kern<<<grid, TS_THREADS, tsmem, stream>>>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, d_skip, y,    \
-                                              y_stride, state, state_stride, seq_slot, seq_start, heads,        \
-                                              groups, P, most);                                                 \
+    fg_launch_pdl(kern, grid, dim3(TS_THREADS), tsmem, stream, xbc, xbc_stride, dt_raw, dt_stride, dt_bias,     \
+                  a_log, d_skip, y, y_stride, state, state_stride, seq_slot, seq_start, heads, groups, P, most); \
   } while (0)
     if (N == 64) TILED(2);
     else if (N == 128) TILED(4);
@@ -1087,8 +1094,8 @@ extern "C" int fg_gated_part_norm(const float* y, long y_stride, const void* z, 
   if ((dtype == FG_F32 || dtype == FG_BF16) && (part == 128 || part == 256 || part == 512 || part == 1024)) {
     const int blocks = (int)(((long)n_tokens * parts + GW_WARPS - 1) / GW_WARPS);
 #define GATED(T, I)                                                                                                       \
-  gated_part_norm_whole_kernel<T, I><<<blocks, GW_WARPS * 32, 0, stream>>>(y, y_stride, (const T*)z, z_stride, w, (T*)out, \
-                                                                           out_stride, req, n_tokens, parts, eps)
+  fg_launch_pdl(gated_part_norm_whole_kernel<T, I>, dim3(blocks), dim3(GW_WARPS * 32), 0, stream, y, y_stride, (const T*)z, \
+                z_stride, w, (T*)out, out_stride, req, n_tokens, parts, eps)
 #define GATED_I(T)                      \
   do {                                  \
     if (part == 128) GATED(T, 4);       \
