@@ -47,6 +47,21 @@ __device__ __forceinline__ void lnp_store4(__nv_bfloat16* p, const float* v) {
   *reinterpret_cast<uint2*>(p) = r;
 }
 
+// a norm's weight (or bias: zeros where there is none) for a thread's runs of four columns
+template <int QUADS>
+__device__ __forceinline__ void lnp_weights(float* r, const float* p, int dim) {
+#pragma unroll
+  for (int q = 0; q < QUADS; ++q) {
+    const int d = 4 * ((int)threadIdx.x + LNP_THREADS * q);
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p != nullptr && d < dim) f = __ldg(reinterpret_cast<const float4*>(p + d));
+    r[4 * q] = f.x;
+    r[4 * q + 1] = f.y;
+    r[4 * q + 2] = f.z;
+    r[4 * q + 3] = f.w;
+  }
+}
+
 // VEC: a thread owns QUADS runs of four columns (a multiple of four columns, everything aligned), else
 // 4 * QUADS columns LNP_THREADS apart.
 template <typename TD, typename TO, int QUADS, bool VEC>
@@ -57,6 +72,17 @@ layer_norm_pair_kernel(float* h, LnpTerms terms, const float* __restrict__ wc, c
   __shared__ float scratch[32];
   constexpr int N = 4 * QUADS;
   pdl_trigger();
+  // the norms' weights are the model's: in runs of four columns, and those of a row of up to 2,048 columns on their way
+  // before the wait (column by column, behind the sums that they meet, they were 32 reads of 16 lines each: 1,501 rows of
+  // 2,048 columns 14.9 -> 12.4 us)
+  constexpr bool EARLY = VEC && QUADS <= 2;
+  float weight[N], bias[N], weight2[N], bias2[N];
+  if (EARLY) {
+    lnp_weights<QUADS>(weight, wc, dim);
+    lnp_weights<QUADS>(bias, bc, dim);
+    lnp_weights<QUADS>(weight2, w, dim);
+    lnp_weights<QUADS>(bias2, b, dim);
+  }
   pdl_wait();
   const int tid = threadIdx.x;
   const size_t base = (size_t)(rows ? rows[blockIdx.x] : (int)blockIdx.x) * dim, obase = (size_t)blockIdx.x * dim;
@@ -120,11 +146,15 @@ layer_norm_pair_kernel(float* h, LnpTerms terms, const float* __restrict__ wc, c
   };
   float mean, rstd;
   moments(v, eps_c, mean, rstd);
+  if (VEC && !EARLY) {
+    lnp_weights<QUADS>(weight, wc, dim);
+    lnp_weights<QUADS>(bias, bc, dim);
+  }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const int d = column(i);
-    if (d >= dim) continue;
-    x[i] += (v[i] - mean) * rstd * wc[d] + (bc != nullptr ? bc[d] : 0.f);
+    if (!VEC && d >= dim) continue;
+    x[i] += (v[i] - mean) * rstd * (VEC ? weight[i] : wc[d]) + (VEC ? bias[i] : bc != nullptr ? bc[d] : 0.f);
   }
   if (rows == nullptr) {
 #pragma unroll
@@ -142,10 +172,14 @@ layer_norm_pair_kernel(float* h, LnpTerms terms, const float* __restrict__ wc, c
     }
   }
   moments(x, eps, mean, rstd);
+  if (VEC && !EARLY) {
+    lnp_weights<QUADS>(weight2, w, dim);
+    lnp_weights<QUADS>(bias2, b, dim);
+  }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const int d = column(i);
-    if (d < dim) v[i] = (x[i] - mean) * rstd * w[d] + (b != nullptr ? b[d] : 0.f);
+    if (VEC || d < dim) v[i] = (x[i] - mean) * rstd * (VEC ? weight2[i] : w[d]) + (VEC ? bias2[i] : b != nullptr ? b[d] : 0.f);
   }
 #pragma unroll
   for (int q = 0; q < QUADS; ++q) {
@@ -198,7 +232,7 @@ extern "C" int fg_layer_norm_pair(float* h, const void* const* deltas, const flo
   FG_CHECK_ARG(wc != nullptr && w != nullptr && out != nullptr, "fg_layer_norm_pair: a norm needs its weight");
   LnpTerms terms;
   terms.n = n_terms;
-  bool vec = dim % 4 == 0 && ((uintptr_t)h & 15) == 0 && ((uintptr_t)out & 15) == 0;
+  bool vec = dim % 4 == 0 && (((uintptr_t)h | (uintptr_t)out | (uintptr_t)wc | (uintptr_t)bc | (uintptr_t)w | (uintptr_t)b) & 15) == 0;
   for (int i = 0; i < LNP_MAX_TERMS; ++i) {
     terms.delta[i] = i < n_terms ? deltas[i] : nullptr;
     terms.coef[i] = i < n_terms ? coefs[i] : 0.f;
