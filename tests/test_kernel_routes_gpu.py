@@ -846,3 +846,57 @@ def test_embedding_rows(ops32, dtype, dim, copies):
     want = torch.zeros(5, dim, device=DEV)
     want[:3] = table[tokens[:3].long()].float() * torch.tensor(0.7, device=DEV)
     assert torch.equal(out, want[:, None].expand(5, copies, dim)) and int(status) == 2  # STATUS_BAD_TOKEN
+
+
+# -- the selective scan -------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("inner,N", [(70, 16), (33, 5), (256, 16)])
+def test_selective_scan_in_parts(ops16, inner, N):
+    """Sequences from 768 tokens on run in parts of 384, shorter ones beside them token by token: the outputs and states of
+    the same sequences brought in portions (which are too short for parts), and the states no further from float64."""
+    g = torch.Generator().manual_seed(inner + N)
+    lengths, order = [767, 768, 0, 1501, 1, 1153], [4, 0, -1, 5, 1, 2]
+    starts = [0]
+    for n in lengths:
+        starts.append(starts[-1] + n)
+    t = starts[-1]
+    x, dt, z, low = (_randn(g, t, n).to(torch.bfloat16) for n in (inner, inner, inner, 2 * N + 8))
+    bias, skip = _randn(g, inner) - 2.0, _randn(g, inner)
+    a = -_randn(g, inner, N).exp()
+    state0 = _randn(g, 6, inner * N + 12)
+
+    def run(state, parts):
+        """``parts``: (first token, tokens, slot) of a step's sequences."""
+        begin, end = parts[0][0], parts[-1][0] + parts[-1][1]
+        ctx = SimpleNamespace(n_seqs=len(parts), longest=None,
+                              seq_slot=torch.tensor([p[2] for p in parts], dtype=torch.int32, device=DEV),
+                              seq_start=torch.tensor([p[0] - begin for p in parts] + [end - begin], dtype=torch.int32, device=DEV))
+        rows = slice(begin, end)
+        return ops16.selective_scan(x[rows], dt[rows], low[rows], 8, z[rows], bias, a, skip, state, ctx, N)
+
+    whole, cut = state0.clone(), state0.clone()
+    y = run(whole, list(zip(starts, lengths, order)))
+    for s, n, slot in zip(starts, lengths, order):
+        for at in range(0, n, 700):
+            m = min(700, n - at)
+            part = run(cut, [(s + at, m, slot)])
+            # (one rounding to bfloat16 of sums that differ in their last bits)
+            assert torch.allclose(part.float(), y[s + at : s + at + m].float(), rtol=2.0 ** -7, atol=1e-3), (s, at)
+    assert torch.equal(whole[3], state0[3]) and torch.equal(whole[:, inner * N :], state0[:, inner * N :])
+    assert torch.equal(whole[4], cut[4]) and torch.equal(whole[1], cut[1])  # the short ones: the same walk
+    errors = []
+    for state in (whole, cut):
+        off = total = 0.0
+        for s, n, slot in zip(starts, lengths, order):
+            if n < 768:
+                continue
+            S = state0[slot, : inner * N].double().view(inner, N)
+            d = torch.nn.functional.softplus(dt[s : s + n].double() + bias.double())
+            b = low[s : s + n, 8 : 8 + N].double()
+            for i in range(n):
+                S = torch.exp2(d[i][:, None] * a.double()) * S + (d[i] * x[s + i].double())[:, None] * b[i][None, :]
+            off += float((state[slot, : inner * N].double().view(inner, N) - S).pow(2).sum())
+            total += float(S.pow(2).sum())
+        errors.append((off / total) ** 0.5)
+    # (the norms of two sets of n rounding errors of one size differ by about 1 / sqrt(n) by chance: four times that)
+    assert errors[0] <= errors[1] * (1 + 4 * (3 * inner * N) ** -0.5), errors
