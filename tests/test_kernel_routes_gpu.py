@@ -900,3 +900,24 @@ def test_selective_scan_in_parts(ops16, inner, N):
         errors.append((off / total) ** 0.5)
     # (the norms of two sets of n rounding errors of one size differ by about 1 / sqrt(n) by chance: four times that)
     assert errors[0] <= errors[1] * (1 + 4 * (3 * inner * N) ** -0.5), errors
+
+
+@pytest.mark.parametrize("rows,ffn", [(1, 4), (3, 8), (5, 1020), (777, 1028), (70000, 16), (9, 8192)])
+@pytest.mark.parametrize("act", ["silu", "relu"])
+def test_float32_gate_in_fours(ops32, rows, ffn, act):
+    """Rows on 16 bytes take four elements a thread, others one: the same numbers."""
+    gen = torch.Generator().manual_seed(rows + ffn)
+    x = _randn(gen, rows, 2 * ffn, scale=4.0)
+    moved = torch.empty(x.numel() + 1, device=DEV)[1:].view(x.shape)
+    moved.copy_(x)
+    scale, index = _randn(gen, rows), torch.randperm(rows, generator=gen).to(DEV, torch.int32)
+    count = torch.tensor([rows - rows // 3], dtype=torch.int32, device=DEV)
+    for interleave in (0, 8) if ffn % 8 == 0 else (0,):
+        for more in ((), (scale, index, count)):
+            outs = []
+            for v in (x, moved):
+                out = torch.full((rows, ffn), 7.0, device=DEV)
+                ops32.silu_gate(v, out, interleave, act, *more)
+                outs.append(out)
+            assert torch.equal(*outs)
+            assert not more or bool((outs[0][int(count):] == 7.0).all())
