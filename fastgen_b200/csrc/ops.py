@@ -59,9 +59,7 @@ _CORE_SIGNATURES = {
     "fg_mamba2_scan": [_P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "fg_mamba2_scan_scratch_floats": [_I, _I, _I, _I, _I, _I, _I],
     "fg_gated_part_norm": [_P, _L, _P, _L, _I, _P, _P, _L, _P, _I, _I, _I, _F, _P],
-    "fg_selective_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _I, _P,
-                          _P],
-    "fg_selective_scan_scratch_floats": [_I, _I, _I, _I, _I, _I],
+    "fg_selective_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _L, _I, _P, _P, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _P],
     "fg_layer_norm_pair": [_P, _P, _P, _I, _I, _P, _P, _F, _P, _P, _F, _P, _I, _P, _I, _I, _P],
     "fg_rms_rows": [_P, _L, _I, _P, _F, _P, _L, _I, _I, _P],
     "fg_rotate_part": [_P, _L, _I, _P, _P, _P, _F, _I, _I, _I, _I, _I, _P],
@@ -281,7 +279,6 @@ def core():
         _declare(lib, _CORE_SIGNATURES)
         lib.fg_mamba2_scan_scratch_floats.restype = ctypes.c_longlong
         lib.fg_gemm_f32_split_scratch.restype = ctypes.c_longlong
-        lib.fg_selective_scan_scratch_floats.restype = ctypes.c_longlong
         _core = lib
     return _core
 
@@ -490,7 +487,7 @@ class Ops:
     def selective_scan(self, x, dt, low, b_offset: int, z, dt_bias, a_log2, d_skip, state, ctx,
                        n_state: int) -> torch.Tensor:
         """``S[c, n] <- exp2(d_c a_log2[c, n]) S[c, n] + d_c x_c B_n``, ``y_c = sum_n S[c, n] C_n + D_c x_c`` with
-        ``d = softplus(dt + dt_bias)``, in float32 per (sequence, channel), from and into ``state``
+        ``d = softplus(dt + dt_bias)``, token by token in float32 per (sequence, channel), from and into ``state``
         [slots, .] (its first ``inner * n_state`` numbers); returns ``y * silu(z)`` [T, inner].  ``x``, ``dt``,
         ``z`` [T, inner] and ``low`` (B in the ``n_state`` columns from ``b_offset``, C behind it) are row-strided
         views of the compute dtype, which the result has; ``a_log2`` [inner, n_state] is ``A`` times ``log2 e``."""
@@ -502,16 +499,10 @@ class Ops:
             assert v.dtype == torch.float32 and v.numel() == size and v.is_contiguous()
         assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1] >= inner * n_state
         out = torch.empty((t, inner), dtype=x.dtype, device=x.device)
-        longest = _longest(ctx, t)
-        # (in 16-bit serving sequences of many tokens run in parts, which meet here)
-        need = self.lib.fg_selective_scan_scratch_floats(_code(x.dtype), t, longest, ctx.n_seqs, inner, n_state)
-        parts = torch.empty(need, dtype=torch.float32, device=x.device) if need else None
         _check(self.lib, self.lib.fg_selective_scan(
             _ptr(x), x.stride(0), _ptr(dt), dt.stride(0), _ptr(z), z.stride(0), _ptr(low), low.stride(0), int(b_offset),
             _code(x.dtype), _ptr(dt_bias), _ptr(a_log2), _ptr(d_skip), _ptr(out), out.stride(0), _ptr(state),
-            state.stride(0), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), ctx.n_seqs, inner, n_state, t, longest, _ptr(parts),
-            _stream()))
-        Ops.launches += 2 * (need > 0)
+            state.stride(0), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), ctx.n_seqs, inner, n_state, _stream()))
         return out
 
     def layer_norm_pair(self, h, terms, close_w, close_b, close_eps: float, w, b, eps: float, out, rows=None):

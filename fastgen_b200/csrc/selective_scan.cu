@@ -14,9 +14,14 @@
 // computed.  The sums over a channel's lanes are reduced for a group of tokens at a time by halving exchanges and
 // pass through shared memory, so that outputs leave in runs of channels.  Tokens beyond a sequence's end have
 // d = 0, which leaves the state as it is.  The recurrence runs token by token, so a prompt gives the same numbers
-// however it is cut (up to the order of the sum over n, which follows the number of lanes a channel; in 16-bit serving long
-// sequences run in parts, see below).  The state of a slot is [channels][N] float32, zero at admission.
-#include "long_sequences.cuh"
+// however it is cut (up to the order of the sum over n, which follows the number of lanes a channel).  The state of
+// a slot is [channels][N] float32, zero at admission.
+//
+// Parts of 384 tokens side by side, composed by exp2(A log2(e) sum d), took 70 us instead of 104 for one sequence of
+// 1,501 tokens and 2,048 channels of 16, but a prompt's numbers then depended on how it was cut, an infinity in a state
+// became a NaN where the decays multiply up to zero, and other launches were slower: 4,096 channels 120 instead of 104 us,
+// 8,192 216 and 147, four sequences of 1,000 tokens and 2,048 channels 156 and 99.
+#include "common.cuh"
 
 constexpr int SEL_THREADS = 256;
 
@@ -61,28 +66,14 @@ __device__ __forceinline__ void sel_pairs(const float* p, uint64_t (&v)[PAIRS]) 
   }
 }
 
-// Sequences of many tokens, 16-bit serving: what bounds the walk is its length, and a few sequences do not fill the chip
-// (2,048 channels of 16: 64 blocks of 130 cycles a token).  They run in parts of SEL_PART tokens side by side, in two
-// launches: the first (ENDS) walks every part but a sequence's last from a state of zeros (the first one from the slot's
-// state, which it also keeps for the second launch) and leaves the state it ends with and the sum of its d; the second
-// (OUTPUTS) finds the state that its part starts from,
-//
-//   S <- exp2(A log2(e) sum d) S + end,    over the parts before it,
-//
-// and walks again for the outputs.  1,501 tokens, 2,048 channels of 16: 103 -> 68 us.  The states' errors against float64 (2,048
-// tokens, 1,024 channels): 5.8e-7 in parts, 6.3e-7 in one walk.
-constexpr int SEL_PART = 384;
-constexpr int SEL_LONG = 2 * SEL_PART;  // fewest tokens of a sequence that runs in parts
-enum { SEL_WHOLE = 0, SEL_ENDS = 1, SEL_OUTPUTS = 2 };
-
-template <typename T, int LPC, int NPL, int TOK, int MODE = SEL_WHOLE>
+template <typename T, int LPC, int NPL, int TOK>
 __global__ void __launch_bounds__(SEL_THREADS, 2)
 selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restrict__ dt, long dt_stride,
                       const T* __restrict__ z, long z_stride, const T* __restrict__ low, long low_stride, int b_offset,
                       const float* __restrict__ dt_bias, const float* __restrict__ a_log2,
                       const float* __restrict__ d_skip, T* __restrict__ out, long out_stride, float* __restrict__ state,
                       long state_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int inner,
-                      int N, int vec, int most, int n_seqs, float* parts) {
+                      int N, int vec) {
   constexpr int NP = LPC * NPL;              // state numbers of a channel, padded
   constexpr int PAIRS = NPL / 2;
   constexpr int CH = SEL_THREADS / LPC;      // channels a block
@@ -96,26 +87,10 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
   __shared__ __align__(16) float b_s[2][TOK][NP], c_s[2][TOK][NP];
   __shared__ float y_s[TOK][YLD];
 
-  int slot, start, n_tok, part = 0, n_parts = 1;
-  if (MODE == SEL_WHOLE) {
-    slot = seq_slot[blockIdx.y];
-    if (slot < 0) return;
-    start = seq_start[blockIdx.y];
-    n_tok = seq_start[blockIdx.y + 1] - start;
-    if (n_tok <= 0 || n_tok >= most) return;  // (from `most` tokens on: in parts)
-  } else {
-    const auto found = long_seq::find_chunk<SEL_PART, SEL_THREADS>(seq_slot, seq_start, n_seqs, SEL_LONG, blockIdx.y, nullptr);
-    if (found.seq < 0) return;
-    slot = seq_slot[found.seq];
-    part = blockIdx.y - found.first_chunk;
-    n_parts = (found.tokens + SEL_PART - 1) / SEL_PART;
-    if (MODE == SEL_ENDS && part == n_parts - 1) return;
-    start = seq_start[found.seq] + part * SEL_PART;
-    n_tok = min(SEL_PART, found.tokens - part * SEL_PART);
-  }
-  // of every part: the state it ends with [inner][N], the one its sequence starts from [inner][N], the sum of d [inner]
-  const size_t part_floats = (size_t)inner * (2 * N + 1);
-  float* const my_part = MODE == SEL_WHOLE ? nullptr : parts + blockIdx.y * part_floats;
+  const int slot = seq_slot[blockIdx.y];
+  if (slot < 0) return;
+  const int start = seq_start[blockIdx.y], n_tok = seq_start[blockIdx.y + 1] - start;
+  if (n_tok <= 0) return;
   const int tid = threadIdx.x;
   const int sub = tid % LPC, ch = tid / LPC;
   const int c0 = blockIdx.x * CH;
@@ -133,42 +108,6 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
       const bool ok0 = sub * NPL + 2 * i < N, ok1 = sub * NPL + 2 * i + 1 < N;
       S[i] = sel_pair(ok0 ? st[2 * i] : 0.f, ok1 ? st[2 * i + 1] : 0.f);
       a[i] = sel_pair(ok0 ? ar[2 * i] : 0.f, ok1 ? ar[2 * i + 1] : 0.f);
-    }
-  }
-
-  if (MODE != SEL_WHOLE) {
-    const size_t at = (size_t)(mine ? c0 + ch : 0) * N + sub * NPL;
-    auto numbers = [&](const float* p, int i) {
-      const bool ok0 = sub * NPL + 2 * i < N, ok1 = sub * NPL + 2 * i + 1 < N;
-      return sel_pair(ok0 ? p[2 * i] : 0.f, ok1 ? p[2 * i + 1] : 0.f);
-    };
-    if (MODE == SEL_ENDS && part == 0) {  // (the second launch's last part may write the state before its first one reads it)
-#pragma unroll
-      for (int i = 0; i < PAIRS; ++i) {
-        float s0, s1;
-        sel_split(S[i], s0, s1);
-        float* kept = my_part + (size_t)inner * N + at + 2 * i;
-        if (mine && sub * NPL + 2 * i < N) kept[0] = s0;
-        if (mine && sub * NPL + 2 * i + 1 < N) kept[1] = s1;
-      }
-    } else if (MODE == SEL_ENDS) {
-#pragma unroll
-      for (int i = 0; i < PAIRS; ++i) S[i] = 0;
-    } else {
-      const float* first = my_part - (size_t)part * part_floats;
-#pragma unroll
-      for (int i = 0; i < PAIRS; ++i) S[i] = numbers(first + (part == 0 ? (size_t)inner * N : 0) + at, i);
-      for (int q = 1; q < part; ++q) {
-        const float* p = first + q * part_floats;
-        const float d = p[(size_t)2 * inner * N + (mine ? c0 + ch : 0)];
-        const uint64_t dd = sel_pair(d, d);
-#pragma unroll
-        for (int i = 0; i < PAIRS; ++i) {
-          float e0, e1;
-          sel_split(sel_mul(dd, a[i]), e0, e1);
-          S[i] = sel_fma(sel_pair(sel_ex2(e0), sel_ex2(e1)), S[i], numbers(p + at, i));
-        }
-      }
     }
   }
 
@@ -193,7 +132,7 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
       const bool ok = lc_ok && tt < TOK && tt < left;
       xn[i] = ok ? px[i * STEP * x_stride] : zero;
       dn[i] = ok ? pd[i * STEP * dt_stride] : zero;
-      if (MODE != SEL_ENDS) zn[i] = ok ? pz[i * STEP * z_stride] : zero;
+      zn[i] = ok ? pz[i * STEP * z_stride] : zero;
     }
 #pragma unroll
     for (int i = 0; i < BPT; ++i) {
@@ -201,7 +140,7 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
       const bool ok = tt < TOK && n < N && tt < left;
       const T* row = pl + tt * low_stride + n;
       bn[i] = ok ? row[0] : zero;
-      if (MODE != SEL_ENDS) cn[i] = ok ? row[N] : zero;
+      cn[i] = ok ? row[N] : zero;
     }
     px += TOK * x_stride;
     pd += TOK * dt_stride;
@@ -218,7 +157,7 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
         d = v > 20.f ? v : log1pf(expf(v));
       }
       xc[i] = to_f32<T>(xn[i]);
-      if (MODE != SEL_ENDS) zc[i] = to_f32<T>(zn[i]);
+      zc[i] = to_f32<T>(zn[i]);
       const float dx = d * xc[i];
       if (tt < TOK) *reinterpret_cast<float4*>(dx_s[buf][tt][lc]) = make_float4(d, d, dx, dx);
     }
@@ -227,40 +166,18 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
       const int e = tid + i * SEL_THREADS, tt = e / NP, n = e % NP;
       if (tt < TOK) {
         b_s[buf][tt][n] = to_f32<T>(bn[i]);
-        if (MODE != SEL_ENDS) c_s[buf][tt][n] = to_f32<T>(cn[i]);
+        c_s[buf][tt][n] = to_f32<T>(cn[i]);
       }
     }
   };
 
   const int n_stages = (n_tok + TOK - 1) / TOK;
-  float d_sum = 0.f;  // of the part, a stage's sum at a time
   fetch(n_tok);
   store(0, n_tok);
   __syncthreads();
   for (int stage = 0; stage < n_stages; ++stage) {
     const int buf = stage & 1, nt = min(TOK, n_tok - stage * TOK), left = n_tok - (stage + 1) * TOK;
     if (left > 0) fetch(left);
-    if (MODE == SEL_ENDS) {
-      float stage_sum = 0.f;
-#pragma unroll 8
-      for (int u = 0; u < TOK; ++u) {  // (tokens beyond the part: d = 0)
-        const ulonglong2 dx = *reinterpret_cast<const ulonglong2*>(dx_s[buf][u][ch]);
-        uint64_t b2[PAIRS];
-        sel_pairs<PAIRS>(&b_s[buf][u][sub * NPL], b2);
-        stage_sum += __uint_as_float((uint32_t)dx.x);
-#pragma unroll
-        for (int i = 0; i < PAIRS; ++i) {
-          float e0, e1;
-          sel_split(sel_mul(dx.x, a[i]), e0, e1);
-          S[i] = sel_fma(sel_pair(sel_ex2(e0), sel_ex2(e1)), S[i], sel_mul(dx.y, b2[i]));
-        }
-      }
-      d_sum += stage_sum;
-      __syncthreads();
-      if (left > 0) store(buf ^ 1, left);
-      __syncthreads();
-      continue;
-    }
 #pragma unroll
     for (int g0 = 0; g0 < TOK; g0 += GROUP) {
       if (g0 >= nt) break;
@@ -313,16 +230,12 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
     if (left > 0) store(buf ^ 1, left);
     __syncthreads();  // the next stage is stored, and the outputs' rows are free again
   }
-  if (!mine || (MODE == SEL_OUTPUTS && part < n_parts - 1)) return;
-  if (MODE == SEL_ENDS) {
-    st = my_part + (size_t)(c0 + ch) * N + sub * NPL;
-    if (sub == 0) my_part[(size_t)2 * inner * N + c0 + ch] = d_sum;
-  }
+  if (!mine) return;
 #pragma unroll
   for (int i = 0; i < PAIRS; ++i) {
     float s0, s1;
     sel_split(S[i], s0, s1);
-    if (MODE != SEL_ENDS && vec) {
+    if (vec) {
       *reinterpret_cast<float2*>(st + 2 * i) = make_float2(s0, s1);
     } else {
       if (sub * NPL + 2 * i < N) st[2 * i] = s0;
@@ -334,34 +247,22 @@ selective_scan_kernel(const T* __restrict__ x, long x_stride, const T* __restric
 // x, dt, z: [T, inner] and low: B in the N columns from b_offset, C in the N behind them, all of `dtype` with
 // row strides.  dt_bias, d_skip: float32 [inner]; a_log2: float32 [inner, N], A times log2(e).  out: [T, inner]
 // of `dtype`.  state: float32 [slots, state_stride], a slot's first inner * N numbers.
-// What the parts of long sequences take beside the state, in floats (0: none run in parts): `longest` bounds the tokens of
-// one sequence of the step.
-static bool sel_in_parts(int dtype, int longest, int N) { return dtype == FG_BF16 && longest >= SEL_LONG && N <= 16; }
-extern "C" long long fg_selective_scan_scratch_floats(int dtype, int n_tokens, int longest, int n_seqs, int inner, int N) {
-  if (!sel_in_parts(dtype, longest, N)) return 0;
-  return (long long)long_seq::most_chunks(n_tokens, n_seqs, SEL_LONG, SEL_PART) * inner * (2 * N + 1);
-}
-
 extern "C" int fg_selective_scan(const void* x, long x_stride, const void* dt, long dt_stride, const void* z,
                                  long z_stride, const void* low, long low_stride, long b_offset, int dtype,
                                  const float* dt_bias, const float* a_log2, const float* d_skip, void* out,
                                  long out_stride, float* state, long state_stride, const int* seq_slot,
-                                 const int* seq_start, int n_seqs, int inner, int N, int n_tokens, int longest,
-                                 float* scratch, cudaStream_t stream) {
+                                 const int* seq_start, int n_seqs, int inner, int N, cudaStream_t stream) {
   if (n_seqs == 0) return 0;
   FG_CHECK_ARG(inner > 0 && N >= 1 && N <= 256, "fg_selective_scan: %d channels of %d numbers (1 to 256)", inner, N);
   FG_CHECK_ARG(n_seqs <= 65535, "fg_selective_scan: %d sequences", n_seqs);
   FG_CHECK_ARG(state_stride >= (long)inner * N, "fg_selective_scan: a state of %ld numbers is too small", state_stride);
   FG_CHECK_ARG(dtype == FG_F32 || dtype == FG_BF16, "fg_selective_scan: bad dtype %d", dtype);
-  const bool in_parts = sel_in_parts(dtype, longest, N);
-  const int most = in_parts ? SEL_LONG : 1 << 30;
 #define LAUNCH_T(T, LPC, NPL, TOK)                                                                                     \
   selective_scan_kernel<T, LPC, NPL, TOK><<<dim3((inner + SEL_THREADS / LPC - 1) / (SEL_THREADS / LPC), n_seqs),       \
                                             SEL_THREADS, 0, stream>>>(                                                 \
       (const T*)x, x_stride, (const T*)dt, dt_stride, (const T*)z, z_stride, (const T*)low, low_stride, (int)b_offset, \
       dt_bias, a_log2, d_skip, (T*)out, out_stride, state, state_stride, seq_slot, seq_start, inner, N,                \
-      N == LPC * NPL && state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 && ((uintptr_t)a_log2 & 15) == 0, most, \
-      n_seqs, nullptr)
+      N == LPC * NPL && state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 && ((uintptr_t)a_log2 & 15) == 0)
 #define LAUNCH(LPC, NPL, TOK)                                  \
   do {                                                         \
     if (dtype == FG_F32) LAUNCH_T(float, LPC, NPL, TOK);       \
@@ -380,22 +281,6 @@ extern "C" int fg_selective_scan(const void* x, long x_stride, const void* dt, l
   else LAUNCH(32, 8, 8);
 #undef LAUNCH
 #undef LAUNCH_T
-  if (in_parts) {
-    FG_CHECK_ARG(scratch != nullptr, "fg_selective_scan: scratch is missing");
-    const long parts = long_seq::most_chunks(n_tokens, n_seqs, SEL_LONG, SEL_PART);
-    FG_CHECK_ARG(parts <= 65535, "fg_selective_scan: %d tokens are too many", n_tokens);
-    constexpr int CH = SEL_THREADS / 8;
-    const dim3 grid((inner + CH - 1) / CH, (unsigned)parts);
-    const int vec = N == 16 && state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 && ((uintptr_t)a_log2 & 15) == 0;
-#define PARTS(mode)                                                                                                          \
-  selective_scan_kernel<__nv_bfloat16, 8, 2, 32, mode><<<grid, SEL_THREADS, 0, stream>>>(                                    \
-      (const __nv_bfloat16*)x, x_stride, (const __nv_bfloat16*)dt, dt_stride, (const __nv_bfloat16*)z, z_stride,             \
-      (const __nv_bfloat16*)low, low_stride, (int)b_offset, dt_bias, a_log2, d_skip, (__nv_bfloat16*)out, out_stride, state, \
-      state_stride, seq_slot, seq_start, inner, N, vec, 0, n_seqs, scratch)
-    PARTS(SEL_ENDS);
-    PARTS(SEL_OUTPUTS);
-#undef PARTS
-  }
   FG_CHECK_LAUNCH("fg_selective_scan");
   return 0;
 }

@@ -850,10 +850,10 @@ def test_embedding_rows(ops32, dtype, dim, copies):
 
 # -- the selective scan -------------------------------------------------------------------------------------
 
-@pytest.mark.parametrize("inner,N", [(70, 16), (33, 5), (256, 16)])
-def test_selective_scan_in_parts(ops16, inner, N):
-    """Sequences from 768 tokens on run in parts of 384, shorter ones beside them token by token: the outputs and states of
-    the same sequences brought in portions (which are too short for parts), and the states no further from float64."""
+@pytest.mark.parametrize("inner,N", [(70, 16), (33, 5), (256, 16), (2048, 16)])
+def test_selective_scan_however_cut(ops16, inner, N):
+    """A sequence's outputs and state have the same bits in one step and in portions, whatever is beside it; an infinity stays
+    in the state that it reached."""
     g = torch.Generator().manual_seed(inner + N)
     lengths, order = [767, 768, 0, 1501, 1, 1153], [4, 0, -1, 5, 1, 2]
     starts = [0]
@@ -863,6 +863,9 @@ def test_selective_scan_in_parts(ops16, inner, N):
     x, dt, z, low = (_randn(g, t, n).to(torch.bfloat16) for n in (inner, inner, inner, 2 * N + 8))
     bias, skip = _randn(g, inner) - 2.0, _randn(g, inner)
     a = -_randn(g, inner, N).exp()
+    if N == 16:  # (numbers that fill the lanes up would turn NaN)
+        a[3] = -4.0  # (over some hundred tokens these decays multiply up to zero, one by one they do not)
+        x[starts[3] + 100, 3] = float("inf")
     state0 = _randn(g, 6, inner * N + 12)
 
     def run(state, parts):
@@ -875,31 +878,17 @@ def test_selective_scan_in_parts(ops16, inner, N):
         return ops16.selective_scan(x[rows], dt[rows], low[rows], 8, z[rows], bias, a, skip, state, ctx, N)
 
     whole, cut = state0.clone(), state0.clone()
-    y = run(whole, list(zip(starts, lengths, order)))
+    # (the lanes a channel, and with them the order of an output's sum, go by channels and sequences of a launch: one by one)
+    groups = [[i] for i, n in enumerate(lengths) if n] if inner > 256 else [list(range(len(lengths)))]
+    y = torch.cat([run(whole, [(starts[i], lengths[i], order[i]) for i in group]) for group in groups])
+    bits = lambda v: v.contiguous().view(torch.int16)
     for s, n, slot in zip(starts, lengths, order):
         for at in range(0, n, 700):
             m = min(700, n - at)
-            part = run(cut, [(s + at, m, slot)])
-            # (one rounding to bfloat16 of sums that differ in their last bits)
-            assert torch.allclose(part.float(), y[s + at : s + at + m].float(), rtol=2.0 ** -7, atol=1e-3), (s, at)
+            assert torch.equal(bits(run(cut, [(s + at, m, slot)])), bits(y[s + at : s + at + m])), (s, at)
+    assert torch.equal(whole.view(torch.int32), cut.view(torch.int32))
     assert torch.equal(whole[3], state0[3]) and torch.equal(whole[:, inner * N :], state0[:, inner * N :])
-    assert torch.equal(whole[4], cut[4]) and torch.equal(whole[1], cut[1])  # the short ones: the same walk
-    errors = []
-    for state in (whole, cut):
-        off = total = 0.0
-        for s, n, slot in zip(starts, lengths, order):
-            if n < 768:
-                continue
-            S = state0[slot, : inner * N].double().view(inner, N)
-            d = torch.nn.functional.softplus(dt[s : s + n].double() + bias.double())
-            b = low[s : s + n, 8 : 8 + N].double()
-            for i in range(n):
-                S = torch.exp2(d[i][:, None] * a.double()) * S + (d[i] * x[s + i].double())[:, None] * b[i][None, :]
-            off += float((state[slot, : inner * N].double().view(inner, N) - S).pow(2).sum())
-            total += float(S.pow(2).sum())
-        errors.append((off / total) ** 0.5)
-    # (the norms of two sets of n rounding errors of one size differ by about 1 / sqrt(n) by chance: four times that)
-    assert errors[0] <= errors[1] * (1 + 4 * (3 * inner * N) ** -0.5), errors
+    assert N != 16 or bool(torch.isinf(whole[5].flatten()[3 * N : 4 * N]).all())
 
 
 @pytest.mark.parametrize("rows,ffn", [(1, 4), (3, 8), (5, 1020), (777, 1028), (70000, 16), (9, 8192)])
