@@ -1,14 +1,14 @@
 // Float32 matrix product  C[M, N] = A[M, K] * W[N, K]^T  on the 5th-generation tensor cores, for weights of
 // at least 1,024 x 1,024 (gemm_f32.cu has the others).
 //
-// A float32 number is the sum of three bfloat16 ones (hi + mid + lo, each the rest rounded to nearest: together all 24
-// bits), and a product of two numbers is six of the nine products of their parts; the three left out are below
-// 2^-25 of it.  Products of bfloat16 are exact in float32.  What a tensor core adds up it rounds toward zero, so it adds
-// up only 64 columns of k at a time: lo and mid parts first, hi * hi last, into a tensor-memory tile that starts from
-// nothing.  These partial sums are read back and added with rounding to nearest: in ascending order within an eighth
-// of the chunks of k, and the eighths in ascending order.  That order depends on K alone: an element's value does not
-// depend on M, on the tile it falls in or on how many blocks share the sum.  Errors against float64 are in
-// the comment at fg_gemm_f32_split.
+// A float32 number times 2^16 is exactly the sum of three bfloat16 ones (hi + mid + lo, each the rest rounded to nearest), and a
+// product of two numbers is six of the nine products of their parts; the three left out come to 2^-24 of it at most, to
+// 2^-27 on average (root mean square).  Products of bfloat16 are exact in float32, but what a tensor core adds up it rounds toward zero.  So
+// hi * hi has a tensor-memory tile of its own, which starts from nothing every 64 columns of k: its sums of 16-bit numbers lose
+// little.  The five small products of a segment (an eighth of the chunks of k) are added up in another, where what is
+// cut off is 2^-8 of that.  The sums are read back and added with rounding to nearest: in ascending order within a segment, and the
+// segments in ascending order.  That order depends on K alone: an element's value does not depend on M, on the tile it falls
+// in or on how many blocks share the sum.  Errors against float64 are in the comment at fg_gemm_f32_split.
 //
 // The weights' rows are the 128 rows of the tensor core's tile, the rows of A its columns (T of them):
 // 777 rows against 128,256 x 2,048: 7,870 -> 1,966 us; 5 rows: 287 -> 180 (bytes: 160).  What bounds it now is the way
@@ -19,13 +19,15 @@
 //                   before -> registers
 //   MMA warp:       24 tcgen05.mma a chunk (6 products x 4 steps of 16)
 // The left operand in tensor memory leaves shared memory to A's parts: each of them is read once a product.
+// hi * hi comes last in a chunk: its sums are read during the next chunk's small products, the small ones' during the hi * hi that
+// ends their segment, so that one tile of each is enough.
 // Few rows (T <= 32): the workers also split A; two blocks an SM, bound by reading W.  More rows: A is split once by
 // a kernel of its own, and the tensor core is what bounds the rest.
-// Where the tiles are too few for the chip, a cluster of eight blocks shares a tile, an eighth of the chunks each, and
-// adds the eighths up over distributed shared memory.
+// Where the tiles are too few for the chip, a cluster of two, four or eight blocks shares a tile, its segments evenly, and
+// adds the segments up over distributed shared memory.
 //
-// An element that is not finite (an infinity or NaN among its inputs, or an overflow) is computed again with
-// float32 multiply-adds in ascending k: the parts of an infinity are an infinity and NaNs.
+// An element that is not finite (an infinity or NaN among its inputs, numbers of 2^111 and more, or an overflow) is computed
+// again with float32 multiply-adds in ascending k: the parts of an infinity are an infinity and NaNs.
 #include "tc5_primitives.cuh"
 #include "tensor_map.cuh"
 
@@ -38,6 +40,9 @@ constexpr int SEGMENTS = 8;   // stretches of chunks whose sums are added last
 constexpr int W_BOX = ROWS * 128, W_STAGE = 2 * W_BOX;
 constexpr int WORKERS = 256, THREADS_ALL = WORKERS + 64, LOAD_WARP_ID = 8, MMA_WARP_ID = 9;
 constexpr int A_COLS = 96;    // tensor-memory columns of a chunk of W: three parts of 64 bfloat16
+// What operands are multiplied by before they are split, and what that leaves on a sum.  Float32's smallest number is then
+// bfloat16's smallest, and the smallest result, 2^-149, is 2^-117 in the sums, inside float32's normal range.
+constexpr float SCALE = 0x1p16f, UNSCALE = 0x1p-32f;
 
 // T rows of A a tile; SHARE blocks (a cluster) share a tile
 template <int T_, int SHARE_>
@@ -102,15 +107,27 @@ __device__ __forceinline__ uint32_t cvt_pair(float a, float b) {  // a in the lo
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
   return r;
 }
-// two numbers -> their three parts, packed
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+// a pair of numbers and its rest, both float32, from the pair's bfloat16 (exact)
+__device__ __forceinline__ uint32_t take_part(uint64_t& v) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  const uint32_t part = cvt_pair(a, b);
+  const uint64_t wide = pair_of(__uint_as_float(part << 16), __uint_as_float(part & 0xffff0000u));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v) : "l"(wide), "l"(pair_of(-1.f, -1.f)));
+  return part;
+}
+// two numbers, times SCALE -> their three parts, packed
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = cvt_pair(a, b);
-  a -= __uint_as_float(hi << 16);
-  b -= __uint_as_float(hi & 0xffff0000u);
-  mid = cvt_pair(a, b);
-  a -= __uint_as_float(mid << 16);
-  b -= __uint_as_float(mid & 0xffff0000u);
-  lo = cvt_pair(a, b);
+  uint64_t v = pair_of(a, b);
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(pair_of(SCALE, SCALE)));
+  hi = take_part(v);
+  mid = take_part(v);
+  lo = take_part(v);
 }
 // byte offset of the 16-byte piece `piece` of a row of 128 bytes in a swizzled tile
 __device__ __forceinline__ int swizzled(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
@@ -176,9 +193,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
   unsigned char* const ws = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
   unsigned char* const as = ws + W_STAGES * W_STAGE;
   // w_full / w_empty: a stage of W; a_full / a_empty: a part of A (SPLIT_HERE: unused); op_full: the parts of a chunk of W
-  // are in tensor memory; d_full / d_empty: a chunk's sums
+  // are in tensor memory; d_full / d_empty: a chunk's sums of hi * hi; small_full / small_empty: a segment's other sums
   __shared__ __align__(8) uint64_t w_full[W_STAGES], w_empty[W_STAGES], a_full[S::UNITS], a_empty[S::UNITS], op_full[2],
-      d_full[2], d_empty[2], drained;
+      d_full, d_empty, small_full, small_empty, drained;
   __shared__ uint32_t tmem_base;
   __shared__ int gave_up;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -198,11 +215,11 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
       mbar_init(&a_full[i], 1);
       mbar_init(&a_empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&op_full[i], WORKERS / 32);
-      mbar_init(&d_full[i], 1);
-      mbar_init(&d_empty[i], WORKERS / 32);
-    }
+    for (int i = 0; i < 2; ++i) mbar_init(&op_full[i], WORKERS / 32);
+    mbar_init(&d_full, 1);
+    mbar_init(&d_empty, WORKERS / 32);
+    mbar_init(&small_full, 1);
+    mbar_init(&small_empty, WORKERS / 32);
     mbar_init(&drained, 1);
     mbar_fence_init();
   }
@@ -278,12 +295,13 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
     if (elect_one()) {
       constexpr uint32_t IDESC = instr_desc(T, false);
       const uint64_t a_desc = smem_desc(as, 16);
-      int slot = 0, use = 0;
+      int slot = 0, use = 0, c = 0, in_segment = 0, segments = 0;  // (segments: those begun before this one)
       for (int j = 0; j < total; ++j) {
         const int buf = j & 1;
-        const uint32_t d = tmem + buf * T, op = tmem + S::COL_A + buf * A_COLS;
+        const uint32_t small = tmem, d = tmem + T, op = tmem + S::COL_A + buf * A_COLS;
+        const bool last = in_segment + 1 == per_segment || c + 1 == per_tile;  // chunk of its segment
         mbar_wait(&op_full[buf], (j >> 1) & 1, status, &gave_up);
-        if (j >= 2) mbar_wait(&d_empty[buf], ((j >> 1) - 1) & 1, status, &gave_up);
+        if (in_segment == 0 && segments > 0) mbar_wait(&small_empty, (segments - 1) & 1, status, &gave_up);
         tc_fence_after();
 #pragma unroll
         for (int p = 0; p < 3; ++p) {  // A's lo, mid, hi
@@ -294,10 +312,20 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
           }
           const uint64_t bd = a_desc + (uint64_t)((unit * S::UNIT) >> 4);
 #pragma unroll
-          for (int q = p; q >= 0; --q)  // W's part q (0: hi): lo * hi; mid * mid, mid * hi; hi * lo, hi * mid, hi * hi
+          for (int q = p; q >= 0; --q) {  // W's part q (0: hi): lo * hi; mid * mid, mid * hi; hi * lo, hi * mid, hi * hi
+            const bool main = p == 2 && q == 0;
+            if (main) {
+              if (last) umma_commit(&small_full);
+              if (j > 0) {
+                mbar_wait(&d_empty, (j - 1) & 1, status, &gave_up);
+                tc_fence_after();
+              }
+            }
 #pragma unroll
             for (int kk = 0; kk < KC / 16; ++kk)
-              umma_f16_ts(d, op + q * 32 + kk * 8, bd + (uint64_t)(kk * 32 >> 4), IDESC, (p > 0 || kk > 0) ? 1u : 0u);
+              umma_f16_ts(main ? d : small, op + q * 32 + kk * 8, bd + (uint64_t)(kk * 32 >> 4), IDESC,
+                          main ? (kk > 0 ? 1u : 0u) : (p > 0 || kk > 0 || in_segment > 0 ? 1u : 0u));
+          }
           if (!S::SPLIT_HERE) {
             umma_commit(&a_empty[slot]);
             if (++slot == S::UNITS) {
@@ -306,7 +334,14 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
             }
           }
         }
-        umma_commit(&d_full[buf]);
+        umma_commit(&d_full);
+        if (last) {
+          in_segment = 0;
+          ++segments;
+        } else {
+          ++in_segment;
+        }
+        if (++c == per_tile) c = 0;
       }
       if (*reinterpret_cast<volatile int*>(&gave_up) != 0) {
         umma_commit(&drained);
@@ -340,7 +375,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
       if (++load_c == per_tile) load_c = 0;
     };
     if (S::SPLIT_HERE && total > 0) fetch_a();
-    int slot = 0, use = 0, tile = tile0, c = 0, in_segment = 0, segment = 0;
+    int slot = 0, use = 0, tile = tile0, c = 0, in_segment = 0, segment = 0, segments = 0;  // (of the tile, of all)
     for (int j = 0; j <= total; ++j) {
       if (j < total) {
         const int buf = j & 1;
@@ -384,25 +419,31 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
         if (S::SPLIT_HERE && j + 1 < total) fetch_a();
       }
       if (j == 0) continue;
-      // the sums of the chunk before
-      const int buf = (j - 1) & 1;
-      mbar_wait(&d_full[buf], ((j - 1) >> 1) & 1, status, &gave_up);
-      tc_fence_after();
-      const uint32_t d = tmem + my_lane + buf * T + half * TC;
-      constexpr int G = TC < 48 ? TC : 16;  // columns in flight: what the registers leave
+      // the sums of the chunk before (and of its segment, where it is the last): tensor memory -> acc
+      auto add_sums = [&](uint32_t col, uint64_t* full, uint64_t* empty, int parity) {
+        mbar_wait(full, parity, status, &gave_up);
+        tc_fence_after();
+        const uint32_t d = tmem + my_lane + col + half * TC;
+        constexpr int G = TC < 48 ? TC : 16;  // columns in flight: what the registers leave
 #pragma unroll
-      for (int g = 0; g < TC; g += G) {
-        uint32_t v[G];
+        for (int g = 0; g < TC; g += G) {
+          uint32_t v[G];
 #pragma unroll
-        for (int i = 0; i < G && g + i < TC; i += 8) tmem_ld8(d + g + i, v + i);
-        tmem_ld_wait();
-        if (g + G >= TC) {
-          tc_fence_before();
-          warp_arrive(&d_empty[buf]);
+          for (int i = 0; i < G && g + i < TC; i += 8) tmem_ld8(d + g + i, v + i);
+          tmem_ld_wait();
+          if (g + G >= TC) {
+            tc_fence_before();
+            warp_arrive(empty);
+          }
+#pragma unroll
+          for (int i = 0; i < G && g + i < TC; ++i) acc[g + i] += __uint_as_float(v[i]);
         }
-#pragma unroll
-        for (int i = 0; i < G && g + i < TC; ++i) acc[g + i] += __uint_as_float(v[i]);
+      };
+      if (in_segment + 1 == per_segment || c + 1 == per_tile) {
+        add_sums(0, &small_full, &small_empty, segments & 1);
+        ++segments;
       }
+      add_sums(T, &d_full, &d_empty, (j - 1) & 1);
       ++c;
       if (++in_segment == per_segment || c == per_tile) {
         if (S::SUM_IN_SMEM) {
@@ -446,6 +487,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
           } else {
             v = sum[0][i];
           }
+          v *= UNSCALE;
           if (bias != nullptr) v += add;
           if (n < N && m0 + i < M) {
             C[(size_t)(m0 + i) * ldc + n] = v;
@@ -491,6 +533,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
         bool bad = false;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
+          v[e] *= UNSCALE;
           if (bias != nullptr && n + e < N) v[e] += bias[n + e];
           bad = bad || (n + e < N && !finite(v[e]));
         }
@@ -617,8 +660,11 @@ extern "C" long long fg_gemm_f32_split_scratch(int M, int K) {
   return M <= 32 ? 0 : 3ll * M * ((K + 7) / 8 * 8) * 2;
 }
 
-// Against float64 (2-norm of the error over that of the result; these sums, multiply-adds in ascending k): K = 1,024 9.8e-8 and
-// 6.0e-7, 2,048 1.04e-7 and 8.1e-7, 8,192 1.23e-7 and 1.62e-6.
+// Against float64 (2-norm of the error over that of the result; these sums, multiply-adds in ascending k), numbers drawn from a
+// normal distribution: K = 1,024 9.2e-8 and 5.8e-7, 2,048 9.8e-8 and 8.1e-7, 8,192 1.19e-7 and 1.62e-6, 14,336 1.37e-7 and
+// 2.14e-6.  Rows with few numbers that are not zero (K = 2,048): one 2.6e-8 and 2.5e-8 (at most 9.7e-8 and 6.0e-8 of an element:
+// the products left out), two 3.6e-8 and 3.1e-8 and four 4.5e-8 and 4.1e-8 (a segment's sum is one rounding more), eight 5.3e-8
+// and 5.3e-8, sixteen 6.0e-8 and 7.4e-8, sixty-four 6.5e-8 and 14.5e-8.
 extern "C" int fg_gemm_f32_split(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
                                  const float* bias, void* scratch, int* status, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;

@@ -93,6 +93,46 @@ def test_float32_product_on_tensor_cores(ops32, m, n, k):
     assert bool(((got.double() - other.double()).abs() <= bound)[finite].all())
 
 
+@pytest.mark.parametrize("m,n,k", [(5, 1100, 1024), (20, 1024, 2052), (300, 1500, 1028), (700, 19000, 1024)])
+def test_float32_product_of_few_or_unusual_numbers(ops32, m, n, k):
+    """Rows of few numbers that are not zero, of numbers at either end of float32's range and of very different ones: no further
+    from float64 than the multiply-adds of the general kernel."""
+    g = torch.Generator().manual_seed(m + k)
+    x, w = _randn(g, m, k), _randn(g, n, k)
+    odd = torch.empty(m, k + 1, device=DEV)[:, :k]  # rows off 16 bytes: the general kernel
+
+    def both(x, w):
+        odd.copy_(x)
+        return ops32.linear(x, w), ops32.linear(odd, w)
+
+    for count in (1, 2, 4, 8, 32):
+        at = torch.stack([torch.randperm(k, generator=g)[:count] for _ in range(m)]).to(DEV)
+        few = torch.zeros_like(x).scatter_(1, at, x.gather(1, at))
+        got, other = both(few, w)
+        ref = few.double() @ w.double().T
+        # With z numbers, none in the segment of another, z segments and their z - 1 sums are rounded, of multiply-adds z
+        # results: sqrt(2) of the error at most, and longer chains of multiply-adds make up for it.  The three products of
+        # parts left out come to 2^-24 of a product at most, a fifth of a rounding on average.
+        assert _relative(got, ref) <= (2.0 ** 0.5 if count < 32 else 1.0) * _relative(other, ref), count
+        if count == 1:
+            assert bool(((got.double() - ref).abs() <= (2 + 2.0 ** -6) * EPS * ref.abs()).all())
+    mixed = x * torch.exp2(torch.randint(-40, 41, (m, k), generator=g).float()).to(DEV)
+    for scaled, weights in ((x * 2.0 ** -120, w * 2.0 ** 100), (x * 2.0 ** 100, w * 2.0 ** -125), (x * 2.0 ** -130, w * 2.0 ** 120),
+                            (x.abs() * 2.0 ** -118, w.abs() * 2.0 ** 90), (mixed, w)):
+        got, other = both(scaled, weights)
+        ref = scaled.double() @ weights.double().T
+        assert _relative(got, ref) <= _relative(other, ref) * (1.0 if scaled is not mixed else 2.0 ** 0.5)
+    # results below float32's normal range: one rounding to their spacing, the general kernel's are many
+    got, other = both(x * 2.0 ** -70, w * 2.0 ** -72)
+    ref = (x * 2.0 ** -70).double() @ (w * 2.0 ** -72).double().T
+    assert bool(((got.double() - ref).abs() <= 2.0 ** -149).all())
+    # numbers that the split does not take (2^111 and more): the general kernel's bits
+    got, other = both(x * 2.0 ** 112, w * 2.0 ** -20)
+    large = ((x * 2.0 ** 112).abs() >= 2.0 ** 112).any(1)
+    assert bool(large.any()) and torch.equal(got[large], other[large]) and bool(torch.isfinite(got).all())
+    assert int(ops32.status.flatten()[0]) == 0
+
+
 def _relative(got, ref):
     return float((got.double() - ref).norm() / ref.norm())
 
