@@ -27,7 +27,8 @@
 // adds the segments up over distributed shared memory.
 //
 // An element that is not finite (an infinity or NaN among its inputs, numbers of 2^111 and more, or an overflow) is computed
-// again with float32 multiply-adds in ascending k: the parts of an infinity are an infinity and NaNs.
+// again with float32 multiply-adds in ascending k: the parts of an infinity are an infinity and NaNs.  A block does that
+// when all its tiles are stored and it waits for nothing any more.
 #include "tc5_primitives.cuh"
 #include "tensor_map.cuh"
 
@@ -134,30 +135,95 @@ __device__ __forceinline__ int swizzled(int row, int piece) { return row * 128 +
 
 __device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
-// The elements of C (this warp's 32 columns from n0, rows [m0, m0 + count)) that are not finite, once more in float32.
-// Called by whole warps; a lane has stored its column itself.
-__device__ __noinline__ void repair(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int n0, int m0,
-                                    int count, int N, int K, const float* bias) {
-  const int lane = threadIdx.x & 31, n = n0 + lane;
-  for (int i = 0; i < count; ++i) {
-    const int m = m0 + i;
-    float* c = C + (size_t)m * ldc + n;
-    const bool bad = n < N && !finite(*c);
-    if (!__any_sync(0xffffffffu, bad)) continue;
-    const float* a = A + (size_t)m * lda;
-    bool nan = false;  // a NaN in A's row is one in all of C's
-    for (int k = lane; k < K; k += 32) nan = nan || a[k] != a[k];
-    nan = __any_sync(0xffffffffu, nan);
-    if (bad) {
-      float v = 0.f;
-      if (nan)
-        v = __uint_as_float(0x7fffffffu);
-      else
-        for (int k = 0; k < K; ++k) v = fmaf(a[k], W[(size_t)n * ldw + k], v);
-      *c = bias != nullptr ? v + bias[n] : v;
+// The elements of C that are not finite, in the columns n0 .. n0 + ROWS - 1 of the rows m0, m0 + step, ... (`count` of them, all
+// stored by this block), once more with multiply-adds in ascending k.  Called by the whole block when it waits for nothing any
+// more: rows of A with a NaN give NaNs; the other rows that hold such an element go sixteen at a time, eight elements of one
+// column a thread, so that a reading of W's 128 rows serves sixteen, the next 64 columns of k on their way meanwhile.  (5 rows
+// against 2,048 x 2,048, all infinite: 443 us with a lane an element and W's rows side by side, here 207; 777 rows against 16,384 x
+// 2,048 5,583, and 441 with a NaN in one row.)
+constexpr int R_ROWS = 16, R_K = 64, R_LD = R_K + 4;
+template <int T>
+__device__ __noinline__ void repair(float* smem, const float* A, int lda, const float* W, int ldw, float* C, int ldc, int n0, int m0,
+                                    int step, int count, int N, int K, const float* bias) {
+  __shared__ int bad_rows[T], n_bad;
+  float* const ws = smem;                   // [ROWS][R_LD]
+  float* const as = smem + ROWS * R_LD;     // [R_ROWS][R_K]
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) n_bad = 0;
+  __syncthreads();
+  if (tid < WORKERS)
+    for (int i = tid >> 5; i < count; i += WORKERS / 32) {
+      const int m = m0 + i * step;
+      float* c = C + (size_t)m * ldc + n0;
+      bool bad = false, nan = false;
+      for (int n = lane; n < min(ROWS, N - n0); n += 32) bad = bad || !finite(c[n]);
+      if (!__any_sync(0xffffffffu, bad)) continue;
+      const float* a = A + (size_t)m * lda;
+#pragma unroll 4
+      for (int k = lane * 4; k < K; k += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(a + k);
+        nan = nan || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
+      }
+      if (__any_sync(0xffffffffu, nan)) {
+        for (int n = lane; n < min(ROWS, N - n0); n += 32) c[n] = __uint_as_float(0x7fffffffu);
+      } else if (lane == 0) {
+        bad_rows[atomicAdd(&n_bad, 1)] = m;
+      }
     }
-    __syncwarp();
+  __syncthreads();
+  const int rows = n_bad, col = tid & (ROWS - 1), part = tid / ROWS, n = n0 + col;
+  constexpr int PIECES = (ROWS + R_ROWS) * (R_K / 4) / WORKERS;  // of 16 bytes, a thread: the last is of A
+  static_assert(PIECES * WORKERS == (ROWS + R_ROWS) * (R_K / 4) && R_ROWS * (R_K / 4) == WORKERS, "");
+  const int row = tid / (R_K / 4), quad = tid % (R_K / 4);  // a thread's first piece; the others are 16 rows apart
+  for (int r0 = 0; r0 < rows; r0 += R_ROWS) {
+    float4 next[PIECES];
+    auto fetch = [&](int k0) {
+      const int k = k0 + 4 * quad;
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) {
+        const bool ok = k < K && (i < PIECES - 1 ? n0 + row + 16 * i < N : r0 + row < rows);
+        const float* src = i < PIECES - 1 ? W + (size_t)(n0 + row + 16 * i) * ldw : A + (size_t)(ok ? bad_rows[r0 + row] : 0) * lda;
+        next[i] = ok ? *reinterpret_cast<const float4*>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    float v[R_ROWS / 2];
+#pragma unroll
+    for (int i = 0; i < R_ROWS / 2; ++i) v[i] = 0.f;
+    if (tid < WORKERS) fetch(0);
+    for (int k0 = 0; k0 < K; k0 += R_K) {
+      const int quads = min(R_K, K - k0) / 4;
+      __syncthreads();  // the columns of k before are read
+      if (tid < WORKERS) {
+#pragma unroll
+        for (int i = 0; i < PIECES - 1; ++i) *reinterpret_cast<float4*>(ws + (row + 16 * i) * R_LD + 4 * quad) = next[i];
+        *reinterpret_cast<float4*>(as + row * R_K + 4 * quad) = next[PIECES - 1];
+      }
+      __syncthreads();
+      if (tid < WORKERS) {
+        if (k0 + R_K < K) fetch(k0 + R_K);
+        for (int q = 0; q < quads; ++q) {
+          const float4 w = *reinterpret_cast<const float4*>(ws + col * R_LD + 4 * q);
+#pragma unroll
+          for (int i = 0; i < R_ROWS / 2; ++i) {
+            const float4 a = *reinterpret_cast<const float4*>(as + (part * (R_ROWS / 2) + i) * R_K + 4 * q);
+            v[i] = fmaf(a.x, w.x, v[i]);
+            v[i] = fmaf(a.y, w.y, v[i]);
+            v[i] = fmaf(a.z, w.z, v[i]);
+            v[i] = fmaf(a.w, w.w, v[i]);
+          }
+        }
+      }
+    }
+    if (tid < WORKERS && n < N)
+#pragma unroll
+      for (int i = 0; i < R_ROWS / 2; ++i) {
+        const int r = r0 + part * (R_ROWS / 2) + i;
+        if (r >= rows) break;
+        float* c = C + (size_t)bad_rows[r] * ldc + n;
+        if (!finite(*c)) *c = bias != nullptr ? v[i] + bias[n] : v[i];
+      }
   }
+  __syncthreads();  // the list of rows is read
 }
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -197,7 +263,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
   __shared__ __align__(8) uint64_t w_full[W_STAGES], w_empty[W_STAGES], a_full[S::UNITS], a_empty[S::UNITS], op_full[2],
       d_full, d_empty, small_full, small_empty, drained;
   __shared__ uint32_t tmem_base;
-  __shared__ int gave_up;
+  __shared__ int gave_up, any_bad;  // any_bad: an element that is not finite was stored
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
   pdl_trigger();
@@ -206,7 +272,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
     tmem_relinquish();
   }
   if (tid == 0) {
-    gave_up = 0;
+    gave_up = any_bad = 0;
     for (int i = 0; i < W_STAGES; ++i) {
       mbar_init(&w_full[i], 1);
       mbar_init(&w_empty[i], WORKERS / 32);
@@ -494,7 +560,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
             bad = bad || !finite(v);
           }
         }
-        if (__any_sync(0xffffffffu, bad)) repair(A, lda, W, ldw, C, ldc, n0, m0, min(TC, M - m0), N, K, bias);
+        if (bad) any_bad = 1;
         c = segment = 0;
         tile += tile_step;
       }
@@ -545,10 +611,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
           for (int e = 0; e < 4; ++e)
             if (n + e < N) c[e] = v[e];
         }
-        if (__any_sync(0xffffffffu, bad)) {  // (the vote also orders the stores before the loads)
-          __syncwarp();
-          for (int e = 0; e < 4; ++e) repair(A, lda, W, ldw, C, ldc, n0 + 32 * e, m0 + t, 1, N, K, bias);
-        }
+        if (bad) any_bad = 1;
       }
     }
     __syncwarp();
@@ -558,6 +621,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
   __syncthreads();
   tc_fence_after();
   if (warp == MMA_WARP_ID) tmem_dealloc(tmem, S::TMEM);
+  if (any_bad && !gave_up)
+    for (int tile = tile0; tile < tiles; tile += tile_step) {
+      const int m0 = tile % m_tiles * T, rows = min(T, M - m0);
+      repair<T>(reinterpret_cast<float*>(ws), A, lda, W, ldw, C, ldc, tile / m_tiles * ROWS, m0 + rank, S::SHARE,
+                (rows - rank + S::SHARE - 1) / S::SHARE, N, K, bias);
+    }
 }
 
 // A's rows in three parts: planes [3][M][ld] (hi, mid, lo); bound by its bytes.

@@ -133,6 +133,25 @@ def test_float32_product_of_few_or_unusual_numbers(ops32, m, n, k):
     assert int(ops32.status.flatten()[0]) == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(5, 1100, 8192), (3, 37889, 1024), (32, 1024, 1100), (40, 19000, 1088), (113, 1500, 14336), (777, 4100, 2048)])
+def test_float32_product_of_an_infinite_column(ops32, m, n, k):
+    """An infinity in every row: all elements are computed again, behind the block's waits; the general kernel's bits."""
+    g = torch.Generator().manual_seed(m * 3 + n)
+    x, w, bias = _randn(g, m, k), _randn(g, n, k), _randn(g, n)
+    x[:, k // 3], w[n // 2, k // 3] = float("inf"), 0.0
+    bias[1] = float("-inf")
+    odd_x = torch.empty(m, k + 1, device=DEV)[:, :k]
+    odd_x.copy_(x)
+    wide = torch.full((m, n + 5), 3.0, device=DEV)
+    bits = lambda v: v.contiguous().view(torch.int32)
+    for b in (None, bias):
+        want = ops32.linear(odd_x, w, bias=b)
+        assert torch.equal(bits(ops32.linear(x, w, bias=b)), bits(want)) and not bool(torch.isfinite(want).any())
+        ops32.linear(x, w, bias=b, out=wide[:, :n])
+        assert torch.equal(bits(wide[:, :n]), bits(want)) and bool((wide[:, n:] == 3.0).all())
+    assert int(ops32.status.flatten()[0]) == 0
+
+
 def _relative(got, ref):
     return float((got.double() - ref).norm() / ref.norm())
 
