@@ -71,9 +71,20 @@ extern "C" int fg_attention_simt(const void* q, int q_stride, void* out, int out
   return 0;
 }
 
-// The rows of a block of fg_attention_f32_prompt: tiles hold max(1, rows / min(group, rows)) tokens.  16: that entry is not
-// there for this head size (its tiles would not fit shared memory), fg_attention_simt takes such prompts.
-extern "C" int fg_attention_f32_prompt_rows() { return FG_HEAD_DIM <= 128 ? fg_attn::P_ROWS : fg_attn::ROWS; }
+// The rows of a block for a step's prompts, which make `small` tiles of 16 rows or `large` of 64 (tiles hold max(1, rows /
+// min(group, rows)) tokens): 64 for fg_attention_f32_prompt, 16 for fg_attention_simt, the same bits.  Above head size 128 tiles of
+// 64 rows would not fit shared memory.  A tile of 64 rows takes a block 3.4 us where one of 16 takes it 1.9 to 3.1, whatever part of
+// the rows holds queries, and an SM 1.8 times as long.  So 16 rows where all their blocks have an SM, or where they are not
+// 1.8 times as many.  Measured (32 / 8 heads of 64, 16 and 64 rows, us): one portion of 2 / 8 / 64 tokens on 4,000 keys
+// 291 / 387 / 391 and 430 / 446 / 480; 64 portions of 4 on 500 101 and 191; 16 portions of 8 and of 16 on 1,000 133 / 195 and
+// 117 / 124; prompts of 60 / 300 / 777 10.8 / 61 / 248 and 11.3 / 42 / 146.
+extern "C" int fg_attention_f32_prompt_rows(int small, int large, int n_heads, int n_kv_heads) {
+  using namespace fg_attn;
+  if (FG_HEAD_DIM > 128) return ROWS;
+  const long group = n_heads / n_kv_heads, slices16 = (group + ROWS - 1) / ROWS, slices64 = (group + P_ROWS - 1) / P_ROWS;
+  const long blocks16 = small * n_kv_heads * slices16, blocks64 = large * n_kv_heads * slices64;
+  return blocks16 <= fg_sm_count() || 5 * blocks16 <= 9 * blocks64 ? ROWS : P_ROWS;
+}
 
 // Prompt tiles in float32; pools start on 16 bytes.  Entries of request -1 or without tokens are padding.
 extern "C" int fg_attention_f32_prompt(const float* q, int q_stride, float* out, int out_stride, const float* k_pages,

@@ -20,7 +20,8 @@ __device__ __forceinline__ void cp_async_row16(float* dst, const float* src, boo
 // Prompts: a block holds 64 rows (tokens x heads of a group), a thread the scores of 4 rows x 4 keys and the outputs of the
 // same 4 rows x HD / 8 columns, so that only keys and values meet at a barrier (one a tile; the next tile's arrive by
 // asynchronous copies meanwhile).  What bounds it is shared memory: 8 reads of 16 bytes for 64 multiply-adds.
-// 777 tokens, 32 / 8 heads of 64: 16 rows a block (attention_simt.cuh) 245 us, here 145; 300 tokens 61 and 42, 60 tokens 11 and 11.
+// 777 tokens, 32 / 8 heads of 64: 16 rows a block (attention_simt.cuh) 248 us, here 146; 300 tokens 61 and 42.  Which prompts come
+// here: fg_attention_f32_prompt_rows.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int P_ROWS = 64;
 

@@ -1,7 +1,7 @@
 // Paged causal attention on the CUDA cores, float32 arithmetic throughout.
 //
-// One kernel serves prompt portions and single decoded tokens alike: the host
-// cuts the step's query tokens into tiles (request, first token, token count)
+// Prompt portions of few tokens, and all tokens where pages do not start on 16 bytes (attention_f32.cuh has
+// single tokens and the prompts of many): the host cuts the step's query tokens into tiles (request, first token, token count)
 // and each thread block handles one tile for one group of query heads that
 // share a key/value head.  Keys and values come only from the cache pages
 // (the step's own keys were written before), in tiles of 32 positions that
@@ -18,6 +18,8 @@
 //
 // Storage type T (float or bf16) only affects loads and the final store.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -214,8 +216,11 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
 // The same for float32 pages, bit for bit (every score, weight and output is the same sum in the same order).  A
 // query's keys stay one sequential walk, so what a launch waits for is the walk's length times a tile's latency: the
 // next tile's keys and values arrive by 16-byte asynchronous copies while this one is worked on, its page numbers a
-// tile earlier still, operands are read four numbers at a time, and rows without a query are skipped.
-// 5 single tokens on 100 to 500 keys: 155 -> 34 us; a prompt of 777: 335 -> 247 us (32 / 8 heads of 64).
+// tile earlier still, operands are read four numbers at a time, and rows without a query are skipped.  A key that a row does
+// not see contributes nothing to it here, whatever its value holds.
+// A tile's work is there twice, for tiles that all rows see whole and for the others: with the guard in one body for both, 8
+// tokens on 4,000 keys took 439 us instead of 387 (32 / 8 heads of 64); with as many registers as its blocks leave
+// 387 instead of 392, at head size 128 543 instead of 618.  Which prompts come here: fg_attention_f32_prompt_rows.
 template <int HD>
 struct SimtShape {
   static constexpr int HP = HD + 4, PP = KEYS + 4;  // padded rows: eight lanes read eight bank groups
@@ -223,7 +228,7 @@ struct SimtShape {
 };
 
 template <int HD>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, HD <= 64 ? 5 : 2)
 attention_simt_f32_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, int out_stride,
                           const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                           const int* __restrict__ block_table, int table_width, int page_size, int n_pages,
@@ -236,7 +241,7 @@ attention_simt_f32_kernel(const float* __restrict__ q, int q_stride, float* __re
   float* const Qs = smem_f;                 // [ROWS][HP]
   float* const Ks = Qs + ROWS * HP;         // [2][KEYS][HP]
   float* const Vs = Ks + 2 * KEYS * HP;     // [2][KEYS][HP]
-  float* const Ps = Vs + 2 * KEYS * HP;     // [ROWS][PP]
+  float* const Ps = Vs + 2 * KEYS * HP;     // [ROWS][PP]; -1: a key that the row does not see
   __shared__ float alpha_s[ROWS], l_s[ROWS];
   __shared__ int key_ok[2][KEYS], row_pos[ROWS];
 
@@ -340,73 +345,81 @@ attention_simt_f32_kernel(const float* __restrict__ q, int q_stride, float* __re
     const int after = settle(next + KEYS);
     next_page = page_of(after);
     __syncthreads();
-    const float* kt = Ks + (buf * KEYS + lane) * HP;
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    auto work = [&](auto guard) {
+      constexpr bool guarded = decltype(guard)::value;  // some row does not see some key of the tile
+      const float* kt = Ks + (buf * KEYS + lane) * HP;
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
-    for (int d = 0; d < HD; d += 4) {
-      const float4 kv = *reinterpret_cast<const float4*>(kt + d);
+      for (int d = 0; d < HD; d += 4) {
+        const float4 kv = *reinterpret_cast<const float4*>(kt + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 qv = *reinterpret_cast<const float4*>(Qs + (warp + 4 * i) * HP + d);
+          s[i] = fmaf(qv.x, kv.x, s[i]);
+          s[i] = fmaf(qv.y, kv.y, s[i]);
+          s[i] = fmaf(qv.z, kv.z, s[i]);
+          s[i] = fmaf(qv.w, kv.w, s[i]);
+        }
+      }
+      const int j = k0 + lane;
+      const bool has_key = key_ok[buf][lane] != 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float4 qv = *reinterpret_cast<const float4*>(Qs + (warp + 4 * i) * HP + d);
-        s[i] = fmaf(qv.x, kv.x, s[i]);
-        s[i] = fmaf(qv.y, kv.y, s[i]);
-        s[i] = fmaf(qv.z, kv.z, s[i]);
-        s[i] = fmaf(qv.w, kv.w, s[i]);
+        const int r = warp + 4 * i;
+        const int p = row_pos[r];
+        if (p < 0) continue;  // (the same for the whole warp)
+        const bool visible = has_key && j <= p && (j >= row_lo[i] || j < keep_first);
+        float sc = s[i] * scale;
+        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+        const float sv = visible ? sc : -INFINITY;
+        const float m_tile = warp_max(sv);
+        const float m_new = fmaxf(m_run[i], m_tile);
+        float pr = 0.f, al = 1.f;
+        if (m_new != -INFINITY) {
+          pr = visible ? expf(sv - m_new) : 0.f;
+          al = (m_run[i] == -INFINITY) ? 0.f : expf(m_run[i] - m_new);
+        }
+        const float psum = warp_sum(pr);
+        l_run[i] = l_run[i] * al + psum;
+        m_run[i] = m_new;
+        Ps[r * PP + lane] = visible || !guarded ? pr : -1.f;
+        if (lane == 0) alpha_s[r] = al;
       }
-    }
-    const int j = k0 + lane;
-    const bool has_key = key_ok[buf][lane] != 0;
+      __syncthreads();
+      if (o_live) {
+        const float al = alpha_s[o_row];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = warp + 4 * i;
-      const int p = row_pos[r];
-      if (p < 0) continue;  // (the same for the whole warp)
-      const bool visible = has_key && j <= p && (j >= row_lo[i] || j < keep_first);
-      float sc = s[i] * scale;
-      if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
-      const float sv = visible ? sc : -INFINITY;
-      const float m_tile = warp_max(sv);
-      const float m_new = fmaxf(m_run[i], m_tile);
-      float pr = 0.f, al = 1.f;
-      if (m_new != -INFINITY) {
-        pr = visible ? expf(sv - m_new) : 0.f;
-        al = (m_run[i] == -INFINITY) ? 0.f : expf(m_run[i] - m_new);
-      }
-      const float psum = warp_sum(pr);
-      l_run[i] = l_run[i] * al + psum;
-      m_run[i] = m_new;
-      Ps[r * PP + lane] = pr;
-      if (lane == 0) alpha_s[r] = al;
-    }
-    __syncthreads();
-    if (o_live) {
-      const float al = alpha_s[o_row];
-#pragma unroll
-      for (int i = 0; i < QUADS; ++i) o4[i] = make_float4(o4[i].x * al, o4[i].y * al, o4[i].z * al, o4[i].w * al);
-      o2 = make_float2(o2.x * al, o2.y * al);
-      const float* vt = Vs + buf * KEYS * HP;
+        for (int i = 0; i < QUADS; ++i) o4[i] = make_float4(o4[i].x * al, o4[i].y * al, o4[i].z * al, o4[i].w * al);
+        o2 = make_float2(o2.x * al, o2.y * al);
+        const float* vt = Vs + buf * KEYS * HP;
 #pragma unroll 2
-      for (int c = 0; c < KEYS; c += 4) {
-        const float4 p4 = *reinterpret_cast<const float4*>(Ps + o_row * PP + c);
-        const float pr[4] = {p4.x, p4.y, p4.z, p4.w};
+        for (int c = 0; c < KEYS; c += 4) {
+          const float4 p4 = *reinterpret_cast<const float4*>(Ps + o_row * PP + c);
+          const float pr[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+          for (int e = 0; e < 4; ++e) {
+            auto sum_up = [&](float value, float& o) { o = guarded && pr[e] < 0.f ? o : fmaf(pr[e], value, o); };
 #pragma unroll
-          for (int i = 0; i < QUADS; ++i) {
-            const float4 v = *reinterpret_cast<const float4*>(vt + (c + e) * HP + 32 * i + 4 * o_col);
-            o4[i].x = fmaf(pr[e], v.x, o4[i].x);
-            o4[i].y = fmaf(pr[e], v.y, o4[i].y);
-            o4[i].z = fmaf(pr[e], v.z, o4[i].z);
-            o4[i].w = fmaf(pr[e], v.w, o4[i].w);
-          }
-          if (REST) {
-            const float2 v = *reinterpret_cast<const float2*>(vt + (c + e) * HP + 32 * QUADS + 2 * o_col);
-            o2.x = fmaf(pr[e], v.x, o2.x);
-            o2.y = fmaf(pr[e], v.y, o2.y);
+            for (int i = 0; i < QUADS; ++i) {
+              const float4 v = *reinterpret_cast<const float4*>(vt + (c + e) * HP + 32 * i + 4 * o_col);
+              sum_up(v.x, o4[i].x);
+              sum_up(v.y, o4[i].y);
+              sum_up(v.z, o4[i].z);
+              sum_up(v.w, o4[i].w);
+            }
+            if (REST) {
+              const float2 v = *reinterpret_cast<const float2*>(vt + (c + e) * HP + 32 * QUADS + 2 * o_col);
+              sum_up(v.x, o2.x);
+              sum_up(v.y, o2.y);
+            }
           }
         }
       }
-    }
+    };
+    if (k0 + KEYS - 1 > min_pos || (window != 0 && k0 < first_visible(max_pos, window)))
+      work(std::true_type());
+    else
+      work(std::false_type());
     __syncthreads();  // the tile's buffer, the weights and the factors are free
     k0 = next;
     next = after;

@@ -98,7 +98,7 @@ _CORE_SIGNATURES = {
 _ATTN_SIGNATURES = {
     "fg_attention_simt": [_P, _I, _P, _I, _I, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F,
                           _P, _P, _P],
-    "fg_attention_f32_prompt_rows": [],
+    "fg_attention_f32_prompt_rows": [_I, _I, _I, _I],
     "fg_attention_f32_prompt": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P,
                                 _P],
     "fg_attention_f32_singles": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P,
@@ -127,6 +127,7 @@ _ATTN_SIGNATURES = {
 
 SKINNY_MAX_M = int(os.environ.get("FG_SKINNY_MAX_M", "8"))      # most tokens the weight-streaming product is used for (it takes up to 32)
 SIMT_ROWS = 16       # query rows per block of the float32 attention kernel
+F32_PROMPT_ROWS = 64  # ... of the float32 kernel of larger prompts
 PREFILL_ROWS = 64    # ... of the bfloat16 prompt kernel
 PREFILL_TMA_ROWS = 128  # ... of the bfloat16 prompt kernel with tiled TMA loads
 PREFILL_TMA_KEYS = 64   # key positions per tile of that kernel
@@ -1375,7 +1376,8 @@ class Ops:
         run's :class:`~fastgen_b200.cache.LayerMemory`, ``ctx`` the step's
         context.  bfloat16 runs on the tensor cores: prompt portions in one
         kernel, single tokens in a split-and-combine pair (with tiled TMA loads
-        where the shapes allow); float32 runs one CUDA-core kernel for all.
+        where the shapes allow).  float32 runs on the CUDA cores: single tokens in a kernel of
+        their own, prompt portions in blocks of 16 or 64 rows, all with the same sums in the same order.
 
         ``out_freqs`` (a frequency table, or ``None``): the caller wants the outputs' adjacent
         pairs turned by ``position * frequency``.  Returns ``True`` if the kernels did that for
@@ -1401,9 +1403,12 @@ class Ops:
         if q.dtype == torch.float32:
             rest = (n_heads, n_kv_heads, head_dim, window, keep_first, float(scale), float(softcap or 0.0), _ptr(sinks),
                     _ptr(self.status), _stream())
-            rows, least = lib.fg_attention_f32_prompt_rows(), 2
             if (k_pages.data_ptr() | v_pages.data_ptr()) % 16:
                 rows, least = SIMT_ROWS, 1  # numbers one by one, whatever the tokens
+            else:
+                small, large = (ctx.count_tiles(attention_tiling(n_heads, n_kv_heads, r), 2)
+                                for r in (SIMT_ROWS, F32_PROMPT_ROWS))
+                rows, least = lib.fg_attention_f32_prompt_rows(small, large, n_heads, n_kv_heads), 2
             tiles = ctx.attention_tiles(attention_tiling(n_heads, n_kv_heads, rows), least)
             if tiles.n and rows == SIMT_ROWS:
                 _check(lib, lib.fg_attention_simt(

@@ -112,6 +112,7 @@ class StepContext:
         self.host_seq_start: List[int] = [0]
         self.host_seq_cached: List[int] = []
         self._tiles: Dict[Tuple[int, int], AttentionTiles] = {}
+        self._tile_counts: Dict[Tuple[int, int], int] = {}
         self._singles: Optional[SingleTokens] = None
 
     def attention_tiles(self, tokens_per_tile: int, min_tokens: int = 1) -> AttentionTiles:
@@ -139,6 +140,18 @@ class StepContext:
                 tiles.append((cached + t - start + n_tok, slot, t, n_tok))
         tiles.sort(key=lambda tile: tile[0])
         return tiles
+
+    def count_tiles(self, tokens_per_tile: int, min_tokens: int = 1) -> int:
+        """How many tiles :meth:`attention_tiles` gives (a captured step, whose sequences change
+        from replay to replay: what one sequence of all its tokens would make)."""
+        if not self.host_seq_slot:
+            return -(-self.n_tokens // tokens_per_tile)
+        key = (tokens_per_tile, min_tokens)
+        if key not in self._tile_counts:
+            start = self.host_seq_start
+            self._tile_counts[key] = sum(-(-(b - a) // tokens_per_tile)
+                                         for a, b in zip(start, start[1:]) if b - a >= min_tokens)
+        return self._tile_counts[key]
 
     def _build_tiles(self, tpt: int, min_tokens: int) -> AttentionTiles:
         tiles = self.host_tiles(tpt, min_tokens)

@@ -298,7 +298,7 @@ def _attention_step(lengths, cached, page, heads, kv, hd, dtype, seed):
     return ctx, q, pools, order.to(DEV, torch.int32)
 
 
-@pytest.mark.parametrize("hd,heads,kv", [(64, 8, 2), (16, 3, 3), (48, 20, 1)])
+@pytest.mark.parametrize("hd,heads,kv", [(64, 8, 2), (16, 3, 3), (48, 20, 1), (160, 4, 2), (256, 4, 2)])
 @pytest.mark.parametrize("window,keep", [(0, 0), (40, 0), (40, 5), (-37, 0)])
 def test_float32_attention_on_asynchronous_copies(ops32, hd, heads, kv, window, keep):
     """The bits of the kernel that loads a number at a time (taken for pools that do not start on 16 bytes)."""
@@ -359,6 +359,42 @@ def test_float32_attention_by_tokens(ops32, hd, heads, kv, window, keep):
     keepers = torch.ones(q.shape[0], dtype=torch.bool, device=DEV)
     keepers[130] = False
     assert torch.equal(again[keepers], outs[0][keepers]) and not bool(torch.isfinite(again[130]).all())
+
+
+@pytest.mark.parametrize("hd,heads,kv", [(64, 8, 2), (16, 3, 3), (48, 20, 1), (128, 9, 3)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (40, 5), (300, 70), (-37, 0)])
+def test_float32_prompts_in_tiles_of_16_and_of_64_rows(ops32, hd, heads, kv, window, keep):
+    """Both kernels of prompts on the same steps, few and many tokens: the same bits, and what lies behind a row's keys reaches
+    neither; the rule takes blocks of 16 rows where 64 rows would leave SMs idle or be mostly empty."""
+    from fastgen_b200.csrc.ops import F32_PROMPT_ROWS, SIMT_ROWS, _check, _code, _ptr, _stream, attention_tiling, attn
+    lib, sms = attn(hd), torch.cuda.get_device_properties(0).multi_processor_count
+    tiling = {rows: attention_tiling(heads, kv, rows) for rows in (SIMT_ROWS, F32_PROMPT_ROWS)}
+    assert lib.fg_attention_f32_prompt_rows(sms // kv // 2, 1, heads, kv) == SIMT_ROWS
+    assert lib.fg_attention_f32_prompt_rows(8 * sms, 2 * sms, heads, kv) == F32_PROMPT_ROWS
+    assert lib.fg_attention_f32_prompt_rows(8 * sms, 8 * sms, heads, kv) == (SIMT_ROWS if heads // kv <= 16 else F32_PROMPT_ROWS)
+    for lengths, cached in (([2, 3, 9, 16, 17], [130, 0, 31, 700, 5]), ([64, 63, 65, 200], [0, 330, 31, 12])):
+        ctx, q, pools, table = _attention_step(lengths, cached, 16, heads, kv, hd, torch.float32, hd + window)
+        sinks = torch.linspace(-1, 1, heads, device=DEV)
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+        def run(rows):
+            tiles = ctx.attention_tiles(tiling[rows], 2)
+            assert ctx.count_tiles(tiling[rows], 2) == tiles.n
+            out = torch.full_like(q, 3.0)
+            kernel, dtype = (lib.fg_attention_simt, (_code(q.dtype),)) if rows == SIMT_ROWS else (lib.fg_attention_f32_prompt, ())
+            _check(lib, kernel(
+                _ptr(q), q.stride(0), _ptr(out), out.stride(0), *dtype, _ptr(pools[0]), _ptr(pools[1]), _ptr(table),
+                table.shape[1], 16, pools[0].shape[0], _ptr(ctx.pos), _ptr(tiles.req), _ptr(tiles.tok0), _ptr(tiles.ntok), tiles.n,
+                heads, kv, hd, window, keep, hd ** -0.5, 3.0 if keep == 5 else 0.0, _ptr(sinks), _ptr(status), _stream()))
+            return out
+
+        few, many = run(SIMT_ROWS), run(F32_PROMPT_ROWS)
+        assert torch.equal(few, many) and bool(torch.isfinite(few).all())
+        last = cached[-1] + lengths[-1] - 1  # only the last token sees its entry
+        page, place = int(table[-1, last // 16]), last % 16
+        pools[0][page, :, place], pools[1][page, :, place] = float("nan"), float("inf")
+        again = [run(rows) for rows in (SIMT_ROWS, F32_PROMPT_ROWS)]
+        assert all(torch.equal(v[:-1], few[:-1]) and not bool(torch.isfinite(v[-1]).any()) for v in again) and int(status) == 0
 
 
 @pytest.mark.parametrize("page", [8, 64, 128])
