@@ -134,17 +134,31 @@ extern "C" int fg_attention_f32_singles(const float* q, int q_stride, float* out
                "fg_attention_f32_singles: %d heads over %d kv heads", n_heads, n_kv_heads);
   FG_CHECK_ARG((((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0, "fg_attention_f32_singles: pools off 16 bytes");
   const int group = n_heads / n_kv_heads;
-  auto launch = [&](auto kern, int rows, size_t bytes) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  auto launch = [&](auto kern, auto shape, int rows) {
+    using S = decltype(shape);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
     FG_CHECK_ARG(e == cudaSuccess, "fg_attention_f32_singles: shared memory: %s", cudaGetErrorString(e));
-    fg_launch_pdl(kern, dim3(n_singles, n_kv_heads, (group + rows - 1) / rows), dim3(S_THREADS), bytes, stream, q, q_stride,
+    fg_launch_pdl(kern, dim3(n_singles, n_kv_heads, (group + rows - 1) / rows), dim3(S::THREADS), S::SMEM, stream, q, q_stride,
                   out, out_stride, k_pages, v_pages, block_table, table_width, page_size, n_pages, pos, req_of, single_req,
                   single_tok, n_kv_heads, group, window, keep_first, scale, status, softcap, sinks);
     return 0;
   };
+  auto by_form = [&](auto rows) {  // (why these forms: attention_f32.cuh)
+    constexpr int HD = FG_HEAD_DIM, R = decltype(rows)::value;
+    using S0 = SingleShape<HD, R, 0>;
+    using S1 = SingleShape<HD, R, 1>;
+    using S2 = SingleShape<HD, R, 2>;
+    const long blocks = (long)n_singles * n_kv_heads * ((group + R - 1) / R), sms = fg_sm_count();
+    const int form = blocks <= sms * S0::BLOCKS || (!S1::THERE && !S2::THERE) ? 0
+                     : S1::THERE && (blocks <= sms * S1::BLOCKS || !S2::THERE) ? 1 : 2;
+    if constexpr (S1::THERE)
+      if (form == 1) return launch(attention_single_f32_kernel<HD, R, 1>, S1(), R);
+    if constexpr (S2::THERE)
+      if (form == 2) return launch(attention_single_f32_kernel<HD, R, 2>, S2(), R);
+    return launch(attention_single_f32_kernel<HD, R, 0>, S0(), R);
+  };
   // groups of up to 4 heads without the work of 8
-  const int rc = group <= 4 ? launch(attention_single_f32_kernel<FG_HEAD_DIM, 4>, 4, SingleShape<FG_HEAD_DIM, 4>::SMEM)
-                            : launch(attention_single_f32_kernel<FG_HEAD_DIM, 8>, 8, SingleShape<FG_HEAD_DIM, 8>::SMEM);
+  const int rc = group <= 4 ? by_form(std::integral_constant<int, 4>()) : by_form(std::integral_constant<int, 8>());
   if (rc) return rc;
   FG_CHECK_LAUNCH("fg_attention_f32_singles");
   return 0;

@@ -287,31 +287,43 @@ attention_prompt_f32_kernel(const float* __restrict__ q, int q_stride, float* __
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Single tokens: a block holds one token and R heads of a group (as many as there are, rounded up to 4 or 8).  The walk over the keys is a chain only in the
-// outputs' sums: eight tiles of 32 keys are scored at once, two a warp, their maxima meet in shared memory,
-// every warp finds the running maximum that its tile starts from, and only then the outputs walk the 256 keys, four rows a
-// thread side by side.  The next tiles' keys come by asynchronous copies during that walk, their values behind it.
-// 5 tokens on 100 to 500 keys, 32 / 8 heads of 64: tile after tile (attention_simt.cuh) 38 us, here 16; one on 700 keys
-// 50 and 23, one on 20 5.6 and 5.5, 16 on 600 44 and 21.
+// Single tokens: a block holds one token and R heads of a group (as many as there are, rounded up to 4 or 8).  The walk over the
+// keys is a chain only in the outputs' sums: a run of several tiles of 32 keys is scored at once, a warp one or two of
+// them, their maxima meet in shared memory, every warp finds the running maximum that its tile starts from, and only then
+// the outputs walk the run's keys, four rows a thread side by side.  The next run's keys come by asynchronous copies
+// during that walk, their values behind it.
+//
+// One block's time falls with the run's length, its shared memory grows with it (head size 64: 139 KB at 8 tiles, 71 at 4, 37 at 2),
+// and a launch of more blocks than fit at once takes another turn for the rest.  So the longest run whose blocks fit at
+// once, else the shortest that is there: form 0 (256 threads; 8 tiles up to head size 80, 4 up to 160, 2 beyond), form 1 (128
+// threads, 4 tiles, up to head size 80), form 2 (2 tiles, 48 to 160).  Measured (us; 32 / 8 heads of 64; tile after tile in blocks of 16
+// rows as in attention_simt.cuh, then forms 0, 1, 2): one token on 4,000 keys 320 / 112 / 149 / 203, 32 tokens 365 / 231 / 208 / 272,
+// 64 tokens 501 / 458 / 410 / 300, and on 20 keys 8 / 21 / 10 / 6; 128 tokens on 250 77 / 71 / 47 / 41.  Head size 128, 64 tokens on 1,000
+// 289 / 213 / - / 159.  5 tokens on 100 to 500 keys of 64 38 / 16.  Blocks of 16 rows stay ahead on a few tens of keys at groups of
+// 8 (7 us to 8) and at head sizes 16 and 32 (4 to 5), and with 768 blocks at head size 16 (240 to 276 on 4,000 keys).
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int S_MAX_ROWS = 8, S_TILES = 8, S_THREADS = 256;
-
-template <int HD, int R>
+template <int HD, int R, int FORM>
 struct SingleShape {
-  static constexpr int TILES = HD <= 80 ? S_TILES : HD <= 160 ? S_TILES / 2 : S_TILES / 4;  // what shared memory holds
+  static constexpr bool THERE = FORM == 0 || (FORM == 1 ? HD <= 80 : HD > 32 && HD <= 160);
+  static constexpr int TILES = FORM == 1 ? 4 : FORM == 2 ? 2 : HD <= 80 ? 8 : HD <= 160 ? 4 : 2;  // what shared memory holds
+  static constexpr int THREADS = FORM == 0 ? 256 : 128, A_WARP = FORM == 0 ? 2 : 1;  // tiles that a warp scores
   static constexpr int CHUNK = TILES * KEYS, KP = HD + 4;  // padded rows of keys: eight lanes read eight bank groups
   static constexpr size_t SMEM = sizeof(float) * (CHUNK * (HD + KP) + R * HD + CHUNK * R);
+  // blocks an SM: by shared memory (4 KB beside the above) and by 128 registers a thread (4 rows, 128 threads: 96)
+  static constexpr int FIT = (int)(228 * 1024 / (SMEM + 4096)), MOST = FORM == 0 ? 2 : R == 4 ? 5 : 4;
+  static constexpr int BLOCKS = FIT < 1 ? 1 : FIT < MOST ? FIT : MOST;
 };
 
-template <int HD, int R>
-__global__ void __launch_bounds__(S_THREADS, 1)
+template <int HD, int R, int FORM>
+__global__ void __launch_bounds__(SingleShape<HD, R, FORM>::THREADS, SingleShape<HD, R, FORM>::BLOCKS)
 attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_stride, const float* k_pages,
                             const float* v_pages, const int* __restrict__ block_table, int table_width, int page_size,
                             int n_pages, const int* __restrict__ pos, const int* __restrict__ req_of,
                             const int* __restrict__ single_req, const int* __restrict__ single_tok, int n_kv_heads,
                             int group, int window, int keep_first, float scale, int* status, float softcap,
                             const float* __restrict__ sinks) {
-  constexpr int TILES = SingleShape<HD, R>::TILES, CHUNK = SingleShape<HD, R>::CHUNK, KP = SingleShape<HD, R>::KP;
+  using S = SingleShape<HD, R, FORM>;
+  constexpr int TILES = S::TILES, CHUNK = S::CHUNK, KP = S::KP, THREADS = S::THREADS, H = S::A_WARP;
   extern __shared__ __align__(16) float smem_f[];
   float* const Vs = smem_f;                 // [CHUNK][HD]
   float* const Ks = Vs + CHUNK * HD;        // [CHUNK][KP]
@@ -329,7 +341,7 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
   if (b < 0) {
     // padding of a fixed-size batch: no request; the rows of a token that belongs to none are zeroed
     if (req_of[tok] < 0)
-      for (int i = tid; i < rows * HD; i += S_THREADS) o[i] = 0.f;
+      for (int i = tid; i < rows * HD; i += THREADS) o[i] = 0.f;
     return;
   }
   const int p = pos[tok], lo = first_visible(p, window);
@@ -358,7 +370,7 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
     }
     return ((unsigned)page * n_kv_heads + g) * page_size + j % page_size;
   };
-  for (int i = tid; i < R * HD; i += S_THREADS)
+  for (int i = tid; i < R * HD; i += THREADS)
     Qs[i] = i < rows * HD ? q[(size_t)tok * q_stride + (size_t)(g * group + head0) * HD + i] : 0.f;
 
   // every thread keeps the running maxima; the sums' and outputs' state: thread -> column, four rows
@@ -366,7 +378,7 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
 #pragma unroll
   for (int r = 0; r < R; ++r) m_run[r] = sinks != nullptr && r < rows ? sinks[g * group + head0 + r] : -INFINITY;
   float l_run = sinks != nullptr ? 1.f : 0.f;  // of row `tid` (tid < R)
-  constexpr int SLOTS = (R / 4 * (HD / 2) + S_THREADS - 1) / S_THREADS;  // (two columns, four rows) a thread
+  constexpr int SLOTS = (R / 4 * (HD / 2) + THREADS - 1) / THREADS;  // (two columns, four rows) a thread
   float2 acc[SLOTS][4];
 #pragma unroll
   for (int u = 0; u < SLOTS; ++u)
@@ -374,12 +386,12 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
     for (int r = 0; r < 4; ++r) acc[u][r] = make_float2(0.f, 0.f);
 
   auto look_up = [&](int t0, int buf) {
-    for (int i = tid; i < CHUNK; i += S_THREADS) row_s[buf][i] = key_row(t0 + i / KEYS, i % KEYS);
+    for (int i = tid; i < CHUNK; i += THREADS) row_s[buf][i] = key_row(t0 + i / KEYS, i % KEYS);
   };
   auto copy = [&](float* dst, int stride, const float* pool, int buf, int tiles) {
 #pragma unroll 4
-    for (int u = 0; u < CHUNK * (HD / 4) / S_THREADS; ++u) {
-      const int i = tid + u * S_THREADS, key = i / (HD / 4), c = i % (HD / 4) * 4;
+    for (int u = 0; u < CHUNK * (HD / 4) / THREADS; ++u) {
+      const int i = tid + u * THREADS, key = i / (HD / 4), c = i % (HD / 4) * 4;
       if (key >= tiles * KEYS) break;
       const unsigned row = row_s[buf][key];
       cp_async_row16(dst + key * stride + c, pool + (row != NONE ? (size_t)row * HD + c : 0), row != NONE);
@@ -396,33 +408,35 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
     if (t0 + TILES < n_tiles) look_up(t0 + TILES, buf ^ 1);
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();  // the keys have landed for all
-    // a warp two tiles, a lane a key of each: a read of the queries serves both
-    const int w0 = warp * 2;
-    float s[2][R];
-    bool visible[2] = {false, false};
+    // a warp H tiles, a lane a key of each: a read of the queries serves all
+    const int w0 = warp * H;
+    float s[H][R];
+    bool visible[H];
     if (w0 < tiles) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) s[0][r] = s[1][r] = 0.f;
+      for (int r = 0; r < H * R; ++r) s[r / R][r % R] = 0.f;
       const float* kr = Ks + (w0 * KEYS + lane) * KP;
 #pragma unroll 4
       for (int d = 0; d < HD; d += 4) {
-        const float4 ka = *reinterpret_cast<const float4*>(kr + d), kb = *reinterpret_cast<const float4*>(kr + KEYS * KP + d);
+        float4 kv[H];
+#pragma unroll
+        for (int h = 0; h < H; ++h) kv[h] = *reinterpret_cast<const float4*>(kr + h * KEYS * KP + d);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const float4 qv = *reinterpret_cast<const float4*>(Qs + r * HD + d);
-          s[0][r] = fmaf(qv.x, ka.x, s[0][r]);
-          s[1][r] = fmaf(qv.x, kb.x, s[1][r]);
-          s[0][r] = fmaf(qv.y, ka.y, s[0][r]);
-          s[1][r] = fmaf(qv.y, kb.y, s[1][r]);
-          s[0][r] = fmaf(qv.z, ka.z, s[0][r]);
-          s[1][r] = fmaf(qv.z, kb.z, s[1][r]);
-          s[0][r] = fmaf(qv.w, ka.w, s[0][r]);
-          s[1][r] = fmaf(qv.w, kb.w, s[1][r]);
+#pragma unroll
+          for (int h = 0; h < H; ++h) s[h][r] = fmaf(qv.x, kv[h].x, s[h][r]);
+#pragma unroll
+          for (int h = 0; h < H; ++h) s[h][r] = fmaf(qv.y, kv[h].y, s[h][r]);
+#pragma unroll
+          for (int h = 0; h < H; ++h) s[h][r] = fmaf(qv.z, kv[h].z, s[h][r]);
+#pragma unroll
+          for (int h = 0; h < H; ++h) s[h][r] = fmaf(qv.w, kv[h].w, s[h][r]);
         }
       }
-      float mx[2][R];
+      float mx[H][R];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int h = 0; h < H; ++h) {
         const int j = tile_pos(t0 + w0 + h) + lane;
         visible[h] = w0 + h < tiles && row_s[buf][(w0 + h) * KEYS + lane] != NONE && j <= p && (j >= lo || j < keep_first);
 #pragma unroll
@@ -435,10 +449,10 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int r = 0; r < 2 * R; ++r) mx[r / R][r % R] = fmaxf(mx[r / R][r % R], __shfl_xor_sync(0xffffffffu, mx[r / R][r % R], o));
+        for (int r = 0; r < H * R; ++r) mx[r / R][r % R] = fmaxf(mx[r / R][r % R], __shfl_xor_sync(0xffffffffu, mx[r / R][r % R], o));
       if (lane == 0)
 #pragma unroll
-        for (int r = 0; r < 2 * R; ++r) max_s[w0 + r / R][r % R] = mx[r / R][r % R];
+        for (int r = 0; r < H * R; ++r) max_s[w0 + r / R][r % R] = mx[r / R][r % R];
     }
     __syncthreads();
     // the keys are read: the next ones are on their way during the rest (an empty group keeps the count where there are none)
@@ -447,17 +461,17 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
     else
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     if (w0 < tiles) {
-      float before[2][R], sum[2][R];
+      float before[H][R], sum[H][R];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         float m = m_run[r];
 #pragma unroll
-        for (int u = 0; u < TILES - 2; ++u) m = fmaxf(m, u < w0 ? max_s[u][r] : -INFINITY);
-        before[0][r] = m;
-        before[1][r] = fmaxf(m, max_s[w0][r]);
+        for (int u = 0; u < TILES - H; ++u) m = fmaxf(m, u < w0 ? max_s[u][r] : -INFINITY);
+#pragma unroll
+        for (int h = 0; h < H; ++h) before[h][r] = m = h == 0 ? m : fmaxf(m, max_s[w0 + h - 1][r]);
       }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int h = 0; h < H; ++h) {
         const bool hide = w0 + h < tiles && masked(t0 + w0 + h);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -472,10 +486,10 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int r = 0; r < 2 * R; ++r) sum[r / R][r % R] += __shfl_xor_sync(0xffffffffu, sum[r / R][r % R], o);
+        for (int r = 0; r < H * R; ++r) sum[r / R][r % R] += __shfl_xor_sync(0xffffffffu, sum[r / R][r % R], o);
       if (lane == 0)
 #pragma unroll
-        for (int r = 0; r < 2 * R; ++r) sum_s[w0 + r / R][r % R] = sum[r / R][r % R];
+        for (int r = 0; r < H * R; ++r) sum_s[w0 + r / R][r % R] = sum[r / R][r % R];
     }
 #pragma unroll
     for (int u = 0; u < TILES; ++u)
@@ -487,7 +501,7 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
       for (int u = 0; u < tiles; ++u) l_run = l_run * al_s[u][tid] + sum_s[u][tid];
 #pragma unroll
     for (int u = 0; u < SLOTS; ++u) {
-      const int at = tid + u * S_THREADS, col = at % (HD / 2) * 2, r0 = at / (HD / 2) * 4;
+      const int at = tid + u * THREADS, col = at % (HD / 2) * 2, r0 = at / (HD / 2) * 4;
       if (r0 >= R) continue;
       auto one_tile = [&](int n, bool guarded) {
         const float* vt = Vs + n * KEYS * HD + col;
@@ -525,7 +539,7 @@ attention_single_f32_kernel(const float* q, int q_stride, float* out, int out_st
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < SLOTS; ++u) {
-    const int at = tid + u * S_THREADS, col = at % (HD / 2) * 2, r0 = at / (HD / 2) * 4;
+    const int at = tid + u * THREADS, col = at % (HD / 2) * 2, r0 = at / (HD / 2) * 4;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
       if (r0 + r < rows) {

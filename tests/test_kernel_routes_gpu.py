@@ -397,6 +397,41 @@ def test_float32_prompts_in_tiles_of_16_and_of_64_rows(ops32, hd, heads, kv, win
         assert all(torch.equal(v[:-1], few[:-1]) and not bool(torch.isfinite(v[-1]).any()) for v in again) and int(status) == 0
 
 
+@pytest.mark.parametrize("hd,heads,kv,n", [
+    (64, 32, 8, 18), (64, 32, 8, 19), (64, 32, 8, 55), (64, 32, 8, 56), (64, 20, 4, 140),  # runs of 8, 4, 4, 2 and 2 tiles
+    (16, 9, 3, 99), (16, 9, 3, 400), (32, 5, 5, 140), (48, 40, 5, 90), (48, 40, 5, 130), (80, 24, 24, 13), (80, 24, 24, 20),
+    (128, 32, 8, 40), (160, 8, 4, 80), (256, 4, 2, 90)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (100, 40), (-37, 0)])
+def test_float32_single_tokens_by_their_number(ops32, hd, heads, kv, n, window, keep):
+    """More blocks than fit the chip at once walk their keys in shorter runs: the bits of the kernel that walks tile after tile
+    (taken for pools off 16 bytes), padding tokens zeroed."""
+    from fastgen_b200.engine.step import SingleTokens
+    ctx, q, pools, table = _attention_step([1] * n, [(37 * i) % 90 + 300 * (i % 7 == 3) for i in range(n)], 16, heads, kv, hd,
+                                           torch.float32, hd + n)
+    ctx.req = torch.arange(n, dtype=torch.int32, device=DEV)
+    how = dict(window=max(window, 0) or None, scale=hd ** -0.5, keep_first=keep, softcap=3.0 if keep else None,
+               sinks=torch.linspace(-1, 1, heads, device=DEV) if window else None, chunk=-window if window < 0 else None)
+    outs = []
+    for shift in (0, 1):
+        moved = []
+        for pool in pools:
+            room = torch.empty(pool.numel() + 4, device=DEV)
+            moved.append(room[shift : shift + pool.numel()].view(pool.shape))
+            moved[-1].copy_(pool)
+        memory = SimpleNamespace(k_pages=moved[0], v_pages=moved[1], block_table=table, page_size=16)
+        out = torch.full_like(q, float("nan"))
+        ops32.attention(q, out, memory, ctx, heads, kv, hd, **how)
+        outs.append(out)
+        if shift == 0:  # as in a captured step: the last token belongs to no request
+            padded = torch.full_like(q, float("nan"))
+            ctx.req[-1] = -1
+            ctx._singles = SingleTokens(ctx.req.clone(), torch.arange(n, dtype=torch.int32, device=DEV), n, 400)
+            ops32.attention(q, padded, memory, ctx, heads, kv, hd, **how)
+            ctx._singles, ctx.req[-1] = None, n - 1
+    assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all()) and int(ops32.status) == 0
+    assert torch.equal(padded[:-1], outs[0][:-1]) and not bool(padded[-1].any())
+
+
 @pytest.mark.parametrize("page", [8, 64, 128])
 @pytest.mark.parametrize("keep,window", [(1, 64), (4, 100), (70, 130), (200, 65)])
 def test_kept_positions_in_the_tensor_memory_kernel(ops16, keep, window, page):
