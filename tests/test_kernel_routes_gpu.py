@@ -637,6 +637,155 @@ def test_rotation_and_attention_start_early(ops16):
     assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
+def _graph_against_waits(ops, run, inputs, keep):
+    """``run(wait)`` step by step with ``inputs`` (pairs of a buffer and its contents a step): launches with a wait after each
+    against one graph of them, from the same ``keep`` (buffers that steps change); the results and buffers of both."""
+    first, results = [k.clone() for k in keep], []
+    for graph in (False, True):
+        if graph:
+            stream, replay = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                replay.capture_begin()
+                out = run(lambda: None)
+                replay.capture_end()
+            torch.cuda.current_stream().wait_stream(stream)
+        for k, v in zip(keep, first):
+            k.copy_(v)
+        got = []
+        for step in range(len(inputs[0][1])):
+            for buffer, contents in inputs:
+                buffer.copy_(contents[step])
+            if graph:
+                replay.replay()
+            else:
+                out = run(torch.cuda.synchronize)
+            got.append(out.clone())
+        ops.check_status()
+        results.append(got + [k.clone() for k in keep])
+    return results
+
+
+def test_state_space_layers_start_early(ops16):
+    """Projection, convolution, its state, the recurrence and the gated norm of two layers as programmatic launches behind one
+    another in a graph: the bits of the same launches with a wait after each."""
+    heads, groups, n_state, p, dim, taps, n = 8, 2, 128, 64, 512, 4, 5
+    inner, channels, floats = heads * p, heads * p + 2 * groups * n_state, heads * n_state * p
+    ctx = _sequences([1] * n, slots=[3, 0, -1, 4, 1])
+    ctx.longest, ctx.req = 1, ctx.seq_slot
+    g = torch.Generator().manual_seed(8)
+    layers = [SimpleNamespace(
+        w_in=_randn(g, inner + channels + heads, dim, scale=dim ** -0.5).to(torch.bfloat16),
+        wo=_randn(g, dim, inner, scale=inner ** -0.5).to(torch.bfloat16),
+        conv=_randn(g, channels, taps, scale=0.5), bias=_randn(g, channels), dt_bias=torch.rand(heads, generator=g).to(DEV) * 3.5 - 3,
+        a_log=torch.rand(heads, generator=g).to(DEV) * 2.5 - 1, d=_randn(g, heads), norm=1 + _randn(g, inner, scale=0.1),
+        state=_randn(g, 6, floats + (taps - 1) * channels)) for _ in range(2)]
+    x = torch.zeros(n, dim, dtype=torch.bfloat16, device=DEV)
+
+    def run(wait):
+        h = x
+        for l in layers:
+            proj = ops16.linear(h, l.w_in)
+            wait()
+            xbc = ops16.mamba2_conv(proj, inner, channels, l.conv, l.bias, l.state, floats, taps, ctx)
+            wait()
+            y = ops16.mamba2_scan(xbc, proj, inner + channels, l.dt_bias, l.a_log, l.d, l.state, ctx, heads, groups, n_state, p)
+            wait()
+            h = ops16.linear(ops16.gated_part_norm(y, proj[:, :inner], l.norm, groups, 1e-5, ctx), l.wo)
+            wait()
+        return h
+
+    xs = [_randn(g, n, dim).to(torch.bfloat16) for _ in range(6)]
+    live = ctx.req >= 0
+    a, b = _graph_against_waits(ops16, run, [(x, xs)], [l.state for l in layers])
+    assert all(torch.equal(u[live] if u.shape[0] == n else u, v[live] if v.shape[0] == n else v) for u, v in zip(a, b))
+
+
+def _latent_step(g, first, page, width, entry):
+    """Single tokens at the positions ``first`` and one of no request, and a pool of random entries."""
+    from fastgen_b200.engine.step import AttentionTiles
+    n, n_pages = len(first), len(first) * width + 2
+    to = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    req, tok = to(list(range(n)) + [-1]), to(list(range(n + 1)))
+    ctx = SimpleNamespace(req=req, pos=to(first + [0]), n_tokens=n + 1, n_seqs=n + 1)
+    ctx.attention_tiles = lambda tpt, least=1: AttentionTiles(req, tok, torch.ones_like(req), n + 1)
+    table = torch.randperm(n_pages, generator=g)[: n * width].reshape(n, width).to(DEV, torch.int32)
+    pool = _randn(g, n_pages, 1, page, entry).to(torch.bfloat16)
+    return ctx, SimpleNamespace(k_pages=pool, block_table=table, page_size=page)
+
+
+def test_latent_layers_start_early(ops16):
+    """Projection, cache entry and query norm, query projection, rotation, attention in stretches and their merge, two layers
+    behind one another in a graph: the bits of the same launches with a wait after each."""
+    R, r, heads, hd, q_rank, dim, page = 256, 32, 8, 64, 128, 512, 16
+    g = torch.Generator().manual_seed(9)
+    first = [0, 15, 16, 63, 200, 330]
+    n, qk = len(first), hd + r
+    layers = []
+    for _ in range(2):
+        ctx, memory = _latent_step(g, first, page, 22, R + r)
+        layers.append(SimpleNamespace(
+            memory=memory, down=_randn(g, q_rank + R + r, dim, scale=dim ** -0.5).to(torch.bfloat16),
+            up=_randn(g, heads * qk, q_rank, scale=q_rank ** -0.5).to(torch.bfloat16),
+            uk=_randn(g, heads, hd, R, scale=hd ** -0.5).to(torch.bfloat16), qn=1 + _randn(g, q_rank, scale=0.1),
+            kn=1 + _randn(g, R, scale=0.1), back=_randn(g, dim, heads * R, scale=R ** -0.5).to(torch.bfloat16)))
+    freqs = torch.linspace(1, 0.01, r // 2, device=DEV)
+    x = torch.zeros(n + 1, dim, dtype=torch.bfloat16, device=DEV)
+    lat = torch.zeros(n + 1, heads, R, dtype=torch.bfloat16, device=DEV)
+
+    def run(wait):
+        h = x
+        for l in layers:
+            down = ops16.linear(h, l.down)
+            wait()
+            q = ops16.latent_prepare(down[:, q_rank:], l.kn, 1e-5, freqs, 1.0, l.memory, ctx, R, r, down[:, :q_rank], q_norm=l.qn,
+                                     n_heads=heads, head_size=qk)
+            wait()
+            q = ops16.linear(q, l.up)
+            wait()
+            ops16.rotate_part(q, ctx, freqs, 1.0, heads, qk, hd, r)
+            wait()
+            q = q.view(n + 1, heads, qk)
+            qa = ops16.head_products(q[:, :, :hd], l.uk)
+            wait()
+            ops16.latent_attention(qa, q[:, :, hd:], lat.permute(1, 0, 2), None, l.memory, ctx, heads, R, r, qk ** -0.5)
+            wait()
+            h = ops16.linear(lat.view(n + 1, heads * R), l.back)
+            wait()
+        return h
+
+    steps = 6
+    xs = [_randn(g, n + 1, dim).to(torch.bfloat16) for _ in range(steps)]
+    pos = [torch.tensor([f + s for f in first] + [0], dtype=torch.int32, device=DEV) for s in range(steps)]
+    a, b = _graph_against_waits(ops16, run, [(x, xs), (ctx.pos, pos)], [l.memory.k_pages for l in layers])
+    assert all(torch.equal(u[:n] if u.shape[0] == n + 1 else u, v[:n] if v.shape[0] == n + 1 else v) for u, v in zip(a, b))
+    assert all(bool(torch.isfinite(u[:n]).all()) for u in a[:steps])
+
+
+@pytest.mark.parametrize("rank,rot", [(256, 32), (512, 64), (256, 0)])
+@pytest.mark.parametrize("tokens", [1, 3])
+def test_latent_queries_off_16_bytes(ops16, rank, rot, tokens):
+    """Queries whose rows lie on 16 bytes are copied in pieces of 16, others in pieces of 4: the same bits."""
+    heads, page, n = 6, 16, 5
+    g = torch.Generator().manual_seed(rank + rot + tokens)
+    cached = [0, 15, 40, 129, 200]
+    ctx, _, pools, table = _attention_step([tokens] * n, cached, page, 1, 1, rank + rot, torch.bfloat16, rank + tokens)
+    memory = SimpleNamespace(k_pages=pools[0], block_table=table, page_size=page)
+    t = n * tokens
+    qa, qt = _randn(g, heads, t, rank).to(torch.bfloat16), _randn(g, t, heads, rot).to(torch.bfloat16)
+    outs = []
+    for a_shift, t_shift in ((0, 0), (2, 0), (0, 6), (4, 2)):
+        wide_a = torch.full((heads, t, rank + 8), float("nan"), dtype=torch.bfloat16, device=DEV)
+        wide_t = torch.full((t, heads, rot + 8), float("nan"), dtype=torch.bfloat16, device=DEV)
+        wide_a[:, :, a_shift : a_shift + rank], wide_t[:, :, t_shift : t_shift + rot] = qa, qt
+        out = torch.full((heads, t, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops16.latent_attention(wide_a[:, :, a_shift : a_shift + rank], wide_t[:, :, t_shift : t_shift + rot], out, None, memory, ctx,
+                               heads, rank, rot, rank ** -0.5)
+        ops16.check_status()
+        outs.append(out)
+    assert bool(torch.isfinite(outs[0]).all()) and all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
 # -- recurrences, chunk by chunk ---------------------------------------------------------------------------
 
 LENGTHS = [([64], 0), ([65, 1, 63], 3), ([95, 96, 97], 0), ([2, 130, 64], 1), ([20, 30], 14), ([300], 0),
