@@ -225,10 +225,13 @@ template <int HD>
 struct SimtShape {
   static constexpr int HP = HD + 4, PP = KEYS + 4;  // padded rows: eight lanes read eight bank groups
   static constexpr size_t SMEM = sizeof(float) * ((ROWS + 4 * KEYS) * HP + ROWS * PP);
+  // Blocks an SM: by shared memory (2 KB beside the above), 6 at most.  Up to head size 32 the compiler's own choice (70
+  // registers): 64 portions of 4 tokens on 500 keys 49 us, with room for 7 blocks asked for 54.
+  static constexpr int FIT = (int)(228 * 1024 / (SMEM + 2048)), BLOCKS = HD <= 32 ? 0 : FIT < 1 ? 1 : FIT < 6 ? FIT : 6;
 };
 
 template <int HD>
-__global__ void __launch_bounds__(THREADS, HD <= 64 ? 5 : 2)
+__global__ void __launch_bounds__(THREADS, SimtShape<HD>::BLOCKS)
 attention_simt_f32_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, int out_stride,
                           const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                           const int* __restrict__ block_table, int table_width, int page_size, int n_pages,
