@@ -720,6 +720,10 @@ Plan choose(int M, int N, int K) {
 
 // Whether the product takes this way: by K and N and by how the rows lie, never by M (a row's sums do not
 // depend on the rows beside it).
+// The line lies above the sizes where a single row is slower this way than by multiply-adds.  Measured below it (us; this way, multiply-adds;
+// 1, 5, 16 and 777 rows): 576 x 576 4.6 / 4.7 / 4.9 / 25 and 3.8 / 4.0 / 6.8 / 27, 3,072 x 768 6.4 / 6.6 / 7.1 / 33 and
+// 5.6 / 7.2 / 10.5 / 112, 2,560 x 960 6.6 / 6.7 / 7.2 / 25 and 6.3 / 8.7 / 13 / 116, 8,192 x 512 8.1 / 8.4 / 9.0 / 52 and 6.3 / 8.8 / 19 /
+// 147, 960 x 960 5.1 / 5.2 / 5.6 / 24 and 5.8 / 6.2 / 9.8 / 74.
 extern "C" int fg_gemm_f32_split_takes(const float* A, int lda, const float* W, int ldw, int N, int K) {
   return K >= 1024 && N >= 1024 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
 }

@@ -84,3 +84,17 @@ def test_attention_tiles_are_in_ascending_order_of_keys():
     covered = sorted(t for t0, n in zip(tok0, ntok) for t in range(t0, t0 + n))
     assert covered == list(range(0, 70)) + list(range(71, 201))
     assert ctx.attention_tiles(32, min_tokens=2) is tiles  # cached per (tokens a tile, least tokens)
+
+
+def test_tiles_are_counted_without_a_list():
+    from fastgen_b200.engine.step import StepContext
+
+    ctx = StepContext("cpu")
+    ctx.host_seq_slot, ctx.host_seq_cached = [0, 1, 2, 3], [5, 0, 9, 1]
+    ctx.host_seq_start, ctx.n_tokens = [0, 70, 71, 103, 105], 105
+    for tokens in (1, 4, 16, 32):
+        for least in (1, 2):
+            assert ctx.count_tiles(tokens, least) == len(ctx.host_tiles(tokens, least))
+    captured = StepContext("cpu")  # a captured step has no sequences of its own
+    captured.n_tokens = 33
+    assert captured.count_tiles(16, 2) == 3
